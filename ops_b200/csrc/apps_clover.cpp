@@ -53,6 +53,16 @@ struct Clover {
 
   std::vector<double> summaries;  // per field_summary: step, time, vol, mass, ie, ke, press, dt
 
+  // The cycle as hand-fused loops (kernels_clover_fused.cu) instead of the
+  // reference's. `fused` says whether this run may use them, `keep_all`
+  // whether every dat must end as the reference's loops leave it (a dump):
+  // then the last two steps, which write every cell of every work array,
+  // run the reference's loops.
+  bool fused = false, keep_all = false;
+  bool eos_current = false;  // pressure and soundspeed hold density0's and energy0's
+  int density_n = -1, energy_n = -1, xvel_n = -1, yvel_n = -1;  // the first sweep's results
+  int S2D_box, S2D_box_X, S2D_box_Y;
+
   explicit Clover(Runtime &rt) : r(rt) {
     memset(states, 0, sizeof(states));
     memset(&grid, 0, sizeof(grid));
@@ -178,6 +188,16 @@ struct Clover {
     S2D_00_0P1_STRID2D_Y = strided(2, {0, 0, 0, 1}, {0, 1}, "s2D_00_0P1_stride2D_y");
     S2D_00_M10_STRID2D_X = strided(2, {0, 0, -1, 0}, {1, 0}, "s2D_00_M10_stride2D_x");
     S2D_00_0M1_STRID2D_Y = strided(2, {0, 0, 0, -1}, {0, 1}, "s2D_00_0M1_stride2D_y");
+    if (fused) {
+      size[0] = x_cells + 5; size[1] = y_cells + 5;
+      density_n = D("fused_density"); energy_n = D("fused_energy");
+      size[0]++; size[1]++;
+      xvel_n = D("fused_xvel"); yvel_n = D("fused_yvel");
+      // the reach of the fused column marches
+      S2D_box = stencil(2, {-2, -2, 2, 2}, "-2,-2:2,2");
+      S2D_box_X = strided(2, {-2, 0, 2, 0}, {1, 0}, "-2:2 stride2D_x");
+      S2D_box_Y = strided(2, {0, -2, 0, 2}, {0, 1}, "-2:2 stride2D_y");
+    }
 
     red_local_dt = r.decl_reduction(8, "double", "local_dt");
     red_xl_pos = r.decl_reduction(8, "double", "xl_pos");
@@ -358,13 +378,17 @@ struct Clover {
   // field_summary.cpp:44-110
   void field_summary() {
     int rng[] = {field.x_min, field.x_max, field.y_min, field.y_max};
-    ideal_gas(0);
-    loop("field_summary_kernel", "field_summary_kernel", rng,
-         {dat(volume, S2D_00, ACC_READ), dat(density0, S2D_00, ACC_READ), dat(energy0, S2D_00, ACC_READ),
-          dat(pressure, S2D_00, ACC_READ), dat(xvel0, S2D_00_P10_0P1_P1P1, ACC_READ),
-          dat(yvel0, S2D_00_P10_0P1_P1P1, ACC_READ), arg_reduce(red_vol, 1, ACC_INC),
-          arg_reduce(red_mass, 1, ACC_INC), arg_reduce(red_ie, 1, ACC_INC), arg_reduce(red_ke, 1, ACC_INC),
-          arg_reduce(red_press, 1, ACC_INC)});
+    if (fused) {
+      loop("ideal_gas_summary", "field_summary", rng,
+           {dat(density0, S2D_00, ACC_READ), dat(energy0, S2D_00, ACC_READ), dat(pressure, S2D_00, ACC_WRITE),
+            dat(soundspeed, S2D_00, ACC_WRITE), dat(volume, S2D_00, ACC_READ),
+            dat(xvel0, S2D_00_P10_0P1_P1P1, ACC_READ), dat(yvel0, S2D_00_P10_0P1_P1P1, ACC_READ),
+            arg_reduce(red_vol, 1, ACC_INC), arg_reduce(red_mass, 1, ACC_INC), arg_reduce(red_ie, 1, ACC_INC),
+            arg_reduce(red_ke, 1, ACC_INC), arg_reduce(red_press, 1, ACC_INC)});
+      eos_current = true;
+    } else {
+      field_summary_loops(rng);
+    }
     double vol = 0, mass = 0, ie = 0, ke = 0, press = 0;
     r.reduction_result(red_vol, &vol);
     r.reduction_result(red_mass, &mass);
@@ -373,6 +397,16 @@ struct Clover {
     r.reduction_result(red_press, &press);
     double row[8] = {(double)step, clover_time, vol, mass, ie, ke, press, dt};
     summaries.insert(summaries.end(), row, row + 8);
+  }
+
+  void field_summary_loops(const int *rng) {
+    ideal_gas(0);
+    loop("field_summary_kernel", "field_summary_kernel", rng,
+         {dat(volume, S2D_00, ACC_READ), dat(density0, S2D_00, ACC_READ), dat(energy0, S2D_00, ACC_READ),
+          dat(pressure, S2D_00, ACC_READ), dat(xvel0, S2D_00_P10_0P1_P1P1, ACC_READ),
+          dat(yvel0, S2D_00_P10_0P1_P1P1, ACC_READ), arg_reduce(red_vol, 1, ACC_INC),
+          arg_reduce(red_mass, 1, ACC_INC), arg_reduce(red_ie, 1, ACC_INC), arg_reduce(red_ke, 1, ACC_INC),
+          arg_reduce(red_press, 1, ACC_INC)});
   }
 
   void viscosity_func() {  // viscosity.cpp:41-58
@@ -388,6 +422,18 @@ struct Clover {
   void calc_dt(double *local_dt, double *xl_pos, double *yl_pos, int *jldt, int *kldt) {
     double jk_control = 1.1;
     int rng[] = {field.x_min, field.x_max, field.y_min, field.y_max};
+    if (fused) {  // the controlling cell's position (calc_dt_kernel_get) is not reported anywhere
+      loop("calc_dt_fused", "calc_dt", rng,
+           {dat(celldx, S2D_00_P10_STRID2D_X, ACC_READ), dat(celldy, S2D_00_0P1_STRID2D_Y, ACC_READ),
+            dat(soundspeed, S2D_00, ACC_READ), dat(viscosity, S2D_00, ACC_READ), dat(density0, S2D_00, ACC_READ),
+            dat(xvel0, S2D_00_P10_0P1_P1P1, ACC_READ), dat(xarea, S2D_00_P10, ACC_READ),
+            dat(volume, S2D_00, ACC_READ), dat(yvel0, S2D_00_P10_0P1_P1P1, ACC_READ),
+            dat(yarea, S2D_00_0P1, ACC_READ), arg_reduce(red_local_dt, 1, ACC_MIN)});
+      *jldt = *kldt = 1;
+      r.reduction_result(red_local_dt, local_dt);
+      check_dt(local_dt);
+      return;
+    }
     loop("calc_dt_kernel", "calc_dt_kernel", rng,
          {dat(celldx, S2D_00_P10_STRID2D_X, ACC_READ), dat(celldy, S2D_00_0P1_STRID2D_Y, ACC_READ),
           dat(soundspeed, S2D_00, ACC_READ), dat(viscosity, S2D_00, ACC_READ), dat(density0, S2D_00, ACC_READ),
@@ -406,6 +452,9 @@ struct Clover {
     r.reduction_result(red_local_dt, local_dt);
     r.reduction_result(red_xl_pos, xl_pos);
     r.reduction_result(red_yl_pos, yl_pos);
+    check_dt(local_dt);
+  }
+  void check_dt(double *local_dt) {
     *local_dt = op_min(*local_dt, g_big);
     if (*local_dt < dtmin) throw Error(E_STATE, "cloverleaf: timestep below dtmin (calc_dt.cpp:99-125)");
   }
@@ -414,7 +463,7 @@ struct Clover {
   void timestep() {
     double dtlp, xl_pos = 0.0, yl_pos = 0.0;
     int jldt, kldt;
-    ideal_gas(0);
+    if (!(fused && eos_current)) ideal_gas(0);
     set_fields({FIELD_DENSITY0, FIELD_ENERGY0, FIELD_PRESSURE, FIELD_XVEL0, FIELD_YVEL0});
     update_halo(fields, 1);
     viscosity_func();
@@ -634,6 +683,86 @@ struct Clover {
           dat(yvel1, S2D_00, ACC_READ)});
   }
 
+  // One step from PdV to reset_field on the fused loops; every dat that a
+  // later loop reads before it is written ends as the reference's loops leave
+  // it, work arrays, energy1 and {x,y}vel1 do not.
+  void fused_step() {
+    const int x_min = field.x_min, x_max = field.x_max, y_min = field.y_min, y_max = field.y_max;
+    int cells[] = {x_min, x_max, y_min, y_max}, nodes[] = {x_min, x_max + 1, y_min, y_max + 1};
+    loop("PdV_predict_pressure", "PdV_predict", cells,
+         {dat(xarea, S2D_00_P10, ACC_READ), dat(xvel0, S2D_00_P10_0P1_P1P1, ACC_READ),
+          dat(yarea, S2D_00_0P1, ACC_READ), dat(yvel0, S2D_00_P10_0P1_P1P1, ACC_READ),
+          dat(volume, S2D_00, ACC_READ), dat(pressure, S2D_00, ACC_RW), dat(density0, S2D_00, ACC_READ),
+          dat(viscosity, S2D_00, ACC_READ), dat(energy0, S2D_00, ACC_READ)});
+    eos_current = false;
+    set_fields({FIELD_PRESSURE});
+    update_halo(fields, 1);
+    loop("lagrange", "lagrange", nodes,
+         {dat(density0, S2D_box, ACC_READ), dat(volume, S2D_box, ACC_READ), dat(pressure, S2D_box, ACC_READ),
+          dat(viscosity, S2D_box, ACC_READ), dat(xvel0, S2D_box, ACC_READ), dat(yvel0, S2D_box, ACC_READ),
+          dat(xarea, S2D_box, ACC_READ), dat(yarea, S2D_box, ACC_READ), dat(energy0, S2D_box, ACC_READ),
+          dat(xvel1, S2D_00, ACC_WRITE), dat(yvel1, S2D_00, ACC_WRITE), dat(density1, S2D_00, ACC_WRITE),
+          dat(energy1, S2D_00, ACC_WRITE), dat(vol_flux_x, S2D_00, ACC_WRITE), dat(vol_flux_y, S2D_00, ACC_WRITE)});
+    set_fields({FIELD_DENSITY1, FIELD_ENERGY1, FIELD_VOL_FLUX_X, FIELD_VOL_FLUX_Y});
+    update_halo(fields, 2);
+    const bool x_first = advect_x != 0;
+    fused_cell(x_first, 1, density1, energy1, density_n, energy_n);
+    // the boundary copies of the first sweep's results
+    std::swap(density1, density_n);
+    set_fields({FIELD_DENSITY1, FIELD_XVEL1, FIELD_YVEL1, x_first ? FIELD_MASS_FLUX_X : FIELD_MASS_FLUX_Y});
+    std::swap(energy1, energy_n);
+    fields[FIELD_ENERGY1] = 1;
+    update_halo(fields, 2);
+    fused_mom(x_first, 1, nodes, density1, xvel1, yvel1, xvel_n, yvel_n);
+    std::swap(density1, density_n);
+    std::swap(energy1, energy_n);
+    fused_cell(!x_first, 2, density_n, energy_n, density1, energy0);
+    std::swap(xvel1, xvel_n);
+    std::swap(yvel1, yvel_n);
+    set_fields({FIELD_DENSITY1, FIELD_XVEL1, FIELD_YVEL1, x_first ? FIELD_MASS_FLUX_Y : FIELD_MASS_FLUX_X});
+    update_halo(fields, 2);
+    fused_mom(!x_first, 2, nodes, density1, xvel1, yvel1, xvel0, yvel0);
+    std::swap(xvel1, xvel_n);
+    std::swap(yvel1, yvel_n);
+  }
+  void fused_cell(bool x, int sweep, int d, int e, int dout, int eout) {
+    const int x_min = field.x_min, x_max = field.x_max, y_min = field.y_min, y_max = field.y_max;
+    int rx[] = {x_min, x_max + 2, y_min, y_max}, ry[] = {x_min, x_max, y_min, y_max + 2};
+    const int vf = x ? vol_flux_x : vol_flux_y, mf = x ? mass_flux_x : mass_flux_y;
+    const int vd = x ? vertexdx : vertexdy, sd = x ? S2D_box_X : S2D_box_Y;
+    const int *rng = x ? rx : ry;
+    if (sweep == 1)
+      loop(x ? "advec_cell_fused_x1" : "advec_cell_fused_y1", "advec_cell", rng,
+           {dat(vf, S2D_box, ACC_READ), dat(volume, S2D_box, ACC_READ), dat(vd, sd, ACC_READ),
+            dat(d, S2D_box, ACC_READ), dat(e, S2D_box, ACC_READ),
+            dat(x ? vol_flux_y : vol_flux_x, S2D_box, ACC_READ), dat(mf, S2D_00, ACC_WRITE),
+            dat(dout, S2D_00, ACC_WRITE), dat(eout, S2D_00, ACC_WRITE)});
+    else
+      loop(x ? "advec_cell_fused_x2" : "advec_cell_fused_y2", "advec_cell", rng,
+           {dat(vf, S2D_box, ACC_READ), dat(volume, S2D_box, ACC_READ), dat(vd, sd, ACC_READ),
+            dat(d, S2D_box, ACC_READ), dat(e, S2D_box, ACC_READ), dat(mf, S2D_00, ACC_WRITE),
+            dat(dout, S2D_00, ACC_WRITE), dat(eout, S2D_00, ACC_WRITE), dat(density0, S2D_00, ACC_WRITE)});
+  }
+  void fused_mom(bool x, int sweep, const int *nodes, int d, int xv, int yv, int xout, int yout) {
+    const int mf = x ? mass_flux_x : mass_flux_y, cd = x ? celldx : celldy, sd = x ? S2D_box_X : S2D_box_Y;
+    if (sweep == 1)
+      loop(x ? "advec_mom_fused_x1" : "advec_mom_fused_y1", "advec_mom", nodes,
+           {dat(mf, S2D_box, ACC_READ), dat(volume, S2D_box, ACC_READ), dat(cd, sd, ACC_READ),
+            dat(d, S2D_box, ACC_READ), dat(xv, S2D_box, ACC_READ), dat(yv, S2D_box, ACC_READ),
+            dat(xout, S2D_00, ACC_WRITE), dat(yout, S2D_00, ACC_WRITE),
+            dat(x ? vol_flux_y : vol_flux_x, S2D_box, ACC_READ)});
+    else
+      loop(x ? "advec_mom_fused_x2" : "advec_mom_fused_y2", "advec_mom", nodes,
+           {dat(mf, S2D_box, ACC_READ), dat(volume, S2D_box, ACC_READ), dat(cd, sd, ACC_READ),
+            dat(d, S2D_box, ACC_READ), dat(xv, S2D_box, ACC_READ), dat(yv, S2D_box, ACC_READ),
+            dat(xout, S2D_00, ACC_WRITE), dat(yout, S2D_00, ACC_WRITE)});
+  }
+  // Whether this step (its dt known) and the one after it are both followed
+  // by another: the next dt is at most dt * dtrise.
+  bool two_more_steps() const {
+    return step + 1 < end_step && clover_time + dt + op_min(dt * dtrise, dtmax) + g_small <= end_time;
+  }
+
   // clover_leaf.cpp:133-160 + start.cpp:44-112
   void setup(const ops_b200_clover_deck &deck) {
     read_input(deck);
@@ -670,13 +799,20 @@ struct Clover {
   // One hydro cycle (clover_leaf.cpp:185-212). Returns true when complete.
   bool cycle() {
     step = step + 1;
+    if (keep_all && step + 1 >= end_step) fused = false;
     timestep();
-    PdV(1);
-    accelerate();
-    PdV(0);
-    flux_calc();
-    advection();
-    reset_field();
+    if (keep_all && !two_more_steps()) fused = false;
+    if (fused) {
+      fused_step();
+    } else {
+      PdV(1);
+      accelerate();
+      PdV(0);
+      flux_calc();
+      advection();
+      reset_field();
+      eos_current = false;
+    }
     advect_x = advect_x ? 0 : 1;
     clover_time = clover_time + dt;
     if (summary_frequency != 0)
@@ -705,6 +841,8 @@ extern "C" int ops_b200_app_cloverleaf(const ops_b200_clover_deck *deck, int war
     ReleaseScope scope(r);
     const Runtime::Mark &mk = scope.mark();
     clover::Clover c(r);
+    c.fused = r.hand_fusion() && r.nranks() <= 1;
+    c.keep_all = dump_dir != nullptr;
     c.setup(*deck);
     EventPair ev;
     cudaEvent_t e0 = ev.a, e1 = ev.b;
@@ -734,6 +872,7 @@ extern "C" int ops_b200_app_cloverleaf(const ops_b200_clover_deck *deck, int war
     if (dump_dir) {
       for (int i = mk.dats; i < r.ndats(); i++) {
         Dat &d = r.dat(i);
+        if (d.name.compare(0, 6, "fused_") == 0) continue;  // not a dat of the reference app
         std::vector<char> buf(r.dat_data_bytes(i));  // the rank's owned part when partitioned
         r.dat_fetch_data(i, buf.data(), buf.size());
         std::string path = std::string(dump_dir) + "/" + d.name + ".bin";

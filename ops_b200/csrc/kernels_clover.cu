@@ -12,6 +12,7 @@
 #include <cstddef>
 
 #include "clover_common.h"
+#include "clover_flux.cuh"
 #include "fused_exec.cuh"
 #include "runtime.h"
 
@@ -448,7 +449,6 @@ template <class View>
 __device__ __forceinline__ void advec_cell_flux(double vol_flux, const View &pre_vol, int cell_max_test,
                                                 const View &vertexd, const View &density1, const View &energy1,
                                                 double &mass_flux, double &ener_flux) {
-  const double one_by_six = 1.0 / 6.0;
   int upwind, donor, downwind, dif;
   if (vol_flux > 0.0) {
     upwind = -2; donor = -1; downwind = 0; dif = donor;
@@ -457,28 +457,8 @@ __device__ __forceinline__ void advec_cell_flux(double vol_flux, const View &pre
   } else {
     upwind = 0; donor = 0; downwind = -1; dif = upwind;
   }
-  double sigmat = qdiv(fabs(vol_flux), pre_vol(donor));
-  double sigma3 = (1.0 + sigmat) * qratio(vertexd(0), vertexd(dif));
-  double sigma4 = 2.0 - sigmat;
-  double sigmav = sigmat;
-  double diffuw = density1(donor) - density1(upwind);
-  double diffdw = density1(downwind) - density1(donor);
-  double limiter;
-  if ((diffuw * diffdw) > 0.0)
-    limiter = (1.0 - sigmav) * op_sign(1.0, diffdw) *
-              op_min(op_min(fabs(diffuw), fabs(diffdw)), one_by_six * (sigma3 * fabs(diffuw) + sigma4 * fabs(diffdw)));
-  else
-    limiter = 0.0;
-  mass_flux = (vol_flux) * (density1(donor) + limiter);
-  double sigmam = qdiv(fabs(mass_flux), density1(donor) * pre_vol(donor));
-  diffuw = energy1(donor) - energy1(upwind);
-  diffdw = energy1(downwind) - energy1(donor);
-  if ((diffuw * diffdw) > 0.0)
-    limiter = (1.0 - sigmam) * op_sign(1.0, diffdw) *
-              op_min(op_min(fabs(diffuw), fabs(diffdw)), one_by_six * (sigma3 * fabs(diffuw) + sigma4 * fabs(diffdw)));
-  else
-    limiter = 0.0;
-  ener_flux = mass_flux * (energy1(donor) + limiter);
+  advec_cell_face(vol_flux, pre_vol(donor), qratio(vertexd(0), vertexd(dif)), density1(donor), density1(upwind),
+                  density1(downwind), energy1(donor), energy1(upwind), energy1(downwind), mass_flux, ener_flux);
 }
 
 struct XView {
@@ -629,21 +609,8 @@ __device__ __forceinline__ double advec_mom_flux(double node_flux, const View &n
   } else {
     upwind = -1; donor = 0; downwind = 1; dif = upwind;
   }
-  double sigma = qdiv(fabs(node_flux), node_mass_pre(donor));
-  double width = celld(0);
-  double vdiffuw = vel1(donor) - vel1(upwind);
-  double vdiffdw = vel1(downwind) - vel1(donor);
-  double limiter = 0.0;
-  if (vdiffuw * vdiffdw > 0.0) {
-    double auw = fabs(vdiffuw);
-    double adw = fabs(vdiffdw);
-    double wind = 1.0;
-    if (vdiffdw <= 0.0) wind = -1.0;
-    limiter = wind * op_min(width * ((2.0 - sigma) * adw / width + (1.0 + sigma) * auw / celld(dif)) / 6.0,
-                            op_min(auw, adw));
-  }
-  double advec_vel_temp = vel1(donor) + (1.0 - sigma) * limiter;
-  return advec_vel_temp * node_flux;
+  return advec_mom_face(node_flux, qdiv(fabs(node_flux), node_mass_pre(donor)), celld(0), celld(dif), vel1(donor),
+                        vel1(upwind), vel1(downwind));
 }
 
 struct advec_mom_kernel1_x_nonvector {  // :139

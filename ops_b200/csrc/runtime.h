@@ -272,6 +272,10 @@ class Runtime {
   long long list_loops() const { return list_loops_; }
   long long loops_skipped() const { return loops_skipped_; }
   int fusion_enabled() const { return fusion_on_; }
+  // Whether the app drivers may queue hand-fused loops for runs of their own
+  // (off with either fusion option, and when a tuning candidate of the fuser
+  // is forced, which wants the reference's loops to chain).
+  bool hand_fusion() const { return fusion_on_ && tiling_on_ && tile_candidate_ < 0; }
   int diags() const { return diags_; }
   void reset_counters() { kernels_launched_ = graphs_launched_ = loops_enqueued_ = 0; }
   char *red_scratch() const { return red_scratch_; }

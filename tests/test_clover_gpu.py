@@ -77,3 +77,28 @@ def test_summary_invariants_and_determinism(gpu_runtime):
     b, _ = apps.cloverleaf(deck)
     assert np.array_equal(a, b)
     np.testing.assert_allclose(a[:, 2], a[0, 2], rtol=1e-13)   # volume
+
+
+@pytest.mark.parametrize("nx,ny", [(2, 2), (3, 70), (29, 5), (30, 31), (57, 64), (130, 33)])
+def test_fused_loops_leave_what_the_reference_loops_leave(gpu_runtime, tmp_path, nx, ny):
+    """The hand-fused cycle against the reference's loops (option tiling 0),
+    meshes at the edges of the column strips (28, 30, 31 and 32 columns a
+    warp, 4 rows): every dumped dat and every summary row, bit for bit."""
+    from ops_b200 import ops as O
+    deck = config2_deck(nx, ny, 7, 3)
+    outs = []
+    for tiling in (1, 0):
+        d = tmp_path / str(tiling)
+        d.mkdir()
+        O.set_option("tiling", tiling)
+        try:
+            summ, _ = apps.cloverleaf(deck, dump_dir=str(d))
+            undumped, _ = apps.cloverleaf(deck)
+        finally:
+            O.set_option("tiling", 1)
+        assert np.array_equal(summ, undumped)
+        outs.append((summ, {p.name: p.read_bytes() for p in sorted(d.iterdir())}))
+    assert np.array_equal(outs[0][0], outs[1][0])
+    assert outs[0][1].keys() == outs[1][1].keys()
+    for name, data in outs[0][1].items():
+        assert data == outs[1][1][name], name
