@@ -61,6 +61,15 @@ struct Clover3D {
   int red_local_dt, red_xl_pos, red_yl_pos, red_zl_pos, red_vol, red_mass, red_ie, red_ke, red_press, red_output;
 
   std::vector<double> summaries;  // per field_summary: step, time, vol, mass, ie, ke, press, dt
+
+  // The cycle as hand-fused loops (kernels_clover3d_fused.cu) instead of the
+  // reference's; `keep_all`: every dat must end as the reference's loops
+  // leave it (a dump), so the last two steps, which write every cell of
+  // every work array, run them.
+  bool fused = false, keep_all = false;
+  bool eos_current = false;  // pressure and soundspeed hold density0's and energy0's
+  int density_n = -1, energy_n = -1, xvel_n = -1, yvel_n = -1, zvel_n = -1;  // a sweep's results
+  int S_box, S_box_X, S_box_Y, S_box_Z;
   long long halo_loops_skipped = 0;
 
   explicit Clover3D(Runtime &rt) : r(rt) {
@@ -226,6 +235,18 @@ struct Clover3D {
     S_P100_M100_M200_STRID_X = strided(4, {0, 0, 0, 1, 0, 0, 2, 0, 0, -1, 0, 0}, {1, 0, 0}, "x4");
     S_0P10_0M10_0M20_STRID_Y = strided(4, {0, 0, 0, 0, 1, 0, 0, 2, 0, 0, -1, 0}, {0, 1, 0}, "y4");
     S_00P1_00M1_00M2_STRID_Z = strided(4, {0, 0, 0, 0, 0, 1, 0, 0, 2, 0, 0, -1}, {0, 0, 1}, "z4");
+
+    if (fused) {
+      size[0] = xc + 5; size[1] = yc + 5; size[2] = zc + 5;
+      density_n = D("fused_density"); energy_n = D("fused_energy");
+      size[0]++; size[1]++; size[2]++;
+      xvel_n = D("fused_xvel"); yvel_n = D("fused_yvel"); zvel_n = D("fused_zvel");
+      // the reach of the fused marches
+      S_box = stencil(2, {-2, -2, -2, 2, 2, 2}, "-2:2");
+      S_box_X = strided(2, {-2, 0, 0, 2, 0, 0}, {1, 0, 0}, "-2:2 stride x");
+      S_box_Y = strided(2, {0, -2, 0, 0, 2, 0}, {0, 1, 0}, "-2:2 stride y");
+      S_box_Z = strided(2, {0, 0, -2, 0, 0, 2}, {0, 0, 1}, "-2:2 stride z");
+    }
 
     red_local_dt = r.decl_reduction(8, "double", "local_dt");
     red_xl_pos = r.decl_reduction(8, "double", "xl_pos");
@@ -441,12 +462,20 @@ struct Clover3D {
 
   void field_summary() {  // field_summary.cpp:40-113
     int rng[6];
-    ideal_gas(0);
-    loop("field_summary_kernel", inner(rng),
-         {dat(volume, S000, ACC_READ), dat(density0, S000, ACC_READ), dat(energy0, S000, ACC_READ),
-          dat(pressure, S000, ACC_READ), dat(xvel0, S_fP1P1P1, ACC_READ), dat(yvel0, S_fP1P1P1, ACC_READ),
-          dat(zvel0, S_fP1P1P1, ACC_READ), arg_reduce(red_vol, 1, ACC_INC), arg_reduce(red_mass, 1, ACC_INC),
-          arg_reduce(red_ie, 1, ACC_INC), arg_reduce(red_ke, 1, ACC_INC), arg_reduce(red_press, 1, ACC_INC)});
+    if (fused) {
+      loop("ideal_gas_summary", inner(rng),
+           {rd(density0), rd(energy0), wr(pressure), wr(soundspeed), rd(volume), rd(xvel0), rd(yvel0), rd(zvel0),
+            arg_reduce(red_vol, 1, ACC_INC), arg_reduce(red_mass, 1, ACC_INC), arg_reduce(red_ie, 1, ACC_INC),
+            arg_reduce(red_ke, 1, ACC_INC), arg_reduce(red_press, 1, ACC_INC)});
+      eos_current = true;
+    } else {
+      ideal_gas(0);
+      loop("field_summary_kernel", inner(rng),
+           {dat(volume, S000, ACC_READ), dat(density0, S000, ACC_READ), dat(energy0, S000, ACC_READ),
+            dat(pressure, S000, ACC_READ), dat(xvel0, S_fP1P1P1, ACC_READ), dat(yvel0, S_fP1P1P1, ACC_READ),
+            dat(zvel0, S_fP1P1P1, ACC_READ), arg_reduce(red_vol, 1, ACC_INC), arg_reduce(red_mass, 1, ACC_INC),
+            arg_reduce(red_ie, 1, ACC_INC), arg_reduce(red_ke, 1, ACC_INC), arg_reduce(red_press, 1, ACC_INC)});
+    }
     double vol = 0, mass = 0, ie = 0, ke = 0, press = 0;
     r.reduction_result(red_vol, &vol);
     r.reduction_result(red_mass, &mass);
@@ -459,6 +488,13 @@ struct Clover3D {
 
   void viscosity_func() {  // viscosity.cpp:38-62
     int rng[6];
+    if (fused) {
+      loop("viscosity_fused", inner(rng),
+           {rd(xvel0), rd(yvel0), rd(zvel0), rd(pressure), rd(density0), rd(xarea), rd(yarea), rd(zarea),
+            dat(celldx, S_box_X, ACC_READ), dat(celldy, S_box_Y, ACC_READ), dat(celldz, S_box_Z, ACC_READ),
+            wr(viscosity)});
+      return;
+    }
     loop("viscosity_kernel", inner(rng),
          {dat(xvel0, S_fP1P1P1, ACC_READ), dat(yvel0, S_fP1P1P1, ACC_READ), dat(celldx, S_P100_STRID_X, ACC_READ),
           dat(celldy, S_0P10_STRID_Y, ACC_READ), dat(pressure, S_6PT, ACC_READ), dat(density0, S000, ACC_READ),
@@ -471,6 +507,16 @@ struct Clover3D {
     int rng[6];
     double jk_control = 1.1;
     inner(rng);
+    if (fused) {  // the controlling cell's position (calc_dt_kernel_get) is not reported anywhere
+      loop("calc_dt_fused", rng,
+           {rd(soundspeed), rd(viscosity), rd(density0), rd(xvel0), rd(yvel0), rd(zvel0), rd(xarea), rd(yarea),
+            rd(zarea), rd(volume), dat(celldx, S_box_X, ACC_READ), dat(celldy, S_box_Y, ACC_READ),
+            dat(celldz, S_box_Z, ACC_READ), arg_reduce(red_local_dt, 1, ACC_MIN)});
+      *jldt = *kldt = 1;
+      r.reduction_result(red_local_dt, local_dt);
+      check_dt(local_dt);
+      return;
+    }
     loop("calc_dt_kernel", rng,
          {dat(celldx, S_P100_STRID_X, ACC_READ), dat(celldy, S_0P10_STRID_Y, ACC_READ),
           dat(soundspeed, S000, ACC_READ), dat(viscosity, S000, ACC_READ), dat(density0, S000, ACC_READ),
@@ -489,6 +535,9 @@ struct Clover3D {
     r.reduction_result(red_local_dt, local_dt);
     r.reduction_result(red_xl_pos, xl_pos);
     r.reduction_result(red_yl_pos, yl_pos);
+    check_dt(local_dt);
+  }
+  void check_dt(double *local_dt) {
     *local_dt = op_min(*local_dt, g_big);
     if (*local_dt < dtmin) throw Error(E_STATE, "cloverleaf3d: timestep below dtmin (calc_dt.cpp:104-140)");
   }
@@ -497,7 +546,7 @@ struct Clover3D {
   void timestep() {
     double dtlp, xl_pos = 0.0, yl_pos = 0.0;
     int jldt, kldt;
-    ideal_gas(0);
+    if (!(fused && eos_current)) ideal_gas(0);
     set_fields({FIELD_DENSITY0, FIELD_ENERGY0, FIELD_PRESSURE, FIELD_XVEL0, FIELD_YVEL0});
     update_halo(fields, 1);
     viscosity_func();
@@ -771,6 +820,96 @@ struct Clover3D {
           dat(yvel1, S000, ACC_READ), dat(zvel0, S000, ACC_WRITE), dat(zvel1, S000, ACC_READ)});
   }
 
+  // One step from PdV to reset_field on the fused loops; every dat that a
+  // later loop reads before it is written ends as the reference's loops leave
+  // it. The boundary copies that the reference repeats on unchanged fields
+  // (before the second cell sweep) are made once.
+  Arg rd(int d) { return dat(d, S_box, ACC_READ); }
+  Arg wr(int d) { return dat(d, S000, ACC_WRITE); }
+  void fused_step() {
+    int cells[6], nodes[6];
+    inner(cells);
+    inner(nodes, 1, 1, 1);
+    loop("PdV_predict_pressure", cells,
+         {rd(xarea), rd(xvel0), rd(yarea), rd(yvel0), rd(zarea), rd(zvel0), rd(volume), dat(pressure, S000, ACC_RW),
+          rd(density0), rd(viscosity), rd(energy0)});
+    eos_current = false;
+    set_fields({FIELD_PRESSURE});
+    update_halo(fields, 1);
+    loop("accelerate_fused", nodes,
+         {rd(density0), rd(volume), rd(pressure), rd(viscosity), rd(xarea), rd(yarea), rd(zarea), rd(xvel0), rd(yvel0),
+          rd(zvel0), wr(xvel1), wr(yvel1), wr(zvel1)});
+    loop("PdV_flux", nodes,
+         {rd(xarea), rd(yarea), rd(zarea), rd(xvel0), rd(xvel1), rd(yvel0), rd(yvel1), rd(zvel0), rd(zvel1),
+          rd(volume), rd(pressure), rd(density0), rd(viscosity), rd(energy0), wr(density1), wr(energy1),
+          wr(vol_flux_x), wr(vol_flux_y), wr(vol_flux_z)});
+    set_fields({FIELD_DENSITY1, FIELD_ENERGY1, FIELD_VOL_FLUX_X, FIELD_VOL_FLUX_Y, FIELD_VOL_FLUX_Z});
+    update_halo(fields, 2);
+    auto swap_cells = [&] {
+      std::swap(density1, density_n);
+      std::swap(energy1, energy_n);
+    };
+    auto swap_vels = [&] {
+      std::swap(xvel1, xvel_n);
+      std::swap(yvel1, yvel_n);
+      std::swap(zvel1, zvel_n);
+    };
+    const bool xf = advect_x != 0;
+    // first sweep: {density, energy, vel}1 -> the _n dats
+    const int dir1 = xf ? G_XDIR : G_ZDIR, dir3 = xf ? G_ZDIR : G_XDIR;
+    fused_cell(dir1, xf ? "advec_cell_fused_x1" : "advec_cell_fused_z1", density_n, energy_n, -1);
+    swap_cells();
+    fused_mom_halo(dir1, 1);
+    fused_mom(dir1, xf ? "advec_mom_fused_x1" : "advec_mom_fused_z1", nodes, xvel_n, yvel_n, zvel_n);
+    swap_vels();
+    // second: back
+    fused_cell(G_YDIR, xf ? "advec_cell_fused_y2x" : "advec_cell_fused_y2z", density_n, energy_n, -1);
+    swap_cells();
+    fused_mom_halo(G_YDIR, 1);
+    fused_mom(G_YDIR, xf ? "advec_mom_fused_y2x" : "advec_mom_fused_y2z", nodes, xvel_n, yvel_n, zvel_n);
+    swap_vels();
+    // third: into the next step's fields
+    fused_cell(dir3, xf ? "advec_cell_fused_z3" : "advec_cell_fused_x3", density_n, energy0, density0);
+    std::swap(density1, density_n);
+    fused_mom_halo(dir3, 0);
+    fused_mom(dir3, xf ? "advec_mom_fused_z3" : "advec_mom_fused_x3", nodes, xvel0, yvel0, zvel0);
+    std::swap(density1, density_n);
+  }
+  void fused_mom_halo(int dir, int energy) {
+    set_fields({FIELD_DENSITY1, FIELD_XVEL1, FIELD_YVEL1, FIELD_ZVEL1});
+    fields[FIELD_ENERGY1] = energy;
+    fields[FIELD_MASS_FLUX_X] = (dir == G_XDIR);
+    fields[FIELD_MASS_FLUX_Y] = (dir == G_YDIR);
+    fields[FIELD_MASS_FLUX_Z] = (dir == G_ZDIR);
+    update_halo(fields, 2);
+  }
+  Arg width(int dir, int x, int y, int z) {
+    return dir == G_XDIR ? dat(x, S_box_X, ACC_READ) : dir == G_YDIR ? dat(y, S_box_Y, ACC_READ) : dat(z, S_box_Z, ACC_READ);
+  }
+  int flux_of(int dir) const { return dir == G_XDIR ? mass_flux_x : dir == G_YDIR ? mass_flux_y : mass_flux_z; }
+  void fused_cell(int dir, const char *k, int dout, int eout, int d0out) {
+    int rng[6];
+    inner(rng);
+    if (dir == G_XDIR) rng[1] += 2;
+    if (dir == G_YDIR) rng[3] += 2, rng[5] += 2;
+    if (dir == G_ZDIR) rng[5] += 2;
+    std::vector<Arg> a = {rd(volume), rd(vol_flux_x), rd(vol_flux_y), rd(vol_flux_z),
+                          width(dir, vertexdx, vertexdy, vertexdz), rd(density1), rd(energy1), wr(flux_of(dir)),
+                          wr(dout), wr(eout)};
+    if (d0out >= 0) a.push_back(wr(d0out));
+    r.par_loop(loops.get(k), k, clover_grid, 3, rng, a.data(), (int)a.size());
+  }
+  void fused_mom(int dir, const char *k, const int *nodes, int xo, int yo, int zo) {
+    loop(k, nodes,
+         {rd(volume), rd(vol_flux_x), rd(vol_flux_y), rd(vol_flux_z), width(dir, celldx, celldy, celldz),
+          rd(flux_of(dir)), rd(density1), rd(xvel1), rd(yvel1), rd(zvel1), wr(xo), wr(yo), wr(zo)});
+  }
+  // Whether this step (its dt known) and the one after it are both followed
+  // by another: the next dt is at most dt * dtrise.
+  bool two_more_steps() const {
+    return step + 1 < end_step && clover_time + dt + op_min(dt * dtrise, dtmax) + g_small <= end_time;
+  }
+
   // clover_leaf.cpp:133-169 + start.cpp:37-100
   void setup(const ops_b200_clover3d_deck &deck) {
     read_input(deck);
@@ -812,13 +951,20 @@ struct Clover3D {
   // One hydro cycle (clover_leaf.cpp:176-210). Returns true when complete.
   bool cycle() {
     step = step + 1;
+    if (keep_all && step + 1 >= end_step) fused = false;
     timestep();
-    PdV(1);
-    accelerate();
-    PdV(0);
-    flux_calc();
-    advection();
-    reset_field();
+    if (keep_all && !two_more_steps()) fused = false;
+    if (fused) {
+      fused_step();
+    } else {
+      PdV(1);
+      accelerate();
+      PdV(0);
+      flux_calc();
+      advection();
+      reset_field();
+      eos_current = false;
+    }
     advect_x = advect_x ? 0 : 1;
     clover_time = clover_time + dt;
     if (summary_frequency != 0)
@@ -848,6 +994,8 @@ extern "C" int ops_b200_app_cloverleaf3d(const ops_b200_clover3d_deck *deck, int
     ReleaseScope scope(r);
     const Runtime::Mark &mk = scope.mark();
     clover3d::Clover3D c(r);
+    c.fused = r.hand_fusion() && r.nranks() <= 1;
+    c.keep_all = dump_dir != nullptr;
     c.setup(*deck);
     EventPair ev;
     cudaEvent_t e0 = ev.a, e1 = ev.b;
@@ -877,6 +1025,7 @@ extern "C" int ops_b200_app_cloverleaf3d(const ops_b200_clover3d_deck *deck, int
     if (dump_dir) {
       for (int i = mk.dats; i < r.ndats(); i++) {
         Dat &d = r.dat(i);
+        if (d.name.compare(0, 6, "fused_") == 0) continue;  // not a dat of the reference app
         std::vector<char> buf(r.dat_data_bytes(i));  // the rank's owned part when partitioned
         r.dat_fetch_data(i, buf.data(), buf.size());
         std::string path = std::string(dump_dir) + "/" + d.name + ".bin";

@@ -75,3 +75,33 @@ def test_determinism_and_volume(gpu_runtime):
     b, _ = apps.cloverleaf3d(deck)
     assert np.array_equal(a, b)
     np.testing.assert_allclose(a[:, 2], a[0, 2], rtol=1e-13)
+
+
+@pytest.mark.parametrize("nx,ny,nz", [(2, 2, 2), (29, 3, 5), (31, 9, 4), (33, 6, 70), (57, 5, 6)])
+def test_fused_loops_leave_what_the_reference_loops_leave(gpu_runtime, tmp_path, nx, ny, nz):
+    """The hand-fused cycle against the reference's loops (option tiling 0) on
+    meshes at the edges of the marches (28, 30, 31 and 32 columns a warp, 4
+    rows): every dumped dat bit for bit; the summaries' sums, taken in
+    another order, to 1e-12 (n additions of positive terms: n * 2^-53 each
+    way at most, n < 2^14), dt exactly."""
+    from ops_b200 import ops as O
+    deck = apps.clover3d_deck(x_cells=nx, y_cells=ny, z_cells=nz, xmax=10.0, ymax=10.0, zmax=10.0,
+                              initial_timestep=0.04, timestep_rise=1.5, max_timestep=0.04, end_step=7,
+                              summary_frequency=1, states=seeded.clover3d_states(nx, ny, nz, 6))
+    outs = []
+    for tiling in (1, 0):
+        d = tmp_path / str(tiling)
+        d.mkdir()
+        O.set_option("tiling", tiling)
+        try:
+            summ, _ = apps.cloverleaf3d(deck, dump_dir=str(d))
+            undumped, _ = apps.cloverleaf3d(deck)
+        finally:
+            O.set_option("tiling", 1)
+        np.testing.assert_allclose(summ, undumped, rtol=1e-12, atol=0)
+        outs.append((summ, {p.name: p.read_bytes() for p in sorted(d.iterdir())}))
+    np.testing.assert_allclose(outs[0][0], outs[1][0], rtol=1e-12, atol=0)
+    assert np.array_equal(outs[0][0][:, 7], outs[1][0][:, 7])
+    assert outs[0][1].keys() == outs[1][1].keys()
+    for name, data in outs[0][1].items():
+        assert data == outs[1][1][name], name
