@@ -488,13 +488,6 @@ struct Clover3D {
 
   void viscosity_func() {  // viscosity.cpp:38-62
     int rng[6];
-    if (fused) {
-      loop("viscosity_fused", inner(rng),
-           {rd(xvel0), rd(yvel0), rd(zvel0), rd(pressure), rd(density0), rd(xarea), rd(yarea), rd(zarea),
-            dat(celldx, S_box_X, ACC_READ), dat(celldy, S_box_Y, ACC_READ), dat(celldz, S_box_Z, ACC_READ),
-            wr(viscosity)});
-      return;
-    }
     loop("viscosity_kernel", inner(rng),
          {dat(xvel0, S_fP1P1P1, ACC_READ), dat(yvel0, S_fP1P1P1, ACC_READ), dat(celldx, S_P100_STRID_X, ACC_READ),
           dat(celldy, S_0P10_STRID_Y, ACC_READ), dat(pressure, S_6PT, ACC_READ), dat(density0, S000, ACC_READ),
@@ -509,9 +502,11 @@ struct Clover3D {
     inner(rng);
     if (fused) {  // the controlling cell's position (calc_dt_kernel_get) is not reported anywhere
       loop("calc_dt_fused", rng,
-           {rd(soundspeed), rd(viscosity), rd(density0), rd(xvel0), rd(yvel0), rd(zvel0), rd(xarea), rd(yarea),
-            rd(zarea), rd(volume), dat(celldx, S_box_X, ACC_READ), dat(celldy, S_box_Y, ACC_READ),
-            dat(celldz, S_box_Z, ACC_READ), arg_reduce(red_local_dt, 1, ACC_MIN)});
+           {dat(celldx, S_P100_STRID_X, ACC_READ), dat(celldy, S_0P10_STRID_Y, ACC_READ),
+            dat(soundspeed, S000, ACC_READ), dat(viscosity, S000, ACC_READ), dat(density0, S000, ACC_READ),
+            dat(xvel0, S_fP1P1P1, ACC_READ), dat(xarea, S000, ACC_READ), dat(volume, S000, ACC_READ),
+            dat(yvel0, S_fP1P1P1, ACC_READ), dat(yarea, S000, ACC_READ), arg_reduce(red_local_dt, 1, ACC_MIN),
+            dat(celldz, S_00P1_STRID_Z, ACC_READ), dat(zvel0, S_fP1P1P1, ACC_READ), dat(zarea, S000, ACC_READ)});
       *jldt = *kldt = 1;
       r.reduction_result(red_local_dt, local_dt);
       check_dt(local_dt);

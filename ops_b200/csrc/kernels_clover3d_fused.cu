@@ -6,7 +6,8 @@
 // Every value is computed by the reference's expressions in the reference's
 // order, so fields and dt are the same bits; the summary's sums are taken in
 // another order. Measured at 256^3: 12.4 -> 7.7 ms of kernels a step, a
-// 4-step run with its set-up 58.5 -> 36.9 ms.
+// 4-step run with its set-up 58.5 -> 36.9 ms; with every march's loads issued
+// one row ahead of their use (Raw, Row below) 32.0 ms.
 //
 // Each warp marches along y or z with one column of x per lane: the marched
 // axis's neighbours are kept from row to row, x neighbours come by shuffles,
@@ -133,17 +134,13 @@ __device__ __forceinline__ void reduce_grid(const LoopParams &lp, int first, con
 // right neighbours.
 struct Quad {
   double v00, v10, v01, v11;
-  __device__ __forceinline__ void load(const Fld &f, int y, int z) {
-    v00 = f(y, z);
-    v01 = f(y + 1, z);
-    v10 = from_right(v00);
-    v11 = from_right(v01);
-  }
+  __device__ __forceinline__ Quad(double a, double b) : v00(a), v10(from_right(a)), v01(b), v11(from_right(b)) {}
+  __device__ __forceinline__ Quad(const Fld &f, int y, int z) : Quad(f(y, z), f(y + 1, z)) {}
 };
 
 // ideal_gas_kernel then field_summary_kernel. A node's kinetic term is the
 // same product at each of the eight cells around it.
-__global__ void __launch_bounds__(32 * kWarps, 6) summary_kernel(const __grid_constant__ LoopParams lp, int rows) {
+__global__ void __launch_bounds__(32 * kWarps, 5) summary_kernel(const __grid_constant__ LoopParams lp, int rows) {
   const March<31, 0, 2> m(lp, rows);
   const int X = min(m.X, lp.end[0]);
   const Fld density0(lp.a[0], X), energy0(lp.a[1], X), pressure(lp.a[2], X), soundspeed(lp.a[3], X), volume(lp.a[4], X),
@@ -151,17 +148,24 @@ __global__ void __launch_bounds__(32 * kWarps, 6) summary_kernel(const __grid_co
   double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
   if (m.live) {
     const int y = m.o;
-    auto kin = [&](int yy, int z) {
-      const double a = xvel0(yy, z), b = yvel0(yy, z), c = zvel0(yy, z);
-      return 0.125 * (a * a + b * b + c * c);
+    auto kin = [](double a, double b, double c) { return 0.125 * (a * a + b * b + c * c); };
+    struct Raw {  // velocities of plane z + 1 at rows y and y + 1, cell values of plane z
+      double u0, u1, v0, v1, w0, w1, d, e, vol;
     };
-    double k0 = kin(y, m.m0), k1 = kin(y + 1, m.m0);
+    auto load = [&](int z) {
+      return Raw{xvel0(y, z + 1), xvel0(y + 1, z + 1), yvel0(y, z + 1), yvel0(y + 1, z + 1), zvel0(y, z + 1),
+                 zvel0(y + 1, z + 1), density0(y, z), energy0(y, z), volume(y, z)};
+    };
+    double k0 = kin(xvel0(y, m.m0), yvel0(y, m.m0), zvel0(y, m.m0));
+    double k1 = kin(xvel0(y + 1, m.m0), yvel0(y + 1, m.m0), zvel0(y + 1, m.m0));
     double k0r = from_right(k0), k1r = from_right(k1);
+    Raw c = load(m.m0);
     for (int z = m.m0; z < m.m1; z++) {
-      const double n0 = kin(y, z + 1), n1 = kin(y + 1, z + 1);
+      const Raw n = load(min(z + 1, m.m1 - 1));
+      const double n0 = kin(c.u0, c.v0, c.w0), n1 = kin(c.u1, c.v1, c.w1);
       const double n0r = from_right(n0), n1r = from_right(n1);
       if (m.own) {
-        const double d = density0(y, z), e = energy0(y, z), cell_vol = volume(y, z);
+        const double d = c.d, e = c.e, cell_vol = c.vol;
         const double v = 1.0 / d;
         const double p = (1.4 - 1.0) * d * e;
         pressure.put(y, z, p);
@@ -189,6 +193,7 @@ __global__ void __launch_bounds__(32 * kWarps, 6) summary_kernel(const __grid_co
       k1 = n1;
       k0r = n0r;
       k1r = n1r;
+      c = n;
     }
   }
   reduce_grid<5>(lp, 8, sum);
@@ -202,148 +207,44 @@ struct ideal_gas_summary {
   static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2>(lp, s, summary_kernel); }
 };
 
-// viscosity_kernel.
-__global__ void __launch_bounds__(32 * kWarps, 4) viscosity_march(const __grid_constant__ LoopParams lp, int rows) {
-  const March<30, 1, 2> m(lp, rows);
-  if (!m.live) return;
-  const int X = min(m.X, lp.end[0]), y = m.o;
-  const Fld xvel0(lp.a[0], X), yvel0(lp.a[1], X), zvel0(lp.a[2], X), pressure(lp.a[3], X), density0(lp.a[4], X),
-      xarea(lp.a[5], X), yarea(lp.a[6], X), zarea(lp.a[7], X), viscosity(lp.a[11], X);
-  const Widths<0> cdx(lp.a[8]);
-  const Widths<1> cdy(lp.a[9]);
-  const Widths<2> cdz(lp.a[10]);
-  const double dx = cdx(X), dx2 = dx + cdx(X + 1), dy = cdy(y), dy2 = dy + cdy(y + 1);
-  Quad u, v, w;
-  u.load(xvel0, y, m.m0);
-  v.load(yvel0, y, m.m0);
-  w.load(zvel0, y, m.m0);
-  double pm = pressure(y, m.m0 - 1), p0 = pressure(y, m.m0);
-  for (int z = m.m0; z < m.m1; z++) {
-    Quad un, vn, wn;
-    un.load(xvel0, y, z + 1);
-    vn.load(yvel0, y, z + 1);
-    wn.load(zvel0, y, z + 1);
-    const double pn = pressure(y, z + 1), ps = pressure(y - 1, z), pt = pressure(y + 1, z);
-    const double pl = from_left(p0), pr = from_right(p0);
-    const double ugradx1 = u.v00 + u.v01 + un.v00 + un.v01;
-    const double vgradx1 = v.v00 + v.v01 + vn.v00 + vn.v01;
-    const double wgradx1 = w.v00 + w.v01 + wn.v00 + wn.v01;
-    const double ugradx2 = from_right(ugradx1), vgradx2 = from_right(vgradx1), wgradx2 = from_right(wgradx1);
-    if (m.own) {
-      const double ugrady1 = u.v00 + u.v10 + un.v00 + un.v10, ugrady2 = u.v01 + u.v11 + un.v01 + un.v11;
-      const double ugradz1 = u.v00 + u.v10 + u.v01 + u.v11, ugradz2 = un.v00 + un.v10 + un.v01 + un.v11;
-      const double vgrady1 = v.v00 + v.v10 + vn.v00 + vn.v10, vgrady2 = v.v01 + v.v11 + vn.v01 + vn.v11;
-      const double vgradz1 = v.v00 + v.v10 + v.v01 + v.v11, vgradz2 = vn.v00 + vn.v10 + vn.v01 + vn.v11;
-      const double wgrady1 = w.v00 + w.v10 + wn.v00 + wn.v10, wgrady2 = w.v01 + w.v11 + wn.v01 + wn.v11;
-      const double wgradz1 = w.v00 + w.v10 + w.v01 + w.v11, wgradz2 = wn.v00 + wn.v10 + wn.v01 + wn.v11;
-      const double dz = cdz(z), dz2 = dz + cdz(z + 1);
-      const double div = xarea(y, z) * (ugradx2 - ugradx1) + yarea(y, z) * (vgrady2 - vgrady1) +
-                         zarea(y, z) * (wgradz2 - wgradz1);
-      const double xx = qdiv(0.25 * (ugradx2 - ugradx1), dx);
-      const double yy = qdiv(0.25 * (vgrady2 - vgrady1), dy);
-      const double zz = qdiv(0.25 * (wgradz2 - wgradz1), dz);
-      const double xy = qdiv(0.25 * (ugrady2 - ugrady1), dy) + qdiv(0.25 * (vgradx2 - vgradx1), dx);
-      const double xz = qdiv(0.25 * (ugradz2 - ugradz1), dz) + qdiv(0.25 * (wgradx2 - wgradx1), dx);
-      const double yz = qdiv(0.25 * (vgradz2 - vgradz1), dz) + qdiv(0.25 * (wgrady2 - wgrady1), dy);
-      double pgradx = qdiv(pr - pl, dx2), pgrady = qdiv(pt - ps, dy2), pgradz = qdiv(pn - pm, dz2);
-      const double pgradx2 = pgradx * pgradx, pgrady2 = pgrady * pgrady, pgradz2 = pgradz * pgradz;
-      const double limiter = qdiv(xx * pgradx2 + yy * pgrady2 + zz * pgradz2 + xy * pgradx * pgrady +
-                                      xz * pgradx * pgradz + yz * pgrady * pgradz,
-                                  op_max(pgradx2 + pgrady2 + pgradz2, 1.0e-16));
-      double out = 0.0;
-      if (!((limiter > 0.0) || (div >= 0.0))) {
-        pgradx = op_sign(op_max(1.0e-16, fabs(pgradx)), pgradx);
-        pgrady = op_sign(op_max(1.0e-16, fabs(pgrady)), pgrady);
-        pgradz = op_sign(op_max(1.0e-16, fabs(pgradz)), pgradz);
-        const double pgrad = sqrt(pgradx * pgradx + pgrady * pgrady + pgradz * pgradz);
-        const double xgrad = fabs(dx * pgrad / pgradx);
-        const double ygrad = fabs(dy * pgrad / pgrady);
-        const double zgrad = fabs(dz * pgrad / pgradz);
-        const double grad = op_min(xgrad, op_min(ygrad, zgrad));
-        const double grad2 = grad * grad;
-        out = 2.0 * (density0(y, z)) * grad2 * limiter * limiter;
-      }
-      viscosity.put(y, z, out);
-    }
-    u = un;
-    v = vn;
-    w = wn;
-    pm = p0;
-    p0 = pn;
-  }
-}
-
-struct viscosity_fused {
-  C3_LOOP(viscosity_fused);
-  __device__ void operator()(const D &xvel0, const D &yvel0, const D &zvel0, const D &pressure, const D &density0,
-                             const D &xarea, const D &yarea, const D &zarea, const D &celldx, const D &celldy,
-                             const D &celldz, D &viscosity) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<30, 2>(lp, s, viscosity_march); }
-};
-
-// calc_dt_kernel with calc_dt_kernel_min folded in.
-__global__ void __launch_bounds__(32 * kWarps, 5) calc_dt_march(const __grid_constant__ LoopParams lp, int rows) {
-  const March<31, 0, 2> m(lp, rows);
-  const int X = min(m.X, lp.end[0]), y = m.o;
-  const Fld soundspeed(lp.a[0], X), viscosity(lp.a[1], X), density0(lp.a[2], X), xvel0(lp.a[3], X), yvel0(lp.a[4], X),
-      zvel0(lp.a[5], X), xarea(lp.a[6], X), yarea(lp.a[7], X), zarea(lp.a[8], X), volume(lp.a[9], X);
-  const Widths<0> cdx(lp.a[10]);
-  const Widths<1> cdy(lp.a[11]);
-  const Widths<2> cdz(lp.a[12]);
-  double dt_min[1] = {RedTraits<double>::big()};
-  if (m.live) {
-    const double dxy = op_min(cdx(X), cdy(y));
-    double u0 = xvel0(y, m.m0), u1 = xvel0(y + 1, m.m0);
-    Quad v, w;
-    v.load(yvel0, y, m.m0);
-    w.load(zvel0, y, m.m0);
-    for (int z = m.m0; z < m.m1; z++) {
-      const double u0n = xvel0(y, z + 1), u1n = xvel0(y + 1, z + 1);
-      Quad vn, wn;
-      vn.load(yvel0, y, z + 1);
-      wn.load(zvel0, y, z + 1);
-      const double us = u0 + u1 + u0n + u1n, usr = from_right(us);
-      if (m.own) {
-        const double vol = volume(y, z), xa = xarea(y, z), ya = yarea(y, z), za = zarea(y, z);
-        double ds = op_min(dxy, cdz(z));
-        ds = 1.0 / (ds * ds);
-        const double c = soundspeed(y, z);
-        double cc = c * c;
-        cc = cc + qdiv(2.0 * viscosity(y, z), density0(y, z));
-        double dtct = ds * cc;
-        dtct = c3.dtc_safe * 1.0 / op_max(sqrt(dtct), c3.g_small);
-        const double du1 = us * xa, du2 = usr * xa;
-        const double dtut = c3.dtu_safe * 4.0 * vol / op_max(op_max(fabs(du1), fabs(du2)), 1.0e-5 * vol);
-        const double dv1 = (v.v00 + v.v10 + vn.v00 + vn.v10) * ya, dv2 = (v.v01 + v.v11 + vn.v01 + vn.v11) * ya;
-        const double dtvt = c3.dtv_safe * 4.0 * vol / op_max(op_max(fabs(dv1), fabs(dv2)), 1.0e-5 * vol);
-        const double dw1 = (w.v00 + w.v01 + w.v10 + w.v11) * za, dw2 = (wn.v00 + wn.v01 + wn.v10 + wn.v11) * za;
-        const double dtwt = c3.dtw_safe * 4.0 * vol / op_max(op_max(fabs(dw1), fabs(dw2)), 1.0e-5 * vol);
-        const double div = du2 - du1 + dv2 - dv1 + dw2 - dw1;
-        const double dtdivt = c3.dtdiv_safe * 4.0 * (vol) / op_max(vol * 1.0e-05, fabs(div));
-        dt_min[0] = op_min(dt_min[0], op_min(op_min(op_min(dtct, dtut), op_min(dtvt, dtdivt)), dtwt));
-      }
-      u0 = u0n;
-      u1 = u1n;
-      v = vn;
-      w = wn;
-    }
-  }
-  reduce_grid<1>(lp, 13, dt_min);
-}
-
+// calc_dt_kernel with calc_dt_kernel_min folded in. Point by point: the six
+// divisions and the square root of a cell want the many warps that the plain
+// executor keeps resident, so a z march gained nothing (0.49 ms at 256^3
+// against 0.50 ms; viscosity_kernel as a march took 0.66 ms against 0.47 ms
+// and stays the reference's loop).
 struct calc_dt_fused {
   C3_LOOP(calc_dt_fused);
-  __device__ void operator()(const D &soundspeed, const D &viscosity, const D &density0, const D &xvel0,
-                             const D &yvel0, const D &zvel0, const D &xarea, const D &yarea, const D &zarea,
-                             const D &volume, const D &celldx, const D &celldy, const D &celldz,
-                             RED<double> &dt_min) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2>(lp, s, calc_dt_march); }
+  static constexpr int min_blocks = 4;
+  __device__ void operator()(const D &celldx, const D &celldy, const D &soundspeed, const D &viscosity,
+                             const D &density0, const D &xvel0, const D &xarea, const D &volume, const D &yvel0,
+                             const D &yarea, RED<double> &dt_min, const D &celldz, const D &zvel0,
+                             const D &zarea) const {
+    double div, ds, dtut, dtvt, dtct, dtwt, dtdivt, cc, dv1, dv2, du1, du2, dw1, dw2;
+    ds = op_min(op_min(celldx(0, 0, 0), celldy(0, 0, 0)), celldz(0, 0, 0));
+    ds = 1.0 / (ds * ds);
+    cc = soundspeed(0, 0, 0) * soundspeed(0, 0, 0);
+    cc = cc + qdiv(2.0 * viscosity(0, 0, 0), density0(0, 0, 0));
+    dtct = ds * cc;
+    dtct = c3.dtc_safe * 1.0 / op_max(sqrt(dtct), c3.g_small);
+    du1 = (xvel0(0, 0, 0) + xvel0(0, 1, 0) + xvel0(0, 0, 1) + xvel0(0, 1, 1)) * xarea(0, 0, 0);
+    du2 = (xvel0(1, 0, 0) + xvel0(1, 1, 0) + xvel0(1, 0, 1) + xvel0(1, 1, 1)) * xarea(0, 0, 0);
+    dtut = c3.dtu_safe * 4.0 * volume(0, 0, 0) / op_max(op_max(fabs(du1), fabs(du2)), 1.0e-5 * volume(0, 0, 0));
+    dv1 = (yvel0(0, 0, 0) + yvel0(1, 0, 0) + yvel0(0, 0, 1) + yvel0(1, 0, 1)) * yarea(0, 0, 0);
+    dv2 = (yvel0(0, 1, 0) + yvel0(1, 1, 0) + yvel0(0, 1, 1) + yvel0(1, 1, 1)) * yarea(0, 0, 0);
+    dtvt = c3.dtv_safe * 4.0 * volume(0, 0, 0) / op_max(op_max(fabs(dv1), fabs(dv2)), 1.0e-5 * volume(0, 0, 0));
+    dw1 = (zvel0(0, 0, 0) + zvel0(0, 1, 0) + zvel0(1, 0, 0) + zvel0(1, 1, 0)) * zarea(0, 0, 0);
+    dw2 = (zvel0(0, 0, 1) + zvel0(0, 1, 1) + zvel0(1, 0, 1) + zvel0(1, 1, 1)) * zarea(0, 0, 0);
+    dtwt = c3.dtw_safe * 4.0 * volume(0, 0, 0) / op_max(op_max(fabs(dw1), fabs(dw2)), 1.0e-5 * volume(0, 0, 0));
+    div = du2 - du1 + dv2 - dv1 + dw2 - dw1;
+    dtdivt = c3.dtdiv_safe * 4.0 * (volume(0, 0, 0)) / op_max(volume(0, 0, 0) * 1.0e-05, fabs(div));
+    *dt_min = op_min(*dt_min, op_min(op_min(op_min(dtct, dtut), op_min(dtvt, dtdivt)), dtwt));
+  }
 };
 
 // PdV_kernel_predict then the ideal gas pressure of the predicted state; the
 // predicted density and energy are nothing else's inputs (revert_kernel
 // restores them and PdV_kernel_nopredict overwrites them unread).
-__global__ void __launch_bounds__(32 * kWarps, 5) predict_march(const __grid_constant__ LoopParams lp, int rows) {
+__global__ void __launch_bounds__(32 * kWarps, 4) predict_march(const __grid_constant__ LoopParams lp, int rows) {
   const March<31, 0, 2> m(lp, rows);
   if (!m.live) return;
   const int X = min(m.X, lp.end[0]), y = m.o;
@@ -351,41 +252,46 @@ __global__ void __launch_bounds__(32 * kWarps, 5) predict_march(const __grid_con
       zvel0(lp.a[5], X), volume(lp.a[6], X), pressure(lp.a[7], X), density0(lp.a[8], X), viscosity(lp.a[9], X),
       energy0(lp.a[10], X);
   const double dt = c3.dt;
-  double u0 = xvel0(y, m.m0), u1 = xvel0(y + 1, m.m0);
-  Quad v, w;
-  v.load(yvel0, y, m.m0);
-  w.load(zvel0, y, m.m0);
-  auto zflux = [&](const Quad &q, int z) {
-    return (zarea(y, z) * (q.v00 + q.v10 + q.v01 + q.v11 + q.v00 + q.v10 + q.v01 + q.v11)) * 0.125 * dt * 0.5;
+  struct Raw {  // plane z + 1: velocities at rows y and y + 1, z area; plane z: the rest
+    double u0, u1, v0, v1, w0, w1, za, xa, ya, yt, vol, p, d, q, e;
   };
-  double back_flux = zflux(w, m.m0);
+  auto load = [&](int z) {
+    return Raw{xvel0(y, z + 1),     xvel0(y + 1, z + 1), yvel0(y, z + 1), yvel0(y + 1, z + 1), zvel0(y, z + 1),
+               zvel0(y + 1, z + 1), zarea(y, z + 1),     xarea(y, z),     yarea(y, z),         yarea(y + 1, z),
+               volume(y, z),        *pressure.at(y, z),  density0(y, z),  viscosity(y, z),     energy0(y, z)};
+  };
+  double u0 = xvel0(y, m.m0), u1 = xvel0(y + 1, m.m0);
+  Quad v(yvel0, y, m.m0);
+  auto zflux = [&](const Quad &q, double za) {
+    return (za * (q.v00 + q.v10 + q.v01 + q.v11 + q.v00 + q.v10 + q.v01 + q.v11)) * 0.125 * dt * 0.5;
+  };
+  double back_flux = zflux(Quad(zvel0, y, m.m0), zarea(y, m.m0));
+  Raw c = load(m.m0);
   for (int z = m.m0; z < m.m1; z++) {
-    const double u0n = xvel0(y, z + 1), u1n = xvel0(y + 1, z + 1);
-    Quad vn, wn;
-    vn.load(yvel0, y, z + 1);
-    wn.load(zvel0, y, z + 1);
-    const double left_flux = (xarea(y, z) * (u0 + u1 + u0n + u1n + u0 + u1 + u0n + u1n)) * 0.125 * dt * 0.5;
+    const Raw n = load(min(z + 1, m.m1 - 1));
+    const double u0n = c.u0, u1n = c.u1;
+    const Quad vn(c.v0, c.v1);
+    const double left_flux = (c.xa * (u0 + u1 + u0n + u1n + u0 + u1 + u0n + u1n)) * 0.125 * dt * 0.5;
     const double right_flux = from_right(left_flux);
-    const double front_flux = zflux(wn, z + 1);
+    const double front_flux = zflux(Quad(c.w0, c.w1), c.za);
     if (m.own) {
       const double bottom_flux =
-          (yarea(y, z) * (v.v00 + v.v10 + vn.v00 + vn.v10 + v.v00 + v.v10 + vn.v00 + vn.v10)) * 0.125 * dt * 0.5;
+          (c.ya * (v.v00 + v.v10 + vn.v00 + vn.v10 + v.v00 + v.v10 + vn.v00 + vn.v10)) * 0.125 * dt * 0.5;
       const double top_flux =
-          (yarea(y + 1, z) * (v.v01 + v.v11 + vn.v01 + vn.v11 + v.v01 + v.v11 + vn.v01 + vn.v11)) * 0.125 * dt * 0.5;
+          (c.yt * (v.v01 + v.v11 + vn.v01 + vn.v11 + v.v01 + v.v11 + vn.v01 + vn.v11)) * 0.125 * dt * 0.5;
       const double total_flux = right_flux - left_flux + top_flux - bottom_flux + front_flux - back_flux;
-      const double vol = volume(y, z), d0 = density0(y, z);
-      const double volume_change = (vol) / (vol + total_flux);
-      const double recip_volume = 1.0 / vol;
-      double *pp = pressure.at(y, z);
-      const double energy_change = (*pp / d0 + qdiv(viscosity(y, z), d0)) * total_flux * recip_volume;
-      const double energy1 = energy0(y, z) - energy_change;
-      const double density1 = d0 * volume_change;
-      *pp = (1.4 - 1.0) * density1 * energy1;
+      const double volume_change = (c.vol) / (c.vol + total_flux);
+      const double recip_volume = 1.0 / c.vol;
+      const double energy_change = (c.p / c.d + qdiv(c.q, c.d)) * total_flux * recip_volume;
+      const double energy1 = c.e - energy_change;
+      const double density1 = c.d * volume_change;
+      pressure.put(y, z, (1.4 - 1.0) * density1 * energy1);
     }
     u0 = u0n;
     u1 = u1n;
     v = vn;
     back_flux = front_flux;
+    c = n;
   }
 }
 
@@ -399,7 +305,7 @@ struct PdV_predict_pressure {
 
 // accelerate_kernel. A plane's share of a node's mass and forces is computed
 // once and kept for the node above.
-__global__ void __launch_bounds__(32 * kWarps, 4) accelerate_march(const __grid_constant__ LoopParams lp, int rows) {
+__global__ void __launch_bounds__(32 * kWarps, 3) accelerate_march(const __grid_constant__ LoopParams lp, int rows) {
   const March<31, 1, 2> m(lp, rows);
   if (!m.live) return;
   const int X = min(m.X, lp.end[0] - 1), y = m.o;
@@ -413,40 +319,49 @@ __global__ void __launch_bounds__(32 * kWarps, 4) accelerate_march(const __grid_
     double xp0, xp1, xq0, xq1;        // x forces of rows y, y - 1
     double yp, ypl, yq, yql;          // y forces at the column and left of it
   };
+  struct Raw {  // the plane's own values at rows y and y - 1
+    double d0, d1, v0, v1, p0, p1, q0, q1, xa0, xa1, ya, za0, za1, xv, yv, zv;
+  };
   auto load = [&](int z) {
+    return Raw{density0(y, z),  density0(y - 1, z),  volume(y, z),  volume(y - 1, z), pressure(y, z), pressure(y - 1, z),
+               viscosity(y, z), viscosity(y - 1, z), xarea(y, z),   xarea(y - 1, z),  yarea(y, z),    zarea(y, z),
+               zarea(y - 1, z), xvel0(y, z),         yvel0(y, z),   zvel0(y, z)};
+  };
+  auto plane = [&](const Raw &w) {
     Plane r;
-    r.m0 = density0(y, z) * volume(y, z);
-    r.m1 = density0(y - 1, z) * volume(y - 1, z);
+    r.m0 = w.d0 * w.v0;
+    r.m1 = w.d1 * w.v1;
     r.m0l = from_left(r.m0);
     r.m1l = from_left(r.m1);
-    r.p0 = pressure(y, z);
-    r.p1 = pressure(y - 1, z);
-    r.q0 = viscosity(y, z);
-    r.q1 = viscosity(y - 1, z);
-    const double xa0 = xarea(y, z), xa1 = xarea(y - 1, z), ya = yarea(y, z);
-    r.xp0 = xa0 * (r.p0 - from_left(r.p0));
-    r.xp1 = xa1 * (r.p1 - from_left(r.p1));
-    r.xq0 = xa0 * (r.q0 - from_left(r.q0));
-    r.xq1 = xa1 * (r.q1 - from_left(r.q1));
-    r.yp = ya * (r.p0 - r.p1);
-    r.yq = ya * (r.q0 - r.q1);
+    r.p0 = w.p0;
+    r.p1 = w.p1;
+    r.q0 = w.q0;
+    r.q1 = w.q1;
+    r.xp0 = w.xa0 * (r.p0 - from_left(r.p0));
+    r.xp1 = w.xa1 * (r.p1 - from_left(r.p1));
+    r.xq0 = w.xa0 * (r.q0 - from_left(r.q0));
+    r.xq1 = w.xa1 * (r.q1 - from_left(r.q1));
+    r.yp = w.ya * (r.p0 - r.p1);
+    r.yq = w.ya * (r.q0 - r.q1);
     r.ypl = from_left(r.yp);
     r.yql = from_left(r.yq);
     return r;
   };
-  Plane b = load(m.m0 - 1);
+  Raw w = load(m.m0);
+  Plane b = plane(load(m.m0 - 1));
   for (int z = m.m0; z < m.m1; z++) {
-    const double za0 = zarea(y, z), za1 = zarea(y - 1, z);
-    const Plane c = load(z);
+    const Raw n = load(min(z + 1, m.m1 - 1));
+    const Plane c = plane(w);
+    const double za0 = w.za0, za1 = w.za1;
     const double zp0 = za0 * (c.p0 - b.p0), zp1 = za1 * (c.p1 - b.p1);
     const double zq0 = za0 * (c.q0 - b.q0), zq1 = za1 * (c.q1 - b.q1);
     const double zp0l = from_left(zp0), zp1l = from_left(zp1), zq0l = from_left(zq0), zq1l = from_left(zq1);
     if (m.own) {
       const double nodal_mass = (c.m1l + c.m1 + c.m0 + c.m0l + b.m1l + b.m1 + b.m0 + b.m0l) * 0.125;
       const double stepbymass = qdt / nodal_mass;
-      double xv = xvel0(y, z) - stepbymass * (c.xp0 + c.xp1 + b.xp0 + b.xp1);
-      double yv = yvel0(y, z) - stepbymass * (c.yp + c.ypl + b.yp + b.ypl);
-      double zv = zvel0(y, z) - stepbymass * (zp0 + zp1 + zp0l + zp1l);
+      double xv = w.xv - stepbymass * (c.xp0 + c.xp1 + b.xp0 + b.xp1);
+      double yv = w.yv - stepbymass * (c.yp + c.ypl + b.yp + b.ypl);
+      double zv = w.zv - stepbymass * (zp0 + zp1 + zp0l + zp1l);
       xv = xv - stepbymass * (c.xq0 + c.xq1 + b.xq0 + b.xq1);
       yv = yv - stepbymass * (c.yq + c.yql + b.yq + b.yql);
       zv = zv - stepbymass * (zq0 + zq1 + zq0l + zq1l);
@@ -455,6 +370,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4) accelerate_march(const __grid_
       zvel1.put(y, z, zv);
     }
     b = c;
+    w = n;
   }
 }
 
@@ -468,7 +384,7 @@ struct accelerate_fused {
 
 // PdV_kernel_nopredict and flux_calc_kernel{x,y,z} over the nodes; each
 // flux stops one short of the nodes in the directions across its face.
-__global__ void __launch_bounds__(32 * kWarps, 4) pdv_flux_march(const __grid_constant__ LoopParams lp, int rows) {
+__global__ void __launch_bounds__(32 * kWarps, 3) pdv_flux_march(const __grid_constant__ LoopParams lp, int rows) {
   const March<31, 0, 2> m(lp, rows);
   if (!m.live) return;
   const int X = min(m.X, lp.end[0]), y = m.o;
@@ -479,32 +395,36 @@ __global__ void __launch_bounds__(32 * kWarps, 4) pdv_flux_march(const __grid_co
   const double dt = c3.dt, edt = 0.125 * c3.dt;
   const int zcell = lp.end[2] - 1;
   const bool cx = m.own && m.X < lp.end[0] - 1, cy = y < lp.end[1] - 1;
+  struct Raw {  // plane z + 1: both velocities at rows y and y + 1, z area; plane z: the rest
+    double u0, u1, t0, t1, v0, v1, s0, s1, w0, w1, r0, r1, za, xa, ya, yt, vol, p, d, q, e;
+  };
+  auto load = [&](int z) {
+    return Raw{xvel0(y, z + 1), xvel0(y + 1, z + 1), xvel1(y, z + 1), xvel1(y + 1, z + 1), yvel0(y, z + 1),
+               yvel0(y + 1, z + 1), yvel1(y, z + 1), yvel1(y + 1, z + 1), zvel0(y, z + 1), zvel0(y + 1, z + 1),
+               zvel1(y, z + 1), zvel1(y + 1, z + 1), zarea(y, z + 1), xarea(y, z), yarea(y, z), yarea(y + 1, z),
+               volume(y, z), pressure(y, z), density0(y, z), viscosity(y, z), energy0(y, z)};
+  };
   double u0 = xvel0(y, m.m0), u1 = xvel0(y + 1, m.m0), t0 = xvel1(y, m.m0), t1 = xvel1(y + 1, m.m0);
-  Quad v, s;
-  v.load(yvel0, y, m.m0);
-  s.load(yvel1, y, m.m0);
+  Quad v(yvel0, y, m.m0), s(yvel1, y, m.m0);
   // the z face of plane z: its flux of volume (the reference's flux_calc reads
   // zvel0(1,0,0) twice) and the PdV flux through it
-  auto zface = [&](int z, double &flux, double &vflux) {
-    Quad w, r;
-    w.load(zvel0, y, z);
-    r.load(zvel1, y, z);
-    const double za = zarea(y, z);
+  auto zface = [&](const Quad &w, const Quad &r, double za, double &flux, double &vflux) {
     flux = (za * (w.v00 + w.v10 + w.v01 + w.v11 + r.v00 + r.v10 + r.v01 + r.v11)) * 0.125 * dt;
     vflux = edt * za * (w.v00 + w.v10 + w.v10 + w.v11 + r.v00 + r.v10 + r.v01 + r.v11);
   };
   double back_flux, vfz;
-  zface(m.m0, back_flux, vfz);
+  zface(Quad(zvel0, y, m.m0), Quad(zvel1, y, m.m0), zarea(y, m.m0), back_flux, vfz);
+  const int zlast = min(m.m1, zcell) - 1;  // the last plane with cells
+  Raw c = load(min(m.m0, zcell - 1));
   for (int z = m.m0; z < m.m1; z++) {
     if (cx && cy) vol_flux_z.put(y, z, vfz);
     if (z == zcell) break;
-    const double u0n = xvel0(y, z + 1), u1n = xvel0(y + 1, z + 1), t0n = xvel1(y, z + 1), t1n = xvel1(y + 1, z + 1);
-    Quad vn, sn;
-    vn.load(yvel0, y, z + 1);
-    sn.load(yvel1, y, z + 1);
+    const Raw n = load(min(z + 1, zlast));
+    const double u0n = c.u0, u1n = c.u1, t0n = c.t0, t1n = c.t1;
+    const Quad vn(c.v0, c.v1), sn(c.s0, c.s1);
     double front_flux;
-    zface(z + 1, front_flux, vfz);
-    const double xa = xarea(y, z), ya = yarea(y, z);
+    zface(Quad(c.w0, c.w1), Quad(c.r0, c.r1), c.za, front_flux, vfz);
+    const double xa = c.xa, ya = c.ya;
     const double xsum = u0 + u1 + u0n + u1n + t0 + t1 + t0n + t1n;
     const double ysum = v.v00 + v.v10 + vn.v00 + vn.v10 + s.v00 + s.v10 + sn.v00 + sn.v10;
     const double left_flux = (xa * xsum) * 0.125 * dt;
@@ -515,15 +435,13 @@ __global__ void __launch_bounds__(32 * kWarps, 4) pdv_flux_march(const __grid_co
       if (cy) {
         const double bottom_flux = (ya * ysum) * 0.125 * dt;
         const double top_flux =
-            (yarea(y + 1, z) * (v.v01 + v.v11 + vn.v01 + vn.v11 + s.v01 + s.v11 + sn.v01 + sn.v11)) * 0.125 * dt;
+            (c.yt * (v.v01 + v.v11 + vn.v01 + vn.v11 + s.v01 + s.v11 + sn.v01 + sn.v11)) * 0.125 * dt;
         const double total_flux = right_flux - left_flux + top_flux - bottom_flux + front_flux - back_flux;
-        const double vol = volume(y, z), d0 = density0(y, z);
-        const double volume_change = (vol) / (vol + total_flux);
-        const double recip_volume = 1.0 / vol;
-        const double energy_change =
-            (pressure(y, z) / d0 + qdiv(viscosity(y, z), d0)) * total_flux * recip_volume;
-        energy1.put(y, z, energy0(y, z) - energy_change);
-        density1.put(y, z, d0 * volume_change);
+        const double volume_change = (c.vol) / (c.vol + total_flux);
+        const double recip_volume = 1.0 / c.vol;
+        const double energy_change = (c.p / c.d + qdiv(c.q, c.d)) * total_flux * recip_volume;
+        energy1.put(y, z, c.e - energy_change);
+        density1.put(y, z, c.d * volume_change);
       }
     }
     u0 = u0n;
@@ -533,6 +451,7 @@ __global__ void __launch_bounds__(32 * kWarps, 4) pdv_flux_march(const __grid_co
     v = vn;
     s = sn;
     back_flux = front_flux;
+    c = n;
   }
 }
 
@@ -736,8 +655,9 @@ __global__ void __launch_bounds__(32 * kWarps, 4) advec_mom_x_march(const __grid
       density(lp.a[6], X);
   const Widths<0> cd(lp.a[4]);
   const double w0 = cd(X), wl = cd(X - 1), wr = cd(X + 1);
-  struct Row {  // mass flux and density x volume on lines z and z - 1, at X and its neighbour
-    double m0, m1, v0, v1;
+  const Fld xvel(lp.a[7], X), yvel(lp.a[8], X), zvel(lp.a[9], X);
+  struct Row {  // mass flux and density x volume on lines z and z - 1; velocities
+    double m0, m1, v0, v1, vel[3];
   };
   auto load = [&](int y) {
     Row r;
@@ -745,6 +665,9 @@ __global__ void __launch_bounds__(32 * kWarps, 4) advec_mom_x_march(const __grid
     r.m1 = mflux(y, z - 1);
     r.v0 = density(y, z) * post_volume<0, VOL>(volume, vfx, vfy, vfz, y, z);
     r.v1 = density(y, z - 1) * post_volume<0, VOL>(volume, vfx, vfy, vfz, y, z - 1);
+    r.vel[0] = xvel(y, z);
+    r.vel[1] = yvel(y, z);
+    r.vel[2] = zvel(y, z);
     return r;
   };
   Row b = load(m.m0 - 1);
@@ -762,8 +685,8 @@ __global__ void __launch_bounds__(32 * kWarps, 4) advec_mom_x_march(const __grid
     const double wdif = neg ? wr : wl;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-      const Fld vel(lp.a[7 + k], X), out(lp.a[10 + k], X);
-      const double v = vel(y, z);
+      const Fld out(lp.a[10 + k], X);
+      const double v = c.vel[k];
       const double vr = from_right(v), vrr = from_right2(v), vl = from_left(v);
       const double mom = advec_mom_face(nf, sigma, w0, wdif, neg ? vr : v, neg ? vrr : vl, neg ? v : vr);
       const double moml = from_left(mom);
@@ -795,26 +718,17 @@ __global__ void __launch_bounds__(32 * kWarps, 3) advec_mom_march(const __grid_c
   struct Flux {  // mass flux of one row: this line and the one before, and left of them
     double a, al, b, bl;
   };
-  auto flux = [&](int r) {
-    Flux f;
-    f.a = mflux(yy(r, 0), zz(r, 0));
-    f.b = mflux(yy(r, 1), zz(r, 1));
-    f.al = from_left(f.a);
-    f.bl = from_left(f.b);
-    return f;
-  };
+  auto pair = [](double a, double b) { return Flux{a, from_left(a), b, from_left(b)}; };
+  auto flux = [&](int r) { return pair(mflux(yy(r, 0), zz(r, 0)), mflux(yy(r, 1), zz(r, 1))); };
   // (-1,0) + (0,0) + (-1,1) + (0,1) along (x, sweep), then the line before
   auto node_flux = [&](const Flux &p, const Flux &q) {
     return 0.125 * (p.al + p.a + q.al + q.a + p.bl + p.b + q.bl + q.b);
   };
-  auto mass = [&](int r) {
-    Flux f;
-    f.a = density(yy(r, 0), zz(r, 0)) * post_volume<DIR, VOL>(volume, vfx, vfy, vfz, yy(r, 0), zz(r, 0));
-    f.b = density(yy(r, 1), zz(r, 1)) * post_volume<DIR, VOL>(volume, vfx, vfy, vfz, yy(r, 1), zz(r, 1));
-    f.al = from_left(f.a);
-    f.bl = from_left(f.b);
-    return f;
+  auto dvol = [&](int r, int back) {
+    const int y = yy(r, back), z = zz(r, back);
+    return density(y, z) * post_volume<DIR, VOL>(volume, vfx, vfy, vfz, y, z);
   };
+  auto mass = [&](int r) { return pair(dvol(r, 0), dvol(r, 1)); };
   // (x, y, z) order of the reference: (0,-1,0) (0,0,0) (-1,-1,0) (-1,0,0),
   // then the same at z - 1; p is the row before q
   auto node_mass = [&](const Flux &p, const Flux &q) {
@@ -836,11 +750,23 @@ __global__ void __launch_bounds__(32 * kWarps, 3) advec_mom_march(const __grid_c
   vel3(r0 - 1, vb);
   vel3(r0, vc);
   vel3(r0 + 1, vn);
+  struct Row {  // row r + 2's velocities and mass fluxes, row r + 1's density x volume (this line, the one before)
+    double v[3], fa, fb, ma, mb;
+  };
+  auto load = [&](int r) {
+    Row w;
+    vel3(r + 2, w.v);
+    w.fa = mflux(yy(r + 2, 0), zz(r + 2, 0));
+    w.fb = mflux(yy(r + 2, 1), zz(r + 2, 1));
+    w.ma = dvol(r + 1, 0);
+    w.mb = dvol(r + 1, 1);
+    return w;
+  };
+  Row c = load(r0);
   for (int r = r0; r < m.m1; r++) {
-    double vnn[3];
-    vel3(r + 2, vnn);
-    const Flux f2 = flux(r + 2);
-    const Flux ms1 = mass(r + 1);
+    const Row n = load(min(r + 1, m.m1 - 1));
+    const double *vnn = c.v;
+    const Flux f2 = pair(c.fa, c.fb), ms1 = pair(c.ma, c.mb);
     const double nf1 = node_flux(f1, f2);
     const double mass_post1 = node_mass(ms, ms1);
     const double mass_pre1 = mass_post1 - nf + nf1;
@@ -865,6 +791,7 @@ __global__ void __launch_bounds__(32 * kWarps, 3) advec_mom_march(const __grid_c
     nf = nf1;
     mass_post = mass_post1;
     mass_pre = mass_pre1;
+    c = n;
   }
 }
 
@@ -884,7 +811,7 @@ ADVEC_MOM(advec_mom_fused_z1, (launch_march<31, 2>(lp, s, advec_mom_march<2, VOL
 ADVEC_MOM(advec_mom_fused_z3, (launch_march<31, 2>(lp, s, advec_mom_march<2, VOL_LAST>)))
 
 #define REG(K) OPSB_REGISTER_LOOP(K);
-REG(ideal_gas_summary) REG(viscosity_fused) REG(calc_dt_fused) REG(PdV_predict_pressure) REG(accelerate_fused)
+REG(ideal_gas_summary) REG(calc_dt_fused) REG(PdV_predict_pressure) REG(accelerate_fused)
 REG(PdV_flux) REG(advec_cell_fused_x1) REG(advec_cell_fused_x3) REG(advec_cell_fused_y2x) REG(advec_cell_fused_y2z)
 REG(advec_cell_fused_z1) REG(advec_cell_fused_z3) REG(advec_mom_fused_x1) REG(advec_mom_fused_x3)
 REG(advec_mom_fused_y2x) REG(advec_mom_fused_y2z) REG(advec_mom_fused_z1) REG(advec_mom_fused_z3)
