@@ -166,7 +166,7 @@ struct Heat3DWorkspace {
     cudaFree(buf);
     buf = nullptr;
     nx = ny = nz = 0;
-    const size_t one = (size_t)pt * (y + 2) * (zz + 2);
+    const size_t one = ((size_t)pt * (y + 2) * (zz + 2) + 15) / 16 * 16;  // 128-byte aligned volumes
     OPSB_CUDA(cudaMalloc(&buf, 5 * one * sizeof(double)));
     OPSB_CUDA(cudaMemsetAsync(buf, 0, 5 * one * sizeof(double), s));
     const size_t first = (size_t)pt * (y + 2) + pt + 1;

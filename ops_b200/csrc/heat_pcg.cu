@@ -1,23 +1,30 @@
 // Device-resident Jacobi-PCG for the TeaLeaf 2D heat operator; interface and
 // algorithm notes in heat_pcg.h.
 //
-// Per iteration (tea_leaf_cg.cpp:103-214, one kernel per reference routine):
-//   k_w   w = A p, pw = p.w                  -> last block: alpha = rro / pw
-//   k_ur  u += alpha p, r -= alpha w, z = Mi r, rz = r.z
-//                                            -> last block: beta, rro, stop test
-//   k_p   p = beta p + z
+// Per iteration (tea_leaf_cg.cpp:103-214) two kernels, each one pass:
+//   k_pw  p = beta p + z, w = A p, pw = p.w, and u += alpha p for the
+//         previous iteration's direction and step -> last block: alpha = rro / pw
+//   k_r   r -= alpha w, rz = r.(Mi r)       -> last block: beta, rro, stop test
+// and after the loop k_flush, the last iteration's u update. The reference's
+// sequence (w; u, r, z; p) passes p through HBM three times and z and u twice
+// as often: 120 B per cell and iteration in FP64, 96 B here (u, p, w, r once
+// in and once out, the faces once in k_pw, Mi once in k_r). The new direction
+// goes to a second buffer, since a cell's neighbours still read the old one;
+// `iters` says which of the two is current.
 // The arithmetic of every cell is the reference's, in its order (this file
 // builds without FMA contraction). Grid sums finish in a fixed order (each
 // block's partial, then the last block to arrive adds the partials by block
 // index), so a solve is bit-reproducible run to run. Once the stop test has
 // fired every later kernel returns at entry, so a chunk of iterations that
 // runs past convergence costs only its launch latency.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
 
 #include "heat_pcg.h"
+#include "march_grid.h"
 #include "runtime.h"
 
 namespace opsb {
@@ -42,6 +49,7 @@ struct Scalars {
   int iters;
   int max_iters;
   int first;
+  int pend;  // u += alpha p of the last k_pw is still to be made
   // FCG restart test on the device (replayed chunks): ||r|| of the last
   // iterations since the last (re)start, `window` 0 when the test is off
   int window, hcount;
@@ -121,61 +129,115 @@ __device__ __forceinline__ T smvp(const T *__restrict__ Kx, const T *__restrict_
   for (int y = blockIdx.y * BY + threadIdx.y; y < (g).ny; y += gridDim.y * BY)                 \
     for (int x = blockIdx.x * BX + threadIdx.x; x < (g).nx; x += gridDim.x * BX)
 
-// tea_leaf_cg_calc_w_reduce_kernel (tea_leaf_cg_kernels.h:8) + alpha = rro/pw.
+// How k_pw gets z: the residual itself, Mi r with Mi read, or Mi r with
+// Mi = 1 / diag(A) computed from the faces it holds anyway (FP64: the same
+// bits as tea_leaf_common_init_diag_init_kernel's Mi, 8 B a cell less).
+enum { Z_R = 0, Z_MI = 1, Z_DIAG = 2 };
+
+// tea_leaf_axpby_kernel (p = beta p + z), tea_leaf_cg_calc_w_reduce_kernel
+// (w = A p, p.w; tea_leaf_cg_kernels.h:8) and the previous iteration's
+// tea_leaf_axpy_kernel on u; then alpha = rro / pw. A warp marches up a strip
+// of 32 columns, one per lane, 30 of them its own: p of the rows below and
+// above stays in registers, p of the columns beside comes by shuffles. The
+// ring's p never changes and is read from the first buffer.
+// A row's loads are issued two rows ahead; FP32 rows are half the bytes, so
+// four CTAs an SM there, three in FP64.
 template <class T>
-__global__ void __launch_bounds__(NT, kResident) k_w(Geom g, const T *__restrict__ Kx, const T *__restrict__ Ky,
-                                          const T *__restrict__ p, T *__restrict__ w, T rx, T ry, Scalars *s,
-                                          double *part, unsigned *cnt) {
+constexpr int kPwBlocks = sizeof(T) == 4 ? 4 : 3;
+template <class T, int Z>
+__global__ void __launch_bounds__(NT, kPwBlocks<T>) k_pw(Geom g, const T *__restrict__ Kx, const T *__restrict__ Ky, T *pa, T *pb,
+                                              const T *__restrict__ r, const T *__restrict__ Mi, T *__restrict__ u,
+                                              T *__restrict__ w, T rx, T ry, int rows, Scalars *s, double *part,
+                                              unsigned *cnt) {
   __shared__ double sm[kWarps];
   __shared__ int last;
   if (s->done) return;
+  const int odd = s->iters & 1;
+  const T *pin = odd ? pb : pa;
+  T *pout = odd ? pa : pb;
+  const bool first = s->iters == 0 && !s->pend, pend = s->pend != 0;
+  const T alpha = (T)s->alpha, beta = (T)s->beta;
+  const int ncol = (g.nx + 29) / 30, nst = (g.ny + rows - 1) / rows;
+  const int wi = blockIdx.x * kWarps + (tid_() >> 5), lane = tid_() & 31;
   double acc[1] = {0.0};
-  HEAT_CELLS(g) {
-    const long long i = (long long)y * g.pitch + x;
-    const T wv = smvp(Kx, Ky, p, i, g.pitch, rx, ry);
-    w[i] = wv;
-    acc[0] = acc[0] + (double)wv * (double)p[i];
+  if (wi < ncol * nst) {
+    const int x = (wi % ncol) * 30 + lane - 1, y0 = (wi / ncol) * rows, y1 = min(y0 + rows, g.ny);
+    const bool in = x >= 0 && x < g.nx, own = in && lane >= 1 && lane <= 30, ring = x == -1 || x == g.nx;
+    const long long P = g.pitch;
+    struct Row {
+      T kx0, kx1, ky1, r, p, m, u;
+    };
+    auto load = [&](int y) {
+      Row v{};
+      const long long i = (long long)y * P + x;
+      if (in && y >= 0 && y < g.ny) {
+        v.kx0 = Kx[i];
+        if (lane == 31) v.kx1 = Kx[i + 1];  // the other lanes' comes from their neighbour
+        v.ky1 = Ky[i + P];
+        v.r = r[i];
+        v.p = pin[i];
+        if (Z == Z_MI) v.m = Mi[i];
+        if (pend && own && y >= y0 && y < y1) v.u = u[i];
+      } else if (in || (ring && y >= 0 && y < g.ny)) {
+        v.p = pa[i];
+        if (x == g.nx) v.kx0 = Kx[i];  // the last column's right face
+      }
+      return v;
+    };
+    // the new direction at row y; d is the diagonal of A there
+    auto dir = [&](Row &v, int y, T ky0, T &d) {
+      const T kr = __shfl_down_sync(0xffffffffu, v.kx0, 1);
+      if (lane < 31) v.kx1 = kr;
+      d = T(1) + ry * (v.ky1 + ky0) + rx * (v.kx1 + v.kx0);
+      if (!in || y < 0 || y >= g.ny) return v.p;
+      const T z = Z == Z_R ? v.r : Z == Z_MI ? v.m * v.r : (T(1) / d) * v.r;
+      return first ? z : beta * v.p + z;
+    };
+    auto face = [&](int y) { return in && y >= 0 && y < g.ny ? Ky[(long long)y * P + x] : T(0); };
+    Row b = load(y0 - 1);
+    T d;
+    T pm = dir(b, y0 - 1, face(y0 - 1), d);
+    T ky0 = face(y0);
+    Row c = load(y0), n = load(y0 + 1);
+    T pc = dir(c, y0, ky0, d);
+    for (int y = y0; y < y1; y++) {
+      const Row nn = load(min(y + 2, y1));
+      const T ky1 = c.ky1;
+      T dn;
+      const T pn = dir(n, y + 1, ky1, dn);
+      const T pl = __shfl_up_sync(0xffffffffu, pc, 1), pr = __shfl_down_sync(0xffffffffu, pc, 1);
+      if (own) {
+        const long long i = (long long)y * P + x;
+        const T wv = d * pc - ry * (ky1 * pn + ky0 * pm) - rx * (c.kx1 * pr + c.kx0 * pl);
+        w[i] = wv;
+        pout[i] = pc;
+        if (pend) u[i] = c.u + alpha * c.p;
+        acc[0] = acc[0] + (double)wv * (double)pc;
+      }
+      pm = pc;
+      pc = pn;
+      d = dn;
+      ky0 = ky1;
+      c = n;
+      n = nn;
+    }
   }
   if (publish<1>(acc, part, cnt, sm, &last)) {
     const double t = grid_total<1>(part, 0, sm);
     if (tid_() == 0) {
       s->pw = t;
       s->alpha = s->rro / t;
+      s->pend = 1;
       *cnt = 0u;
     }
   }
 }
 
-// tea_leaf_axpy_kernel on u and r, tea_leaf_zeqxty_kernel (z = Mi r) and
-// tea_leaf_dot_kernel (r.z), or tea_leaf_cg_calc_ur_r_reduce_kernel (r.r)
-// without preconditioner; then beta = rrn/rro and the stop test.
-template <class T, bool PREC, int STOP>
-__global__ void __launch_bounds__(NT, kResident) k_ur(Geom g, T *__restrict__ u, const T *__restrict__ p, T *__restrict__ r,
-                                           const T *__restrict__ w, const T *__restrict__ Mi, T *__restrict__ z,
-                                           Scalars *s, double *part, unsigned *cnt) {
-  constexpr int NV = (STOP == STOP_TRUE && PREC) ? 2 : 1;
-  __shared__ double sm[kWarps];
-  __shared__ int last;
-  if (s->done) return;
-  const T alpha = (T)s->alpha;
-  double acc[NV];
-#pragma unroll
-  for (int k = 0; k < NV; k++) acc[k] = 0.0;
-  HEAT_CELLS(g) {
-    const long long i = (long long)y * g.pitch + x;
-    u[i] = u[i] + alpha * p[i];
-    const T rv = r[i] - alpha * w[i];
-    r[i] = rv;
-    if (PREC) {
-      const T zv = Mi[i] * rv;
-      z[i] = zv;
-      acc[0] = acc[0] + (double)rv * (double)zv;
-    } else {
-      acc[0] = acc[0] + (double)rv * (double)rv;
-    }
-    if (NV == 2) acc[NV - 1] = acc[NV - 1] + (double)rv * (double)rv;
-  }
-  if (publish<NV>(acc, part, cnt, sm, &last)) {
+// The last block's part of k_r: beta = rrn / rro and the stop test.
+template <int NV, int STOP>
+__device__ __forceinline__ void finish_r(const double (&acc)[NV], Scalars *s, double *part, unsigned *cnt, double *sm,
+                                         int *last) {
+  if (publish<NV>(acc, part, cnt, sm, last)) {
     const double t = grid_total<NV>(part, 0, sm);
     const double rr = NV == 2 ? grid_total<NV>(part, NV - 1, sm) : t;
     if (tid_() == 0) {
@@ -193,14 +255,45 @@ __global__ void __launch_bounds__(NT, kResident) k_ur(Geom g, T *__restrict__ u,
   }
 }
 
-// tea_leaf_axpby_kernel with alpha = beta, beta = 1 (tea_leaf_cg.cpp:188-214).
-template <class T>
-__global__ void __launch_bounds__(NT, kResident) k_p(Geom g, T *__restrict__ p, const T *__restrict__ z, const Scalars *s) {
+// tea_leaf_axpy_kernel on r, tea_leaf_zeqxty_kernel (z = Mi r) and
+// tea_leaf_dot_kernel (r.z), or tea_leaf_cg_calc_ur_r_reduce_kernel's r.r
+// without preconditioner.
+template <class T, bool PREC, int STOP>
+__global__ void __launch_bounds__(NT, kResident) k_r(Geom g, T *__restrict__ r, const T *__restrict__ w,
+                                                     const T *__restrict__ Mi, Scalars *s, double *part,
+                                                     unsigned *cnt) {
+  constexpr int NV = (STOP == STOP_TRUE && PREC) ? 2 : 1;
+  __shared__ double sm[kWarps];
+  __shared__ int last;
   if (s->done) return;
-  const T beta = (T)s->beta;
+  const T alpha = (T)s->alpha;
+  double acc[NV] = {};
   HEAT_CELLS(g) {
     const long long i = (long long)y * g.pitch + x;
-    p[i] = beta * p[i] + z[i];
+    const T rv = r[i] - alpha * w[i];
+    r[i] = rv;
+    const T zv = PREC ? Mi[i] * rv : rv;
+    acc[0] = acc[0] + (double)rv * (double)zv;
+    if (NV == 2) acc[NV - 1] = acc[NV - 1] + (double)rv * (double)rv;
+  }
+  finish_r<NV, STOP>(acc, s, part, cnt, sm, &last);
+}
+
+// After the loop: the pending u += alpha p, the current direction back in the
+// first buffer and, when `z` is wanted, z = Mi r.
+template <class T>
+__global__ void __launch_bounds__(NT, kResident) k_flush(Geom g, T *__restrict__ u, T *pa, const T *pb,
+                                                         const T *__restrict__ r, const T *__restrict__ Mi, T *z,
+                                                         const Scalars *s) {
+  if (!s->pend) return;
+  const T alpha = (T)s->alpha;
+  const bool odd = s->iters & 1;
+  HEAT_CELLS(g) {
+    const long long i = (long long)y * g.pitch + x;
+    const T p = odd ? pb[i] : pa[i];
+    u[i] = u[i] + alpha * p;
+    if (odd) pa[i] = p;
+    if (z) z[i] = Mi[i] * r[i];
   }
 }
 
@@ -264,6 +357,7 @@ __global__ void __launch_bounds__(NT, kResident) k_init(Geom g, const double *__
       s->iters = 0;
       s->max_iters = max_iters;
       s->done = 0;
+      s->pend = 0;
       *cnt = 0u;
     }
   }
@@ -272,15 +366,15 @@ __global__ void __launch_bounds__(NT, kResident) k_init(Geom g, const double *__
 // Reliable update of the FP32 loop (Sleijpen and van der Vorst 1996, "Reliable
 // updated residuals in hybrid Bi-CG methods"): the recursive FP32 residual is
 // replaced by the FP64 residual r64 = u0 - A u, z32 = Mi32 r32, and the search
-// direction is kept: beta = rz_new / rz_prev, followed by k_p. The first call
-// starts the loop (beta = 0 with p32 = 0, so p = z) and fixes the estimate
+// direction is kept: beta = rz_new / rz_prev, which the next k_pw applies. The
+// first call starts the loop (no direction yet, so p = z) and fixes the estimate
 // threshold eps * sqrt(rz0); `scale` tightens it after an estimate that the
 // FP64 check did not confirm. The next update is due once sqrt(rz) has fallen
 // by `delta`.
 template <bool PREC>
 __global__ void __launch_bounds__(NT, kResident) k_reinit32(Geom g, Geom g32, const double *__restrict__ r64,
-                                                 float *__restrict__ r, const float *__restrict__ Mi,
-                                                 float *__restrict__ z, int first, double eps, double scale,
+                                                 float *__restrict__ r, const float *__restrict__ Mi, int first,
+                                                 double eps, double scale,
                                                  double delta, int max_iters, Scalars *s, double *part,
                                                  unsigned *cnt) {
   __shared__ double sm[kWarps];
@@ -291,11 +385,7 @@ __global__ void __launch_bounds__(NT, kResident) k_reinit32(Geom g, Geom g32, co
     const long long j = (long long)y * g32.pitch + x;
     const float rv = (float)r64[i];
     r[j] = rv;
-    float zv = rv;
-    if (PREC) {
-      zv = Mi[j] * rv;
-      z[j] = zv;
-    }
+    const float zv = PREC ? Mi[j] * rv : rv;
     acc[0] = acc[0] + (double)rv * (double)zv;
   }
   if (publish<1>(acc, part, cnt, sm, &last)) {
@@ -313,17 +403,24 @@ __global__ void __launch_bounds__(NT, kResident) k_reinit32(Geom g, Geom g32, co
       s->ref = delta * sqrt(fabs(t));
       s->rro = t;
       s->done = 0;
+      s->pend = 0;
       *cnt = 0u;
     }
   }
 }
 
-// Reliable update, FP64 side: u += e, e = 0.
-__global__ void __launch_bounds__(NT, kResident) k_update(Geom g, Geom g32, double *__restrict__ u, float *__restrict__ e) {
+// Reliable update, FP64 side: e += alpha p (the last iteration's), u += e, e = 0.
+__global__ void __launch_bounds__(NT, kResident) k_update(Geom g, Geom g32, double *__restrict__ u,
+                                                          float *__restrict__ e, const float *__restrict__ pa,
+                                                          const float *__restrict__ pb, const Scalars *s) {
+  const float alpha = (float)s->alpha;
+  const float *p = s->iters & 1 ? pb : pa;
+  const bool pend = s->pend != 0;
   HEAT_CELLS(g) {
     const long long i = (long long)y * g.pitch + x;
     const long long j = (long long)y * g32.pitch + x;
-    u[i] = u[i] + (double)e[j];
+    const float ev = pend ? e[j] + alpha * p[j] : e[j];
+    u[i] = u[i] + (double)ev;
     e[j] = 0.0f;
   }
 }
@@ -338,10 +435,263 @@ __global__ void __launch_bounds__(NT, kResident) k_to_float(Geom g, Geom g32, co
       const long long i = (long long)y * g.pitch + x, j = (long long)y * g32.pitch + x;
       fa[j] = (float)a[i];
       fb[j] = (float)b[i];
-      if (c) fc[j] = (float)c[i];
+      if (c) fc[j] = x >= 0 && x < g.nx && y >= 0 && y < g.ny ? (float)c[i] : 0.0f;  // Mi: zero on the ring
     }
 }
 
+
+// ---- the whole loop in one kernel, for grids that fit the registers ---------
+// Up to kTargetBlocks blocks of 128 x 2 cells (303 K cells, 550^2) an iteration
+// of the two kernels above is launch and drain latency: 14 us at 128^2, 17 us
+// at 512^2. Here a CTA keeps K such blocks, one above the other: its cells' r,
+// u and coefficients stay in registers, the direction p in shared memory with a
+// one-cell halo, for the whole loop. CTAs exchange only z along their edges
+// and the partial sums (a neighbour's p is beta p + z, tracked in the halo):
+// 64^2 14.1 -> 3.7 us an iteration, 128^2 14.0 -> 4.5, 256^2 14.2 -> 5.4, 512^2
+// 17.3 -> 10.8 (FP64).
+// Each block's partial is its own, and the totals are taken, in the order that
+// the launched kernels use (publish, grid_total), so alpha, beta and every
+// iterate are the same bits as an iteration of single-cell threads gave.
+//
+// A value travels as two 64-bit words, each with half of it and the number of
+// the exchange, so a reader knows a whole value without a fence or a counter;
+// two slots alternate, since a CTA can be one exchange ahead of another. The CTAs wait for one another, so the launch is cooperative, and
+// every wait ends after two seconds with an error.
+constexpr unsigned long long kWaitNs = 2000000000ull;
+
+__device__ __forceinline__ void ll_put(ulonglong2 *slot, double v, unsigned tag) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
+  asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
+               : "memory");
+}
+// The value tagged `tag`; false when it did not arrive in time.
+__device__ __forceinline__ bool ll_get(const ulonglong2 *slot, unsigned tag, double *v) {
+  unsigned long long t0 = 0;
+  for (unsigned i = 0;; i++) {
+    unsigned long long a, b;
+    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(slot) : "memory");
+    if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag) {
+      *v = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+      return true;
+    }
+    if ((i & 255u) == 255u) {
+      unsigned long long now;
+      asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+      if (!t0) t0 = now;
+      else if (now - t0 > kWaitNs) return false;
+    }
+  }
+}
+
+template <class T, int Z, int STOP, int K>
+__global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restrict__ Kx, const T *__restrict__ Ky,
+                                                        T *__restrict__ p, T *__restrict__ r, const T *__restrict__ Mi,
+                                                        T *__restrict__ u, T *__restrict__ zout, T rx, T ry, int gx,
+                                                        Scalars *s, ulonglong2 *slots, int *err) {
+  constexpr int NV = (STOP == STOP_TRUE && Z != Z_R) ? 2 : 1;
+  __shared__ T ps[2 * K + 2][BX + 2];
+  __shared__ double ws[NV * K][kWarps], sm[kWarps], tot[2];
+  __shared__ int expired;
+  if (s->done) return;
+  const int tx = threadIdx.x, ty = threadIdx.y, t = tid_(), lane = t & 31, warp = t >> 5;
+  const int bx = blockIdx.x % gx, by = blockIdx.x / gx, y0 = by * 2 * K, x = bx * BX + tx;
+  const int gy = (g.ny + BY - 1) / BY, nb = gx * gy;  // the launched kernels' blocks
+  const long long P = g.pitch;
+  const bool first = s->iters == 0;
+  double rro = s->rro, rro_prev = s->rro_prev, alpha = s->alpha, beta = s->beta, pw = s->pw, e = s->err;
+  int iters = s->iters;
+  const int max_iters = s->max_iters;
+  const double stop = s->stop, ref = s->ref;
+  if (t == 0) expired = 0;
+
+  T kx0[K], kx1[K], ky0[K], ky1[K], d[K], mi[K], rv[K], uv[K], pv[K], zv[K], wv[K];
+  auto row = [&](int k) { return y0 + 2 * k + ty; };
+  auto cell = [&](int xx, int yy) { return xx >= 0 && xx < g.nx && yy >= 0 && yy < g.ny; };
+  // a ring cell beside the interior holds a constant direction
+  auto ring = [&](int xx, int yy) {
+    return ((xx == -1 || xx == g.nx) && yy >= 0 && yy < g.ny) || ((yy == -1 || yy == g.ny) && xx >= 0 && xx < g.nx);
+  };
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const int y = row(k);
+    const long long i = (long long)y * P + x;
+    kx0[k] = kx1[k] = ky0[k] = ky1[k] = d[k] = mi[k] = rv[k] = uv[k] = pv[k] = zv[k] = T(0);
+    if (cell(x, y)) {
+      kx0[k] = Kx[i];
+      kx1[k] = Kx[i + 1];
+      ky0[k] = Ky[i];
+      ky1[k] = Ky[i + P];
+      d[k] = T(1) + ry * (ky1[k] + ky0[k]) + rx * (kx1[k] + kx0[k]);
+      mi[k] = Z == Z_R ? T(1) : Mi[i];
+      rv[k] = r[i];
+      uv[k] = u[i];
+      if (!first) pv[k] = p[i];
+      zv[k] = Z == Z_R ? rv[k] : mi[k] * rv[k];
+    } else {
+      ps[1 + 2 * k + ty][1 + tx] = ring(x, y) ? p[i] : T(0);
+    }
+  }
+  // z on a CTA's edges: its first row, last row, first column, last column,
+  // in one of two buffers
+  constexpr int kEdge = 2 * BX + 4 * K;
+  ulonglong2 *edges = slots + 4 * kTargetBlocks;
+  auto edge = [&](int cx, int cy, int at, unsigned buf) {
+    return edges + ((size_t)(cx + cy * gx) * 2 + buf) * kEdge + at;
+  };
+  // this thread's halo cells: above or below its column, and one at the side
+  struct Halo {
+    T *at;  // its place in ps
+    const ulonglong2 *from;  // its CTA's edge slot, first buffer
+    bool live;  // an interior cell of another CTA
+    T p, z;
+  };
+  auto halo = [&](int xx, int yy, int cx, int cy, int slot) {
+    const long long i = (long long)yy * P + xx;
+    Halo h{&ps[yy - y0 + 1][xx - bx * BX + 1], nullptr, cell(xx, yy), T(0), T(0)};
+    if (h.live) {
+      h.from = edge(cx, cy, slot, 0);
+      h.z = Z == Z_R ? r[i] : Mi[i] * r[i];
+      if (!first) h.p = p[i];
+    } else {
+      *h.at = ring(xx, yy) ? p[i] : T(0);
+    }
+    return h;
+  };
+  Halo hv = ty ? halo(x, y0 + 2 * K, bx, by + 1, tx) : halo(x, y0 - 1, bx, by - 1, BX + tx), hs{};
+  if (t < 2 * K) hs = halo(bx * BX - 1, y0 + t, bx - 1, by, 2 * BX + 2 * K + t);
+  else if (t < 4 * K) hs = halo(bx * BX + BX, y0 + t - 2 * K, bx + 1, by, 2 * BX + t - 2 * K);
+
+  // the grid's sums of acc[v * K + k], block k of this CTA; `meanwhile` runs
+  // between this CTA's share and the wait for the others'
+  auto total = [&](auto &acc, auto nv, unsigned tag, auto meanwhile) {
+    constexpr int N = decltype(nv)::value;
+#pragma unroll
+    for (int q = 0; q < N * K; q++) {
+      double v = acc[q];
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      if (lane == 0) ws[q][warp] = v;
+    }
+    __syncthreads();
+    ulonglong2 *buf = slots + (size_t)(tag & 1u) * 2 * kTargetBlocks;
+    for (int q = warp; q < N * K; q += kWarps) {
+      double v = lane < kWarps ? ws[q][lane] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+      const int k = q % K, vb = y0 / 2 + k;
+      if (lane == 0 && vb < gy) ll_put(buf + (size_t)(q / K) * kTargetBlocks + bx + vb * gx, v, tag);
+    }
+    meanwhile();
+#pragma unroll
+    for (int n = 0; n < N; n++) {
+      double v = 0.0;
+      for (int b = t; b < nb; b += NT) {
+        double q = 0.0;
+        if (!ll_get(buf + (size_t)n * kTargetBlocks + b, tag, &q)) expired = 1;
+        v += q;
+      }
+      v = block_sum(v, sm);
+      if (t == 0) tot[n] = v;
+    }
+    __syncthreads();
+  };
+
+  unsigned tag = 0;
+  int done = 0;
+  bool fresh = first;
+  while (true) {
+    const T bt = (T)beta;
+#pragma unroll
+    for (int k = 0; k < K; k++) {
+      pv[k] = fresh ? zv[k] : bt * pv[k] + zv[k];
+      if (cell(x, row(k))) ps[1 + 2 * k + ty][1 + tx] = pv[k];
+    }
+    if (hv.live) *hv.at = hv.p = fresh ? hv.z : bt * hv.p + hv.z;
+    if (hs.live) *hs.at = hs.p = fresh ? hs.z : bt * hs.p + hs.z;
+    fresh = false;
+    __syncthreads();
+    {
+      double acc[K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        const int yy = 1 + 2 * k + ty, xx = 1 + tx;
+        wv[k] = d[k] * pv[k] - ry * (ky1[k] * ps[yy + 1][xx] + ky0[k] * ps[yy - 1][xx]) -
+                rx * (kx1[k] * ps[yy][xx + 1] + kx0[k] * ps[yy][xx - 1]);
+        acc[k] = (double)wv[k] * (double)pv[k];
+      }
+      total(acc, std::integral_constant<int, 1>{}, ++tag, [] {});
+    }
+    if (expired) break;
+    pw = tot[0];
+    alpha = rro / pw;
+    const T al = (T)alpha;
+    {
+      double acc[NV * K];
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        uv[k] = uv[k] + al * pv[k];
+        rv[k] = rv[k] - al * wv[k];
+        zv[k] = Z == Z_R ? rv[k] : mi[k] * rv[k];
+        acc[k] = (double)rv[k] * (double)zv[k];
+        if (NV == 2) acc[(NV - 1) * K + k] = (double)rv[k] * (double)rv[k];
+      }
+      ++tag;
+      const unsigned buf = (tag >> 1) & 1u;
+#pragma unroll
+      for (int k = 0; k < K; k++) {
+        if (!cell(x, row(k))) continue;
+        const int q = 2 * k + ty;
+        const double zd = (double)zv[k];
+        if (q == 0) ll_put(edge(bx, by, tx, buf), zd, tag);
+        if (q == 2 * K - 1) ll_put(edge(bx, by, BX + tx, buf), zd, tag);
+        if (tx == 0) ll_put(edge(bx, by, 2 * BX + q, buf), zd, tag);
+        if (tx == BX - 1) ll_put(edge(bx, by, 2 * BX + 2 * K + q, buf), zd, tag);
+      }
+      total(acc, std::integral_constant<int, NV>{}, tag, [&] {
+        double z = 0.0;
+        if (hv.live) {
+          if (!ll_get(hv.from + (size_t)buf * kEdge, tag, &z)) expired = 1;
+          hv.z = (T)z;
+        }
+        if (hs.live) {
+          if (!ll_get(hs.from + (size_t)buf * kEdge, tag, &z)) expired = 1;
+          hs.z = (T)z;
+        }
+      });
+    }
+    if (expired) break;
+    const double rz = tot[0], rr = tot[NV - 1];
+    rro_prev = rro;
+    beta = rz / rro;
+    rro = rz;
+    iters++;
+    e = STOP == STOP_TRUE ? sqrt(fabs(rr)) : sqrt(fabs(rz));
+    if (fabs(e) < stop) done = 1;
+    else if (STOP == STOP_RELIABLE && e < ref) done = 3;
+    else if (iters >= max_iters) done = 2;
+    if (done) break;
+  }
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    if (!cell(x, row(k))) continue;
+    const long long i = (long long)row(k) * P + x;
+    u[i] = uv[k];
+    r[i] = rv[k];
+    p[i] = pv[k];
+    if (zout) zout[i] = zv[k];
+  }
+  if (blockIdx.x == 0 && t == 0) {
+    s->rro = rro;
+    s->rro_prev = rro_prev;
+    s->alpha = alpha;
+    s->beta = beta;
+    s->pw = pw;
+    s->err = e;
+    s->iters = iters;
+    s->done = done;
+  }
+  if (t == 0 && expired) *err = 1;
+}
 
 // ---- flexible CG (Notay 2000, FCG with one-step truncation) ----------------
 // k_fw: w = A p, pw = p.w, pr = p.r -> alpha = pr / pw; a non-positive pw
@@ -482,31 +832,175 @@ __device__ __forceinline__ T smvp3(const T *__restrict__ Kx, const T *__restrict
          ry * (ky1 * u[i + P] + ky0 * u[i - P]) - rx * (kx1 * u[i + 1] + kx0 * u[i - 1]);
 }
 
-// w = A p on the interior, pw = p.w -> alpha = rro / pw (k_w in 3D; FP64, or
-// FP32 for the mixed solver's inner iterations).
+// k_pw in 3D (FP64, or FP32 for the mixed solver's inner iterations), with z =
+// Mi r. A CTA marches along z over a tile of 30 x (kTileY - 2) cells, one
+// column a thread, its outermost threads computing p for their neighbours:
+// p of the planes below and above stays in registers, p of the columns beside
+// comes by shuffles in x and through shared memory in y (three planes, so that
+// one barrier a plane is enough). Halo cells hold p = 0.
+constexpr int kTileY = 16;
+
 template <class T>
-__global__ void __launch_bounds__(NT, kResident) k_w3(Geom3 g, const T *__restrict__ Kx, const T *__restrict__ Ky,
-                                                     const T *__restrict__ Kz, const T *__restrict__ p,
-                                                     T *__restrict__ w, T rx, T ry, T rz, Scalars *s, double *part,
-                                                     unsigned *cnt) {
+__global__ void __launch_bounds__(32 * kTileY, 2) k_pw3(Geom3 g, const T *__restrict__ Kx, const T *__restrict__ Ky,
+                                                       const T *__restrict__ Kz, T *pa, T *pb,
+                                                       const T *__restrict__ r, const T *__restrict__ Mi,
+                                                       T *__restrict__ u, T *__restrict__ w, T rx, T ry, T rz, int tx,
+                                                       int ty, int planes, Scalars *s, double *part, unsigned *cnt) {
+  __shared__ double sm[kTileY];
+  __shared__ T ps[3][kTileY][32];
+  __shared__ int last;
+  if (s->done) return;
+  const int odd = s->iters & 1;
+  const T *pin = odd ? pb : pa;
+  T *pout = odd ? pa : pb;
+  const bool first = s->iters == 0 && !s->pend, pend = s->pend != 0;
+  const T alpha = (T)s->alpha, beta = (T)s->beta;
+  const int lane = threadIdx.x, row = threadIdx.y;
+  const int bx = blockIdx.x % tx, by = (blockIdx.x / tx) % ty, bz = blockIdx.x / (tx * ty);
+  const int x = bx * 30 + lane - 1, y = by * (kTileY - 2) + row - 1;
+  const int z0 = bz * planes, z1 = min(z0 + planes, g.nz);
+  const bool in = x >= 0 && x < g.nx && y >= 0 && y < g.ny;
+  const bool own = in && lane >= 1 && lane <= 30 && row >= 1 && row <= kTileY - 2;
+  const long long P = g.pitch, Q = g.plane, base = (long long)y * P + x;
+  struct Raw {
+    T r, p, m;
+  };
+  auto load = [&](int z) {
+    Raw v{};
+    if (in && z >= 0 && z < g.nz) {
+      const long long i = base + (long long)z * Q;
+      v.r = r[i];
+      v.p = pin[i];
+      v.m = Mi[i];
+    }
+    return v;
+  };
+  auto dir = [&](const Raw &v) {
+    const T z = v.m * v.r;
+    return first ? z : beta * v.p + z;
+  };
+  double acc = 0.0;
+  const Raw b = load(z0 - 1);
+  Raw c = load(z0), n = load(z0 + 1);
+  T pm = dir(b), pc = dir(c);
+  ps[z0 % 3][row][lane] = pc;
+  T kz0 = own ? Kz[base + (long long)z0 * Q] : T(0);
+  struct Face {
+    T kx0, kx1, ky0, ky1, kz1, u;
+  };
+  auto faces = [&](int z) {
+    Face f{};
+    if (own) {
+      const long long i = base + (long long)z * Q;
+      f.kx0 = Kx[i];
+      f.kx1 = Kx[i + 1];
+      f.ky0 = Ky[i];
+      f.ky1 = Ky[i + P];
+      f.kz1 = Kz[i + Q];
+      if (pend) f.u = u[i];
+    }
+    return f;
+  };
+  // FP32 has the registers to load a plane's faces one plane ahead too
+  constexpr bool kAhead = sizeof(T) == 4;
+  Face f{};
+  if (kAhead) f = faces(z0);
+  for (int z = z0; z < z1; z++) {
+    const long long i = base + (long long)z * Q;
+    if (!kAhead) f = faces(z);
+    const Face c_f = f;
+    if (kAhead) f = faces(min(z + 1, z1 - 1));
+    const Raw nn = load(min(z + 2, z1));
+    const T pn = dir(n);
+    ps[(z + 1) % 3][row][lane] = pn;
+    __syncthreads();
+    const T pl = __shfl_up_sync(0xffffffffu, pc, 1), pr = __shfl_down_sync(0xffffffffu, pc, 1);
+    if (own) {
+      const T kx0 = c_f.kx0, kx1 = c_f.kx1, ky0 = c_f.ky0, ky1 = c_f.ky1, kz1 = c_f.kz1;
+      const T ps0 = ps[z % 3][row - 1][lane], ps1 = ps[z % 3][row + 1][lane];
+      const T wv = (T(1) + rz * (kz1 + kz0) + ry * (ky1 + ky0) + rx * (kx1 + kx0)) * pc - rz * (kz1 * pn + kz0 * pm) -
+                   ry * (ky1 * ps1 + ky0 * ps0) - rx * (kx1 * pr + kx0 * pl);
+      w[i] = wv;
+      pout[i] = pc;
+      if (pend) u[i] = c_f.u + alpha * c.p;
+      acc = acc + (double)wv * (double)pc;
+    }
+    kz0 = c_f.kz1;
+    pm = pc;
+    pc = pn;
+    c = n;
+    n = nn;
+  }
+  // the block's partial, then the last block's total, as publish / grid_total
+  auto sum = [&](double v) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if (lane == 0) sm[row] = v;
+    __syncthreads();
+    double t = 0.0;
+    if (row == 0) {
+      t = lane < kTileY ? sm[lane] : 0.0;
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) t += __shfl_down_sync(0xffffffffu, t, o);
+    }
+    return t;
+  };
+  const double bs = sum(acc);
+  const bool lead = lane == 0 && row == 0;
+  if (lead) {
+    part[blockIdx.x] = bs;
+    __threadfence();
+    last = atomicAdd(cnt, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double v = 0.0;
+  for (int k = row * 32 + lane; k < (int)gridDim.x; k += 32 * kTileY) v += __ldcg(part + k);
+  const double t = sum(v);
+  if (lead) {
+    s->pw = t;
+    s->alpha = s->rro / t;
+    s->pend = 1;
+    *cnt = 0u;
+  }
+}
+
+// k_r over n consecutive values (the padded volume: its halo cells hold zeros
+// and stay zero), 16 bytes a load: rows of 194 values or so would leave a
+// quarter of a row-wise grid idle. The fields start on 16-byte boundaries.
+constexpr int kFlatBlocks = 4;  // CTAs per SM: 64 registers hold a vector of each field
+template <class T, int STOP>
+__global__ void __launch_bounds__(NT, kFlatBlocks) k_r_flat(T *__restrict__ r, const T *__restrict__ w,
+                                                          const T *__restrict__ Mi, long long n, Scalars *s,
+                                                          double *part, unsigned *cnt) {
+  constexpr int NV = STOP == STOP_TRUE ? 2 : 1, V = 16 / sizeof(T);
   __shared__ double sm[kWarps];
   __shared__ int last;
   if (s->done) return;
-  double acc[1] = {0.0};
-  HEAT_CELLS3(g) {
-    const long long i = (long long)z * g.plane + (long long)y * g.pitch + x;
-    const T wv = smvp3<T>(Kx, Ky, Kz, p, i, g.pitch, g.plane, rx, ry, rz);
-    w[i] = wv;
-    acc[0] = acc[0] + (double)wv * (double)p[i];
+  const T alpha = (T)s->alpha;
+  double acc[NV] = {};
+  struct alignas(16) Vec {
+    T v[V];
+  };
+  auto cell = [&](T rin, T wv, T m) {
+    const T rv = rin - alpha * wv;
+    acc[0] = acc[0] + (double)rv * (double)(m * rv);
+    if (NV == 2) acc[NV - 1] = acc[NV - 1] + (double)rv * (double)rv;
+    return rv;
+  };
+  const long long nv = n / V, step = (long long)gridDim.x * NT;
+  for (long long k = (long long)blockIdx.x * NT + tid_(); k < nv; k += step) {
+    Vec a = reinterpret_cast<Vec *>(r)[k];
+    const Vec b = reinterpret_cast<const Vec *>(w)[k], c = reinterpret_cast<const Vec *>(Mi)[k];
+#pragma unroll
+    for (int j = 0; j < V; j++) a.v[j] = cell(a.v[j], b.v[j], c.v[j]);
+    reinterpret_cast<Vec *>(r)[k] = a;
   }
-  if (publish<1>(acc, part, cnt, sm, &last)) {
-    const double t = grid_total<1>(part, 0, sm);
-    if (tid_() == 0) {
-      s->pw = t;
-      s->alpha = s->rro / t;
-      *cnt = 0u;
-    }
-  }
+  if (blockIdx.x == 0)
+    for (long long k = nv * V + tid_(); k < n; k += NT) r[k] = cell(r[k], w[k], Mi[k]);
+  finish_r<NV, STOP>(acc, s, part, cnt, sm, &last);
 }
 
 // r = u0 - A u, rr = r.r; the first call of a solve fixes ||r0|| and the stop
@@ -585,9 +1079,15 @@ struct Solver::Impl {
   float *f32 = nullptr;
   size_t f32_bytes = 0;
   long long pitch32 = 0;
-  float *Kx = nullptr, *Ky = nullptr, *Mi = nullptr, *r = nullptr, *p = nullptr, *w = nullptr, *z = nullptr,
+  float *Kx = nullptr, *Ky = nullptr, *Mi = nullptr, *r = nullptr, *p = nullptr, *w = nullptr, *p2 = nullptr,
         *e = nullptr;
+  // the FP64 direction's second buffer, interior at p64b + its field's offset
+  double *p64b = nullptr;
+  size_t p64b_n = 0;
   float *Kz = nullptr;  // 3D only
+  ulonglong2 *slots = nullptr;  // k_pcg_resident's exchange, then its error word
+  // 2 x 2 partials a block, and the edges of up to 256 CTAs of 16 rows
+  static constexpr size_t kSlotBytes = (4 * (size_t)kTargetBlocks + 256 * 2 * (2 * BX + 32)) * sizeof(ulonglong2);
   // replayed iteration chunks, rebuilt when any argument changes
   struct Chunk {
     cudaGraphExec_t exec = nullptr;
@@ -604,6 +1104,50 @@ struct Solver::Impl {
     cudaFree(part);
     cudaFree(cnt);
     cudaFree(f32);
+    cudaFree(p64b);
+    cudaFree(slots);
+  }
+
+  // The loop of one PCG run by k_pcg_resident when the grid fits it (returns
+  // false otherwise): s must hold what k_init or k_reinit32 left.
+  template <class T, int Z, int STOP>
+  bool resident(const Geom &g, const T *Kx, const T *Ky, T *p, T *r, const T *Mi, T *u, T *zout, T rx, T ry, Scalars *s,
+                cudaStream_t st) {
+    const int gx = (g.nx + BX - 1) / BX, gy = (g.ny + BY - 1) / BY;
+    if ((long long)gx * gy > kTargetBlocks) return false;
+    int dev = 0, sms = 0, coop = 0;
+    OPSB_CUDA(cudaGetDevice(&dev));
+    OPSB_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    OPSB_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+    if (!coop) return false;
+    int K = 1;
+    sms = std::min(sms, 256);
+    while (K <= 8 && gx * ((gy + K - 1) / K) > sms) K *= 2;
+    if (K > 8) return false;
+    if (!slots) OPSB_CUDA(cudaMalloc(&slots, kSlotBytes + 64));
+    OPSB_CUDA(cudaMemsetAsync(slots, 0, kSlotBytes + 64, st));
+    int *err = reinterpret_cast<int *>(reinterpret_cast<char *>(slots) + kSlotBytes);
+    const void *f = K == 1 ? (const void *)k_pcg_resident<T, Z, STOP, 1>
+                  : K == 2 ? (const void *)k_pcg_resident<T, Z, STOP, 2>
+                  : K == 4 ? (const void *)k_pcg_resident<T, Z, STOP, 4>
+                           : (const void *)k_pcg_resident<T, Z, STOP, 8>;
+    Geom gg = g;
+    int gxx = gx;
+    void *args[] = {&gg, &Kx, &Ky, &p, &r, &Mi, &u, &zout, &rx, &ry, &gxx, &s, &slots, &err};
+    OPSB_CUDA(cudaLaunchCooperativeKernel(f, dim3(gx * ((gy + K - 1) / K)), dim3(BX, BY), args, 0, st));
+    OPSB_CUDA(cudaMemcpyAsync(h_flag, err, sizeof(int), cudaMemcpyDeviceToHost, st));
+    OPSB_CUDA(cudaStreamSynchronize(st));
+    if (h_flag[0]) throw Error(E_TIMEOUT, "heat solver: a wait between thread blocks expired");
+    return true;
+  }
+
+  void ensure_p64(size_t n) {
+    if (n <= p64b_n) return;
+    cudaFree(p64b);
+    p64b = nullptr;
+    p64b_n = 0;
+    OPSB_CUDA(cudaMalloc(&p64b, n * sizeof(double)));
+    p64b_n = n;
   }
 
   void ensure_base() {
@@ -618,8 +1162,10 @@ struct Solver::Impl {
   }
 
   // The 3D mixed solver's nine FP32 fields, each a padded volume of nf
-  // values in the FP64 fields' flat layout, zero on every halo cell.
+  // values in the FP64 fields' flat layout, zero on every halo cell; each
+  // field starts on a 128-byte boundary.
   void ensure_f32_flat(size_t nf, cudaStream_t st) {
+    nf = (nf + 31) / 32 * 32;
     const size_t bytes = 9 * nf * sizeof(float);
     if (bytes != f32_bytes || pitch32 != -1) {
       cudaFree(f32);
@@ -630,7 +1176,7 @@ struct Solver::Impl {
       chunk32.key.clear();
     }
     OPSB_CUDA(cudaMemsetAsync(f32, 0, bytes, st));
-    float **fields[9] = {&Kx, &Ky, &Kz, &Mi, &r, &p, &w, &z, &e};
+    float **fields[9] = {&Kx, &Ky, &Kz, &Mi, &r, &p, &w, &p2, &e};
     for (int k = 0; k < 9; k++) *fields[k] = f32 + k * nf;
   }
 
@@ -649,7 +1195,7 @@ struct Solver::Impl {
       chunk32.key.clear();
     }
     OPSB_CUDA(cudaMemsetAsync(f32, 0, bytes, st));
-    float **fields[8] = {&Kx, &Ky, &Mi, &r, &p, &w, &z, &e};
+    float **fields[8] = {&Kx, &Ky, &Mi, &r, &p, &w, &p2, &e};
     for (int k = 0; k < 8; k++) *fields[k] = f32 + k * one + pitch + 32;
   }
 };
@@ -667,6 +1213,27 @@ dim3 grid_for(int nx, int ny) {
   if (gy > rows) gy = rows;
   if (gy < 1) gy = 1;
   return dim3(gx, gy);
+}
+
+// k_pw's strips and k_pw3's tiles (two CTAs).
+void pw_grid(int nx, int ny, int per_sm, int *rows, int *blocks) {
+  const long long ncol = (nx + 29) / 30;
+  *rows = march_rows(ncol, ny, 2, 148LL * per_sm * kWarps, (long long)kMaxBlocks * kWarps);
+  *blocks = (int)((ncol * ((ny + *rows - 1) / *rows) + kWarps - 1) / kWarps);
+  if (*blocks > kMaxBlocks) throw Error(E_UNSUPPORTED, "heat solver: rows too long");
+}
+struct Grid3 {
+  int tx, ty, planes, blocks;
+};
+Grid3 pw3_grid(int nx, int ny, int nz) {
+  Grid3 q;
+  q.tx = (nx + 29) / 30;
+  q.ty = (ny + kTileY - 3) / (kTileY - 2);
+  const long long tiles = (long long)q.tx * q.ty;
+  if (tiles > kMaxBlocks) throw Error(E_UNSUPPORTED, "heat solver 3D: cross-section too large");
+  q.planes = march_rows(tiles, nz, 2, 148LL * 2, kMaxBlocks);
+  q.blocks = (int)(tiles * ((nz + q.planes - 1) / q.planes));
+  return q;
 }
 
 std::string key_of(std::initializer_list<const void *> ptrs, std::initializer_list<double> vals) {
@@ -751,32 +1318,50 @@ void Solver::pcg_fp64(const Field2D &f, double rx, double ry, bool precond, bool
   check_launch("heat solver init");
   launches_ += 2;
   if (max_iters > 0) {
-    const std::string key = key_of({f.Kx, f.Ky, f.u, f.r, f.w, f.p, f.z, f.Mi},
-                                   {rx, ry, (double)f.nx, (double)f.ny, (double)f.pitch, precond ? 1.0 : 0.0,
-                                    true_stop ? 1.0 : 0.0});
-    if (m.chunk64.key != key) {
-      if (m.chunk64.exec) cudaGraphExecDestroy(m.chunk64.exec);
-      m.chunk64.exec = nullptr;
-      m.chunk64.key.clear();
-      double *zsrc = precond ? f.z : f.r;
-      m.chunk64.exec = capture(st, [&] {
-        for (int it = 0; it < kChunk; it++) {
-          k_w<double><<<grid, block, 0, st>>>(g, f.Kx, f.Ky, f.p, f.w, rx, ry, m.s64, m.part, m.cnt);
-          if (precond && true_stop)
-            k_ur<double, true, STOP_TRUE><<<grid, block, 0, st>>>(g, f.u, f.p, f.r, f.w, f.Mi, f.z, m.s64, m.part,
-                                                                  m.cnt);
-          else if (precond)
-            k_ur<double, true, STOP_TEALEAF><<<grid, block, 0, st>>>(g, f.u, f.p, f.r, f.w, f.Mi, f.z, m.s64,
-                                                                     m.part, m.cnt);
-          else
-            k_ur<double, false, STOP_TEALEAF><<<grid, block, 0, st>>>(g, f.u, f.p, f.r, f.w, f.Mi, f.z, m.s64,
-                                                                      m.part, m.cnt);
-          k_p<double><<<grid, block, 0, st>>>(g, f.p, zsrc, m.s64);
-        }
-      });
-      m.chunk64.key = key;
+    m.ensure_p64((size_t)f.pitch * f.ny);
+    double *pb = m.p64b;
+    bool ran;
+    if (precond && true_stop)
+      ran = m.resident<double, Z_MI, STOP_TRUE>(g, f.Kx, f.Ky, f.p, f.r, f.Mi, f.u, f.z, rx, ry, m.s64, st);
+    else if (precond)
+      ran = m.resident<double, Z_MI, STOP_TEALEAF>(g, f.Kx, f.Ky, f.p, f.r, f.Mi, f.u, f.z, rx, ry, m.s64, st);
+    else
+      ran = m.resident<double, Z_R, STOP_TEALEAF>(g, f.Kx, f.Ky, f.p, f.r, f.Mi, f.u, nullptr, rx, ry, m.s64, st);
+    if (ran) {
+      launches_ += 1;
+    } else {
+      int rows, blocks;
+      pw_grid(f.nx, f.ny, kPwBlocks<double>, &rows, &blocks);
+      const std::string key = key_of({f.Kx, f.Ky, f.u, f.r, f.w, f.p, pb, f.Mi},
+                                     {rx, ry, (double)f.nx, (double)f.ny, (double)f.pitch, precond ? 1.0 : 0.0,
+                                      true_stop ? 1.0 : 0.0});
+      if (m.chunk64.key != key) {
+        if (m.chunk64.exec) cudaGraphExecDestroy(m.chunk64.exec);
+        m.chunk64.exec = nullptr;
+        m.chunk64.key.clear();
+        m.chunk64.exec = capture(st, [&] {
+          for (int it = 0; it < kChunk; it++) {
+            if (precond)
+              k_pw<double, Z_DIAG><<<blocks, block, 0, st>>>(g, f.Kx, f.Ky, f.p, pb, f.r, f.Mi, f.u, f.w, rx, ry, rows,
+                                                             m.s64, m.part, m.cnt);
+            else
+              k_pw<double, Z_R><<<blocks, block, 0, st>>>(g, f.Kx, f.Ky, f.p, pb, f.r, f.Mi, f.u, f.w, rx, ry, rows,
+                                                          m.s64, m.part, m.cnt);
+            if (precond && true_stop)
+              k_r<double, true, STOP_TRUE><<<grid, block, 0, st>>>(g, f.r, f.w, f.Mi, m.s64, m.part, m.cnt);
+            else if (precond)
+              k_r<double, true, STOP_TEALEAF><<<grid, block, 0, st>>>(g, f.r, f.w, f.Mi, m.s64, m.part, m.cnt);
+            else
+              k_r<double, false, STOP_TEALEAF><<<grid, block, 0, st>>>(g, f.r, f.w, f.Mi, m.s64, m.part, m.cnt);
+          }
+        });
+        m.chunk64.key = key;
+      }
+      launches_ += run_chunks(m.chunk64.exec, m.s64, max_iters, m.h_flag, m.ev, st, 2 * kChunk);
+      k_flush<double><<<grid, block, 0, st>>>(g, f.u, f.p, pb, f.r, f.Mi, precond ? f.z : nullptr, m.s64);
+      check_launch("heat solver flush");
+      launches_ += 1;
     }
-    launches_ += run_chunks(m.chunk64.exec, m.s64, max_iters, m.h_flag, m.ev, st, 3 * kChunk);
   }
   OPSB_CUDA(cudaMemcpyAsync(&h, m.s64, sizeof(h), cudaMemcpyDeviceToHost, st));
   OPSB_CUDA(cudaStreamSynchronize(st));
@@ -809,6 +1394,9 @@ void Solver::pcg_mixed(const Field2D &f, double rx, double ry, bool precond, dou
   launches_ = 0;
   const Geom g{f.nx, f.ny, f.pitch}, g32{f.nx, f.ny, m.pitch32};
   const dim3 grid = grid_for(f.nx, f.ny), block(BX, BY);
+  // a whole FP32 field: its ring and row ends hold zeros
+  const long long o32 = m.pitch32 + 32, n32 = m.pitch32 * (f.ny + 2);
+  const int gridr = (int)std::min<long long>((n32 / 4 + NT - 1) / NT, 148 * kFlatBlocks);
   const float rxf = (float)rx, ryf = (float)ry;
   k_to_float<<<grid_for(f.nx + 2, f.ny + 2), block, 0, st>>>(g, g32, f.Kx, f.Ky, precond ? f.Mi : nullptr, m.Kx,
                                                               m.Ky, m.Mi);
@@ -821,29 +1409,32 @@ void Solver::pcg_mixed(const Field2D &f, double rx, double ry, bool precond, dou
   OPSB_CUDA(cudaStreamSynchronize(st));
   const double r0 = sqrt(fabs(h.rr0));
   out->initial_residual = r0;
-  const std::string key = key_of({m.Kx, m.Ky, m.e, m.r, m.w, m.p, m.z, m.Mi},
+  int rows, blocks;
+  pw_grid(f.nx, f.ny, kPwBlocks<float>, &rows, &blocks);
+  const std::string key = key_of({m.Kx, m.Ky, m.e, m.r, m.w, m.p, m.p2, m.Mi},
                                  {(double)rxf, (double)ryf, (double)f.nx, (double)f.ny, (double)m.pitch32,
                                   precond ? 1.0 : 0.0});
-  if (m.chunk32.key != key) {
+  auto capture_chunk = [&] {
+    if (m.chunk32.key == key) return;
     if (m.chunk32.exec) cudaGraphExecDestroy(m.chunk32.exec);
     m.chunk32.exec = nullptr;
     m.chunk32.key.clear();
-    float *zsrc = precond ? m.z : m.r;
     m.chunk32.exec = capture(st, [&] {
       for (int it = 0; it < kChunk; it++) {
-        k_w<float><<<grid, block, 0, st>>>(g32, m.Kx, m.Ky, m.p, m.w, rxf, ryf, m.s32, m.part, m.cnt);
-        if (precond)
-          k_ur<float, true, STOP_RELIABLE><<<grid, block, 0, st>>>(g32, m.e, m.p, m.r, m.w, m.Mi, m.z, m.s32,
-                                                                   m.part, m.cnt);
-        else
-          k_ur<float, false, STOP_RELIABLE><<<grid, block, 0, st>>>(g32, m.e, m.p, m.r, m.w, m.Mi, m.z, m.s32,
-                                                                    m.part, m.cnt);
-        k_p<float><<<grid, block, 0, st>>>(g32, m.p, zsrc, m.s32);
+        if (precond) {
+          k_pw<float, Z_MI><<<blocks, block, 0, st>>>(g32, m.Kx, m.Ky, m.p, m.p2, m.r, m.Mi, m.e, m.w, rxf, ryf, rows,
+                                                      m.s32, m.part, m.cnt);
+          k_r_flat<float, STOP_RELIABLE><<<gridr, block, 0, st>>>(m.r - o32, m.w - o32, m.Mi - o32, n32, m.s32, m.part,
+                                                                  m.cnt);
+        } else {
+          k_pw<float, Z_R><<<blocks, block, 0, st>>>(g32, m.Kx, m.Ky, m.p, m.p2, m.r, m.Mi, m.e, m.w, rxf, ryf, rows,
+                                                     m.s32, m.part, m.cnt);
+          k_r<float, false, STOP_RELIABLE><<<grid, block, 0, st>>>(g32, m.r, m.w, m.Mi, m.s32, m.part, m.cnt);
+        }
       }
     });
     m.chunk32.key = key;
-  }
-  float *zsrc = precond ? m.z : m.r;
+  };
   int updates = 0, iters = 0;
   double scale = 1.0;
   bool done = h.done == 1 || r0 == 0.0;
@@ -851,17 +1442,27 @@ void Solver::pcg_mixed(const Field2D &f, double rx, double ry, bool precond, dou
   memset(&in, 0, sizeof(in));
   while (!done) {
     if (precond)
-      k_reinit32<true><<<grid, block, 0, st>>>(g, g32, f.r, m.r, m.Mi, m.z, updates == 0, eps, scale, delta,
-                                               max_iters, m.s32, m.part, m.cnt);
+      k_reinit32<true><<<grid, block, 0, st>>>(g, g32, f.r, m.r, m.Mi, updates == 0, eps, scale, delta, max_iters,
+                                               m.s32, m.part, m.cnt);
     else
-      k_reinit32<false><<<grid, block, 0, st>>>(g, g32, f.r, m.r, m.Mi, m.z, updates == 0, eps, scale, delta,
-                                                max_iters, m.s32, m.part, m.cnt);
-    k_p<float><<<grid, block, 0, st>>>(g32, m.p, zsrc, m.s32);
+      k_reinit32<false><<<grid, block, 0, st>>>(g, g32, f.r, m.r, m.Mi, updates == 0, eps, scale, delta, max_iters,
+                                                m.s32, m.part, m.cnt);
     check_launch("heat solver reliable update");
-    launches_ += 2;
-    launches_ += run_chunks(m.chunk32.exec, m.s32, max_iters, m.h_flag, m.ev, st, 3 * kChunk);
+    launches_ += 1;
+    const bool ran =
+        max_iters > 0 &&
+        (precond ? m.resident<float, Z_MI, STOP_RELIABLE>(g32, m.Kx, m.Ky, m.p, m.r, m.Mi, m.e, nullptr, rxf, ryf, m.s32,
+                                                          st)
+                 : m.resident<float, Z_R, STOP_RELIABLE>(g32, m.Kx, m.Ky, m.p, m.r, m.Mi, m.e, nullptr, rxf, ryf, m.s32,
+                                                         st));
+    if (ran) {
+      launches_ += 1;
+    } else {
+      capture_chunk();
+      launches_ += run_chunks(m.chunk32.exec, m.s32, max_iters, m.h_flag, m.ev, st, 2 * kChunk);
+    }
     OPSB_CUDA(cudaMemcpyAsync(&in, m.s32, sizeof(in), cudaMemcpyDeviceToHost, st));
-    k_update<<<grid, block, 0, st>>>(g, g32, f.u, m.e);
+    k_update<<<grid, block, 0, st>>>(g, g32, f.u, m.e, m.p, m.p2, m.s32);
     k_resid<<<grid, block, 0, st>>>(g, f.Kx, f.Ky, f.u, f.u0, f.r, rx, ry, eps, m.s64, m.part, m.cnt);
     check_launch("heat solver reliable update");
     launches_ += 2;
@@ -914,8 +1515,12 @@ void Solver::pcg3d(const Field3D &f, double rx, double ry, double rz, bool true_
   const int rows = (f.ny + 2) * (f.nz + 2);
   const Geom gf{(int)f.pitch, rows, f.pitch};
   const dim3 gridf = grid_for((int)f.pitch, rows);
-  double *u = f.u - off, *r = f.r - off, *w = f.w - off, *p = f.p - off, *z = f.z - off;
+  double *r = f.r - off, *w = f.w - off, *p = f.p - off, *z = f.z - off;
   const double *Mi = f.Mi - off;
+  const long long nf = f.plane * (f.nz + 2);
+  if (((uintptr_t)r | (uintptr_t)w | (uintptr_t)Mi) & 15) throw Error(E_ARG, "heat solver 3D: misaligned field");
+  const Grid3 q = pw3_grid(f.nx, f.ny, f.nz);
+  const int gridr = (int)std::min<long long>((nf / 2 + NT - 1) / NT, 148 * kFlatBlocks);
   Scalars h = fresh(0.0);
   OPSB_CUDA(cudaMemcpyAsync(m.s64, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   k_resid3<<<grid3, block, 0, st>>>(g, f.Kx, f.Ky, f.Kz, f.u, f.u0, f.r, rx, ry, rz, eps, m.s64, m.part, m.cnt);
@@ -932,17 +1537,21 @@ void Solver::pcg3d(const Field3D &f, double rx, double ry, double rz, bool true_
       m.chunk64.key.clear();
       m.chunk64.exec = capture(st, [&] {
         for (int it = 0; it < kChunk; it++) {
-          k_w3<double><<<grid3, block, 0, st>>>(g, f.Kx, f.Ky, f.Kz, f.p, f.w, rx, ry, rz, m.s64, m.part, m.cnt);
+          // f.z is the direction's second buffer
+          k_pw3<double><<<q.blocks, dim3(32, kTileY), 0, st>>>(g, f.Kx, f.Ky, f.Kz, f.p, f.z, f.r, f.Mi, f.u, f.w, rx,
+                                                               ry, rz, q.tx, q.ty, q.planes, m.s64, m.part, m.cnt);
           if (true_stop)
-            k_ur<double, true, STOP_TRUE><<<gridf, block, 0, st>>>(gf, u, p, r, w, Mi, z, m.s64, m.part, m.cnt);
+            k_r_flat<double, STOP_TRUE><<<gridr, block, 0, st>>>(r, w, Mi, nf, m.s64, m.part, m.cnt);
           else
-            k_ur<double, true, STOP_TEALEAF><<<gridf, block, 0, st>>>(gf, u, p, r, w, Mi, z, m.s64, m.part, m.cnt);
-          k_p<double><<<gridf, block, 0, st>>>(gf, p, z, m.s64);
+            k_r_flat<double, STOP_TEALEAF><<<gridr, block, 0, st>>>(r, w, Mi, nf, m.s64, m.part, m.cnt);
         }
       });
       m.chunk64.key = key;
     }
-    launches_ += run_chunks(m.chunk64.exec, m.s64, max_iters, m.h_flag, m.ev, st, 3 * kChunk);
+    launches_ += run_chunks(m.chunk64.exec, m.s64, max_iters, m.h_flag, m.ev, st, 2 * kChunk);
+    k_flush<double><<<gridf, block, 0, st>>>(gf, f.u - off, p, z, r, Mi, nullptr, m.s64);
+    check_launch("heat solver 3D flush");
+    launches_ += 1;
   }
   OPSB_CUDA(cudaMemcpyAsync(&h, m.s64, sizeof(h), cudaMemcpyDeviceToHost, st));
   OPSB_CUDA(cudaStreamSynchronize(st));
@@ -977,6 +1586,8 @@ void Solver::pcg3d_mixed(const Field3D &f, double rx, double ry, double rz, doub
   const Geom gf{(int)f.pitch, rows, f.pitch};
   const dim3 gridf = grid_for((int)f.pitch, rows);
   const dim3 grid1((unsigned)std::min<long long>(((long long)nf + NT - 1) / NT, 148LL * 16));
+  const Grid3 q = pw3_grid(f.nx, f.ny, f.nz);
+  const int gridr = (int)std::min<long long>(((long long)nf / 4 + NT - 1) / NT + 1, 148 * kFlatBlocks);
   const float rxf = (float)rx, ryf = (float)ry, rzf = (float)rz;
   k_flat_to_float<<<grid1, block, 0, st>>>(f.Kx - off, m.Kx, (long long)nf);
   k_flat_to_float<<<grid1, block, 0, st>>>(f.Ky - off, m.Ky, (long long)nf);
@@ -991,7 +1602,7 @@ void Solver::pcg3d_mixed(const Field3D &f, double rx, double ry, double rz, doub
   OPSB_CUDA(cudaStreamSynchronize(st));
   const double r0 = sqrt(fabs(h.rr0));
   out->initial_residual = r0;
-  const std::string key = "3d" + key_of({m.Kx, m.Ky, m.Kz, m.e, m.r, m.w, m.p, m.z, m.Mi},
+  const std::string key = "3d" + key_of({m.Kx, m.Ky, m.Kz, m.e, m.r, m.w, m.p, m.p2, m.Mi},
                                         {(double)rxf, (double)ryf, (double)rzf, (double)f.nx, (double)f.ny,
                                          (double)f.nz, (double)f.pitch});
   if (m.chunk32.key != key) {
@@ -1000,11 +1611,10 @@ void Solver::pcg3d_mixed(const Field3D &f, double rx, double ry, double rz, doub
     m.chunk32.key.clear();
     m.chunk32.exec = capture(st, [&] {
       for (int it = 0; it < kChunk; it++) {
-        k_w3<float><<<grid3, block, 0, st>>>(g, m.Kx + off, m.Ky + off, m.Kz + off, m.p + off, m.w + off, rxf, ryf,
-                                             rzf, m.s32, m.part, m.cnt);
-        k_ur<float, true, STOP_RELIABLE><<<gridf, block, 0, st>>>(gf, m.e, m.p, m.r, m.w, m.Mi, m.z, m.s32, m.part,
-                                                                  m.cnt);
-        k_p<float><<<gridf, block, 0, st>>>(gf, m.p, m.z, m.s32);
+        k_pw3<float><<<q.blocks, dim3(32, kTileY), 0, st>>>(g, m.Kx + off, m.Ky + off, m.Kz + off, m.p + off,
+                                                            m.p2 + off, m.r + off, m.Mi + off, m.e + off, m.w + off,
+                                                            rxf, ryf, rzf, q.tx, q.ty, q.planes, m.s32, m.part, m.cnt);
+        k_r_flat<float, STOP_RELIABLE><<<gridr, block, 0, st>>>(m.r, m.w, m.Mi, (long long)nf, m.s32, m.part, m.cnt);
       }
     });
     m.chunk32.key = key;
@@ -1015,14 +1625,13 @@ void Solver::pcg3d_mixed(const Field3D &f, double rx, double ry, double rz, doub
   Scalars in;
   memset(&in, 0, sizeof(in));
   while (!done) {
-    k_reinit32<true><<<gridf, block, 0, st>>>(gf, gf, f.r - off, m.r, m.Mi, m.z, updates == 0, eps, scale, delta,
+    k_reinit32<true><<<gridf, block, 0, st>>>(gf, gf, f.r - off, m.r, m.Mi, updates == 0, eps, scale, delta,
                                               max_iters, m.s32, m.part, m.cnt);
-    k_p<float><<<gridf, block, 0, st>>>(gf, m.p, m.z, m.s32);
     check_launch("heat solver 3D reliable update");
-    launches_ += 2;
-    launches_ += run_chunks(m.chunk32.exec, m.s32, max_iters, m.h_flag, m.ev, st, 3 * kChunk);
+    launches_ += 1;
+    launches_ += run_chunks(m.chunk32.exec, m.s32, max_iters, m.h_flag, m.ev, st, 2 * kChunk);
     OPSB_CUDA(cudaMemcpyAsync(&in, m.s32, sizeof(in), cudaMemcpyDeviceToHost, st));
-    k_update<<<gridf, block, 0, st>>>(gf, gf, f.u - off, m.e);
+    k_update<<<gridf, block, 0, st>>>(gf, gf, f.u - off, m.e, m.p, m.p2, m.s32);
     k_resid3<<<grid3, block, 0, st>>>(g, f.Kx, f.Ky, f.Kz, f.u, f.u0, f.r, rx, ry, rz, eps, m.s64, m.part, m.cnt);
     check_launch("heat solver 3D reliable update");
     launches_ += 2;

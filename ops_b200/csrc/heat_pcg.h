@@ -1,7 +1,7 @@
 // Device-resident Jacobi-preconditioned CG for the TeaLeaf 2D heat operator
 // (apps/c/TeaLeaf/tea_solve.cpp:139-356 with tea_leaf_cg.cpp:53-214): the
 // scalars alpha, beta and the stopping test live in device memory, so an
-// iteration is three kernel launches and no host round trip; iterations are
+// iteration is two kernel launches and no host round trip; iterations are
 // replayed from a CUDA graph in chunks and the host polls one chunk behind.
 //
 // Two precisions:

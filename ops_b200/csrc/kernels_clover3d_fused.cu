@@ -19,6 +19,7 @@
 
 #include "clover3d_common.h"
 #include "clover_flux.cuh"
+#include "march_grid.h"
 #include "runtime.h"
 
 namespace opsb {
@@ -87,21 +88,24 @@ struct March {
   }
 };
 
-// Rows per march: at most 64 (the rows read before the first owned one then
-// cost 2-5 %), fewer when the mesh would not give every SM 32 warps, and at
-// least 4; never more CTAs than a reduction has slots for.
-template <int OWN, int M, class F>
+// HALO: rows a march reads beyond its own.
+template <int OWN, int M, int HALO, class F>
 void launch_march(const LoopParams &lp, cudaStream_t s, F kernel) {
+  static int per_sm = 0;  // resident CTAs, per kernel
+  if (!per_sm) {
+    int n = 0;
+    OPSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 32 * kWarps, 0));
+    per_sm = std::max(n, 1);
+  }
   constexpr int O = M == 1 ? 2 : 1;
-  const long long nx = lp.end[0] - lp.start[0], nm = lp.end[M] - lp.start[M], no = lp.end[O] - lp.start[O];
-  const long long ncol = (nx + OWN - 1) / OWN;
-  constexpr long long kTarget = 148LL * 32;
-  long long rows = std::max(4LL, std::min(64LL, nm * no * ncol / kTarget));
-  auto blocks = [&] { return (ncol * no * ((nm + rows - 1) / rows) + kWarps - 1) / kWarps; };
-  while (blocks() > Runtime::kMaxRedBlocks && rows < nm) rows *= 2;
-  if (blocks() > Runtime::kMaxRedBlocks && lp.nred > 0)
+  const long long nx = lp.end[0] - lp.start[0], no = lp.end[O] - lp.start[O];
+  const int nm = lp.end[M] - lp.start[M];
+  const long long columns = (nx + OWN - 1) / OWN * no;
+  const int rows = march_rows(columns, nm, HALO, 148LL * per_sm * kWarps, (long long)Runtime::kMaxRedBlocks * kWarps);
+  const long long blocks = (columns * ((nm + rows - 1) / rows) + kWarps - 1) / kWarps;
+  if (blocks > Runtime::kMaxRedBlocks && lp.nred > 0)
     throw Error(E_UNSUPPORTED, "cloverleaf3d: mesh too large for one reduction");
-  kernel<<<(unsigned)blocks(), 32 * kWarps, 0, s>>>(lp, (int)rows);
+  kernel<<<(unsigned)blocks, 32 * kWarps, 0, s>>>(lp, rows);
 }
 
 // The grid's reductions: `v[k]` belongs to argument first + k (every thread
@@ -204,7 +208,7 @@ struct ideal_gas_summary {
   __device__ void operator()(const D &density0, const D &energy0, D &pressure, D &soundspeed, const D &volume,
                              const D &xvel0, const D &yvel0, const D &zvel0, RED<double> &vol, RED<double> &mass,
                              RED<double> &ie, RED<double> &ke, RED<double> &press) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2>(lp, s, summary_kernel); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, summary_kernel); }
 };
 
 // calc_dt_kernel with calc_dt_kernel_min folded in. Point by point: the six
@@ -300,7 +304,7 @@ struct PdV_predict_pressure {
   __device__ void operator()(const D &xarea, const D &xvel0, const D &yarea, const D &yvel0, const D &zarea,
                              const D &zvel0, const D &volume, D &pressure, const D &density0, const D &viscosity,
                              const D &energy0) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2>(lp, s, predict_march); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, predict_march); }
 };
 
 // accelerate_kernel. A plane's share of a node's mass and forces is computed
@@ -379,7 +383,7 @@ struct accelerate_fused {
   __device__ void operator()(const D &density0, const D &volume, const D &pressure, const D &viscosity,
                              const D &xarea, const D &yarea, const D &zarea, const D &xvel0, const D &yvel0,
                              const D &zvel0, D &xvel1, D &yvel1, D &zvel1) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2>(lp, s, accelerate_march); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, accelerate_march); }
 };
 
 // PdV_kernel_nopredict and flux_calc_kernel{x,y,z} over the nodes; each
@@ -461,7 +465,7 @@ struct PdV_flux {
                              const D &yvel0, const D &yvel1, const D &zvel0, const D &zvel1, const D &volume,
                              const D &pressure, const D &density0, const D &viscosity, const D &energy0, D &density1,
                              D &energy1, D &vol_flux_x, D &vol_flux_y, D &vol_flux_z) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2>(lp, s, pdv_flux_march); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, pdv_flux_march); }
 };
 
 // ---- advection -------------------------------------------------------------------
@@ -631,12 +635,12 @@ __global__ void __launch_bounds__(32 * kWarps, 5) advec_cell_march(const __grid_
                                D &density0) const;                                                                  \
     static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { LAUNCH; }                                \
   };
-ADVEC_CELL(advec_cell_fused_x1, (launch_march<28, 1>(lp, s, advec_cell_x_march<VOL_FIRST>)))
-ADVEC_CELL(advec_cell_fused_z1, (launch_march<32, 2>(lp, s, advec_cell_march<2, VOL_FIRST>)))
-ADVEC_CELL(advec_cell_fused_y2x, (launch_march<32, 1>(lp, s, advec_cell_march<1, VOL_YZ>)))
-ADVEC_CELL(advec_cell_fused_y2z, (launch_march<32, 1>(lp, s, advec_cell_march<1, VOL_YX>)))
-ADVEC_CELL_LAST(advec_cell_fused_x3, (launch_march<28, 1>(lp, s, advec_cell_x_march<VOL_LAST>)))
-ADVEC_CELL_LAST(advec_cell_fused_z3, (launch_march<32, 2>(lp, s, advec_cell_march<2, VOL_LAST>)))
+ADVEC_CELL(advec_cell_fused_x1, (launch_march<28, 1, 0>(lp, s, advec_cell_x_march<VOL_FIRST>)))
+ADVEC_CELL(advec_cell_fused_z1, (launch_march<32, 2, 3>(lp, s, advec_cell_march<2, VOL_FIRST>)))
+ADVEC_CELL(advec_cell_fused_y2x, (launch_march<32, 1, 3>(lp, s, advec_cell_march<1, VOL_YZ>)))
+ADVEC_CELL(advec_cell_fused_y2z, (launch_march<32, 1, 3>(lp, s, advec_cell_march<1, VOL_YX>)))
+ADVEC_CELL_LAST(advec_cell_fused_x3, (launch_march<28, 1, 0>(lp, s, advec_cell_x_march<VOL_LAST>)))
+ADVEC_CELL_LAST(advec_cell_fused_z3, (launch_march<32, 2, 3>(lp, s, advec_cell_march<2, VOL_LAST>)))
 
 // One momentum sweep of the three velocities: node fluxes and masses (alike
 // for all three), momentum fluxes and updates, into other dats than the
@@ -803,12 +807,12 @@ __global__ void __launch_bounds__(32 * kWarps, 3) advec_mom_march(const __grid_c
                                const D &zvel, D &xout, D &yout, D &zout) const;                                     \
     static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { LAUNCH; }                                \
   };
-ADVEC_MOM(advec_mom_fused_x1, (launch_march<28, 1>(lp, s, advec_mom_x_march<VOL_FIRST>)))
-ADVEC_MOM(advec_mom_fused_x3, (launch_march<28, 1>(lp, s, advec_mom_x_march<VOL_LAST>)))
-ADVEC_MOM(advec_mom_fused_y2x, (launch_march<31, 1>(lp, s, advec_mom_march<1, VOL_YZ>)))
-ADVEC_MOM(advec_mom_fused_y2z, (launch_march<31, 1>(lp, s, advec_mom_march<1, VOL_YX>)))
-ADVEC_MOM(advec_mom_fused_z1, (launch_march<31, 2>(lp, s, advec_mom_march<2, VOL_FIRST>)))
-ADVEC_MOM(advec_mom_fused_z3, (launch_march<31, 2>(lp, s, advec_mom_march<2, VOL_LAST>)))
+ADVEC_MOM(advec_mom_fused_x1, (launch_march<28, 1, 1>(lp, s, advec_mom_x_march<VOL_FIRST>)))
+ADVEC_MOM(advec_mom_fused_x3, (launch_march<28, 1, 1>(lp, s, advec_mom_x_march<VOL_LAST>)))
+ADVEC_MOM(advec_mom_fused_y2x, (launch_march<31, 1, 3>(lp, s, advec_mom_march<1, VOL_YZ>)))
+ADVEC_MOM(advec_mom_fused_y2z, (launch_march<31, 1, 3>(lp, s, advec_mom_march<1, VOL_YX>)))
+ADVEC_MOM(advec_mom_fused_z1, (launch_march<31, 2, 3>(lp, s, advec_mom_march<2, VOL_FIRST>)))
+ADVEC_MOM(advec_mom_fused_z3, (launch_march<31, 2, 3>(lp, s, advec_mom_march<2, VOL_LAST>)))
 
 #define REG(K) OPSB_REGISTER_LOOP(K);
 REG(ideal_gas_summary) REG(calc_dt_fused) REG(PdV_predict_pressure) REG(accelerate_fused)

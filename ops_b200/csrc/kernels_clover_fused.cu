@@ -25,6 +25,7 @@
 
 #include "clover_common.h"
 #include "clover_flux.cuh"
+#include "march_grid.h"
 #include "runtime.h"
 
 namespace opsb {
@@ -164,24 +165,20 @@ struct Strip {
   }
 };
 
-// Rows per strip: long enough that the rows read before the first owned one
-// cost little, short enough that every SM gets `kTarget` warps. At 3840^2 the
-// target is met with 64 rows; small meshes take the 4-row minimum.
-template <int OWN>
-void strip_grid(const LoopParams &lp, int &rows, int &blocks) {
-  const long long nx = lp.end[0] - lp.start[0], ny = lp.end[1] - lp.start[1];
-  const long long ncol = (nx + OWN - 1) / OWN;
-  constexpr long long kTarget = 148LL * 32;
-  rows = (int)std::max(4LL, std::min(64LL, ny * ncol / kTarget));
-  const long long warps = ncol * ((ny + rows - 1) / rows);
-  blocks = (int)((warps + kWarps - 1) / kWarps);
-}
-
-template <int OWN, class F>
+// HALO: rows a strip reads beyond its own.
+template <int OWN, int HALO, class F>
 void launch_strips(const LoopParams &lp, cudaStream_t s, F kernel) {
-  int rows, blocks;
-  strip_grid<OWN>(lp, rows, blocks);
-  kernel<<<blocks, 32 * kWarps, 0, s>>>(lp, rows);
+  static int per_sm = 0;  // resident CTAs, per kernel
+  if (!per_sm) {
+    int n = 0;
+    OPSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 32 * kWarps, 0));
+    per_sm = std::max(n, 1);
+  }
+  const int nx = lp.end[0] - lp.start[0], ny = lp.end[1] - lp.start[1];
+  const long long ncol = (nx + OWN - 1) / OWN;
+  const int rows = march_rows(ncol, ny, HALO, 148LL * per_sm * kWarps);
+  const long long warps = ncol * ((ny + rows - 1) / rows);
+  kernel<<<(unsigned)((warps + kWarps - 1) / kWarps), 32 * kWarps, 0, s>>>(lp, rows);
 }
 
 // accelerate_kernel, PdV_kernel_nopredict and flux_calc_kernel{x,y}
@@ -285,7 +282,7 @@ struct lagrange {
   __device__ void operator()(const D &density0, const D &volume, const D &pressure, const D &viscosity,
                              const D &xvel0, const D &yvel0, const D &xarea, const D &yarea, const D &energy0,
                              D &xvel1, D &yvel1, D &density1, D &energy1, D &vol_flux_x, D &vol_flux_y) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<30>(lp, s, lagrange_kernel); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<30, 2>(lp, s, lagrange_kernel); }
 };
 
 // advec_cell_kernel{1,2}, 3 and 4 of an x sweep (advec_cell.cpp:38-147). The
@@ -417,21 +414,21 @@ __global__ void __launch_bounds__(32 * kWarps, 5) advec_cell_y_kernel(const __gr
   }
 }
 
-#define ADVEC_CELL(NAME, OWN, KERNEL)                                                                          \
+#define ADVEC_CELL(NAME, OWN, HALO, KERNEL)                                                                          \
   struct NAME##1 {                                                                                             \
     CL_LOOP(NAME##1);                                                                                          \
     __device__ void operator()(const D &vol_flux, const D &volume, const D &vertexd, const D &density,         \
                                const D &energy, const D &vol_flux_t, D &mass_flux, D &dout, D &eout) const;    \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN>(lp, s, KERNEL<true>); }  \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<true>); }  \
   };                                                                                                           \
   struct NAME##2 {                                                                                             \
     CL_LOOP(NAME##2);                                                                                          \
     __device__ void operator()(const D &vol_flux, const D &volume, const D &vertexd, const D &density,         \
                                const D &energy, D &mass_flux, D &dout, D &eout, D &d0out) const;               \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN>(lp, s, KERNEL<false>); } \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<false>); } \
   };
-ADVEC_CELL(advec_cell_fused_x, 28, advec_cell_x_kernel)
-ADVEC_CELL(advec_cell_fused_y, 32, advec_cell_y_kernel)
+ADVEC_CELL(advec_cell_fused_x, 28, 0, advec_cell_x_kernel)
+ADVEC_CELL(advec_cell_fused_y, 32, 3, advec_cell_y_kernel)
 
 // The x momentum sweep of both velocities (advec_mom.cpp:40-163): node
 // fluxes and masses, the two momentum fluxes and the updates; the node
@@ -574,21 +571,21 @@ __global__ void __launch_bounds__(32 * kWarps, 4) advec_mom_y_kernel(const __gri
   }
 }
 
-#define ADVEC_MOM(NAME, OWN, KERNEL)                                                                             \
+#define ADVEC_MOM(NAME, OWN, HALO, KERNEL)                                                                             \
   struct NAME##1 {                                                                                               \
     CL_LOOP(NAME##1);                                                                                            \
     __device__ void operator()(const D &mass_flux, const D &volume, const D &celld, const D &density,            \
                                const D &xvel, const D &yvel, D &xout, D &yout, const D &vol_flux_t) const;       \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN>(lp, s, KERNEL<true>); }    \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<true>); }    \
   };                                                                                                             \
   struct NAME##2 {                                                                                               \
     CL_LOOP(NAME##2);                                                                                            \
     __device__ void operator()(const D &mass_flux, const D &volume, const D &celld, const D &density,            \
                                const D &xvel, const D &yvel, D &xout, D &yout) const;                            \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN>(lp, s, KERNEL<false>); }   \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<false>); }   \
   };
-ADVEC_MOM(advec_mom_fused_x, 28, advec_mom_x_kernel)
-ADVEC_MOM(advec_mom_fused_y, 31, advec_mom_y_kernel)
+ADVEC_MOM(advec_mom_fused_x, 28, 1, advec_mom_x_kernel)
+ADVEC_MOM(advec_mom_fused_y, 31, 3, advec_mom_y_kernel)
 
 #define REG(K) OPSB_REGISTER_LOOP(K);
 REG(ideal_gas_summary) REG(calc_dt_fused) REG(PdV_predict_pressure) REG(lagrange)

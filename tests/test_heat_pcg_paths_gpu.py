@@ -1,0 +1,52 @@
+"""The Jacobi-PCG loops of the heat solver at the edges of their kernels: the
+one-kernel loop (tiles of 128 x 2 cells, 1 to 8 of them a CTA, grids up to 1184
+tiles) and the two-kernel loop beyond it (strips of 30 columns), FP64 and
+mixed. Held to the FP64 residual recomputed by numpy and, as far as the two
+residuals allow them to differ, to the solution of the flexible CG with
+Jacobi (other kernels, the same solve)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def residual(Kx, Ky, u, u0, rx):
+    c, e, n = (slice(1, -1), slice(1, -1)), (slice(1, -1), slice(2, None)), (slice(2, None), slice(1, -1))
+    w, s = (slice(1, -1), slice(None, -2)), (slice(None, -2), slice(1, -1))
+    return u0[c] - ((1.0 + rx * (Ky[n] + Ky[c] + Kx[e] + Kx[c])) * u[c] - rx * (Ky[n] * u[n] + Ky[c] * u[s])
+                    - rx * (Kx[e] * u[e] + Kx[c] * u[w]))
+
+
+# nx, ny: one cell; a tile's last column and the next CTA's first; 2, 4 and 8
+# tiles a CTA with ragged ends; the largest grid of the one-kernel loop (8 x
+# 148 tiles) and the first beyond it; strips of 30, 31 and 61 columns
+@pytest.mark.parametrize("nx,ny", [(1, 1), (128, 2), (129, 3), (127, 33), (61, 600), (257, 301), (1024, 296),
+                                   (1024, 298), (31, 2400), (150, 1190), (1230, 61)])
+@pytest.mark.parametrize("method", ["PCG_TRUE", "PCG", "MIXED"])
+def test_loops_reach_the_residual(gpu_runtime, nx, ny, method):
+    import torch
+
+    from ops_b200 import lmg
+    rng = np.random.default_rng(nx * 7 + ny)
+    rho = np.exp(rng.uniform(np.log(0.1), np.log(10.0), (ny, nx)))
+    Kx, Ky, u0 = lmg.padded_problem(rho, rng.uniform(0.0, 1.0, (ny, nx)))
+    # open edges too: a non-zero boundary face next to the ring's zero
+    Kx[1:-1, 1] = Kx[1:-1, -1] = 0.3
+    k = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (Kx, Ky, u0)]
+    u, v = k[2].clone(), k[2].clone()
+    u[0], u[-1], u[:, 0], u[:, -1] = 0.0, 0.0, 0.0, 0.0
+    v.copy_(u)
+    st = lmg.solve(*k, u, 20.0, 20.0, method=getattr(lmg, method), eps=1e-10)
+    ref = lmg.solve(*k, v, 20.0, 20.0, method=lmg.FCG_JACOBI, eps=1e-12)
+    assert st["converged"] and ref["converged"]
+    a, b = u.cpu().numpy(), v.cpu().numpy()
+    r = np.linalg.norm(residual(Kx, Ky, a, u0, 20.0))
+    # PCG stops on sqrt|r.z| < eps ||r0|| (TeaLeaf's rule), so ||r|| < sqrt(max D) eps ||r0|| with
+    # D <= 1 + 20 * 4 * 10 (faces are at most 1 / 0.1): a factor of 28.3
+    bound = (1.5 if method != "PCG" else 30.0) * 1e-10 * st["initial_residual"]
+    assert r <= max(bound, 1e-13 * np.linalg.norm(u0)), (r, bound)
+    # A is the identity plus a positive semidefinite operator: ||u - v|| <= ||A (u - v)||
+    s = np.linalg.norm(residual(Kx, Ky, b, u0, 20.0))
+    assert np.linalg.norm(a - b) <= r + s + 1e-12 * np.linalg.norm(b)
+    if method == "PCG_TRUE" and ref["iterations"] > 3:
+        assert st["iterations"] < ref["iterations"]
