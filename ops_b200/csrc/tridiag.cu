@@ -41,38 +41,32 @@ struct Sys {
   int nl0, nl1;    // line counts along the two non-solve dimensions (fastest first)
   long long ss;    // stride along the solve dimension (elements)
   long long s0, s1;
-  long long line0 = 0;  // line kernel: first line number of this system in the launch
-  long long scr0 = 0;   // line kernel: first scratch element of this system
+  long long line0 = 0;  // line kernel: first group of 16 lines of this system
 };
 
 struct Work {
   int sys, l0, l1;  // system, first line along dim 0, line index along dim 1
 };
 
-// Reciprocal by Newton-Raphson refinement (Newton's method for 1/x,
-// e = 1 - x r, r' = r + r e, which doubles the correct bits per step) from a
-// hardware approximation. It is accurate to about 1 ulp without the
-// out-of-line slow path of IEEE division, whose call would force the
-// per-thread coefficient arrays out of registers. Valid for finite normal
-// pivots with 2^-1000 < |x| < 2^1000; the solver's tolerance is relative
-// (1e-12 in FP64), not bit-exact.
+// Reciprocal: the hardware's approximation r (rcp.approx.ftz.f64, about 20 bits)
+// and one third-order step of Newton's iteration for 1/x (e = 1 - x r,
+// r' = r + r (e + e^2), whose error is e^3, beyond FP64). About 1 ulp, without
+// the out-of-line slow path of IEEE division, whose call would force the
+// per-thread coefficient arrays out of registers, and short: the reciprocal is
+// most of the chain from row to row (a single-precision seed with its
+// conversions, scaling and two second-order steps took twice as long). Valid
+// for finite normal pivots with 2^-1000 < |x| < 2^1000; the solver's tolerance
+// is relative (1e-12 in FP64), not bit-exact.
 __device__ __forceinline__ float recip(float x) {
   float r = __fdividef(1.0f, x);
   const float e = fmaf(-x, r, 1.0f);
   return fmaf(r, e, r);
 }
 __device__ __forceinline__ double recip(double x) {
-  // Scale x to [1, 2) by its exponent so the single-precision seed never
-  // over- or underflows, refine twice, then undo the scaling.
-  const long long bits = __double_as_longlong(x);
-  const long long ex = (bits >> 52) & 0x7ff;
-  const double m = __longlong_as_double((bits & ~(0x7ffLL << 52)) | (1023LL << 52));
-  double r = (double)__fdividef(1.0f, (float)m);
-  double e = fma(-m, r, 1.0);
-  r = fma(r, e, r);
-  e = fma(-m, r, 1.0);
-  r = fma(r, e, r);
-  return r * __longlong_as_double((2046LL - ex) << 52);
+  double r;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
+  const double e = fma(-x, r, 1.0);
+  return fma(r, fma(e, e, e), r);
 }
 
 // One work item = L neighbouring lines x n rows of one system, staged in
@@ -330,7 +324,10 @@ __global__ void __launch_bounds__(kTileThreads, kCtasPerSm) trid_tile_kernel(con
 // recurrences as trid_tile_kernel, each line's 2 P chunk end rows are solved
 // by parallel cyclic reduction over shuffles within its lane group, and the
 // lanes substitute back and store through the strip. A warp keeps all its
-// lines' 4 n loads in flight at once.
+// lines' 4 n loads in flight at once. Its time is its instructions (FP64 chains
+// and reduction steps): with the short reciprocal and one of them a reduced row
+// and step instead of two, 256^3 FP64 0.248 -> 0.168 ms, FP32 0.135 -> 0.120, the
+// 64-block batch 0.837 -> 0.587 and 0.480 -> 0.402.
 constexpr int kWarpLines = 8;  // warps per CTA
 
 template <int R>
@@ -389,7 +386,7 @@ __global__ void __launch_bounds__(32 * kWarpLines, sizeof(T) == 4 ? 3 : 2)
     const int r0 = ro + gl * n / kact, m = (gl + 1) * n / kact - gl * n / kact;
     const bool act = g < nlines && gl < kact && n > 1;
     T ra[R], rc[R], rd[R];
-    T fa[2] = {T(0), T(0)}, fb[2] = {T(1), T(1)}, fc[2] = {T(0), T(0)}, fd[2] = {T(0), T(0)};
+    T fa[2] = {T(0), T(0)}, fc[2] = {T(0), T(0)}, fd[2] = {T(0), T(0)};
     if (act) {
       T pa = T(0), pc = T(0), pd = T(0);
 #pragma unroll
@@ -457,30 +454,28 @@ __global__ void __launch_bounds__(32 * kWarpLines, sizeof(T) == 4 ? 3 : 2)
     // 2. each line's 2 P chunk end rows (row 2 gl + j), parallel cyclic
     // reduction over shuffles within the line's lane group; lanes without a
     // chunk hold identity rows
+    // (the rows enter with b = 1 and every step divides its row by the new b, so
+    // a step takes one reciprocal a row and the solution is the last d)
     const int N = 2 * P;
     for (int h = 1; h < N; h *= 2) {
-      T ma[2], mb[2], mc[2], md[2], pa[2], pb[2], pc[2], pd[2];
+      T ma[2], mc[2], md[2], pa[2], pc[2], pd[2];
       if (h == 1) {
         ma[0] = __shfl_up_sync(0xffffffffu, fa[1], 1, P);
-        mb[0] = __shfl_up_sync(0xffffffffu, fb[1], 1, P);
         mc[0] = __shfl_up_sync(0xffffffffu, fc[1], 1, P);
         md[0] = __shfl_up_sync(0xffffffffu, fd[1], 1, P);
         pa[1] = __shfl_down_sync(0xffffffffu, fa[0], 1, P);
-        pb[1] = __shfl_down_sync(0xffffffffu, fb[0], 1, P);
         pc[1] = __shfl_down_sync(0xffffffffu, fc[0], 1, P);
         pd[1] = __shfl_down_sync(0xffffffffu, fd[0], 1, P);
-        pa[0] = fa[1]; pb[0] = fb[1]; pc[0] = fc[1]; pd[0] = fd[1];
-        ma[1] = fa[0]; mb[1] = fb[0]; mc[1] = fc[0]; md[1] = fd[0];
+        pa[0] = fa[1]; pc[0] = fc[1]; pd[0] = fd[1];
+        ma[1] = fa[0]; mc[1] = fc[0]; md[1] = fd[0];
       } else {
         const int q = h >> 1;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
           ma[j] = __shfl_up_sync(0xffffffffu, fa[j], q, P);
-          mb[j] = __shfl_up_sync(0xffffffffu, fb[j], q, P);
           mc[j] = __shfl_up_sync(0xffffffffu, fc[j], q, P);
           md[j] = __shfl_up_sync(0xffffffffu, fd[j], q, P);
           pa[j] = __shfl_down_sync(0xffffffffu, fa[j], q, P);
-          pb[j] = __shfl_down_sync(0xffffffffu, fb[j], q, P);
           pc[j] = __shfl_down_sync(0xffffffffu, fc[j], q, P);
           pd[j] = __shfl_down_sync(0xffffffffu, fd[j], q, P);
         }
@@ -488,32 +483,17 @@ __global__ void __launch_bounds__(32 * kWarpLines, sizeof(T) == 4 ? 3 : 2)
 #pragma unroll
       for (int j = 0; j < 2; j++) {
         const int k = 2 * gl + j;
-        T ak = fa[j], bk = fb[j], ck = fc[j], dk = fd[j];
-        if (k - h >= 0) {
-          const T al = -ak * recip(mb[j]);
-          ak = al * ma[j];
-          bk = bk + al * mc[j];
-          dk = dk + al * md[j];
-        } else {
-          ak = T(0);
-        }
-        if (k + h < N) {
-          const T gg = -ck * recip(pb[j]);
-          ck = gg * pc[j];
-          bk = bk + gg * pa[j];
-          dk = dk + gg * pd[j];
-        } else {
-          ck = T(0);
-        }
-        fa[j] = ak;
-        fb[j] = bk;
-        fc[j] = ck;
-        fd[j] = dk;
+        // a row without a neighbour there has no coefficient for it either
+        const T ak = k - h >= 0 ? fa[j] : T(0), ck = k + h < N ? fc[j] : T(0);
+        const T r = recip(T(1) - ak * mc[j] - ck * pa[j]);
+        fa[j] = -ak * ma[j] * r;
+        fc[j] = -ck * pc[j] * r;
+        fd[j] = (fd[j] - ak * md[j] - ck * pd[j]) * r;
       }
     }
     // 3. substitute back, then store through the strip with the loads' mapping
     if (act) {
-      const T xf = fd[0] * recip(fb[0]), xl = fd[1] * recip(fb[1]);
+      const T xf = fd[0], xl = fd[1];
 #pragma unroll
       for (int i = 0; i < R; i++)
         if (i < m) Sd[strip_pos(r0 + i)] = (i == 0) ? xf : (i == m - 1) ? xl : rd[i] - ra[i] * xf - rc[i] * xl;
@@ -533,110 +513,208 @@ __global__ void __launch_bounds__(32 * kWarpLines, sizeof(T) == 4 ? 3 : 2)
   }
 }
 
-// Lines strided along the solve dimension and contiguous across lines (the
-// y and z sweeps): one thread per line runs the Thomas algorithm straight
-// from HBM, neighbouring threads reading neighbouring lines so every access
-// coalesces. The forward pass keeps c' and d' in a scratch array laid out
-// row-major over the system's lines (coalesced too) and the backward pass
-// reads them back: 72 bytes per FP64 unknown (80 for _Inc) against the
-// tile kernel's 40, but no staging, no barriers and several rows of loads in
-// flight per thread, which is what the strided sweeps lacked. Rows in
-// flight: 8 (one 32-byte sector of each line per array in FP32, two in
-// FP64), or 4 in FP64 when the lines fill the GPU (more than 1024 a SM): a
-// grid of few lines leaves the registers free and gains from the deeper
-// pipeline (256^3 FP64 y sweep 0.239 -> 0.219 ms), while the 64-block batch
-// (about 0.5 M lines) lost 7-20 % with it. The arithmetic is the textbook
-// Thomas elimination:
+// ---- strided sweeps -----------------------------------------------------------
+// The y and z sweeps run the textbook Thomas elimination straight from HBM:
 //   c'_0 = c_0 / b_0, d'_0 = d_0 / b_0; for i >= 1, r = 1 / (b_i - a_i c'_{i-1}),
 //   c'_i = c_i r, d'_i = (d_i - a_i d'_{i-1}) r; x_{n-1} = d'_{n-1},
 //   x_i = d'_i - c'_i x_{i+1}.
-constexpr int kLineThreads = 128;
-constexpr long long kLinesDeep = 148LL * 1024;  // at most this many lines: 8 rows in flight in FP64
+// It needs a fraction of the partition method's instructions, but c' and d' have
+// to wait for the backward pass. They go to a scratch that stays in L2: the
+// grid keeps only so many lines in flight that their c' and d' fit
+// (kScratchBytes), each thread reuses its own slot line after line, the scratch
+// is marked evict-last and everything else evict-first. HBM then sees the
+// compulsory 40 B per FP64 unknown (48 with _Inc). With every line in flight
+// the scratch went through HBM too (68 to 77 B). 256^3 FP64: y sweep 0.213 ->
+// 0.167 ms, z sweep (_Inc) 0.289 -> 0.209 ms; the 64-block batch's 0.548 -> 0.478
+// and 0.655 -> 0.544 ms, in FP32 0.297 -> 0.273 and 0.432 -> 0.307 ms. Scratches of
+// 60 to 400 MB measured within 7 % of one another, 40 MB 1.3x slower.
+constexpr size_t kScratchBytes = 64ull << 20;
 
-template <class T, int kLineUnroll>
+__device__ __forceinline__ uint64_t policy_last() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+__device__ __forceinline__ uint64_t policy_first() {
+  uint64_t p;
+  asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+  return p;
+}
+template <class T>
+__device__ __forceinline__ void cp_async_hint(T *dst, const T *src, uint64_t pol) {
+  asm volatile("cp.async.ca.shared.global.L2::cache_hint [%0], [%1], %2, %3;" ::"r"(smem_addr(dst)), "l"(src),
+               "n"((int)sizeof(T)), "l"(pol)
+               : "memory");
+}
+__device__ __forceinline__ double ld_hint(const double *p, uint64_t pol) {
+  double v;
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol) : "memory");
+  return v;
+}
+__device__ __forceinline__ float ld_hint(const float *p, uint64_t pol) {
+  float v;
+  asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol) : "memory");
+  return v;
+}
+__device__ __forceinline__ void st_hint(double *p, double v, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.f64 [%0], %1, %2;" ::"l"(p), "d"(v), "l"(pol) : "memory");
+}
+__device__ __forceinline__ void st_hint(float *p, float v, uint64_t pol) {
+  asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(pol) : "memory");
+}
+
+// Lines strided along the solve dimension and contiguous across lines (the y
+// and z sweeps). A warp solves 16 neighbouring lines, two lanes each: one
+// eliminates from the top, its partner (lane + 16) from the bottom with a and c
+// in each other's place, they meet in the middle,
+//   x_m = (d'_m - c'_m d''_{m+1}) / (1 - c'_m a''_{m+1}),
+// and substitute outwards. So a line's chain is half as long and the lines
+// whose c' and d' fit L2 keep twice the threads busy. The rows ahead come by
+// cp.async into the thread's own column of a ring of kLineStages stages of
+// kLineRows rows (no barrier: nobody else reads it); the backward pass reads
+// c' and d' kLineRows rows ahead into registers.
+constexpr int kLineThreads = 128, kLineRows = 8, kLineStages = 3;
+
+template <class T>
+constexpr int kLineSmem = kLineStages * kLineRows * 4 * kLineThreads * (int)sizeof(T);
+
+template <class T>
 __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__restrict__ sys, int nsys,
-                                                                 long long total, T *__restrict__ scr_c,
-                                                                 T *__restrict__ scr_d) {
-  for (long long g = (long long)blockIdx.x * kLineThreads + threadIdx.x; g < total;
-       g += (long long)gridDim.x * kLineThreads) {
-    int lo = 0, hi = nsys - 1;  // last system whose first line is <= g
+                                                                 long long groups, T *scr, int slots) {
+  constexpr int U = kLineRows;
+  extern __shared__ __align__(16) unsigned char smraw[];
+  T *ring = reinterpret_cast<T *>(smraw) + threadIdx.x;  // element (stage, row, array) every kLineThreads
+  const uint64_t keep = policy_last(), pass = policy_first();
+  const int slot = blockIdx.x * kLineThreads + threadIdx.x, lane = threadIdx.x & 31, half = lane >> 4;
+  T *cp = scr + slot;  // c' of row i at [2 i slots], d' at [(2 i + 1) slots]
+  for (long long g = slot >> 5; g < groups; g += slots >> 5) {
+    int lo = 0, hi = nsys - 1;  // last system whose first group of lines is <= g
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (sys[mid].line0 <= g) lo = mid;
       else hi = mid - 1;
     }
     const Sys &s = sys[lo];
-    const long long k = g - s.line0, nlines = (long long)s.nl0 * s.nl1;
-    const int n = s.n;
-    const long long base = (k % s.nl0) * s.s0 + (k / s.nl0) * s.s1, ss = s.ss;
-    const T *a = reinterpret_cast<const T *>(s.a) + base;
+    const long long lines = (long long)s.nl0 * s.nl1, l = (g - s.line0) * 16 + (lane & 15);
+    const int n = s.n, len = l < lines ? (half ? n / 2 : (n + 1) / 2) : 0;
+    const long long ss = half ? -s.ss : s.ss;
+    const long long base = (l % s.nl0) * s.s0 + (l / s.nl0) * s.s1 + (half ? (long long)(n - 1) * s.ss : 0);
+    const T *a = reinterpret_cast<const T *>(half ? s.c : s.a) + base;
     const T *b = reinterpret_cast<const T *>(s.b) + base;
-    const T *c = reinterpret_cast<const T *>(s.c) + base;
-    const T *d = reinterpret_cast<const T *>(s.d) + base;
-    T *x = reinterpret_cast<T *>(s.d) + base;
+    const T *c = reinterpret_cast<const T *>(half ? s.a : s.c) + base;
+    T *d = reinterpret_cast<T *>(s.d) + base;
     T *u = s.u ? reinterpret_cast<T *>(s.u) + base : nullptr;
-    T *cp = scr_c + s.scr0 + k, *dp = scr_d + s.scr0 + k;
-    if (n <= 0) continue;
-    T r = recip(b[0]);
-    T pc = c[0] * r, pd = d[0] * r;
-    cp[0] = pc;
-    dp[0] = pd;
-    int i = 1;
-    for (; i + kLineUnroll <= n; i += kLineUnroll) {
-      T ai[kLineUnroll], bi[kLineUnroll], ci[kLineUnroll], di[kLineUnroll];
+    const int nst = ((n + 1) / 2 + U - 1) / U, full = (n / 2) / U;  // stages; those that every live lane fills
+    long long ahead = 0;  // offset of the next row to fetch
+    auto fetch_row = [&](T *t) {
+      cp_async_hint(t, a + ahead, pass);
+      cp_async_hint(t + kLineThreads, b + ahead, pass);
+      cp_async_hint(t + 2 * kLineThreads, c + ahead, pass);
+      cp_async_hint(t + 3 * kLineThreads, (const T *)d + ahead, pass);
+      ahead += ss;
+    };
+    auto fetch = [&](int st) {
+      T *t = ring + (st % kLineStages) * (U * 4 * kLineThreads);
+      if (st < full && len) {
 #pragma unroll
-      for (int j = 0; j < kLineUnroll; j++) {
-        const long long q = (long long)(i + j) * ss;
-        ai[j] = a[q];
-        bi[j] = b[q];
-        ci[j] = c[q];
-        di[j] = d[q];
+        for (int j = 0; j < U; j++) fetch_row(t + 4 * j * kLineThreads);
+      } else {
+        for (int j = 0; j < min(U, len - st * U); j++) fetch_row(t + 4 * j * kLineThreads);
       }
+      asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    for (int st = 0; st < kLineStages - 1; st++) fetch(st);
+    // the chain from row to row is one product and the reciprocal:
+    // b_i - a_i c'_{i-1} = b_i - (a_i c_{i-1}) r_{i-1}
+    T rc = T(0), lc = T(0), pd = T(0);
+    T *q = cp;
+    auto eliminate = [&](T ai, T bi, T ci, T di) {
+      rc = recip(bi - (ai * lc) * rc);
+      lc = ci;
+      pd = (di - ai * pd) * rc;
+      st_hint(q, lc * rc, keep);
+      st_hint(q + slots, pd, keep);
+      q += 2 * slots;
+    };
+    for (int st = 0; st < nst; st++) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kLineStages - 2) : "memory");
+      T *t = ring + (st % kLineStages) * (U * 4 * kLineThreads);
+      if (st == 0) t[0] = T(0);  // the first row has no neighbour before it
+      if (st < full) {
+        T v[U][4];
 #pragma unroll
-      for (int j = 0; j < kLineUnroll; j++) {
-        r = recip(bi[j] - ai[j] * pc);
-        pc = ci[j] * r;
-        pd = (di[j] - ai[j] * pd) * r;
-        cp[(long long)(i + j) * nlines] = pc;
-        dp[(long long)(i + j) * nlines] = pd;
-      }
-    }
-    for (; i < n; i++) {
-      const long long q = (long long)i * ss;
-      const T ai = a[q];
-      r = recip(b[q] - ai * pc);
-      pc = c[q] * r;
-      pd = (d[q] - ai * pd) * r;
-      cp[(long long)i * nlines] = pc;
-      dp[(long long)i * nlines] = pd;
-    }
-    T xv = pd;  // x_{n-1}
-    {
-      const long long q = (long long)(n - 1) * ss;
-      if (u) u[q] += xv;
-      else x[q] = xv;
-    }
-    int j = n - 2;
-    for (; j - kLineUnroll + 1 >= 0; j -= kLineUnroll) {
-      T cj[kLineUnroll], dj[kLineUnroll];
+        for (int j = 0; j < U; j++)
 #pragma unroll
-      for (int t = 0; t < kLineUnroll; t++) {
-        cj[t] = cp[(long long)(j - t) * nlines];
-        dj[t] = dp[(long long)(j - t) * nlines];
-      }
+          for (int f = 0; f < 4; f++) v[j][f] = t[(4 * j + f) * kLineThreads];
+        fetch(st + kLineStages - 1);
+        if (len) {
 #pragma unroll
-      for (int t = 0; t < kLineUnroll; t++) {
-        xv = dj[t] - cj[t] * xv;
-        const long long q = (long long)(j - t) * ss;
-        if (u) u[q] += xv;
-        else x[q] = xv;
+          for (int j = 0; j < U; j++) eliminate(v[j][0], v[j][1], v[j][2], v[j][3]);
+        }
+      } else {
+        for (int j = 0; j < min(U, len - st * U); j++) {
+          const T *r = t + 4 * j * kLineThreads;
+          eliminate(r[0], r[kLineThreads], r[2 * kLineThreads], r[3 * kLineThreads]);
+        }
+        fetch(st + kLineStages - 1);
       }
     }
-    for (; j >= 0; j--) {
-      xv = dp[(long long)j * nlines] - cp[(long long)j * nlines] * xv;
-      const long long q = (long long)j * ss;
-      if (u) u[q] += xv;
-      else x[q] = xv;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    const T pc = n > 1 ? lc * rc : T(0);  // a line of one row has no c
+    const T oc = __shfl_xor_sync(0xffffffffu, pc, 16), od = __shfl_xor_sync(0xffffffffu, pd, 16);
+    T xv = n > 1 ? (pd - pc * od) * recip(T(1) - pc * oc) : pd;
+    // outwards, from the row before the middle
+    long long out = (long long)(len - 1) * ss;
+    auto put = [&](T ui) {
+      if (u) __stcs(u + out, ui + xv);
+      else __stcs(d + out, xv);
+      out -= ss;
+    };
+    if (len) put(u ? u[out] : T(0));
+    q = cp + (long long)(len - 2) * 2 * slots;
+    struct Back {
+      T c[U], d[U], u[U];
+    };
+    long long uo = out;
+    auto back = [&](int i, Back &w) {  // rows i .. i - U + 1
+      if (i >= U - 1) {
+#pragma unroll
+        for (int j = 0; j < U; j++) {
+          w.c[j] = ld_hint(q, keep);
+          w.d[j] = ld_hint(q + slots, keep);
+          q -= 2 * slots;
+        }
+        if (u) {
+#pragma unroll
+          for (int j = 0; j < U; j++, uo -= ss) w.u[j] = __ldcs(u + uo);
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < U; j++)
+          if (i - j >= 0) {
+            w.c[j] = ld_hint(q, keep);
+            w.d[j] = ld_hint(q + slots, keep);
+            q -= 2 * slots;
+            if (u) w.u[j] = __ldcs(u + uo);
+            uo -= ss;
+          }
+      }
+    };
+    auto substitute = [&](int i, const Back &w) {
+#pragma unroll
+      for (int j = 0; j < U; j++)
+        if (i - j >= 0) {
+          xv = w.d[j] - w.c[j] * xv;
+          put(w.u[j]);
+        }
+    };
+    Back w0, w1;
+    back(len - 2, w0);
+    for (int i = len - 2; i >= 0; i -= 2 * U) {
+      back(i - U, w1);
+      substitute(i, w0);
+      back(i - 2 * U, w0);
+      substitute(i - U, w1);
     }
   }
 }
@@ -646,7 +724,7 @@ struct Buffers {
   Sys *sys = nullptr;
   Work *work = nullptr;
   size_t sys_cap = 0, work_cap = 0;
-  void *scr = nullptr;  // line kernel scratch (c' then d')
+  void *scr = nullptr;  // c' and d' of the lines in flight
   size_t scr_bytes = 0;
 };
 Buffers &buffers() {
@@ -655,46 +733,54 @@ Buffers &buffers() {
 }
 
 // The y/z sweeps (solve dimension strided, lines contiguous) by the line
-// kernel; returns false when some system does not have that shape (the x
-// sweeps stay with the tile kernel: a warp-transposing variant of the line
-// kernel for them measured 0.70 ms against the tile kernel's 0.41 ms on the
-// 256^3 FP64 x sweep).
+// kernel; returns false when some system does not have that shape.
 template <class T>
-bool launch_lines(std::vector<Sys> systems, cudaStream_t stream, long long *kernels) {
-  long long lines = 0, unknowns = 0;
-  for (Sys &s : systems) {
-    if (s.ss == 1 || s.s0 != 1) return false;
-    s.line0 = lines;
-    s.scr0 = unknowns;
-    const long long nl = (long long)s.nl0 * s.nl1;
-    lines += s.n > 0 ? nl : 0;
-    unknowns += s.n > 0 ? nl * s.n : 0;
-  }
+bool launch_lines(const std::vector<Sys> &systems, int maxn, cudaStream_t stream, long long *kernels) {
+  long long groups = 0;
   std::vector<Sys> live;  // systems with no rows or no lines take no part
-
-  for (const Sys &s : systems)
-    if (s.n > 0 && (long long)s.nl0 * s.nl1 > 0) live.push_back(s);
+  for (const Sys &s : systems) {
+    if (s.ss == 1 || s.s0 != 1) return false;
+    const long long nl = (long long)s.nl0 * s.nl1;
+    if (s.n <= 0 || nl <= 0) continue;
+    live.push_back(s);
+    live.back().line0 = groups;
+    groups += (nl + 15) / 16;
+  }
   if (live.empty()) return true;
+  static int per_sm = 0;  // resident threads, per type
+  if (!per_sm) {
+    int k = 0;
+    OPSB_CUDA(cudaFuncSetAttribute(trid_line_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLineSmem<T>));
+    OPSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, trid_line_kernel<T>, kLineThreads, kLineSmem<T>));
+    per_sm = std::max(k, 1) * kLineThreads;
+  }
+  // threads: what is resident, no more than kScratchBytes hold half lines for
+  // (but a CTA an SM at least), nor than there are groups
+  const int rows = (maxn + 1) / 2;
+  const size_t line = 2 * sizeof(T) * (size_t)rows;
+  const long long fit = (long long)(kScratchBytes / line) / 148 / kLineThreads * kLineThreads;
+  long long slots = 148 * std::max<long long>(kLineThreads, std::min<long long>(per_sm, fit));
+  slots = std::min(slots, (32 * groups + kLineThreads - 1) / kLineThreads * kLineThreads);
   Buffers &B = buffers();
   if (B.sys_cap < live.size()) {
     if (B.sys) cudaFree(B.sys);
-    B.sys_cap = std::max<size_t>(live.size(), 64);
-    OPSB_CUDA(cudaMalloc(&B.sys, B.sys_cap * sizeof(Sys)));
+    B.sys = nullptr;
+    B.sys_cap = 0;
+    const size_t cap = std::max<size_t>(live.size(), 64);
+    OPSB_CUDA(cudaMalloc(&B.sys, cap * sizeof(Sys)));
+    B.sys_cap = cap;
   }
-  const size_t need = 2 * (size_t)unknowns * sizeof(T);
+  const size_t need = (size_t)slots * line;
   if (B.scr_bytes < need) {
     if (B.scr) cudaFree(B.scr);
     B.scr = nullptr;
+    B.scr_bytes = 0;
     OPSB_CUDA(cudaMalloc(&B.scr, need));
     B.scr_bytes = need;
   }
   OPSB_CUDA(cudaMemcpyAsync(B.sys, live.data(), live.size() * sizeof(Sys), cudaMemcpyHostToDevice, stream));
-  T *sc = static_cast<T *>(B.scr), *sd = sc + unknowns;
-  const int grid = (int)std::min<long long>((lines + kLineThreads - 1) / kLineThreads, 148LL * 16);
-  if (sizeof(T) == 4 || lines <= kLinesDeep)
-    trid_line_kernel<T, 8><<<grid, kLineThreads, 0, stream>>>(B.sys, (int)live.size(), lines, sc, sd);
-  else
-    trid_line_kernel<T, 4><<<grid, kLineThreads, 0, stream>>>(B.sys, (int)live.size(), lines, sc, sd);
+  trid_line_kernel<T><<<(unsigned)(slots / kLineThreads), kLineThreads, kLineSmem<T>, stream>>>(
+      B.sys, (int)live.size(), groups, static_cast<T *>(B.scr), (int)slots);
   OPSB_CUDA(cudaGetLastError());
   if (kernels) (*kernels)++;
   return true;
@@ -731,7 +817,7 @@ void launch(const std::vector<Sys> &systems, int solvedim, cudaStream_t stream, 
   int maxn = 0;
   for (const Sys &s : systems) maxn = std::max(maxn, s.n);
   if (maxn == 0) return;
-  if (launch_lines<T>(systems, stream, kernels)) return;
+  if (launch_lines<T>(systems, maxn, stream, kernels)) return;
   bool contig = true;
   for (const Sys &s : systems) contig = contig && (s.n == 0 || s.ss == 1);
   // x sweeps of lines up to 256 rows: a warp per 1, 2 or 4 lines

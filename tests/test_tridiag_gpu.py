@@ -185,3 +185,31 @@ def test_full_size_256_cube_residual(gpu_runtime):
         r[..., 1:] += am[..., 1:] * xm[..., :-1]
         r[..., :-1] += cm[..., :-1] * xm[..., 1:]
         assert np.abs(r).max() / np.abs(dm).max() < 1e-14
+
+
+@pytest.mark.parametrize("dtype,rtol", [(np.float64, 1e-12), (np.float32, 2e-4)])
+@pytest.mark.parametrize("inc", [False, True])
+def test_more_strided_lines_than_threads(gpu_runtime, orc, dtype, rtol, inc):
+    """y sweeps of uneven systems in one launch with more groups of 16 lines
+    than the grid has warps (a thread takes several lines and reuses its
+    scratch), line counts that leave a group part empty, odd, even and one-row
+    lines."""
+    import torch
+    shapes = [(3, 41, 9001), (1, 1, 333), (2, 40, 16), (5, 7, 5003)]
+    sets, systems = [], []
+    for i, shape in enumerate(shapes):
+        a, b, c, d = seeded.trid_system(shape, 1, 31 + i, dtype)
+        u = seeded.uniform(7 + i, np.arange(d.size, dtype=np.uint64), -1, 1).reshape(d.shape).astype(dtype)
+        t = [torch.from_numpy(v).cuda() for v in (a, b, c, d, u)]
+        sets.append(((a, b, c, d, u), t))
+        systems.append(dict(a=t[0].data_ptr(), b=t[1].data_ptr(), c=t[2].data_ptr(), d=t[3].data_ptr(),
+                            u=t[4].data_ptr() if inc else None, dims=list(shape[::-1]), pads=list(shape[::-1])))
+    O.trid_batch(np.dtype(dtype).itemsize, 1, systems, None)
+    torch.cuda.synchronize()
+    for (a, b, c, d, u), t in sets:
+        ref = d.copy()
+        oracle_solve(orc, a, b, c, ref, 1)
+        if inc:
+            assert np.array_equal(t[3].cpu().numpy(), d)
+            ref = u + ref
+        np.testing.assert_allclose(t[4 if inc else 3].cpu().numpy(), ref, rtol=rtol, atol=rtol * np.abs(ref).max())
