@@ -322,20 +322,28 @@ __global__ void k_anorm(Fields f, const float *d, const double *e, float *G, dou
   }
 }
 
-// Per image: E[n] = ||e||^2 (or e.Ae); loss = mean_n d.d / E[n] (or d.Ad / E[n]) (one thread).
-__global__ void k_loss_finish(const double *part, int nblk, int n, double *E, double *loss) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  double L = 0.0;
-  for (int i = 0; i < n; i++) {
+// Per image: E[n] = ||e||^2 (or e.Ae); loss = mean_n d.d / E[n] (or d.Ad /
+// E[n]). One block, an image a thread, its partials added in block order with
+// their loads ahead (one thread for everything took 38 us of a 16 x 64^2 step);
+// the images' ratios, left in `part`, are added in order too.
+__global__ void k_loss_finish(double *part, int nblk, int n, double *E, double *loss) {
+  for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    double *p = part + (size_t)i * nblk * 2;
     double a = 0.0, b = 0.0;
+#pragma unroll 8
     for (int k = 0; k < nblk; k++) {
-      a += part[(i * nblk + k) * 2];
-      b += part[(i * nblk + k) * 2 + 1];
+      a += p[2 * k];
+      b += p[2 * k + 1];
     }
     if (!(b > 0.0)) b = 1.0;
     E[i] = b;
-    L += a / b;
+    p[0] = a / b;
   }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  double L = 0.0;
+#pragma unroll 4
+  for (int i = 0; i < n; i++) L += part[(size_t)i * nblk * 2];
   *loss = L / (double)n;
 }
 
@@ -378,22 +386,40 @@ __global__ void k_out_bwd(Fields f, const double *s, const double *E, const floa
   }
 }
 
-// Weight gradient of one 3x3 layer: dW[tap][co][ci] = sum_p g[p][co] x[p + tap][ci]
-// (x zero outside the image), db[co] = sum_p g[p][co]. blockIdx.y = tap (9 =
-// bias); each CTA sums its pixel tiles; partial[blockIdx.x][...] in W layout.
+// Weight gradients of the 3x3 layers: dW[tap][co][ci] = sum_p g[p][co] x[p + tap][ci]
+// (x zero outside the image), db[co] = sum_p g[p][co]. All layers run in one
+// launch, a CTA per layer, share of the pixel tiles and row of three taps; it
+// sums its tiles in order and leaves partial[share][...] in W layout. A thread
+// holds RO x RI outputs of each of the three taps, so a pixel's values are
+// loaded and converted once for 3 RO RI products (one CTA a tap, one output a
+// thread at a time and a launch a layer before: 343 us of a 16 x 64^2 step, now
+// 140 us). Every output is still one chain over the pixels in the same order.
+struct WgLayer {
+  const bf16 *x, *g;
+  float *partial;  // this layer's shares
+  float *grad;
+  int h, w, tiles, shares, len, first;  // first: this layer's first CTA
+};
+struct WgPlan {
+  WgLayer l[kLayers];
+  // the output layer's partials (k_out_bwd)
+  const float *opart;
+  float *ograd;
+  int oparts;
+};
+
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kT) k_wgrad(const bf16 *x, const bf16 *g, int n, int h, int w, float *partial) {
-  constexpr int NO = CIN * COUT, PER = (NO + kT - 1) / kT, LEN = 9 * NO + COUT;
-  __shared__ __align__(16) bf16 gs[kWgTile * COUT];
-  __shared__ __align__(16) bf16 xs[kWgTile * CIN];
-  const int tap = blockIdx.y;
-  const int dy = tap / 3 - 1, dx = tap % 3 - 1;
+__device__ __forceinline__ void wgrad_share(const WgLayer &L, int share, int dyi, uint4 *smem) {
+  constexpr int NO = CIN * COUT, PER = NO / kT > 0 ? NO / kT : 1;
+  constexpr int RI = PER >= 4 ? 4 : PER >= 2 ? 2 : 1, RO = PER / RI;  // outputs a thread: RO co x RI ci
+  static_assert(NO >= kT && RO * RI == PER, "wgrad tiling");
+  constexpr int XW = 18;  // 16 pixels and a column either side
+  bf16 *gs = reinterpret_cast<bf16 *>(smem), *xs = gs + kWgTile * COUT;
+  const int h = L.h, w = L.w, dy = dyi - 1;
   const int tx = (w + 15) / 16, ty = (h + 7) / 8;
-  const int tiles = n * tx * ty;
-  float acc[PER];
-#pragma unroll
-  for (int k = 0; k < PER; k++) acc[k] = 0.0f;
-  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+  const int ci0 = (threadIdx.x % (CIN / RI)) * RI, co0 = (threadIdx.x / (CIN / RI)) * RO;
+  float acc[3][RO][RI] = {}, bacc = 0.0f;
+  for (int t = share; t < L.tiles; t += L.shares) {
     const int img = t / (tx * ty), rem = t - img * tx * ty;
     const int y0 = (rem / tx) * 8, x0 = (rem % tx) * 16;
     __syncthreads();
@@ -401,56 +427,102 @@ __global__ void __launch_bounds__(kT) k_wgrad(const bf16 *x, const bf16 *g, int 
       const int p = v / (COUT / 8), cg = v % (COUT / 8);
       const int y = y0 + p / 16, xx = x0 + p % 16;
       uint4 val = make_uint4(0, 0, 0, 0);
-      if (y < h && xx < w) val = *reinterpret_cast<const uint4 *>(g + (((long long)img * h + y) * w + xx) * COUT + cg * 8);
+      if (y < h && xx < w)
+        val = *reinterpret_cast<const uint4 *>(L.g + (((long long)img * h + y) * w + xx) * COUT + cg * 8);
       *reinterpret_cast<uint4 *>(gs + p * COUT + cg * 8) = val;
     }
-    if (tap < 9) {
-      for (int v = threadIdx.x; v < kWgTile * (CIN / 8); v += kT) {
-        const int p = v / (CIN / 8), cg = v % (CIN / 8);
-        const int y = y0 + p / 16 + dy, xx = x0 + p % 16 + dx;
-        uint4 val = make_uint4(0, 0, 0, 0);
-        if (y >= 0 && y < h && xx >= 0 && xx < w && y0 + p / 16 < h && x0 + p % 16 < w)
-          val = *reinterpret_cast<const uint4 *>(x + (((long long)img * h + y) * w + xx) * CIN + cg * 8);
-        *reinterpret_cast<uint4 *>(xs + p * CIN + cg * 8) = val;
-      }
+    for (int v = threadIdx.x; v < 8 * XW * (CIN / 8); v += kT) {
+      const int p = v / (CIN / 8), cg = v % (CIN / 8);
+      const int y = y0 + p / XW + dy, xx = x0 + p % XW - 1;
+      uint4 val = make_uint4(0, 0, 0, 0);
+      if (y >= 0 && y < h && xx >= 0 && xx < w)
+        val = *reinterpret_cast<const uint4 *>(L.x + (((long long)img * h + y) * w + xx) * CIN + cg * 8);
+      *reinterpret_cast<uint4 *>(xs + p * CIN + cg * 8) = val;
     }
     __syncthreads();
-    if (tap < 9) {
+    for (int r = 0; r < 8; r++) {
+      const bf16 *gr = gs + r * 16 * COUT + co0, *xr = xs + r * XW * CIN + ci0;
+      float x[3][RI];  // the columns left of, at and right of the pixel
+      auto ldx = [&](int c, float (&o)[RI]) {
 #pragma unroll
-      for (int k = 0; k < PER; k++) {
-        const int o = threadIdx.x + k * kT;
-        if (o < NO) {
-          const int co = o / CIN, ci = o - co * CIN;
-          float a = acc[k];
-          for (int p = 0; p < kWgTile; p++) a += __bfloat162float(gs[p * COUT + co]) * __bfloat162float(xs[p * CIN + ci]);
-          acc[k] = a;
+        for (int k = 0; k < RI; k++) o[k] = __bfloat162float(xr[c * CIN + k]);
+      };
+      ldx(0, x[0]);
+      ldx(1, x[1]);
+#pragma unroll 4
+      for (int p = 0; p < 16; p++) {
+        ldx(p + 2, x[2]);
+        float g[RO];
+#pragma unroll
+        for (int o = 0; o < RO; o++) g[o] = __bfloat162float(gr[p * COUT + o]);
+#pragma unroll
+        for (int d = 0; d < 3; d++)
+#pragma unroll
+          for (int o = 0; o < RO; o++)
+#pragma unroll
+            for (int k = 0; k < RI; k++) acc[d][o][k] += g[o] * x[d][k];
+#pragma unroll
+        for (int k = 0; k < RI; k++) {
+          x[0][k] = x[1][k];
+          x[1][k] = x[2][k];
         }
       }
-    } else if (threadIdx.x < COUT) {
-      float a = acc[0];
-      for (int p = 0; p < kWgTile; p++) a += __bfloat162float(gs[p * COUT + threadIdx.x]);
-      acc[0] = a;
     }
+    if (dyi == 0 && threadIdx.x < COUT)
+      for (int p = 0; p < kWgTile; p++) bacc += __bfloat162float(gs[p * COUT + threadIdx.x]);
   }
-  float *out = partial + (size_t)blockIdx.x * LEN;
-  if (tap < 9) {
+  float *out = L.partial + (size_t)share * L.len;
 #pragma unroll
-    for (int k = 0; k < PER; k++) {
-      const int o = threadIdx.x + k * kT;
-      if (o < NO) out[tap * NO + o] = acc[k];
-    }
-  } else if (threadIdx.x < COUT) {
-    out[9 * NO + threadIdx.x] = acc[0];
+  for (int d = 0; d < 3; d++)
+#pragma unroll
+    for (int o = 0; o < RO; o++)
+#pragma unroll
+      for (int k = 0; k < RI; k++) out[(dyi * 3 + d) * NO + (co0 + o) * CIN + ci0 + k] = acc[d][o][k];
+  if (dyi == 0 && threadIdx.x < COUT) out[9 * NO + threadIdx.x] = bacc;
+}
+
+__global__ void __launch_bounds__(kT) k_wgrad(const __grid_constant__ WgPlan P) {
+  __shared__ uint4 smem[(kWgTile * 64 + 8 * 18 * 64) / 8];
+  int l = 0;
+  while (l + 1 < kLayers && (int)blockIdx.x >= P.l[l + 1].first) l++;
+  const WgLayer &L = P.l[l];
+  const int b = blockIdx.x - L.first, share = b / 3, dyi = b % 3;
+  switch (l) {
+    case C0: case C0U: wgrad_share<16, 16>(L, share, dyi, smem); break;
+    case C1A: wgrad_share<16, 32>(L, share, dyi, smem); break;
+    case C1B: wgrad_share<32, 32>(L, share, dyi, smem); break;
+    case C2A: wgrad_share<32, 64>(L, share, dyi, smem); break;
+    case C2U: wgrad_share<64, 32>(L, share, dyi, smem); break;
+    case C1U: wgrad_share<32, 16>(L, share, dyi, smem); break;
+    default: wgrad_share<64, 64>(L, share, dyi, smem); break;
   }
 }
 
-// grad[i] = sum_k partial[k * len + i], k in order.
-__global__ void k_sum_parts(const float *partial, int nparts, int len, float *grad) {
-  for (int i = blockIdx.x * kT + threadIdx.x; i < len; i += gridDim.x * kT) {
-    float t = 0.0f;
-    for (int k = 0; k < nparts; k++) t += partial[(size_t)k * len + i];
-    grad[i] = t;
+// grad[i] = sum_k partial[k * len + i], k in order, eight loads ahead.
+__device__ __forceinline__ float sum_parts(const float *p, int nparts, int len) {
+  float t = 0.0f;
+  int k = 0;
+  for (; k + 8 <= nparts; k += 8) {
+    float v[8];
+#pragma unroll
+    for (int j = 0; j < 8; j++) v[j] = __ldcg(p + (size_t)(k + j) * len);
+#pragma unroll
+    for (int j = 0; j < 8; j++) t += v[j];
   }
+  for (; k < nparts; k++) t += __ldcg(p + (size_t)k * len);
+  return t;
+}
+// Every layer's gradient from its partials, blockIdx.y = layer; the last is
+// the output layer.
+__global__ void k_sum_parts(const __grid_constant__ WgPlan P) {
+  if (blockIdx.y == kLayers) {
+    const int i = blockIdx.x * kT + threadIdx.x;
+    if (i < 17) P.ograd[i] = sum_parts(P.opart + i, P.oparts, 17);
+    return;
+  }
+  const WgLayer &L = P.l[blockIdx.y];
+  for (int i = blockIdx.x * kT + threadIdx.x; i < L.len; i += gridDim.x * kT)
+    L.grad[i] = sum_parts(L.partial + i, L.shares, L.len);
 }
 
 __global__ void k_adam(float *p, const float *g, float *m, float *v, int np, float lr_t, float b1, float b2,
@@ -465,16 +537,23 @@ __global__ void k_adam(float *p, const float *g, float *m, float *v, int np, flo
   }
 }
 
-// BF16 copies of one layer's weights: forward [9][cout][cin] and, for the
-// input gradient, flipped and transposed [9][cin][cout] with tap' = 8 - tap.
-__global__ void k_prep(const float *W, int cin, int cout, bf16 *wf, bf16 *wt) {
+// BF16 copies of every layer's weights (blockIdx.y = layer): forward
+// [9][cout][cin] and, for the input gradient, flipped and transposed
+// [9][cin][cout] with tap' = 8 - tap.
+struct PrepPlan {
+  const float *W[kLayers];
+  bf16 *wf[kLayers], *wt[kLayers];
+  int cin[kLayers], cout[kLayers];
+};
+__global__ void k_prep(const __grid_constant__ PrepPlan P) {
+  const int l = blockIdx.y, cin = P.cin[l], cout = P.cout[l];
   const int total = 9 * cin * cout;
   for (int i = blockIdx.x * kT + threadIdx.x; i < total; i += gridDim.x * kT) {
     const int tap = i / (cin * cout), rem = i - tap * cin * cout;
     const int co = rem / cin, ci = rem - co * cin;
-    const bf16 v = __float2bfloat16_rn(W[i]);
-    wf[i] = v;
-    wt[(8 - tap) * cin * cout + ci * cout + co] = v;
+    const bf16 v = __float2bfloat16_rn(P.W[l][i]);
+    P.wf[l][i] = v;
+    P.wt[l][(8 - tap) * cin * cout + ci * cout + co] = v;
   }
 }
 
@@ -502,6 +581,18 @@ struct Rng {
   double normal() { return sqrt(-2.0 * log(u01())) * cos(6.283185307179586 * u01()); }
 };
 
+}  // namespace
+
+namespace {
+// Level of each layer's grid (0 the finest), its pixel tiles, shares of them
+// and length of a partial.
+constexpr int kLevel[kLayers] = {0, 1, 1, 2, 2, 3, 3, 2, 1, 0};
+int wg_tiles(int l, int n, int h, int w) {
+  const int hl = h >> kLevel[l], wl = w >> kLevel[l];
+  return n * ((wl + 15) / 16) * ((hl + 7) / 8);
+}
+int wg_shares(int l, int n, int h, int w) { return std::min(kWgX, wg_tiles(l, n, h, w)); }
+int wg_len(int l) { return 9 * kDefs[l].cin * kDefs[l].cout + kDefs[l].cout; }
 }  // namespace
 
 struct Net::Impl {
@@ -547,9 +638,9 @@ struct Net::Impl {
     zblk = (int)std::max<long long>(1, std::min<long long>(std::min<long long>(1024, 148 * 8 / n),
                                                             (h * (long long)w + kT - 1) / kT));
     const size_t pred_b = ((size_t)P0 * 4 + 255) / 256 * 256;
-    int maxlen = 0;
-    for (int l = 0; l < kLayers; l++) maxlen = std::max(maxlen, 9 * kDefs[l].cin * kDefs[l].cout + kDefs[l].cout);
-    const size_t wpart_b = ((size_t)kWgX * maxlen * 4 + 255) / 256 * 256;
+    size_t wpart_n = 0;
+    for (int l = 0; l < kLayers; l++) wpart_n += (size_t)wg_shares(l, n, h, w) * wg_len(l);
+    const size_t wpart_b = (wpart_n * 4 + 255) / 256 * 256;
     const size_t opart_b = ((size_t)148 * 16 * 17 * 4 + 255) / 256 * 256;
     const size_t dscal_b = ((size_t)(2 * n + 1 + 2 * n * zblk) * 8 + 255) / 256 * 256;
     check(cudaMalloc(&act, bytes + 2 * pred_b + wpart_b + opart_b + dscal_b), "learned preconditioner buffers");
@@ -631,10 +722,16 @@ void conv(const bf16 *x, const bf16 *w, int n, int h, int wd, int cin, int cout,
 static void forward(Net::Impl &m, const Fields &f, cudaStream_t s, long long &launches) {
   const Offsets &o = offs();
   if (!m.prepped) {
-    for (int l = 0; l < kLayers; l++)
-      k_prep<<<blocks_for(9 * kDefs[l].cin * kDefs[l].cout), kT, 0, s>>>(m.params + o.w[l], kDefs[l].cin,
-                                                                         kDefs[l].cout, m.wf[l], m.wt[l]);
-    launches += kLayers;
+    PrepPlan P;
+    for (int l = 0; l < kLayers; l++) {
+      P.W[l] = m.params + o.w[l];
+      P.wf[l] = m.wf[l];
+      P.wt[l] = m.wt[l];
+      P.cin[l] = kDefs[l].cin;
+      P.cout[l] = kDefs[l].cout;
+    }
+    k_prep<<<dim3(16, kLayers), kT, 0, s>>>(P);
+    launches += 1;
     m.prepped = true;
   }
   const int n = f.n, h = f.h, w = f.w;
@@ -674,17 +771,6 @@ void Net::apply(const Fields &f, double *out, cudaStream_t s) {
   launches_ += 1;
 }
 
-namespace {
-template <int CI, int CO>
-void wgrad(const bf16 *x, const bf16 *g, int n, int h, int w, float *wpart, float *grad, cudaStream_t s) {
-  const int tiles = n * ((w + 15) / 16) * ((h + 7) / 8);
-  const int gx = std::min(kWgX, tiles);
-  k_wgrad<CI, CO><<<dim3(gx, 10), kT, 0, s>>>(x, g, n, h, w, wpart);
-  const int len = 9 * CI * CO + CO;
-  k_sum_parts<<<blocks_for(len), kT, 0, s>>>(wpart, gx, len, grad);
-}
-}  // namespace
-
 double Net::loss_and_grad(const Fields &f, const double *e, int kind, cudaStream_t s) {
   Impl &m = *m_;
   m.ensure(f.n, f.h, f.w);
@@ -701,11 +787,10 @@ double Net::loss_and_grad(const Fields &f, const double *e, int kind, cudaStream
     G = m.gbuf;
     launches_ += 1;
   }
-  k_loss_finish<<<1, 32, 0, s>>>(lpart, m.zblk, n, E, loss);
+  k_loss_finish<<<1, std::min(1024, (n + 31) / 32 * 32), 0, s>>>(lpart, m.zblk, n, E, loss);
   const int ob = blocks_for((long long)n * h * w);
   k_out_bwd<<<ob, kT, 0, s>>>(f, m.dscal, E, G, m.h0, m.params, o.wout, m.g0u, m.opart);
-  k_sum_parts<<<1, kT, 0, s>>>(m.opart, ob, 17, m.grads + o.wout);
-  launches_ += 6;
+  launches_ += 5;
   const int h1 = h / 2, w1 = w / 2, h2 = h / 4, w2 = w / 4, h3 = h / 8, w3 = w / 8;
   // input gradients (tensor cores, flipped/transposed weights)
   conv(m.g0u, m.wt[C0U], n, h, w, 16, 16, nullptr, nullptr, m.du0, cnn::CONV_PLAIN, s);
@@ -725,19 +810,33 @@ double Net::loss_and_grad(const Fields &f, const double *e, int kind, cudaStream
   k_add_poolT_mask<<<blocks_for((long long)n * h * w * 2), kT, 0, s>>>(m.du0, m.dp1, m.e0, m.ge0, n, h, w, 16);
   launches_ += 16;
   // weight gradients (CUDA cores, fixed-order partial sums)
-  float *WG = m.grads;
-  wgrad<16, 16>(m.u0, m.g0u, n, h, w, m.wpart, WG + o.w[C0U], s);
-  wgrad<32, 16>(m.u1, m.g1u, n, h1, w1, m.wpart, WG + o.w[C1U], s);
-  wgrad<64, 32>(m.u2, m.g2u, n, h2, w2, m.wpart, WG + o.w[C2U], s);
-  wgrad<64, 64>(m.a3, m.g3b, n, h3, w3, m.wpart, WG + o.w[C3B], s);
-  wgrad<64, 64>(m.p3, m.ga3, n, h3, w3, m.wpart, WG + o.w[C3A], s);
-  wgrad<64, 64>(m.a2, m.ge2, n, h2, w2, m.wpart, WG + o.w[C2B], s);
-  wgrad<32, 64>(m.p2, m.ga2, n, h2, w2, m.wpart, WG + o.w[C2A], s);
-  wgrad<32, 32>(m.a1, m.ge1, n, h1, w1, m.wpart, WG + o.w[C1B], s);
-  wgrad<16, 32>(m.p1, m.ga1, n, h1, w1, m.wpart, WG + o.w[C1A], s);
-  wgrad<16, 16>(m.x0, m.ge0, n, h, w, m.wpart, WG + o.w[C0], s);
+  WgPlan P;
+  const bf16 *xin[kLayers] = {m.x0, m.p1, m.a1, m.p2, m.a2, m.p3, m.a3, m.u2, m.u1, m.u0};
+  const bf16 *gout[kLayers] = {m.ge0, m.ga1, m.ge1, m.ga2, m.ge2, m.ga3, m.g3b, m.g2u, m.g1u, m.g0u};
+  float *part = m.wpart;
+  int ctas = 0;
+  for (int l = 0; l < kLayers; l++) {
+    WgLayer &L = P.l[l];
+    L.x = xin[l];
+    L.g = gout[l];
+    L.partial = part;
+    L.grad = m.grads + o.w[l];
+    L.h = h >> kLevel[l];
+    L.w = w >> kLevel[l];
+    L.tiles = wg_tiles(l, n, h, w);
+    L.shares = wg_shares(l, n, h, w);
+    L.len = wg_len(l);
+    L.first = ctas;
+    ctas += 3 * L.shares;
+    part += (size_t)L.shares * L.len;
+  }
+  P.opart = m.opart;
+  P.ograd = m.grads + o.wout;
+  P.oparts = ob;
+  k_wgrad<<<ctas, kT, 0, s>>>(P);
+  k_sum_parts<<<dim3(148, kLayers + 1), kT, 0, s>>>(P);
   check(cudaGetLastError(), "learned preconditioner backward");
-  launches_ += 20;
+  launches_ += 2;
   double L = 0.0;
   check(cudaMemcpyAsync(&L, loss, 8, cudaMemcpyDeviceToHost, s), "loss readback");
   check(cudaStreamSynchronize(s), "learned preconditioner step");
