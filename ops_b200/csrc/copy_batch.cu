@@ -89,6 +89,7 @@ bool plan(const std::vector<Desc> &q, size_t i, int n, Planned &out) {
   Runtime &rt = Runtime::get();
   struct Item { CopyStrip s; Box w, r; const char *data; int batch; };
   std::vector<Item> items;
+  std::unordered_map<const char *, std::vector<int>> of_dat;  // items of one storage, in queue order
   for (int j = 0; j < n; j++) {
     const Desc &d = q[i + j];
     const CopyLoopSpec *sp = find_copy_loop(d.loop);
@@ -120,9 +121,12 @@ bool plan(const std::vector<Desc> &q, size_t i, int n, Planned &out) {
       if (meet(it.w, it.r)) return false;  // a strip reading its own cells: keep the loop
       it.data = dt.data_d;
       it.batch = 0;
-      for (const Item &e : items)
-        if (e.data == it.data && e.batch >= it.batch && (meet(it.w, e.w) || meet(it.w, e.r) || meet(it.r, e.w)))
-          it.batch = e.batch + 1;
+      std::vector<int> &same = of_dat[it.data];
+      for (int k : same) {
+        const Item &e = items[k];
+        if (e.batch >= it.batch && (meet(it.w, e.w) || meet(it.w, e.r) || meet(it.r, e.w))) it.batch = e.batch + 1;
+      }
+      same.push_back((int)items.size());
       items.push_back(it);
     }
   }

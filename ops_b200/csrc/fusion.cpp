@@ -779,10 +779,18 @@ void Runtime::plan_fusion(const std::vector<Desc> &q, std::vector<FusedItem> &it
   auto bit = S.bounds.find(qk);
   if (bit == S.bounds.end()) {
     std::vector<std::pair<size_t, size_t>> b;
+    // A chain has two compute loops or more, so one that has fewer is not
+    // analysed, and a start from which the eligible run has fewer is passed
+    // over (analysing every stretch of a boundary refresh's 40 copy loops
+    // took 1.5 ms of host time a step structure).
+    std::vector<char> kind(q.size());  // 0 ineligible, 1 copy loop, 2 compute loop
+    for (size_t k = 0; k < q.size(); k++) {
+      int g;
+      kind[k] = !fp.eligible(q[k], &g) ? 0 : find_copy_loop(q[k].loop) ? 1 : 2;
+    }
     size_t i = 0;
     while (i < q.size()) {
-      int g;
-      if (!fp.eligible(q[i], &g)) {
+      if (!kind[i]) {
         i++;
         continue;
       }
@@ -790,9 +798,10 @@ void Runtime::plan_fusion(const std::vector<Desc> &q, std::vector<FusedItem> &it
       size_t best = 0;
       double best_saved = 0.0;
       ChainAnalysis A;
-      for (size_t j = i + 1; j <= q.size(); j++) {
-        int gj;
-        if (!fp.eligible(q[j - 1], &gj)) break;
+      int ncompute = 0;
+      for (size_t j = i + 1; j <= q.size() && kind[j - 1]; j++) {
+        ncompute += kind[j - 1] == 2;
+        if (ncompute < 2 && j - i <= (size_t)kMaxLoops) continue;
         if (fp.analyse(q, i, j - i, A)) {
           const double saved = A.loop_bytes - A.fused_bytes;
           if (saved > best_saved) {

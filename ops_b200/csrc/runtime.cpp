@@ -230,9 +230,13 @@ int Runtime::decl_dat(int blk, int dim, const int *size, const int *base, const 
     const Dat &dd = *dats_[idx];
     dat_set_data(idx, data, (size_t)dd.size[0] * dd.size[1] * dd.size[2] * dd.elem_size);
   }
-  OPSB_CUDA(cudaStreamSynchronize(stream_));
-  // a dat declared on a block already partitioned gets its slab at once
-  if (blk < (int)slabs_.size()) window_dat(*dats_[idx]);
+  // The zeros are ordered before every use on the runtime's stream; other
+  // ranks reach a dat only once its block is partitioned.
+  if (blk < (int)slabs_.size()) {
+    OPSB_CUDA(cudaStreamSynchronize(stream_));
+    // a dat declared on a block already partitioned gets its slab at once
+    window_dat(*dats_[idx]);
+  }
   return idx;
 }
 
@@ -303,16 +307,18 @@ void Runtime::decl_const(const char *name, int dim, const char *type, const void
       seen = it->second.bytes;
     }
   }
-  bool any = false;
+  // The loops that read a constant run on the same stream, so nothing waits
+  // here: the value goes through a pageable buffer of our own, which the
+  // driver stages before the call returns (the caller's may be pinned).
+  std::vector<char> buf;
   for (auto it = range.first; it != range.second; ++it) {
     if (!scope.empty() && it->second.scope != scope) continue;
     size_t bytes = ts > 0 ? (size_t)ts * dim : it->second.bytes;
     bytes = std::min(bytes, it->second.bytes);
-    OPSB_CUDA(cudaMemcpyToSymbolAsync(it->second.symbol, data, bytes, it->second.offset, cudaMemcpyHostToDevice,
-                                      stream_));
-    any = true;
+    if (data) buf.assign((const char *)data, (const char *)data + bytes);
+    OPSB_CUDA(cudaMemcpyToSymbolAsync(it->second.symbol, data ? buf.data() : nullptr, bytes, it->second.offset,
+                                      cudaMemcpyHostToDevice, stream_));
   }
-  if (any) OPSB_CUDA(cudaStreamSynchronize(stream_));
 }
 
 // ---------------------------------------------------------------------------
