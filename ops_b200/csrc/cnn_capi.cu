@@ -79,11 +79,13 @@ struct HeatWorkspace {
     if (x == nx && y == ny && pt == pitch && buf) return;
     cudaFree(buf);
     buf = nullptr;
-    const size_t one = (size_t)pt * (y + 2);
+    // each field's interior starts a 128-byte line (an even pitch then leaves
+    // the pairs of columns the multigrid cycle loads on 16 bytes)
+    const size_t first = ((size_t)pt + 1 + 15) / 16 * 16, one = ((size_t)pt * (y + 1) + first + 15) / 16 * 16;
     OPSB_CUDA(cudaMalloc(&buf, 6 * one * sizeof(double)));
     OPSB_CUDA(cudaMemsetAsync(buf, 0, 6 * one * sizeof(double), s));
     double **f[6] = {&r, &w, &p, &z, &Mi, &t};
-    for (int k = 0; k < 6; k++) *f[k] = buf + k * one + pt + 1;
+    for (int k = 0; k < 6; k++) *f[k] = buf + k * one + first;
     nx = x;
     ny = y;
     pitch = pt;

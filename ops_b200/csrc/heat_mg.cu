@@ -9,15 +9,16 @@
 // domain hold zero, so their terms are dropped while their face weights stay
 // in the diagonal (as the halo of the FP64 operator does).
 //
-// Every kernel is a streaming pass over one level (HBM-bound on the fine
-// levels): the fine level of one cycle costs five passes (first pre-sweep
-// with the FP64 -> FP32 copy of r, second pre-sweep, residual + restriction,
-// prolongation fused into the first post-sweep, last post-sweep writing the
-// FP64 result), about 106 bytes per fine cell; the coarser levels add a third.
+// A level above the coarsest costs two passes: k_cycle on the way down (both
+// pre-sweeps, the residual and its restriction) and k_cycle on the way up
+// (the correction and both post-sweeps). On level 0 that is 21 and 29 bytes a
+// cell; the coarser levels add a third.
 #include <algorithm>
+#include <cstdint>
 #include <string>
 
 #include "heat_mg.h"
+#include "march_grid.h"
 #include "runtime.h"
 
 namespace opsb {
@@ -55,108 +56,187 @@ __device__ __forceinline__ float diag(const LV &L, long long i, float aw, float 
   return (UNIT ? 1.0f : L.m[i]) + aw + ae + as + an;
 }
 
-// r - A z at (x, y), with z read through `zf(x, y)`; also returns the diagonal.
-template <bool UNIT, class ZF>
-__device__ __forceinline__ float resid(const LV &L, int x, int y, float rv, const ZF &zf, float &c) {
-  const long long i = (long long)y * L.P + x;
-  const float aw = L.ax[i], ae = L.ax[i + 1], as = L.ay[i], an = L.ay[i + L.P];
-  c = diag<UNIT>(L, i, aw, ae, as, an);
-  float s = rv - c * zf(x, y);
-  if (x > 0) s += aw * zf(x - 1, y);
-  if (x < L.nx - 1) s += ae * zf(x + 1, y);
-  if (y > 0) s += as * zf(x, y - 1);
-  if (y < L.ny - 1) s += an * zf(x, y + 1);
-  return s;
+// omega / c: the reciprocal approximation (1 ulp) with one Newton step (1/c =
+// q + q (1 - c q)), whose error is that of a rounded reciprocal; a division
+// and its range checks, two per cell and pass, were half of a pass's
+// instructions.
+__device__ __forceinline__ float over(float omega, float c) {
+  float q;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(q) : "f"(c));
+  return omega * fmaf(q, fmaf(-c, q, 1.0f), q);
 }
 
-// First pre-sweep from z = 0: z = omega r / c. On level 0 (R64) r arrives in
-// FP64 with the fields' pitch `fp` and its FP32 copy is kept in `r32`.
-template <bool UNIT, bool R64>
-__global__ void __launch_bounds__(BX *BY) k_pre_first(LV L, const double *__restrict__ r64, long long fp,
-                                                      float *__restrict__ r32, float *__restrict__ zout,
-                                                      float omega) {
-  MG_CELLS(L) {
-    const long long i = (long long)y * L.P + x;
-    float rv;
-    if (R64) {
-      rv = (float)r64[(long long)y * fp + x];
-      r32[i] = rv;
-    } else {
-      rv = r32[i];
-    }
-    const float c = diag<UNIT>(L, i, L.ax[i], L.ax[i + 1], L.ay[i], L.ay[i + L.P]);
-    zout[i] = omega * rv / c;
-  }
-}
+constexpr int kCycleWarps = 4;
+constexpr int cycle_blocks(bool up) { return up ? 4 : 5; }
 
-// zout = zin + omega (r - A zin) / c; with OUT64 the result goes to the FP64
-// field z64 (pitch fp) instead.
-template <bool UNIT, bool OUT64>
-__global__ void __launch_bounds__(BX *BY) k_smooth(LV L, const float *__restrict__ r, const float *__restrict__ zin,
-                                                   float *__restrict__ zout, double *__restrict__ z64, long long fp,
-                                                   float omega) {
-  auto zf = [&](int xx, int yy) { return zin[(long long)yy * L.P + xx]; };
-  MG_CELLS(L) {
-    const long long i = (long long)y * L.P + x;
-    float c;
-    const float s = resid<UNIT>(L, x, y, r[i], zf, c);
-    const float v = zin[i] + omega * s / c;
-    if (OUT64) z64[(long long)y * fp + x] = (double)v;
-    else zout[i] = v;
-  }
-}
-
-// First post-sweep with the coarse correction folded in: z' = zin + P e
-// (each cell takes its aggregate's value of e), then one damped-Jacobi sweep
-// on z'.
-template <bool UNIT, bool OUT64>
-__global__ void __launch_bounds__(BX *BY) k_post_first(LV L, const float *__restrict__ r, const float *__restrict__ zin,
-                                                       const float *__restrict__ e, long long eP,
-                                                       float *__restrict__ zout, double *__restrict__ z64,
-                                                       long long fp, float omega) {
-  MG_CELLS(L) {
-    const long long i = (long long)y * L.P + x;
-    // the cell's aggregate value and, across the aggregate's edge on each
-    // axis, the neighbouring aggregate's (the other side shares the cell's)
-    const float *ec = e + (long long)(y >> 1) * eP + (x >> 1);
-    const float e0 = ec[0];
-    const float ew = (x & 1) ? e0 : (x > 0 ? ec[-1] : 0.f);
-    const float ee = (x & 1) ? (x < L.nx - 1 ? ec[1] : 0.f) : e0;
-    const float es = (y & 1) ? e0 : (y > 0 ? ec[-eP] : 0.f);
-    const float en = (y & 1) ? (y < L.ny - 1 ? ec[eP] : 0.f) : e0;
-    auto zf = [&](int xx, int yy) {
-      const float zv = zin[(long long)yy * L.P + xx];
-      return zv + (xx < x ? ew : xx > x ? ee : yy < y ? es : yy > y ? en : e0);
-    };
-    float c;
-    const float s = resid<UNIT>(L, x, y, r[i], zf, c);
-    const float v = zf(x, y) + omega * s / c;
-    if (OUT64) z64[(long long)y * fp + x] = (double)v;
-    else zout[i] = v;
-  }
-}
-
-// Coarse right-hand side: rc(I, J) = sum of r - A z over the aggregate's
-// cells, in a fixed order (rows, then columns).
-template <bool UNIT>
-__global__ void __launch_bounds__(BX *BY) k_restrict(LV L, const float *__restrict__ r, const float *__restrict__ z,
-                                                     int cnx, int cny, long long cP, float *__restrict__ rc) {
-  auto zf = [&](int xx, int yy) { return z[(long long)yy * L.P + xx]; };
-  for (int J = blockIdx.y * BY + threadIdx.y; J < cny; J += gridDim.y * BY)
-    for (int I = blockIdx.x * BX + threadIdx.x; I < cnx; I += gridDim.x * BX) {
-      float acc = 0.0f;
-      for (int dy = 0; dy < 2; dy++) {
-        const int y = 2 * J + dy;
-        if (y >= L.ny) break;
-        for (int dx = 0; dx < 2; dx++) {
-          const int x = 2 * I + dx;
-          if (x >= L.nx) break;
-          float c;
-          acc += resid<UNIT>(L, x, y, r[(long long)y * L.P + x], zf, c);
+// One level on the way down (UP false):
+//    z0 = omega r / c;  z = z0 + omega (r - A z0) / c, kept in `zmid`;
+//    rc = the sum of r - A z over each aggregate (rows, then columns)
+// or up: z0 = zmid + P e (each cell its aggregate's value of e), then two
+// damped-Jacobi sweeps on it, the second one written out. On level 0 (R64,
+// OUT64) r is read from and z written to the FP64 fields (pitch `fp`; `vec`
+// says that their pairs of columns are 16-byte aligned).
+// Each of the sweeps used to be a pass of its own, 106 bytes a fine cell and
+// cycle. Here a warp marches up a strip of `rows` rows: a lane owns an
+// aggregate's two columns (30 lanes' own, one beside on each side), rows y of
+// z0, y - 1 of the first sweep and y - 2 of the second stage are in registers
+// at a time, neighbours beside come by shuffles, and a row is loaded two rows
+// or three ahead. Bound by memory on the fine levels (4096^2: 76 us down and
+// 89 up, 4.5 and 5.4 TB/s, where the five passes took 419), by latency on the
+// coarse ones (5 to 6 us a pass, launch included, below 512^2). A CTA of four
+// warps, five an SM down and four up, is what holds a pass in its registers
+// (with 80 registers a pass up spilled and took 134 us).
+template <bool UP, bool UNIT, bool R64, bool OUT64>
+__global__ void __launch_bounds__(32 * kCycleWarps, cycle_blocks(UP))
+    k_cycle(LV L, const double *__restrict__ r64, long long fp, int vec, const float *__restrict__ r32, float *zmid,
+            const float *__restrict__ e, long long cP, float *__restrict__ out, double *__restrict__ z64, float omega,
+            int rows) {
+  const int lane = threadIdx.x & 31, wi = blockIdx.x * kCycleWarps + (threadIdx.x >> 5);
+  const int ncol = ((L.nx + 1) / 2 + 29) / 30, nst = (L.ny + rows - 1) / rows;
+  if (wi >= ncol * nst) return;
+  const int I = (wi % ncol) * 30 + lane - 1, x = 2 * I, y0 = (wi / ncol) * rows, y1 = min(y0 + rows, L.ny);
+  const bool in0 = I >= 0 && x < L.nx, in1 = I >= 0 && x + 1 < L.nx, own = in0 && lane >= 1 && lane <= 30;
+  const long long P = L.P;
+  struct Row {
+    double2 r64;
+    float2 r, a, n, m, z;
+    float ae, e;
+  };
+  // a pair's second column may be the row's padding: it is masked below
+  auto pair = [](const float *q) { return *reinterpret_cast<const float2 *>(q); };
+  auto load = [&](int y) {
+    Row v{};
+    const long long i = (long long)y * P + x;
+    if (in0 && y >= -1 && y < L.ny) v.n = pair(L.ay + i + P);
+    if (I >= 0 && x <= L.nx && y >= 0 && y < L.ny) {
+      v.a = pair(L.ax + i);
+      if (lane == 31 && x + 2 <= L.nx) v.ae = L.ax[i + 2];  // the other lanes' comes from their neighbour
+      if (in0) {
+        if (R64) {
+          const double *q = r64 + (long long)y * fp + x;
+          if (vec && in1) {
+            v.r64 = *reinterpret_cast<const double2 *>(q);
+          } else {
+            v.r64.x = q[0];
+            if (in1) v.r64.y = q[1];
+          }
+        } else {
+          v.r = pair(r32 + i);
+        }
+        if (!UNIT) v.m = pair(L.m + i);
+        if (UP) {
+          v.z = pair(zmid + i);
+          v.e = e[(long long)(y >> 1) * cP + I];
         }
       }
-      rc[(long long)J * cP + I] = acc;
     }
+    return v;
+  };
+  struct Cells {
+    float2 r, c, q, a, s, n;  // r, diagonal, omega / diagonal, x-faces, y-faces below and above
+    float ae;
+  };
+  // r - A z on a row's two columns: centre zc, rows below and above zs, zn
+  auto resid = [&](const Cells &q, float2 zc, float2 zs, float2 zn) {
+    const float l = __shfl_up_sync(0xffffffffu, zc.y, 1), r = __shfl_down_sync(0xffffffffu, zc.x, 1);
+    float2 t;
+    t.x = q.r.x - q.c.x * zc.x;
+    t.x += q.a.x * l;
+    t.x += q.a.y * zc.y;
+    t.x += q.s.x * zs.x;
+    t.x += q.n.x * zn.x;
+    t.y = q.r.y - q.c.y * zc.y;
+    t.y += q.a.y * zc.x;
+    t.y += q.ae * r;
+    t.y += q.s.y * zs.y;
+    t.y += q.n.y * zn.y;
+    return t;
+  };
+  float acc = 0.f;
+  // Row y: z0 there, the first sweep on row y - 1 (cells A; z0 of y - 2, y - 1
+  // in za, zb) and the second stage on row y - 2 (cells B; the first sweep's of
+  // y - 3, y - 2 in va, vb), the upper row of an aggregate if ODD.
+  auto step = [&](int y, const Row &cur, float2 south, const Cells &A, const Cells &B, float2 za, float2 zb, float2 va,
+                  float2 vb, bool odd, Cells &C, float2 &z, float2 &v) {
+    const float ae = __shfl_down_sync(0xffffffffu, cur.a.x, 1);
+    C.r = R64 ? make_float2((float)cur.r64.x, (float)cur.r64.y) : cur.r;
+    C.a = cur.a;
+    C.ae = lane == 31 ? cur.ae : ae;
+    C.s = south;
+    C.n = cur.n;
+    C.c.x = (UNIT ? 1.0f : cur.m.x) + C.a.x + C.a.y + C.s.x + C.n.x;
+    C.c.y = (UNIT ? 1.0f : cur.m.y) + C.a.y + C.ae + C.s.y + C.n.y;
+    // outside the level q is 0 (and so is all of r, faces and z): z stays 0 there
+    const bool in = y >= 0 && y < L.ny;
+    C.q.x = in && in0 ? over(omega, C.c.x) : 0.f;
+    C.q.y = in && in1 ? over(omega, C.c.y) : 0.f;
+    if (UP) {
+      z.x = in && in0 ? cur.z.x + cur.e : 0.f;
+      z.y = in && in1 ? cur.z.y + cur.e : 0.f;
+    } else {
+      z.x = C.r.x * C.q.x;
+      z.y = C.r.y * C.q.y;
+    }
+    float2 t = resid(A, zb, za, z);
+    v.x = zb.x + A.q.x * t.x;
+    v.y = zb.y + A.q.y * t.y;
+    if (!UP && own && y - 1 >= y0 && y - 1 < y1) {
+      float *q = zmid + (long long)(y - 1) * P + x;
+      if (in1) *reinterpret_cast<float2 *>(q) = v;
+      else *q = v.x;
+    }
+    t = resid(B, vb, va, v);
+    const int yo = y - 2;
+    if (own && yo >= y0 && yo < y1) {
+      if (UP) {
+        const float2 o = make_float2(vb.x + B.q.x * t.x, vb.y + B.q.y * t.y);
+        if (OUT64) {
+          double *q = z64 + (long long)yo * fp + x;
+          if (vec && in1) {
+            *reinterpret_cast<double2 *>(q) = make_double2((double)o.x, (double)o.y);
+          } else {
+            q[0] = (double)o.x;
+            if (in1) q[1] = (double)o.y;
+          }
+        } else {
+          float *q = out + (long long)yo * P + x;
+          if (in1) *reinterpret_cast<float2 *>(q) = o;
+          else *q = o.x;
+        }
+      } else {
+        acc = odd ? acc + t.x : t.x;
+        if (in1) acc += t.y;
+        if (odd || yo == L.ny - 1) out[(long long)(yo >> 1) * cP + I] = acc;
+      }
+    }
+  };
+  float2 s{};  // the faces below the current row
+  if (in0 && y0 >= 2) s = pair(L.ay + (long long)(y0 - 2) * P + x);
+  Row c0 = load(y0 - 2), c1 = load(y0 - 1);
+  Cells A{}, B{};
+  float2 za{}, zb{}, va{}, vb{};
+  for (int y = y0 - 2; y < y1 + 2; y += 2) {
+    const Row n0 = load(min(y + 2, y1 + 1)), n1 = load(min(y + 3, y1 + 1));
+    Cells C, D;
+    float2 z0, z1, v0, v1;
+    step(y, c0, s, A, B, za, zb, va, vb, false, C, z0, v0);
+    step(y + 1, c1, C.n, C, A, zb, z0, vb, v0, true, D, z1, v1);
+    s = D.n;
+    za = z0;
+    zb = z1;
+    va = v0;
+    vb = v1;
+    B = C;
+    A = D;
+    c0 = n0;
+    c1 = n1;
+  }
+}
+
+// The FP32 copy of r for a cycle whose z overlaps it.
+__global__ void __launch_bounds__(BX *BY) k_copy_r(LV L, const double *__restrict__ r64, long long fp,
+                                                   float *__restrict__ r32) {
+  MG_CELLS(L) r32[(long long)y * L.P + x] = (float)r64[(long long)y * fp + x];
 }
 
 // The coarsest level (at most kCoarsest x kCoarsest cells, one per thread of
@@ -181,7 +261,8 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarsest(LV L, const float *
     c = diag<UNIT>(L, i, aw, ae, as, an);
     rv = IO64 ? (float)r64[(long long)y * fp + x] : r32[i];
   }
-  float v = on ? omega * rv / c : 0.f;
+  const float q = over(omega, c);
+  float v = on ? q * rv : 0.f;
   zs[0][t] = v;
   __syncthreads();
   int cur = 0;
@@ -193,7 +274,7 @@ __global__ void __launch_bounds__(kCoarseThreads) k_coarsest(LV L, const float *
       if (x < L.nx - 1) s += ae * zc[t + 1];
       if (y > 0) s += as * zc[t - L.nx];
       if (y < L.ny - 1) s += an * zc[t + L.nx];
-      v = zc[t] + omega * s / c;
+      v = zc[t] + q * s;
     }
     zs[cur ^ 1][t] = v;
     __syncthreads();
@@ -376,62 +457,67 @@ long long Multigrid::enqueue(const double *r, double *z, cudaStream_t s) {
     check("coarsest level");
     return 1;
   }
-  std::vector<float *> zc(nl), out(nl);
+  static_assert(kSweeps == 2, "k_cycle makes two sweeps a side");
+  // strips of whole aggregates' rows
+  auto strips = [&](const Level &L, bool up, int *rows) {
+    const int ncol = ((L.nx + 1) / 2 + 29) / 30, cny = (L.ny + 1) / 2;
+    *rows = 2 * march_rows(ncol, cny, 2, 148LL * cycle_blocks(up) * kCycleWarps);
+    const long long warps = (long long)ncol * ((L.ny + *rows - 1) / *rows);
+    return (unsigned)((warps + kCycleWarps - 1) / kCycleWarps);
+  };
+  const int nt = 32 * kCycleWarps;
+  // r and z of level 0: strips read r beside the rows they write z to, so
+  // where the two overlap r is taken from a copy
+  const long long span = (long long)(lv_[0].ny - 1) * fpitch_ + lv_[0].nx;
+  const bool apart = z + span <= r || r + span <= z;
+  auto even = [&](const double *p) { return fpitch_ % 2 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0; };
+  const int vr = even(r), vz = even(z);
+  if (!apart) {
+    k_copy_r<<<grid_of(lv_[0].nx, lv_[0].ny), blk, 0, s>>>(view(0), r, fpitch_, lv_[0].r);
+    n++;
+  }
   // down: smooth, then hand the residual to the next level
   for (int l = 0; l + 1 < nl; l++) {
-    Level &L = lv_[l];
+    Level &L = lv_[l], &C = lv_[l + 1];
     const LV v = view(l);
-    const dim3 g = grid_of(L.nx, L.ny);
-    if (l == 0) k_pre_first<true, true><<<g, blk, 0, s>>>(v, r, fpitch_, L.r, L.z0, w);
-    else k_pre_first<false, false><<<g, blk, 0, s>>>(v, nullptr, 0, L.r, L.z0, w);
+    int rows;
+    const unsigned g = strips(L, false, &rows);
+    if (l == 0 && apart)
+      k_cycle<false, true, true, false><<<g, nt, 0, s>>>(v, r, fpitch_, vr, nullptr, L.z0, nullptr, C.pitch, C.r,
+                                                         nullptr, w, rows);
+    else if (l == 0)
+      k_cycle<false, true, false, false><<<g, nt, 0, s>>>(v, nullptr, 0, 0, L.r, L.z0, nullptr, C.pitch, C.r, nullptr,
+                                                          w, rows);
+    else
+      k_cycle<false, false, false, false><<<g, nt, 0, s>>>(v, nullptr, 0, 0, L.r, L.z0, nullptr, C.pitch, C.r,
+                                                           nullptr, w, rows);
     n++;
-    float *cur = L.z0, *oth = L.z1;
-    for (int k = 1; k < kSweeps; k++) {
-      if (l == 0) k_smooth<true, false><<<g, blk, 0, s>>>(v, L.r, cur, oth, nullptr, 0, w);
-      else k_smooth<false, false><<<g, blk, 0, s>>>(v, L.r, cur, oth, nullptr, 0, w);
-      n++;
-      std::swap(cur, oth);
-    }
-    zc[l] = cur;
-    const Level &C = lv_[l + 1];
-    const dim3 gc = grid_of(C.nx, C.ny);
-    if (l == 0) k_restrict<true><<<gc, blk, 0, s>>>(v, L.r, cur, C.nx, C.ny, C.pitch, C.r);
-    else k_restrict<false><<<gc, blk, 0, s>>>(v, L.r, cur, C.nx, C.ny, C.pitch, C.r);
-    n++;
-    check("restriction");
+    check("pre-smoothing and restriction");
   }
   {
     Level &L = lv_[nl - 1];
     k_coarsest<false, false><<<1, kCoarseThreads, 0, s>>>(view(nl - 1), L.r, nullptr, 0, L.z1, nullptr,
                                                           kCoarseSweeps, w);
     n++;
-    out[nl - 1] = L.z1;
     check("coarsest level");
   }
   // up: correct with the coarse solution, then post-smooth
   for (int l = nl - 2; l >= 0; l--) {
-    Level &L = lv_[l];
+    Level &L = lv_[l], &C = lv_[l + 1];
     const LV v = view(l);
-    const dim3 g = grid_of(L.nx, L.ny);
-    const float *e = out[l + 1];
-    const long long eP = lv_[l + 1].pitch;
-    float *cur = zc[l], *oth = (cur == L.z0) ? L.z1 : L.z0;
-    const bool last_first = kSweeps == 1;
-    if (l == 0 && last_first) k_post_first<true, true><<<g, blk, 0, s>>>(v, L.r, cur, e, eP, nullptr, z, fpitch_, w);
-    else if (l == 0) k_post_first<true, false><<<g, blk, 0, s>>>(v, L.r, cur, e, eP, oth, nullptr, 0, w);
-    else k_post_first<false, false><<<g, blk, 0, s>>>(v, L.r, cur, e, eP, oth, nullptr, 0, w);
+    int rows;
+    const unsigned g = strips(L, true, &rows);
+    if (l == 0 && apart)
+      k_cycle<true, true, true, true><<<g, nt, 0, s>>>(v, r, fpitch_, vr && vz, nullptr, L.z0, C.z1, C.pitch, nullptr, z,
+                                                       w, rows);
+    else if (l == 0)
+      k_cycle<true, true, false, true><<<g, nt, 0, s>>>(v, nullptr, fpitch_, vz, L.r, L.z0, C.z1, C.pitch, nullptr, z,
+                                                        w, rows);
+    else
+      k_cycle<true, false, false, false><<<g, nt, 0, s>>>(v, nullptr, 0, 0, L.r, L.z0, C.z1, C.pitch, L.z1, nullptr, w,
+                                                          rows);
     n++;
-    std::swap(cur, oth);
-    for (int k = 1; k < kSweeps; k++) {
-      const bool last = k == kSweeps - 1;
-      if (l == 0 && last) k_smooth<true, true><<<g, blk, 0, s>>>(v, L.r, cur, nullptr, z, fpitch_, w);
-      else if (l == 0) k_smooth<true, false><<<g, blk, 0, s>>>(v, L.r, cur, oth, nullptr, 0, w);
-      else k_smooth<false, false><<<g, blk, 0, s>>>(v, L.r, cur, oth, nullptr, 0, w);
-      n++;
-      std::swap(cur, oth);
-    }
-    out[l] = cur;
-    check("prolongation / post-smoothing");
+    check("prolongation and post-smoothing");
   }
   return n;
 }

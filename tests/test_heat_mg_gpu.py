@@ -157,3 +157,18 @@ def test_fcg_mg_is_deterministic(gpu_runtime):
         outs.append((u, st["iterations"]))
     assert outs[0][1] == outs[1][1]
     assert torch.equal(outs[0][0], outs[1][0])
+
+
+@pytest.mark.parametrize("ny,nx", [(17, 120), (34, 61), (200, 59), (257, 60), (18, 241), (400, 17)])
+@pytest.mark.parametrize("in_place", [False, True])
+def test_vcycle_strip_edges(gpu_runtime, ny, nx, in_place):
+    """The level passes' strips (30 aggregates wide, whole aggregates high):
+    one and two strips, a lone last column or row, several strips high; and z
+    written over r. Bound as above."""
+    from ops_b200 import lmg
+    Kx, Ky, r = random_problem(ny, nx, 11 * ny + nx)
+    z = cuda(r if in_place else np.zeros_like(r))
+    lmg.mg_apply(cuda(Kx), cuda(Ky), z if in_place else cuda(r), z, 60.0, 45.0)
+    want = vcycle(hierarchy(Kx, Ky, 60.0, 45.0), r[1:-1, 1:-1])
+    got = z.cpu().numpy()[1:-1, 1:-1]
+    assert np.linalg.norm(got - want) / np.linalg.norm(want) < 1e-4
