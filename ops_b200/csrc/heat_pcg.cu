@@ -1072,6 +1072,7 @@ void check_launch(const char *what) {
 struct Solver::Impl {
   Scalars *s64 = nullptr, *s32 = nullptr;
   double *part = nullptr;
+  int part_n = 0;
   unsigned *cnt = nullptr;
   int *h_flag = nullptr;  // pinned, two slots
   cudaEvent_t ev[2] = {nullptr, nullptr};
@@ -1150,11 +1151,24 @@ struct Solver::Impl {
     p64b_n = n;
   }
 
+  // Partials for a grid of more than kMaxBlocks (a strip or tile is a block's
+  // least: 2D rows of a million cells, 3D cross-sections of 1312^2).
+  void ensure_part(int blocks) {
+    if (blocks <= part_n) return;
+    cudaFree(part);
+    part = nullptr;
+    part_n = 0;
+    chunk64.key.clear();  // the captured chunks hold the old address
+    chunk32.key.clear();
+    OPSB_CUDA(cudaMalloc(&part, 2 * (size_t)blocks * sizeof(double)));
+    part_n = blocks;
+  }
+
   void ensure_base() {
     if (s64) return;
     OPSB_CUDA(cudaMalloc(&s64, 2 * sizeof(Scalars)));
     s32 = s64 + 1;
-    OPSB_CUDA(cudaMalloc(&part, 2 * kMaxBlocks * sizeof(double)));
+    ensure_part(kMaxBlocks);
     OPSB_CUDA(cudaMalloc(&cnt, 64));
     OPSB_CUDA(cudaMemset(cnt, 0, 64));
     OPSB_CUDA(cudaMallocHost(&h_flag, 2 * sizeof(int)));
@@ -1220,7 +1234,6 @@ void pw_grid(int nx, int ny, int per_sm, int *rows, int *blocks) {
   const long long ncol = (nx + 29) / 30;
   *rows = march_rows(ncol, ny, 2, 148LL * per_sm * kWarps, (long long)kMaxBlocks * kWarps);
   *blocks = (int)((ncol * ((ny + *rows - 1) / *rows) + kWarps - 1) / kWarps);
-  if (*blocks > kMaxBlocks) throw Error(E_UNSUPPORTED, "heat solver: rows too long");
 }
 struct Grid3 {
   int tx, ty, planes, blocks;
@@ -1230,7 +1243,7 @@ Grid3 pw3_grid(int nx, int ny, int nz) {
   q.tx = (nx + 29) / 30;
   q.ty = (ny + kTileY - 3) / (kTileY - 2);
   const long long tiles = (long long)q.tx * q.ty;
-  if (tiles > kMaxBlocks) throw Error(E_UNSUPPORTED, "heat solver 3D: cross-section too large");
+  if (tiles > 0x7fffffffLL) throw Error(E_UNSUPPORTED, "heat solver 3D: cross-section too large");
   q.planes = march_rows(tiles, nz, 2, 148LL * 2, kMaxBlocks);
   q.blocks = (int)(tiles * ((nz + q.planes - 1) / q.planes));
   return q;
@@ -1332,6 +1345,7 @@ void Solver::pcg_fp64(const Field2D &f, double rx, double ry, bool precond, bool
     } else {
       int rows, blocks;
       pw_grid(f.nx, f.ny, kPwBlocks<double>, &rows, &blocks);
+      m.ensure_part(blocks);
       const std::string key = key_of({f.Kx, f.Ky, f.u, f.r, f.w, f.p, pb, f.Mi},
                                      {rx, ry, (double)f.nx, (double)f.ny, (double)f.pitch, precond ? 1.0 : 0.0,
                                       true_stop ? 1.0 : 0.0});
@@ -1411,6 +1425,7 @@ void Solver::pcg_mixed(const Field2D &f, double rx, double ry, bool precond, dou
   out->initial_residual = r0;
   int rows, blocks;
   pw_grid(f.nx, f.ny, kPwBlocks<float>, &rows, &blocks);
+  m.ensure_part(blocks);
   const std::string key = key_of({m.Kx, m.Ky, m.e, m.r, m.w, m.p, m.p2, m.Mi},
                                  {(double)rxf, (double)ryf, (double)f.nx, (double)f.ny, (double)m.pitch32,
                                   precond ? 1.0 : 0.0});
@@ -1520,6 +1535,7 @@ void Solver::pcg3d(const Field3D &f, double rx, double ry, double rz, bool true_
   const long long nf = f.plane * (f.nz + 2);
   if (((uintptr_t)r | (uintptr_t)w | (uintptr_t)Mi) & 15) throw Error(E_ARG, "heat solver 3D: misaligned field");
   const Grid3 q = pw3_grid(f.nx, f.ny, f.nz);
+  m.ensure_part(q.blocks);
   const int gridr = (int)std::min<long long>((nf / 2 + NT - 1) / NT, 148 * kFlatBlocks);
   Scalars h = fresh(0.0);
   OPSB_CUDA(cudaMemcpyAsync(m.s64, &h, sizeof(h), cudaMemcpyHostToDevice, st));
@@ -1587,6 +1603,7 @@ void Solver::pcg3d_mixed(const Field3D &f, double rx, double ry, double rz, doub
   const dim3 gridf = grid_for((int)f.pitch, rows);
   const dim3 grid1((unsigned)std::min<long long>(((long long)nf + NT - 1) / NT, 148LL * 16));
   const Grid3 q = pw3_grid(f.nx, f.ny, f.nz);
+  m.ensure_part(q.blocks);
   const int gridr = (int)std::min<long long>(((long long)nf / 4 + NT - 1) / NT + 1, 148 * kFlatBlocks);
   const float rxf = (float)rx, ryf = (float)ry, rzf = (float)rz;
   k_flat_to_float<<<grid1, block, 0, st>>>(f.Kx - off, m.Kx, (long long)nf);

@@ -19,9 +19,10 @@ def residual(Kx, Ky, u, u0, rx):
 
 # nx, ny: one cell; a tile's last column and the next CTA's first; 2, 4 and 8
 # tiles a CTA with ragged ends; the largest grid of the one-kernel loop (8 x
-# 148 tiles) and the first beyond it; strips of 30, 31 and 61 columns
+# 148 tiles) and the first beyond it; strips of 30, 31 and 61 columns; more
+# strips than 4096 CTAs hold
 @pytest.mark.parametrize("nx,ny", [(1, 1), (128, 2), (129, 3), (127, 33), (61, 600), (257, 301), (1024, 296),
-                                   (1024, 298), (31, 2400), (150, 1190), (1230, 61)])
+                                   (1024, 298), (31, 2400), (150, 1190), (1230, 61), (990001, 2)])
 @pytest.mark.parametrize("method", ["PCG_TRUE", "PCG", "MIXED"])
 def test_loops_reach_the_residual(gpu_runtime, nx, ny, method):
     import torch
@@ -50,3 +51,20 @@ def test_loops_reach_the_residual(gpu_runtime, nx, ny, method):
     assert np.linalg.norm(a - b) <= r + s + 1e-12 * np.linalg.norm(b)
     if method == "PCG_TRUE" and ref["iterations"] > 3:
         assert st["iterations"] < ref["iterations"]
+
+
+@pytest.mark.parametrize("method", ["PCG_TRUE", "MIXED"])
+def test_wide_cross_section_3d(gpu_runtime, method):
+    """A cross-section of more than 4096 tiles."""
+    import torch
+
+    from ops_b200 import lmg
+    rng = np.random.default_rng(5)
+    rho = np.exp(rng.uniform(np.log(0.1), np.log(10.0), (2, 1400, 1400)))
+    k = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in lmg.faces3d(rho)]
+    u0 = torch.zeros_like(k[0])
+    u0[1:-1, 1:-1, 1:-1] = torch.from_numpy(rng.uniform(0.0, 1.0, rho.shape)).cuda()
+    u = u0.clone()
+    st = lmg.solve3d(*k, u0, u, 5.0, 5.0, 5.0, method=getattr(lmg, method), eps=1e-8)
+    # stopped on the recursive residual (PCG_TRUE) or the FP64 one; they differ by rounding, far below 1e-8 ||r0||
+    assert st["converged"] and st["final_residual"] < 1.5e-8 * st["initial_residual"]
