@@ -50,6 +50,7 @@ struct Scalars {
   int max_iters;
   int first;
   int pend;  // u += alpha p of the last k_pw is still to be made
+  int restart;  // FCG: the next direction is z itself
   // FCG restart test on the device (replayed chunks): ||r|| of the last
   // iterations since the last (re)start, `window` 0 when the test is off
   int window, hcount;
@@ -132,7 +133,8 @@ __device__ __forceinline__ T smvp(const T *__restrict__ Kx, const T *__restrict_
 // How k_pw gets z: the residual itself, Mi r with Mi read, or Mi r with
 // Mi = 1 / diag(A) computed from the faces it holds anyway (FP64: the same
 // bits as tea_leaf_common_init_diag_init_kernel's Mi, 8 B a cell less).
-enum { Z_R = 0, Z_MI = 1, Z_DIAG = 2 };
+// Z_FCG: the flexible CG's z itself in `r`, and the residual in `Mi`.
+enum { Z_R = 0, Z_MI = 1, Z_DIAG = 2, Z_FCG = 3 };
 
 // tea_leaf_axpby_kernel (p = beta p + z), tea_leaf_cg_calc_w_reduce_kernel
 // (w = A p, p.w; tea_leaf_cg_kernels.h:8) and the previous iteration's
@@ -142,6 +144,9 @@ enum { Z_R = 0, Z_MI = 1, Z_DIAG = 2 };
 // ring's p never changes and is read from the first buffer.
 // A row's loads are issued two rows ahead; FP32 rows are half the bytes, so
 // four CTAs an SM there, three in FP64.
+// Z_FCG (Notay 2000, FCG with one-step truncation): alpha = p.r / p.w, p = z
+// after a restart, and a non-positive p.w (the preconditioned direction lost
+// positive curvature) stops with done = 4.
 template <class T>
 constexpr int kPwBlocks = sizeof(T) == 4 ? 4 : 3;
 template <class T, int Z>
@@ -155,11 +160,12 @@ __global__ void __launch_bounds__(NT, kPwBlocks<T>) k_pw(Geom g, const T *__rest
   const int odd = s->iters & 1;
   const T *pin = odd ? pb : pa;
   T *pout = odd ? pa : pb;
-  const bool first = s->iters == 0 && !s->pend, pend = s->pend != 0;
+  const bool first = Z == Z_FCG ? s->restart != 0 : s->iters == 0 && !s->pend, pend = s->pend != 0;
   const T alpha = (T)s->alpha, beta = (T)s->beta;
+  constexpr int NV = Z == Z_FCG ? 2 : 1;
   const int ncol = (g.nx + 29) / 30, nst = (g.ny + rows - 1) / rows;
   const int wi = blockIdx.x * kWarps + (tid_() >> 5), lane = tid_() & 31;
-  double acc[1] = {0.0};
+  double acc[NV] = {};
   if (wi < ncol * nst) {
     const int x = (wi % ncol) * 30 + lane - 1, y0 = (wi / ncol) * rows, y1 = min(y0 + rows, g.ny);
     const bool in = x >= 0 && x < g.nx, own = in && lane >= 1 && lane <= 30, ring = x == -1 || x == g.nx;
@@ -176,7 +182,7 @@ __global__ void __launch_bounds__(NT, kPwBlocks<T>) k_pw(Geom g, const T *__rest
         v.ky1 = Ky[i + P];
         v.r = r[i];
         v.p = pin[i];
-        if (Z == Z_MI) v.m = Mi[i];
+        if (Z == Z_MI || (Z == Z_FCG && own && y >= y0 && y < y1)) v.m = Mi[i];
         if (pend && own && y >= y0 && y < y1) v.u = u[i];
       } else if (in || (ring && y >= 0 && y < g.ny)) {
         v.p = pa[i];
@@ -190,7 +196,7 @@ __global__ void __launch_bounds__(NT, kPwBlocks<T>) k_pw(Geom g, const T *__rest
       if (lane < 31) v.kx1 = kr;
       d = T(1) + ry * (v.ky1 + ky0) + rx * (v.kx1 + v.kx0);
       if (!in || y < 0 || y >= g.ny) return v.p;
-      const T z = Z == Z_R ? v.r : Z == Z_MI ? v.m * v.r : (T(1) / d) * v.r;
+      const T z = Z == Z_R || Z == Z_FCG ? v.r : Z == Z_MI ? v.m * v.r : (T(1) / d) * v.r;
       return first ? z : beta * v.p + z;
     };
     auto face = [&](int y) { return in && y >= 0 && y < g.ny ? Ky[(long long)y * P + x] : T(0); };
@@ -213,6 +219,7 @@ __global__ void __launch_bounds__(NT, kPwBlocks<T>) k_pw(Geom g, const T *__rest
         pout[i] = pc;
         if (pend) u[i] = c.u + alpha * c.p;
         acc[0] = acc[0] + (double)wv * (double)pc;
+        if (Z == Z_FCG) acc[NV - 1] = acc[NV - 1] + (double)pc * (double)c.m;
       }
       pm = pc;
       pc = pn;
@@ -222,12 +229,20 @@ __global__ void __launch_bounds__(NT, kPwBlocks<T>) k_pw(Geom g, const T *__rest
       n = nn;
     }
   }
-  if (publish<1>(acc, part, cnt, sm, &last)) {
-    const double t = grid_total<1>(part, 0, sm);
+  if (publish<NV>(acc, part, cnt, sm, &last)) {
+    const double t = grid_total<NV>(part, 0, sm);
+    const double pr = Z == Z_FCG ? grid_total<NV>(part, NV - 1, sm) : 0.0;
     if (tid_() == 0) {
       s->pw = t;
-      s->alpha = s->rro / t;
-      s->pend = 1;
+      if (Z == Z_FCG) {
+        s->restart = 0;
+        s->pend = t > 0.0;
+        if (t > 0.0) s->alpha = pr / t;
+        else s->done = 4;
+      } else {
+        s->alpha = s->rro / t;
+        s->pend = 1;
+      }
       *cnt = 0u;
     }
   }
@@ -693,40 +708,13 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
   if (t == 0 && expired) *err = 1;
 }
 
-// ---- flexible CG (Notay 2000, FCG with one-step truncation) ----------------
-// k_fw: w = A p, pw = p.w, pr = p.r -> alpha = pr / pw; a non-positive pw
-// (the preconditioned direction lost positive curvature) stops with done = 4.
-__global__ void __launch_bounds__(NT, kResident) k_fw(Geom g, const double *__restrict__ Kx, const double *__restrict__ Ky,
-                                           const double *__restrict__ p, const double *__restrict__ r,
-                                           double *__restrict__ w, double rx, double ry, Scalars *s, double *part,
-                                           unsigned *cnt) {
-  __shared__ double sm[kWarps];
-  __shared__ int last;
-  if (s->done) return;
-  double acc[2] = {0.0, 0.0};
-  HEAT_CELLS(g) {
-    const long long i = (long long)y * g.pitch + x;
-    const double wv = smvp(Kx, Ky, p, i, g.pitch, rx, ry);
-    w[i] = wv;
-    acc[0] = acc[0] + wv * p[i];
-    acc[1] = acc[1] + p[i] * r[i];
-  }
-  if (publish<2>(acc, part, cnt, sm, &last)) {
-    const double pw = grid_total<2>(part, 0, sm);
-    const double pr = grid_total<2>(part, 1, sm);
-    if (tid_() == 0) {
-      s->pw = pw;
-      if (pw > 0.0) s->alpha = pr / pw;
-      else s->done = 4;
-      *cnt = 0u;
-    }
-  }
-}
-
-// u += alpha p, r -= alpha w, rr = r.r; stop when ||r|| < eps ||r0||.
-__global__ void __launch_bounds__(NT, kResident) k_fupd(Geom g, double *__restrict__ u, const double *__restrict__ p,
-                                             double *__restrict__ r, const double *__restrict__ w, Scalars *s,
-                                             double *part, unsigned *cnt) {
+// ---- flexible CG -----------------------------------------------------------
+// An iteration is k_pw<Z_FCG> (direction, w = A p and the previous step of u;
+// they were three passes of 112 B a cell, now one of 72), k_fr, the
+// preconditioner and k_fzw.
+// r -= alpha w, rr = r.r; stop when ||r|| < eps ||r0||.
+__global__ void __launch_bounds__(NT, kResident) k_fr(Geom g, double *__restrict__ r, const double *__restrict__ w,
+                                                      Scalars *s, double *part, unsigned *cnt) {
   __shared__ double sm[kWarps];
   __shared__ int last;
   if (s->done) return;
@@ -734,7 +722,6 @@ __global__ void __launch_bounds__(NT, kResident) k_fupd(Geom g, double *__restri
   double acc[1] = {0.0};
   HEAT_CELLS(g) {
     const long long i = (long long)y * g.pitch + x;
-    u[i] = u[i] + alpha * p[i];
     const double rv = r[i] - alpha * w[i];
     r[i] = rv;
     acc[0] = acc[0] + rv * rv;
@@ -775,17 +762,6 @@ __global__ void __launch_bounds__(NT, kResident) k_fzw(Geom g, const double *__r
       s->beta = -t / s->pw;
       *cnt = 0u;
     }
-  }
-}
-
-// p = z + beta p, or p = z on a restart.
-__global__ void __launch_bounds__(NT, kResident) k_fp(Geom g, double *__restrict__ p, const double *__restrict__ z,
-                                           const Scalars *s, int restart) {
-  if (!restart && s->done) return;  // the solve stopped earlier in a replayed chunk
-  const double beta = restart ? 0.0 : s->beta;
-  HEAT_CELLS(g) {
-    const long long i = (long long)y * g.pitch + x;
-    p[i] = restart ? z[i] : z[i] + beta * p[i];
   }
 }
 
@@ -1697,6 +1673,7 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
   const dim3 grid = grid_for(f.nx, f.ny), block(BX, BY);
   Scalars h = fresh(0.0);
   h.max_iters = max_iters;
+  h.restart = 1;
   OPSB_CUDA(cudaMemcpyAsync(m.s64, &h, sizeof(h), cudaMemcpyHostToDevice, st));
   k_resid<<<grid, block, 0, st>>>(g, f.Kx, f.Ky, f.u, f.u0, f.r, rx, ry, eps, m.s64, m.part, m.cnt);
   check_launch("fcg init");
@@ -1720,10 +1697,35 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
   bool done = h.done == 1 || r0 == 0.0;
   if (!done) {
     // the initial residual kernel leaves done = 0 and iters = 0
+    m.ensure_p64((size_t)f.pitch * f.ny);
     precond();
-    k_fp<<<grid, block, 0, st>>>(g, f.p, f.z, m.s64, 1);
-    launches_ += 1;
   }
+  double *const pb = m.p64b;
+  int rows = 1, blocks = 1;
+  pw_grid(f.nx, f.ny, kPwBlocks<double>, &rows, &blocks);
+  m.ensure_part(blocks);
+  auto step = [&] {
+    k_pw<double, Z_FCG><<<blocks, block, 0, st>>>(g, f.Kx, f.Ky, f.p, pb, f.z, f.r, f.u, f.w, rx, ry, rows, m.s64,
+                                                  m.part, m.cnt);
+    k_fr<<<grid, block, 0, st>>>(g, f.r, f.w, m.s64, m.part, m.cnt);
+    launches_ += 2;
+  };
+  auto beta = [&] {
+    k_fzw<<<grid, block, 0, st>>>(g, f.z, f.w, m.s64, m.part, m.cnt);
+    launches_ += 1;
+  };
+  auto flush = [&] {  // the pending u += alpha p
+    k_flush<double><<<grid, block, 0, st>>>(g, f.u, f.p, pb, f.r, f.Mi, nullptr, m.s64);
+    launches_ += 1;
+  };
+  // after a stop with done 4 or 5: u up to date, and the next direction z
+  auto restart_from = [&] {
+    flush();
+    const int set[3] = {0, 0, 1};  // done; pend, restart
+    OPSB_CUDA(cudaMemcpyAsync(&m.s64->done, set, sizeof(int), cudaMemcpyHostToDevice, st));
+    OPSB_CUDA(cudaMemcpyAsync(&m.s64->pend, set + 1, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
+    precond();
+  };
   bool host_loop = true;
   if (chunked && window < 64 && !done) {
     host_loop = false;
@@ -1744,13 +1746,9 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
           const long long before = launches_;
           graphs[which] = capture(st, [&] {
             for (int it = 0; it < kFcgChunk; it++) {
-              k_fw<<<grid, block, 0, st>>>(g, f.Kx, f.Ky, f.p, f.r, f.w, rx, ry, m.s64, m.part, m.cnt);
-              k_fupd<<<grid, block, 0, st>>>(g, f.u, f.p, f.r, f.w, m.s64, m.part, m.cnt);
-              launches_ += 2;
+              step();
               precond();
-              k_fzw<<<grid, block, 0, st>>>(g, f.z, f.w, m.s64, m.part, m.cnt);
-              k_fp<<<grid, block, 0, st>>>(g, f.p, f.z, m.s64, 0);
-              launches_ += 2;
+              beta();
             }
           });
           per_chunk[which] = launches_ - before;
@@ -1766,12 +1764,9 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
         // done 4 (lost curvature) or 5 (not halved over the window): restart
         if (learned) out->fallbacks++;
         learned = false;
-        const int zero3[3] = {0, 0, 0};  // done = 0; window = hcount = 0 (no restart test on the fallback)
-        OPSB_CUDA(cudaMemcpyAsync(&m.s64->done, zero3, sizeof(int), cudaMemcpyHostToDevice, st));
-        OPSB_CUDA(cudaMemcpyAsync(&m.s64->window, zero3 + 1, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
-        precond();
-        k_fp<<<grid, block, 0, st>>>(g, f.p, f.z, m.s64, 1);
-        launches_ += 1;
+        const int zero2[2] = {0, 0};  // window = hcount = 0 (no restart test on the fallback)
+        OPSB_CUDA(cudaMemcpyAsync(&m.s64->window, zero2, 2 * sizeof(int), cudaMemcpyHostToDevice, st));
+        restart_from();
       }
     } catch (...) {
       for (cudaGraphExec_t x : graphs)
@@ -1783,10 +1778,8 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
   }
   std::vector<double> hist;
   while (!done && host_loop) {
-    k_fw<<<grid, block, 0, st>>>(g, f.Kx, f.Ky, f.p, f.r, f.w, rx, ry, m.s64, m.part, m.cnt);
-    k_fupd<<<grid, block, 0, st>>>(g, f.u, f.p, f.r, f.w, m.s64, m.part, m.cnt);
+    step();
     check_launch("fcg iteration");
-    launches_ += 2;
     OPSB_CUDA(cudaMemcpyAsync(&h, m.s64, sizeof(h), cudaMemcpyDeviceToHost, st));
     OPSB_CUDA(cudaStreamSynchronize(st));
     if (h.done == 1 || h.done == 2) break;
@@ -1802,19 +1795,14 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
       if (learned) out->fallbacks++;
       learned = false;
       hist.clear();
-      int zero = 0;
-      OPSB_CUDA(cudaMemcpyAsync(&m.s64->done, &zero, sizeof(int), cudaMemcpyHostToDevice, st));
-      precond();
-      k_fp<<<grid, block, 0, st>>>(g, f.p, f.z, m.s64, 1);
-      launches_ += 1;
+      restart_from();
       continue;
     }
     precond();
-    k_fzw<<<grid, block, 0, st>>>(g, f.z, f.w, m.s64, m.part, m.cnt);
-    k_fp<<<grid, block, 0, st>>>(g, f.p, f.z, m.s64, 0);
+    beta();
     check_launch("fcg direction");
-    launches_ += 2;
   }
+  if (!done) flush();
   out->iterations = h.iters;
   out->converged = h.done == 1 || done;
   out->error = h.err;
