@@ -229,10 +229,22 @@ struct apply_stencil {
     // even pitch and an aligned dat origin; otherwise one column per thread
     const bool pairs = (lp.start[0] % 2) == 0 && (va.ay % 2) == 0 &&
                        (reinterpret_cast<uintptr_t>(va.ptr) % 16) == 0;
-    if (pairs)
-      launch_march2<256, 32, 4>(lp, s);  // 4.83 TB/s at 4096^2 (generic executor 3.93)
+    if (!pairs) {
+      launch_march<256, 32, 4>(lp, s);  // 4.20 TB/s
+      return;
+    }
+    // 32 rows a CTA stream best where the grid has the CTAs for it; a smaller
+    // one is latency-bound and takes the fewest rows that still run as one
+    // wave of four CTAs an SM (with its host round trip, an iteration takes
+    // 38.2 us instead of 40.2 at 1024^2 with 4 rows, 38.5 instead of 41.0 at
+    // 1500^2 with 8; at 2048^2 32 rows are the fastest)
+    const long long gx = std::max(1, (lp.end[0] - lp.start[0] + 511) / 512), ny = lp.end[1] - lp.start[1];
+    if (gx * ((ny + 3) / 4) <= 592)
+      launch_march2<256, 4, 4>(lp, s);
+    else if (gx * ((ny + 7) / 8) <= 592)
+      launch_march2<256, 8, 4>(lp, s);
     else
-      launch_march<256, 32, 4>(lp, s);   // 4.20 TB/s
+      launch_march2<256, 32, 4>(lp, s);  // 4.83 TB/s at 4096^2 (generic executor 3.93)
   }
 };
 

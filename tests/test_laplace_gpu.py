@@ -104,6 +104,36 @@ def test_python_api_path_matches_oracle(gpu_runtime, orc, graphs, fusion):
     assert np.array_equal(errs, eo)
 
 
+@pytest.mark.parametrize("x0", [-1, 0, 1])
+@pytest.mark.parametrize("nx", [0, 1, 2, 59, 60, 61, 120, 121])
+@pytest.mark.parametrize("ny", [1, 2, 9, 70])
+def test_sweep_on_part_of_a_dat(gpu_runtime, x0, nx, ny):
+    """The sweep at its strips' edges (60 columns) on aligned and odd starts,
+    up to the dat's last readable points: bit-exact, nothing else written."""
+    rng = np.random.default_rng(nx * 100 + ny + x0)
+    f = rng.standard_normal((ny + 2, nx + x0 + 3))
+    blk = O.ops_decl_block(2, "part")
+    size, m, p = [nx + x0 - 1, ny], [-2, -1], [2, 1]
+    if size[0] < 0:
+        pytest.skip("no such dat")
+    A = O.ops_decl_dat(blk, 1, size, [0, 0], m, p, f, "double", "A")
+    g = rng.standard_normal(f.shape)
+    An = O.ops_decl_dat(blk, 1, size, [0, 0], m, p, g, "double", "Anew")
+    S0 = O.ops_decl_stencil(2, 1, [0, 0], "0,0")
+    S5 = O.ops_decl_stencil(2, 5, [0, 0, 1, 0, -1, 0, 0, 1, 0, -1], "5pt")
+    h = O.ops_decl_reduction_handle(8, "double", "error")
+    O.ops_par_loop("laplace2d/apply_stencil", "apply", blk, 2, [x0, x0 + nx, 0, ny],
+                   O.ops_arg_dat(A, 1, S5, "double", O.OPS_READ), O.ops_arg_dat(An, 1, S0, "double", O.OPS_WRITE),
+                   O.ops_arg_reduce(h, 1, "double", O.OPS_MAX))
+    err = O.ops_reduction_result(h)
+    want, c = g.copy(), slice(1, 1 + ny)
+    lo, hi = x0 + 2, x0 + 2 + nx
+    want[c, lo:hi] = 0.25 * (((f[c, lo + 1:hi + 1] + f[c, lo - 1:hi - 1]) + f[:ny, lo:hi]) + f[2:, lo:hi])
+    assert np.array_equal(O.ops_dat_fetch_data(An), want)
+    if nx:
+        assert err == np.abs(want[c, lo:hi] - f[c, lo:hi]).max()
+
+
 def test_copy_elision_and_graphs_are_used(gpu_runtime):
     init = seeded.laplace_field(256, 256, 3)
     O.reset_counters()
