@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(kThreads, G::min_blocks) fused_chain_kernel(co
     v = block_reduce<double>(v, acc, red_smem);
     if (threadIdx.x == 0) {
       double *slot = reinterpret_cast<double *>(P->red[r].slot);
-      *slot = P->red[r].first ? v : red_combine(acc, *slot, v);
+      put_reduction(slot, P->red[r].first ? v : red_combine(acc, *slot, v), P->red_mirror);
     }
   }
   if (threadIdx.x == 0) *P->red_counter = 0u;

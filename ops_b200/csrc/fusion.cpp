@@ -533,6 +533,7 @@ class FusionPlanner {
       }
     }
     P.red_scratch = rt.red_scratch_;
+    P.red_mirror = rt.red_mirror_;
     validate(A, P, buf_of);
   }
 

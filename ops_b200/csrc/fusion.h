@@ -95,6 +95,7 @@ struct FPlan {
   int smem_doubles;        // dynamic shared memory (guards included)
   char *red_scratch;
   unsigned int *red_counter;
+  long long red_mirror;    // as LoopParams'
   FRed red[kMaxRed];
   FLoop L[kMaxLoops];
   FBuf B[kMaxBufs];

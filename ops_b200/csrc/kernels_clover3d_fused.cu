@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(32 * kWarps, 5) summary_kernel(const __grid_co
 
 struct ideal_gas_summary {
   C3_LOOP(ideal_gas_summary);
+  static constexpr bool red_mirror = true;
   __device__ void operator()(const D &density0, const D &energy0, D &pressure, D &soundspeed, const D &volume,
                              const D &xvel0, const D &yvel0, const D &zvel0, RED<double> &vol, RED<double> &mass,
                              RED<double> &ie, RED<double> &ke, RED<double> &press) const;

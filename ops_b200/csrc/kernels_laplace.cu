@@ -212,6 +212,7 @@ void launch_march(const LoopParams &lp, cudaStream_t s) {
 
 struct apply_stencil {
   static constexpr const char *kname = "laplace2d/apply_stencil";
+  static constexpr bool red_mirror = true;
   __device__ void operator()(const ACC2<double> &A, ACC2<double> &Anew, RED<double> &error) const {
     Anew(0, 0) = 0.25f * (A(1, 0) + A(-1, 0) + A(0, -1) + A(0, 1));
     *error = fmax(*error, fabs(Anew(0, 0) - A(0, 0)));

@@ -135,7 +135,18 @@ struct LoopParams {
   char *red_scratch;  // per-block partials: [red_index][block][OPSB_MAX_RED_DIM] x 8 bytes
   unsigned int *red_counter;  // blocks-done counter, reset to 0 by the last block
   ArgView a[OPSB_MAX_ARGS];
+  long long red_mirror;  // bytes from a reduction's slot to its copy in pinned host memory
 };
+
+// The one thread that finishes a reduction also writes the value to the host:
+// the result is there when the stream is, without a copy of its own behind the
+// kernel (an iteration of Laplace at 96 x 64, whose host reads each result,
+// takes 30 us instead of 40).
+template <class T>
+__device__ __forceinline__ void put_reduction(T *slot, T v, long long mirror) {
+  *slot = v;
+  *reinterpret_cast<volatile T *>(reinterpret_cast<char *>(slot) + mirror) = v;
+}
 
 // ----------------------------------------------------------------------------
 // Reduction identities and combine, by element type and access mode
@@ -284,7 +295,7 @@ __device__ void finish_grid_reduction(const ArgView &a, const LoopParams &lp, in
     T v = red_identity<T>(a.acc);
     for (int b = tid; b < nblocks; b += nthr) v = red_combine(a.acc, v, part[(size_t)b * OPSB_MAX_RED_DIM + d]);
     v = block_reduce<T>(v, a.acc, smem);
-    if (tid == 0) slot[d] = a.first ? v : red_combine(a.acc, slot[d], v);
+    if (tid == 0) put_reduction(slot + d, a.first ? v : red_combine(a.acc, slot[d], v), lp.red_mirror);
   }
 }
 

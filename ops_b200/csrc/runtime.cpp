@@ -121,7 +121,10 @@ void Runtime::init(int device, int diags) {
   OPSB_CUDA(cudaMemset(red_counters_, 0, kNumCounters * sizeof(unsigned int)));
   OPSB_CUDA(cudaMalloc(&red_arena_, kRedArenaBytes));
   OPSB_CUDA(cudaMemset(red_arena_, 0, kRedArenaBytes));
-  OPSB_CUDA(cudaMallocHost(&red_host_, kRedArenaBytes));
+  OPSB_CUDA(cudaHostAlloc(&red_host_, kRedArenaBytes, cudaHostAllocMapped));
+  void *mapped = nullptr;
+  OPSB_CUDA(cudaHostGetDevicePointer(&mapped, red_host_, 0));
+  red_mirror_ = (long long)((intptr_t)mapped - (intptr_t)red_arena_);
   const char *g = getenv("OPS_B200_GRAPHS");
   if (g) graphs_on_ = atoi(g);
   const char *f = getenv("OPS_B200_FUSION");
@@ -561,6 +564,7 @@ void Runtime::build_params(const Desc &d, LoopParams &lp, int *nred_out) {
   }
   lp.nred = nred;
   lp.red_scratch = red_scratch_;
+  lp.red_mirror = red_mirror_;
   lp.red_counter = red_counters_;
   if (nred_out) *nred_out = nred;
 }
@@ -895,7 +899,10 @@ void Runtime::add_fusion_stats(const FusionStats &s) {
 }
 
 void Runtime::run_queue(std::vector<Desc> &q) {
-  red_dirty_ = true;
+  red_pending_ = true;
+  for (const Desc &d : q)
+    if (!d.loop->red_mirror && !d.loop->internal)
+      for (const Arg &a : d.args) red_dirty_ |= a.kind == ARG_REDUCE;
   elide_copies(q);
   // OPSB_TRACE_QUEUE=1: every flushed loop to stderr (kernel, range, per dat
   // arg: name, access, stencil points), for analysing loop chains
@@ -998,9 +1005,9 @@ void Runtime::reduction_result(int handle, void *out) {
     const Reduction &last = reductions_.back();
     const size_t used = (size_t)(last.slot_d - red_arena_) + (size_t)last.size;
     OPSB_CUDA(cudaMemcpyAsync(red_host_, red_arena_, used, cudaMemcpyDeviceToHost, stream_));
-    OPSB_CUDA(cudaStreamSynchronize(stream_));
-    red_dirty_ = false;
   }
+  if (red_dirty_ || red_pending_) OPSB_CUDA(cudaStreamSynchronize(stream_));
+  red_dirty_ = red_pending_ = false;
   memcpy(out, red_host_ + (r.slot_d - red_arena_), r.size);
   if (partitioned_ && nranks() > 1) combine_reduction(r, out);
   r.initialized = 0;  // ops_reduction_result_char resets the handle (ops_lib_core.cpp:1143)

@@ -112,6 +112,7 @@ struct LoopInfo {
   int copy_dst = -1, copy_src = -1;  // pure copy kernels: which args are dst/src
   int internal = 0;         // runtime-internal item (not launched through exec_loop)
   int mgrid_ok = 0;         // the kernel maps multigrid (restrict/prolong) stencils
+  int red_mirror = 0;       // its reductions end in put_reduction: the host has the values too
   void (*launch)(const LoopParams &, dim3, dim3, cudaStream_t) = nullptr;
   // several loops of this kernel in one launch (exec_loop_list); null for
   // kernels with their own launch
@@ -384,7 +385,10 @@ class Runtime {
   // there until loops run again.
   char *red_arena_ = nullptr;
   char *red_host_ = nullptr;
-  bool red_dirty_ = true;
+  // What a result still needs: the arena copied to the host (red_dirty_), or
+  // only the stream waited for, its kernels having written the host's copy too.
+  bool red_dirty_ = true, red_pending_ = true;
+  long long red_mirror_ = 0;  // from the arena to the host's copy as a kernel addresses it
 
   struct GraphEntry {
     int seen = 0;
@@ -537,6 +541,11 @@ struct CopyTrait { static constexpr int dst = -1, src = -1; };
 template <class K>
 struct CopyTrait<K, std::void_t<decltype(K::copy_dst)>> { static constexpr int dst = K::copy_dst, src = K::copy_src; };
 
+template <class K, class = void>
+struct RedMirror { static constexpr bool value = false; };
+template <class K>
+struct RedMirror<K, std::void_t<decltype(K::red_mirror)>> { static constexpr bool value = K::red_mirror; };
+
 template <class K>
 LoopInfo make_loop_info(const char *kernel) {
   LoopInfo li;
@@ -556,6 +565,9 @@ LoopInfo make_loop_info(const char *kernel) {
     li.launch_list = &launch_exec_list<K>;
   }
   li.mgrid_ok = LoopMgridOk<K>::value ? 1 : 0;
+  // a kernel with its own launch states `red_mirror` when it finishes its
+  // reductions with finish_grid_reduction, as the generic executor does
+  li.red_mirror = RedMirror<K>::value || !CustomLaunch<K>::value ? 1 : 0;
   return li;
 }
 
