@@ -290,18 +290,18 @@ CL_N = 3840
 # DRAM bytes per cell of one launch of a workload's dominant kernel, from one
 # ncu capture each (dram__bytes_read.sum + dram__bytes_write.sum; the
 # captures are summarised in profiles/, which names the command):
-#   CloverLeaf 2D PdV_kernel_nopredict at 2560^2: 89.3 + 21.0 B
-#     (profiles/cloverleaf2d_2560_dram_per_kernel.md)
-#   CloverLeaf 3D PdV_kernel_nopredict at 160^3: 141.4 + 22.6 B
-#     (profiles/cloverleaf3d_160_pdv_accelerate.md)
+#   CloverLeaf 2D lagrange at 2560^2: 73.7 + 42.3 B
+#     (profiles/fused_loops_dram.md)
+#   CloverLeaf 3D PdV_flux at 160^3: 131.6 + 37.5 B
+#     (profiles/fused_loops_dram.md)
 #   Laplace apply_stencil at 4096^2: 227.4 MB per launch / 4096^2
 #     (profiles/laplace2d_4096_apply_stencil_dram.md)
-#   ADI 256^3 FP64 x / y / z sweeps: 650.1 / 1144.0 / 1283.4 MB per sweep / 256^3
-#     (profiles/adi_cube_256_fp64_dram.md)
+#   ADI 256^3 FP64 x / y / z sweeps: 649.6 / 765.5 / 909.6 MB per sweep / 256^3
+#     (profiles/fused_loops_dram.md)
 # Traffic grows with the cells (or unknowns) a launch processes, so a
 # launch's traffic is the figure times its cells.
-TRAFFIC_PER_CELL = {"clover": 110.3, "clover3d": 164.0, "laplace": 227.4e6 / 4096 ** 2,
-                    "adi_cube_fp64": (650.1e6 / 256 ** 3, 1144.0e6 / 256 ** 3, 1283.4e6 / 256 ** 3)}
+TRAFFIC_PER_CELL = {"clover": 116.0, "clover3d": 169.1, "laplace": 227.4e6 / 4096 ** 2,
+                    "adi_cube_fp64": (649.6e6 / 256 ** 3, 765.5e6 / 256 ** 3, 909.6e6 / 256 ** 3)}
 
 
 def clover_deck(steps, n=CL_N):
@@ -349,9 +349,8 @@ def bench_clover(args, world, rank, local, pg):
     cells = N * N
     K, W = args.steps, args.warmup
 
-    # Untimed: the fused chains' tile shapes are tuned on their first
-    # executions (both sweep orders) and kept in the tuning cache file, which
-    # the timed call reads.
+    # Untimed: first executions (modules, storage; the tile shapes of any
+    # chain the queue's fuser takes, kept in its cache file).
     apps.cloverleaf(clover_deck(24, N))
     barrier(pg, local)
     O.reset_counters()
@@ -405,9 +404,9 @@ def bench_clover(args, world, rank, local, pg):
                    "l2": "inputs larger than L2 (about 30 fields of 118 MB)", "parallelism": f"replicas x{world}"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": TRAFFIC_PER_CELL["clover"] * cells
-                     if dom == "cloverleaf/PdV_kernel_nopredict" else None,
-                     "traffic_source": "ncu capture of PdV_kernel_nopredict at 2560^2, per cell x cells"
-                                       " (profiles/cloverleaf2d_2560_dram_per_kernel.md)", "kernel": dom,
+                     if dom == "cloverleaf/lagrange" else None,
+                     "traffic_source": "ncu capture of lagrange at 2560^2, per cell x cells"
+                                       " (profiles/fused_loops_dram.md)", "kernel": dom,
                      "alg_bytes_per_launch": by / n, "avg_launch_ms": ms / n, "peak_source": f"{peak_kind} hbm_gbs",
                      "step_effective_gbs": tot_by / (tot_ms * 1e-3) / 1e9,
                      "step_alg_bytes_per_cell": tot_by / kp / cells},
@@ -569,9 +568,9 @@ def bench_clover3d(args, world, rank, local, pg):
                    "l2": "inputs larger than L2 (about 40 fields of 140 MB)", "parallelism": f"replicas x{world}"},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": TRAFFIC_PER_CELL["clover3d"] * cells
-                     if dom == "cloverleaf3d/PdV_kernel_nopredict" else None,
-                     "traffic_source": "ncu capture of PdV_kernel_nopredict at 160^3, per cell x cells"
-                                       " (profiles/cloverleaf3d_160_pdv_accelerate.md)", "kernel": dom,
+                     if dom == "cloverleaf3d/PdV_flux" else None,
+                     "traffic_source": "ncu capture of PdV_flux at 160^3, per cell x cells"
+                                       " (profiles/fused_loops_dram.md)", "kernel": dom,
                      "alg_bytes_per_launch": by / n, "avg_launch_ms": ms / n, "peak_source": f"{peak_kind} hbm_gbs",
                      "step_effective_gbs": tot_by / (tot_ms * 1e-3) / 1e9,
                      "step_alg_bytes_per_cell": tot_by / kp / cells},
@@ -756,7 +755,7 @@ def bench_adi(args, world, rank, local, pg):
                      "traffic": TRAFFIC_PER_CELL["adi_cube_fp64"][dom] * unknowns
                      if name == "adi_cube_fp64" else None,
                      "traffic_source": "ncu capture of one x, y and z sweep at 256^3 FP64"
-                                       " (profiles/adi_cube_256_fp64_dram.md); other cases not captured",
+                                       " (profiles/fused_loops_dram.md); other cases not captured",
                      "sweep_ms": sweep_ms, "alg_bytes_per_unknown": byt, "peak_source": f"{peak_kind} hbm_gbs"},
         "e2e": {"value": (total_unknowns if shard else world * unknowns) * 3 / e2e_s, "unit": "unknowns solved/s",
                 "h2d_bytes_per_step": h2d,
@@ -837,8 +836,8 @@ def reference_adi(args, world, rank):
 # Implicit heat conduction (TeaLeaf CG, jac_diag), 4096^2, eps 1e-10
 # ---------------------------------------------------------------------------
 TEA_N = 4096
-TEA_BYTES_FP64 = 120.0   # per cell-iteration: k_w 32 + k_ur 64 + k_p 24 (FP64 words)
-TEA_BYTES_FP32 = 60.0
+TEA_BYTES_FP64 = 96.0   # per cell-iteration: k_pw 64 (r, p, u, Kx, Ky in; p, w, u out) + k_r 32 (r, w, Mi in; r out)
+TEA_BYTES_FP32 = 52.0   # the same in FP32 words, with Mi in k_pw too
 
 
 def tea_deck(steps, n=TEA_N, max_iters=200000, **kw):
@@ -924,7 +923,7 @@ def bench_tea(args, world, rank, local, pg):
     t_mixed = max_over_ranks(pg, float(np.median(sm[:, 6])), local)
     it_p = float(np.mean(sp[:, 0]))
     it_m = float(np.mean(sm[:, 0]))
-    # roofline of the dominant chain: the FP32 inner iteration (k_w + k_ur + k_p)
+    # roofline of the dominant chain: the FP32 inner iteration (k_pw + k_r)
     per_it_m = t_mixed / max(it_m, 1.0)
     per_it_p = t_plain / max(it_p, 1.0)
     ach_m = TEA_BYTES_FP32 * cells / per_it_m / 1e9
@@ -956,7 +955,7 @@ def bench_tea(args, world, rank, local, pg):
                    "reliable_delta": args.reliable_delta, "parallelism": f"replicas x{world}"},
         "roofline": {"bound": "hbm", "achieved": ach_m, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": ach_m / peaks["hbm_gbs"], "traffic": None,
-                     "kernel": "FP32 inner PCG iteration (k_w + k_ur + k_p)",
+                     "kernel": "FP32 inner PCG iteration (k_pw + k_r_flat)",
                      "alg_bytes_per_cell_iteration": TEA_BYTES_FP32, "avg_iteration_ms": per_it_m * 1e3,
                      "peak_source": f"{peak_kind} hbm_gbs",
                      "fp64_iteration": {"achieved": ach_p, "frac": ach_p / peaks["hbm_gbs"],
@@ -1251,11 +1250,10 @@ def bench_mg(args, world, rank, local, pg):
     t_plain = max_over_ranks(pg, float(np.median([s["seconds"] for s in plain])), local)
     it = mg[0]["iterations"]
     # algorithmic bytes of one iteration, per cell: the FP64 flexible-CG
-    # kernels (w = A p with p.w, p.r: Kx Ky p r w 40; u, r update: 48; z.w: 16;
-    # p = z + beta p: 24) and the FP32 V-cycle's fine level (106: r in FP64 and
-    # its FP32 copy, five streaming passes, z out in FP64) plus its coarse
-    # levels (a third of the fine level's 5 x 20 bytes in FP32)
-    per_cell = 128 + 106 + 100 / 3
+    # kernels (p, w = A p and u: 72; r: 24; z.w: 16) and the FP32 V-cycle's
+    # fine level (21 down and 29 up, r and z in FP64) plus its coarse levels (a
+    # third of 46)
+    per_cell = 112 + 50 + 46 / 3
     alg = per_cell * N * N * it
     ach = alg / t_mg / 1e9
 
@@ -1321,10 +1319,11 @@ def bench_mg(args, world, rank, local, pg):
 # 3D heat solve: the 7-point operator at 512^3, FP64 Jacobi-PCG to 1e-10
 # ---------------------------------------------------------------------------
 H3_N = 512
-HEAT3D_BYTES = 128.0  # FP64 per cell-iteration: w = A p (p, Kx, Ky, Kz, w: 40) + u, r, z updates (64) + p (24)
-# DRAM bytes per cell of one iteration (k_w3 + k_ur + k_p) from one ncu capture
-# at 256^3 (profiles/heat3d_256_pcg_iteration_dram.md); they scale with the cells
-HEAT3D_TRAFFIC = 124.8
+# FP64 per cell-iteration: k_pw3 80 (r, Mi, p, u, Kx, Ky, Kz in; p, w, u out) + k_r_flat 32 (r, w, Mi in; r out)
+HEAT3D_BYTES = 112.0
+# DRAM bytes per cell of one iteration from one ncu capture at 256^3
+# (profiles/fused_loops_dram.md); they scale with the cells
+HEAT3D_TRAFFIC = 110.8
 
 
 def heat3d_problem(n, seed, local):
@@ -1419,8 +1418,8 @@ def bench_heat3d(args, world, rank, local, pg):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                      "frac": achieved / peaks["hbm_gbs"], "traffic": HEAT3D_TRAFFIC * cells,
                      "traffic_source": "ncu capture of one iteration at 256^3, per cell x cells"
-                                       " (profiles/heat3d_256_pcg_iteration_dram.md)",
-                     "kernel": "PCG iteration (k_w3 + k_ur + k_p)", "alg_bytes_per_cell_iteration": HEAT3D_BYTES,
+                                       " (profiles/fused_loops_dram.md)",
+                     "kernel": "PCG iteration (k_pw3 + k_r_flat)", "alg_bytes_per_cell_iteration": HEAT3D_BYTES,
                      "avg_iteration_ms": t * 1e3 / max(iters, 1), "peak_source": f"{peak_kind} hbm_gbs"},
         "e2e": {"value": e2e_s, "unit": "s", "h2d_bytes_per_step": sum(h.numel() * 8 for h in hk),
                 "d2h_bytes_per_step": hu.numel() * 8},
