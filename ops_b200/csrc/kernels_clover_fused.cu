@@ -6,9 +6,9 @@
 // 1595 B per cell and step in 43 launches. None of those outlive the step, so
 // each kernel here computes them in registers and moves only the fields that
 // the next kernel needs: 608 B per cell and step in 9 launches plus the
-// boundary copies. Measured at 3840^2: 4.9 -> 2.44 ms of kernels a step, a
-// whole 10-step run 59.1 -> 30.6 ms (250 x 187: 14.1 -> 7.5 ms, half the
-// launches and no chain planning). Every value is computed by the reference's expressions in
+// boundary copies. Measured at 3840^2: 4.9 -> 2.37 ms of kernels a step, a
+// whole 10-step run 58.5 -> 26.1 ms (250 x 187: 14.1 -> 3.5 ms, half the
+// launches, and a queue the planner passes over). Every value is computed by the reference's expressions in
 // the reference's order (clover_flux.cuh, --fmad=false), so fields and dt are
 // the same bits.
 //
