@@ -388,12 +388,16 @@ __global__ void k_out_bwd(Fields f, const double *s, const double *E, const floa
 
 // Weight gradients of the 3x3 layers: dW[tap][co][ci] = sum_p g[p][co] x[p + tap][ci]
 // (x zero outside the image), db[co] = sum_p g[p][co]. All layers run in one
-// launch, a CTA per layer, share of the pixel tiles and row of three taps; it
-// sums its tiles in order and leaves partial[share][...] in W layout. A thread
-// holds RO x RI outputs of each of the three taps, so a pixel's values are
-// loaded and converted once for 3 RO RI products (one CTA a tap, one output a
-// thread at a time and a launch a layer before: 343 us of a 16 x 64^2 step, now
-// 140 us). Every output is still one chain over the pixels in the same order.
+// launch, a CTA per layer and share of the pixel tiles (and row of three taps
+// where the layer has 2048 weights a tap or more); it sums its tiles in order
+// and leaves partial[share][...] in W layout. A thread holds RO x RI outputs of
+// three taps, so a pixel's values are loaded (one word each way) and converted
+// once for 3 RO RI products; a small layer's three rows of taps go to three
+// groups of 64 threads of one CTA for that, and its bias to the fourth. Bound
+// by issue: a product is a multiplication and an addition. (One CTA a tap, one
+// output a thread at a time and a launch a layer: 343 us of a 16 x 64^2 step;
+// all layers in one launch with rows of taps in CTAs of their own 140 us; now
+// 123 us.) Every output is still one chain over the pixels in the same order.
 struct WgLayer {
   const bf16 *x, *g;
   float *partial;  // this layer's shares
@@ -408,16 +412,46 @@ struct WgPlan {
   int oparts;
 };
 
+// bf16 pairs of a word, exactly.
+template <int N>
+__device__ __forceinline__ void unpack(const bf16 *p, float (&o)[N]) {
+  unsigned u[(N + 1) / 2];
+  if constexpr (N == 1) {
+    o[0] = __bfloat162float(*p);
+    return;
+  } else if constexpr (N == 2) {
+    u[0] = *reinterpret_cast<const unsigned *>(p);
+  } else {
+    static_assert(N == 4, "one, two or four values");
+    const uint2 v = *reinterpret_cast<const uint2 *>(p);
+    u[0] = v.x;
+    u[1] = v.y;
+  }
+#pragma unroll
+  for (int k = 0; k < N / 2; k++) {
+    o[2 * k] = __uint_as_float(u[k] << 16);
+    o[2 * k + 1] = __uint_as_float(u[k] & 0xffff0000u);
+  }
+}
+
+// Rows of taps that one CTA takes: all three where 64 threads hold a row's.
+constexpr int wg_rows(int cin, int cout) { return cin * cout <= 1024 ? 3 : 1; }
+
 template <int CIN, int COUT>
-__device__ __forceinline__ void wgrad_share(const WgLayer &L, int share, int dyi, uint4 *smem) {
-  constexpr int NO = CIN * COUT, PER = NO / kT > 0 ? NO / kT : 1;
-  constexpr int RI = PER >= 4 ? 4 : PER >= 2 ? 2 : 1, RO = PER / RI;  // outputs a thread: RO co x RI ci
-  static_assert(NO >= kT && RO * RI == PER, "wgrad tiling");
-  constexpr int XW = 18;  // 16 pixels and a column either side
+__device__ __forceinline__ void wgrad_share(const WgLayer &L, int b, uint4 *smem) {
+  constexpr int ROWS = wg_rows(CIN, COUT), THR = ROWS == 3 ? 64 : kT;
+  constexpr int NO = CIN * COUT, PER = NO / THR;
+  constexpr int RI = PER >= 8 ? 4 : 2, RO = PER / RI;  // outputs a thread: RO co x RI ci
+  static_assert(NO % THR == 0 && RO * RI == PER && RO >= 1 && RO <= 4, "wgrad tiling");
+  constexpr int XW = 18, XH = ROWS == 3 ? 10 : 8;  // 16 pixels and a column either side; a row either side too
   bf16 *gs = reinterpret_cast<bf16 *>(smem), *xs = gs + kWgTile * COUT;
-  const int h = L.h, w = L.w, dy = dyi - 1;
+  const int share = ROWS == 3 ? b : b / 3, group = ROWS == 3 ? threadIdx.x / 64 : 0;
+  const int dyi = ROWS == 3 ? group : b % 3;   // row of taps; group 3 takes the bias
+  const int row0 = ROWS == 3 ? -1 : dyi - 1;   // x's first row in the tile, from the tile's
+  const int h = L.h, w = L.w;
   const int tx = (w + 15) / 16, ty = (h + 7) / 8;
-  const int ci0 = (threadIdx.x % (CIN / RI)) * RI, co0 = (threadIdx.x / (CIN / RI)) * RO;
+  const int q = threadIdx.x % THR, ci0 = (q % (CIN / RI)) * RI, co0 = (q / (CIN / RI)) * RO;
+  const bool bias = ROWS == 3 ? group == 3 && q < COUT : dyi == 0 && q < COUT;
   float acc[3][RO][RI] = {}, bacc = 0.0f;
   for (int t = share; t < L.tiles; t += L.shares) {
     const int img = t / (tx * ty), rem = t - img * tx * ty;
@@ -431,70 +465,69 @@ __device__ __forceinline__ void wgrad_share(const WgLayer &L, int share, int dyi
         val = *reinterpret_cast<const uint4 *>(L.g + (((long long)img * h + y) * w + xx) * COUT + cg * 8);
       *reinterpret_cast<uint4 *>(gs + p * COUT + cg * 8) = val;
     }
-    for (int v = threadIdx.x; v < 8 * XW * (CIN / 8); v += kT) {
+    for (int v = threadIdx.x; v < XH * XW * (CIN / 8); v += kT) {
       const int p = v / (CIN / 8), cg = v % (CIN / 8);
-      const int y = y0 + p / XW + dy, xx = x0 + p % XW - 1;
+      const int y = y0 + p / XW + row0, xx = x0 + p % XW - 1;
       uint4 val = make_uint4(0, 0, 0, 0);
       if (y >= 0 && y < h && xx >= 0 && xx < w)
         val = *reinterpret_cast<const uint4 *>(L.x + (((long long)img * h + y) * w + xx) * CIN + cg * 8);
       *reinterpret_cast<uint4 *>(xs + p * CIN + cg * 8) = val;
     }
     __syncthreads();
-    for (int r = 0; r < 8; r++) {
-      const bf16 *gr = gs + r * 16 * COUT + co0, *xr = xs + r * XW * CIN + ci0;
-      float x[3][RI];  // the columns left of, at and right of the pixel
-      auto ldx = [&](int c, float (&o)[RI]) {
-#pragma unroll
-        for (int k = 0; k < RI; k++) o[k] = __bfloat162float(xr[c * CIN + k]);
-      };
-      ldx(0, x[0]);
-      ldx(1, x[1]);
+    if (group < 3) {
+      for (int r = 0; r < 8; r++) {
+        const bf16 *gr = gs + r * 16 * COUT + co0, *xr = xs + (r + (ROWS == 3 ? dyi : 0)) * XW * CIN + ci0;
+        float x[3][RI];  // the columns left of, at and right of the pixel
+        unpack<RI>(xr, x[0]);
+        unpack<RI>(xr + CIN, x[1]);
 #pragma unroll 4
-      for (int p = 0; p < 16; p++) {
-        ldx(p + 2, x[2]);
-        float g[RO];
+        for (int p = 0; p < 16; p++) {
+          unpack<RI>(xr + (p + 2) * CIN, x[2]);
+          float g[RO];
+          unpack<RO>(gr + p * COUT, g);
 #pragma unroll
-        for (int o = 0; o < RO; o++) g[o] = __bfloat162float(gr[p * COUT + o]);
+          for (int d = 0; d < 3; d++)
 #pragma unroll
-        for (int d = 0; d < 3; d++)
+            for (int o = 0; o < RO; o++)
 #pragma unroll
-          for (int o = 0; o < RO; o++)
+              for (int k = 0; k < RI; k++) acc[d][o][k] += g[o] * x[d][k];
 #pragma unroll
-            for (int k = 0; k < RI; k++) acc[d][o][k] += g[o] * x[d][k];
-#pragma unroll
-        for (int k = 0; k < RI; k++) {
-          x[0][k] = x[1][k];
-          x[1][k] = x[2][k];
+          for (int k = 0; k < RI; k++) {
+            x[0][k] = x[1][k];
+            x[1][k] = x[2][k];
+          }
         }
       }
     }
-    if (dyi == 0 && threadIdx.x < COUT)
-      for (int p = 0; p < kWgTile; p++) bacc += __bfloat162float(gs[p * COUT + threadIdx.x]);
+    if (bias)
+#pragma unroll 8
+      for (int p = 0; p < kWgTile; p++) bacc += __bfloat162float(gs[p * COUT + q]);
   }
   float *out = L.partial + (size_t)share * L.len;
+  if (group < 3)
 #pragma unroll
-  for (int d = 0; d < 3; d++)
+    for (int d = 0; d < 3; d++)
 #pragma unroll
-    for (int o = 0; o < RO; o++)
+      for (int o = 0; o < RO; o++)
 #pragma unroll
-      for (int k = 0; k < RI; k++) out[(dyi * 3 + d) * NO + (co0 + o) * CIN + ci0 + k] = acc[d][o][k];
-  if (dyi == 0 && threadIdx.x < COUT) out[9 * NO + threadIdx.x] = bacc;
+        for (int k = 0; k < RI; k++) out[(dyi * 3 + d) * NO + (co0 + o) * CIN + ci0 + k] = acc[d][o][k];
+  if (bias) out[9 * NO + q] = bacc;
 }
 
 __global__ void __launch_bounds__(kT) k_wgrad(const __grid_constant__ WgPlan P) {
-  __shared__ uint4 smem[(kWgTile * 64 + 8 * 18 * 64) / 8];
+  __shared__ uint4 smem[(kWgTile * 64 + 8 * 18 * 64) / 8];  // 64 to 64 channels; the small layers' rows fit it
   int l = 0;
   while (l + 1 < kLayers && (int)blockIdx.x >= P.l[l + 1].first) l++;
   const WgLayer &L = P.l[l];
-  const int b = blockIdx.x - L.first, share = b / 3, dyi = b % 3;
+  const int b = blockIdx.x - L.first;
   switch (l) {
-    case C0: case C0U: wgrad_share<16, 16>(L, share, dyi, smem); break;
-    case C1A: wgrad_share<16, 32>(L, share, dyi, smem); break;
-    case C1B: wgrad_share<32, 32>(L, share, dyi, smem); break;
-    case C2A: wgrad_share<32, 64>(L, share, dyi, smem); break;
-    case C2U: wgrad_share<64, 32>(L, share, dyi, smem); break;
-    case C1U: wgrad_share<32, 16>(L, share, dyi, smem); break;
-    default: wgrad_share<64, 64>(L, share, dyi, smem); break;
+    case C0: case C0U: wgrad_share<16, 16>(L, b, smem); break;
+    case C1A: wgrad_share<16, 32>(L, b, smem); break;
+    case C1B: wgrad_share<32, 32>(L, b, smem); break;
+    case C2A: wgrad_share<32, 64>(L, b, smem); break;
+    case C2U: wgrad_share<64, 32>(L, b, smem); break;
+    case C1U: wgrad_share<32, 16>(L, b, smem); break;
+    default: wgrad_share<64, 64>(L, b, smem); break;
   }
 }
 
@@ -827,7 +860,7 @@ double Net::loss_and_grad(const Fields &f, const double *e, int kind, cudaStream
     L.shares = wg_shares(l, n, h, w);
     L.len = wg_len(l);
     L.first = ctas;
-    ctas += 3 * L.shares;
+    ctas += wg_rows(kDefs[l].cin, kDefs[l].cout) == 3 ? L.shares : 3 * L.shares;
     part += (size_t)L.shares * L.len;
   }
   P.opart = m.opart;
