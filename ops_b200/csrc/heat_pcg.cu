@@ -57,7 +57,7 @@ struct Scalars {
   double hist[64];
 };
 
-// Stopping quantity of k_ur.
+// Stopping quantity of k_r.
 enum { STOP_TEALEAF = 0,  // sqrt|r.z| < eps ||r0|| (tea_solve.cpp:349-355)
        STOP_TRUE = 1,     // ||r|| < eps ||r0||
        STOP_RELIABLE = 2  // inner FP32 loop: estimate test, or a decade of decrease since the last update
