@@ -451,7 +451,11 @@ typedef struct ops_b200_trid_system {
  * one launch (elem_size 8 = double, 4 = float) on `stream` (cudaStream_t,
  * NULL = default stream). Lines along x (contiguous) run the partition
  * method in shared memory, up to 512 points; lines along y/z (strided,
- * neighbouring lines contiguous) run Thomas per line, any length, with a
+ * neighbouring lines contiguous) are eliminated from both ends at once, any
+ * length; a line whose elimination from the last row meets small pivots is
+ * solved by Thomas from the first row. Neither exchanges rows: the y/z sweeps
+ * need pivots from the first row on, the x sweeps in each chunk of 4 to 8 rows
+ * too (diagonally dominant lines have them all). The y/z sweeps use a
  * c'/d' scratch array of 2 x (unknowns) elements that the library keeps and
  * grows. The work lists and that scratch are shared by all calls: calls on
  * different streams must not overlap. */

@@ -563,6 +563,10 @@ __device__ __forceinline__ void st_hint(float *p, float v, uint64_t pol) {
   asm volatile("st.global.L2::cache_hint.f32 [%0], %1, %2;" ::"l"(p), "f"(v), "l"(pol) : "memory");
 }
 
+// The size of a value as an integer that orders like it: NaN above infinity.
+__device__ __forceinline__ int magnitude(double x) { return __double2hiint(x) & 0x7fffffff; }
+__device__ __forceinline__ int magnitude(float x) { return __float_as_int(x) & 0x7fffffff; }
+
 // Lines strided along the solve dimension and contiguous across lines (the y
 // and z sweeps). A warp solves 16 neighbouring lines, two lanes each: one
 // eliminates from the top, its partner (lane + 16) from the bottom with a and c
@@ -573,6 +577,14 @@ __device__ __forceinline__ void st_hint(float *p, float v, uint64_t pol) {
 // cp.async into the thread's own column of a ring of kLineStages stages of
 // kLineRows rows (no barrier: nobody else reads it); the backward pass reads
 // c' and d' kLineRows rows ahead into registers.
+//
+// A line may have pivots from the top only (b_{n-1} = 0, say). While |c'| stays
+// within kGrowth a pivot's rounding error is that of its row's entries, so the
+// elimination from the bottom is as sound as the rows are; a line whose c' pass
+// it (a vanished pivot leaves infinity or NaN) is solved again from the top
+// alone, a lane a line, in the two lanes' scratch. Diagonally dominant rows
+// have |c'| <= 1.
+constexpr float kGrowth = 16.0f;
 constexpr int kLineThreads = 128, kLineRows = 8, kLineStages = 3;
 
 template <class T>
@@ -627,12 +639,15 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
     // the chain from row to row is one product and the reciprocal:
     // b_i - a_i c'_{i-1} = b_i - (a_i c_{i-1}) r_{i-1}
     T rc = T(0), lc = T(0), pd = T(0);
+    int worst = 0;  // the largest |c'|
     T *q = cp;
     auto eliminate = [&](T ai, T bi, T ci, T di) {
       rc = recip(bi - (ai * lc) * rc);
       lc = ci;
       pd = (di - ai * pd) * rc;
-      st_hint(q, lc * rc, keep);
+      const T ncp = lc * rc;
+      worst = max(worst, magnitude(ncp));
+      st_hint(q, ncp, keep);
       st_hint(q + slots, pd, keep);
       q += 2 * slots;
     };
@@ -662,6 +677,31 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     const T pc = n > 1 ? lc * rc : T(0);  // a line of one row has no c
     const T oc = __shfl_xor_sync(0xffffffffu, pc, 16), od = __shfl_xor_sync(0xffffffffu, pd, 16);
+    const bool ill = __shfl_sync(0xffffffffu, worst, (lane & 15) + 16) > magnitude(T(kGrowth));
+    if (__any_sync(0xffffffffu, ill)) {
+      __syncwarp();  // the partner's scratch changes hands
+      if (ill && !half) {
+        // row i's c' and d': in this lane's scratch, from row len on in its partner's
+        auto row = [&](int i) { return i < len ? cp + 2ll * i * slots : cp + 16 + 2ll * (i - len) * slots; };
+        T tc = T(0), td = T(0);
+        for (int i = 0; i < n; i++) {
+          const long long o = i * ss;
+          const T ai = i ? a[o] : T(0), r = recip(b[o] - ai * tc);
+          tc = c[o] * r;
+          td = (d[o] - ai * td) * r;
+          row(i)[0] = tc;
+          row(i)[slots] = td;
+        }
+        for (int i = n - 1; i >= 0; i--) {
+          const long long o = i * ss;
+          if (i < n - 1) td = row(i)[slots] - row(i)[0] * td;
+          if (u) u[o] += td;
+          else d[o] = td;
+        }
+      }
+      __syncwarp();
+    }
+    const int todo = ill ? 0 : len;  // rows still to substitute
     T xv = n > 1 ? (pd - pc * od) * recip(T(1) - pc * oc) : pd;
     // outwards, from the row before the middle
     long long out = (long long)(len - 1) * ss;
@@ -670,7 +710,7 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       else __stcs(d + out, xv);
       out -= ss;
     };
-    if (len) put(u ? u[out] : T(0));
+    if (todo) put(u ? u[out] : T(0));
     q = cp + (long long)(len - 2) * 2 * slots;
     struct Back {
       T c[U], d[U], u[U];
@@ -709,8 +749,8 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
         }
     };
     Back w0, w1;
-    back(len - 2, w0);
-    for (int i = len - 2; i >= 0; i -= 2 * U) {
+    back(todo - 2, w0);
+    for (int i = todo - 2; i >= 0; i -= 2 * U) {
       back(i - U, w1);
       substitute(i, w0);
       back(i - 2 * U, w0);

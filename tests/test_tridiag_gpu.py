@@ -213,3 +213,35 @@ def test_more_strided_lines_than_threads(gpu_runtime, orc, dtype, rtol, inc):
             assert np.array_equal(t[3].cpu().numpy(), d)
             ref = u + ref
         np.testing.assert_allclose(t[4 if inc else 3].cpu().numpy(), ref, rtol=rtol, atol=rtol * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("dtype,rtol", [(np.float64, 1e-12), (np.float32, 2e-4)])
+@pytest.mark.parametrize("inc", [False, True])
+@pytest.mark.parametrize("solvedim", [1, 2])
+@pytest.mark.parametrize("n", [2, 3, 5, 16, 17, 64, 101])
+def test_strided_lines_with_pivots_from_the_top_only(gpu_runtime, orc, dtype, rtol, inc, solvedim, n):
+    """Lines whose elimination from the last row meets a vanishing or tiny
+    pivot (b_{n-1} = 0, b_{n-1} = a rounding unit, a singular trailing 2 x 2
+    block), between ordinary ones of the same group of 16. From the top they
+    are as well conditioned as the rest: |c'| < 1 up to the last rows."""
+    lines = 37
+    a, b, c, d = seeded.trid_system((lines, n), 1, 3 + n, dtype)
+    k = np.arange(lines) % 4
+    a[k > 0, n - 1] = 1.0
+    b[k == 1, n - 1] = 0.0
+    b[k == 2, n - 1] = np.finfo(dtype).eps
+    if n > 3:
+        for arr, v in ((b, n - 2), (c, n - 2), (b, n - 1)):
+            arr[k == 3, v] = 1.0
+    u = seeded.uniform(5, np.arange(d.size, dtype=np.uint64), -1, 1).reshape(d.shape).astype(dtype)
+    # the solve dimension along y (z = 1) or z (y = 1), the lines along x
+    shape = (1, n, lines) if solvedim == 1 else (n, 1, lines)
+    a, b, c, d, u = (np.ascontiguousarray(v.T).reshape(shape) for v in (a, b, c, d, u))
+    x, ug = run_gpu(a, b, c, d, solvedim, u=u if inc else None)
+    ref = d.copy()
+    oracle_solve(orc, a, b, c, ref, solvedim)
+    assert np.isfinite(ref).all()
+    if inc:
+        assert np.array_equal(x, d)
+        x, ref = ug, u + ref
+    np.testing.assert_allclose(x, ref, rtol=rtol, atol=rtol * np.abs(ref).max())
