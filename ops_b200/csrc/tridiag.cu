@@ -69,6 +69,21 @@ __device__ __forceinline__ double recip(double x) {
   return fma(r, fma(e, e, e), r);
 }
 
+// r = 1 / x and cr = c / x by the same steps: c takes part in the correction, so
+// the two are ready together.
+__device__ __forceinline__ void recip_times(float x, float c, float &r, float &cr) {
+  const float q = __fdividef(1.0f, x), cq = c * q, e = fmaf(-x, q, 1.0f);
+  r = fmaf(q, e, q);
+  cr = fmaf(cq, e, cq);
+}
+__device__ __forceinline__ void recip_times(double x, double c, double &r, double &cr) {
+  double q;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(q) : "d"(x));
+  const double cq = c * q, e = fma(-x, q, 1.0), t = fma(e, e, e);
+  r = fma(q, t, q);
+  cr = fma(cq, t, cq);
+}
+
 // One work item = L neighbouring lines x n rows of one system, staged in
 // shared memory: the four coefficient tiles are loaded with cp.async (rows
 // of the tile along whichever dimension is contiguous in HBM, so the loads
@@ -636,18 +651,18 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       asm volatile("cp.async.commit_group;" ::: "memory");
     };
     for (int st = 0; st < kLineStages - 1; st++) fetch(st);
-    // the chain from row to row is one product and the reciprocal:
-    // b_i - a_i c'_{i-1} = b_i - (a_i c_{i-1}) r_{i-1}
-    T rc = T(0), lc = T(0), pd = T(0);
+    // the chain from row to row is one product and the reciprocal. (A product
+    // a_i c_{i-1} taken ahead would be a cycle shorter but has the square of the
+    // rows' scale: FP32 rows of 1e20 overflow in it.)
+    T pc = T(0), pd = T(0);
     int worst = 0;  // the largest |c'|
     T *q = cp;
     auto eliminate = [&](T ai, T bi, T ci, T di) {
-      rc = recip(bi - (ai * lc) * rc);
-      lc = ci;
-      pd = (di - ai * pd) * rc;
-      const T ncp = lc * rc;
-      worst = max(worst, magnitude(ncp));
-      st_hint(q, ncp, keep);
+      T r;
+      recip_times(bi - ai * pc, ci, r, pc);
+      pd = (di - ai * pd) * r;
+      worst = max(worst, magnitude(pc));
+      st_hint(q, pc, keep);
       st_hint(q + slots, pd, keep);
       q += 2 * slots;
     };
@@ -675,7 +690,7 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    const T pc = n > 1 ? lc * rc : T(0);  // a line of one row has no c
+    if (n == 1) pc = T(0);  // no c
     const T oc = __shfl_xor_sync(0xffffffffu, pc, 16), od = __shfl_xor_sync(0xffffffffu, pd, 16);
     const bool ill = __shfl_sync(0xffffffffu, worst, (lane & 15) + 16) > magnitude(T(kGrowth));
     if (__any_sync(0xffffffffu, ill)) {

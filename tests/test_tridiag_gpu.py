@@ -245,3 +245,18 @@ def test_strided_lines_with_pivots_from_the_top_only(gpu_runtime, orc, dtype, rt
         assert np.array_equal(x, d)
         x, ref = ug, u + ref
     np.testing.assert_allclose(x, ref, rtol=rtol, atol=rtol * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("dtype,rtol,power", [(np.float64, 1e-12, 600), (np.float32, 2e-4, 80)])
+@pytest.mark.parametrize("sign", [1, -1])
+@pytest.mark.parametrize("solvedim", [0, 1, 2])
+def test_rows_of_any_scale(gpu_runtime, orc, dtype, rtol, power, sign, solvedim):
+    """Rows scaled by a power of two whose square leaves the type's range: the
+    solution is that of the unscaled rows."""
+    shape = (9, 14, 33)
+    a, b, c, d = seeded.trid_system(shape, solvedim, 17, dtype)
+    s = dtype(2.0) ** (sign * power)
+    x, _ = run_gpu(a * s, b * s, c * s, d * s, solvedim)
+    ref = d.copy()
+    oracle_solve(orc, a, b, c, ref, solvedim)
+    np.testing.assert_allclose(x, ref, rtol=rtol, atol=rtol * np.abs(ref).max())
