@@ -455,10 +455,12 @@ typedef struct ops_b200_trid_system {
  * length; a line whose elimination from the last row meets small pivots is
  * solved by Thomas from the first row. Neither exchanges rows: the y/z sweeps
  * need pivots from the first row on, the x sweeps in each chunk of 4 to 8 rows
- * too (diagonally dominant lines have them all). The y/z sweeps use a
- * c'/d' scratch array of 2 x (unknowns) elements that the library keeps and
- * grows. The work lists and that scratch are shared by all calls: calls on
- * different streams must not overlap. */
+ * too (diagonally dominant lines have them all). The y/z sweeps keep a
+ * scratch that the library grows: the c' and d' of the lines in flight, 64 MB
+ * as long as 592 groups of 16 lines fit in that and never more than 2 x
+ * (unknowns) elements (rounded up to whole pairs of rows). The work lists and
+ * that scratch are shared by all calls: calls on different streams must not
+ * overlap. */
 int ops_b200_trid_batch(int elem_size, int solvedim, int nsys, const ops_b200_trid_system *systems, void *stream);
 
 /* ---- allocation-free sweep ----------------------------------------------

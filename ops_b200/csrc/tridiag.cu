@@ -41,7 +41,10 @@ struct Sys {
   int nl0, nl1;    // line counts along the two non-solve dimensions (fastest first)
   long long ss;    // stride along the solve dimension (elements)
   long long s0, s1;
-  long long line0 = 0;  // line kernel: first group of 16 lines of this system
+  // line kernel: an entry is a system's groups of `glines` lines from line lofs
+  // on; its first group, and its first group's scratch
+  long long line0 = 0, scr0 = 0, lofs = 0;
+  int glines = 0;
 };
 
 struct Work {
@@ -536,8 +539,8 @@ __global__ void __launch_bounds__(32 * kWarpLines, sizeof(T) == 4 ? 3 : 2)
 // It needs a fraction of the partition method's instructions, but c' and d' have
 // to wait for the backward pass. They go to a scratch that stays in L2: the
 // grid keeps only so many lines in flight that their c' and d' fit
-// (kScratchBytes), each thread reuses its own slot line after line, the scratch
-// is marked evict-last and everything else evict-first. HBM then sees the
+// (kScratchBytes; a CTA an SM at least), each warp reuses its own part group after
+// group, the scratch is marked evict-last and everything else evict-first. HBM then sees the
 // compulsory 40 B per FP64 unknown (48 with _Inc). With every line in flight
 // the scratch went through HBM too (68 to 77 B). 256^3 FP64: y sweep 0.213 ->
 // 0.167 ms, z sweep (_Inc) 0.289 -> 0.209 ms; the 64-block batch's 0.548 -> 0.478
@@ -602,19 +605,23 @@ __device__ __forceinline__ int magnitude(float x) { return __float_as_int(x) & 0
 constexpr float kGrowth = 16.0f;
 constexpr int kLineThreads = 128, kLineRows = 8, kLineStages = 3;
 
+// Scratch of a group: c' and d' of its lines' halves.
+__host__ __device__ inline long long group_scratch(int n, int glines) { return (n + 1) / 2 * 4ll * glines; }
+
 template <class T>
 constexpr int kLineSmem = kLineStages * kLineRows * 4 * kLineThreads * (int)sizeof(T);
 
 template <class T>
 __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__restrict__ sys, int nsys,
-                                                                 long long groups, T *scr, int slots) {
+                                                                 long long groups, T *scr) {
   constexpr int U = kLineRows;
   extern __shared__ __align__(16) unsigned char smraw[];
   T *ring = reinterpret_cast<T *>(smraw) + threadIdx.x;  // element (stage, row, array) every kLineThreads
   const uint64_t keep = policy_last(), pass = policy_first();
-  const int slot = blockIdx.x * kLineThreads + threadIdx.x, lane = threadIdx.x & 31, half = lane >> 4;
-  T *cp = scr + slot;  // c' of row i at [2 i slots], d' at [(2 i + 1) slots]
-  for (long long g = slot >> 5; g < groups; g += slots >> 5) {
+  const int lane = threadIdx.x & 31, half = lane >> 4, warps = gridDim.x * (kLineThreads / 32);
+  const int first = blockIdx.x * (kLineThreads / 32) + (threadIdx.x >> 5);
+  T *part = nullptr;  // the warp's scratch: its first group's, which needs the most
+  for (long long g = first; g < groups; g += warps) {
     int lo = 0, hi = nsys - 1;  // last system whose first group of lines is <= g
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -622,8 +629,11 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       else hi = mid - 1;
     }
     const Sys &s = sys[lo];
-    const long long lines = (long long)s.nl0 * s.nl1, l = (g - s.line0) * 16 + (lane & 15);
-    const int n = s.n, len = l < lines ? (half ? n / 2 : (n + 1) / 2) : 0;
+    const long long l = s.lofs + (g - s.line0) * 16 + (lane & 15);
+    const int n = s.n, len = (lane & 15) < s.glines ? (half ? n / 2 : (n + 1) / 2) : 0;
+    const int width = 2 * s.glines;
+    if (g == first) part = scr + s.scr0 + (g - s.line0) * group_scratch(n, s.glines);
+    T *cp = part + half * s.glines + (lane & 15);  // c' of row i at [2 i width], d' at [(2 i + 1) width]
     const long long ss = half ? -s.ss : s.ss;
     const long long base = (l % s.nl0) * s.s0 + (l / s.nl0) * s.s1 + (half ? (long long)(n - 1) * s.ss : 0);
     const T *a = reinterpret_cast<const T *>(half ? s.c : s.a) + base;
@@ -663,8 +673,8 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       pd = (di - ai * pd) * r;
       worst = max(worst, magnitude(pc));
       st_hint(q, pc, keep);
-      st_hint(q + slots, pd, keep);
-      q += 2 * slots;
+      st_hint(q + width, pd, keep);
+      q += 2 * width;
     };
     for (int st = 0; st < nst; st++) {
       asm volatile("cp.async.wait_group %0;" ::"n"(kLineStages - 2) : "memory");
@@ -697,7 +707,7 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       __syncwarp();  // the partner's scratch changes hands
       if (ill && !half) {
         // row i's c' and d': in this lane's scratch, from row len on in its partner's
-        auto row = [&](int i) { return i < len ? cp + 2ll * i * slots : cp + 16 + 2ll * (i - len) * slots; };
+        auto row = [&](int i) { return i < len ? cp + 2ll * i * width : cp + s.glines + 2ll * (i - len) * width; };
         T tc = T(0), td = T(0);
         for (int i = 0; i < n; i++) {
           const long long o = i * ss;
@@ -705,11 +715,11 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
           tc = c[o] * r;
           td = (d[o] - ai * td) * r;
           row(i)[0] = tc;
-          row(i)[slots] = td;
+          row(i)[width] = td;
         }
         for (int i = n - 1; i >= 0; i--) {
           const long long o = i * ss;
-          if (i < n - 1) td = row(i)[slots] - row(i)[0] * td;
+          if (i < n - 1) td = row(i)[width] - row(i)[0] * td;
           if (u) u[o] += td;
           else d[o] = td;
         }
@@ -726,7 +736,7 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
       out -= ss;
     };
     if (todo) put(u ? u[out] : T(0));
-    q = cp + (long long)(len - 2) * 2 * slots;
+    q = cp + (long long)(len - 2) * 2 * width;
     struct Back {
       T c[U], d[U], u[U];
     };
@@ -736,8 +746,8 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
 #pragma unroll
         for (int j = 0; j < U; j++) {
           w.c[j] = ld_hint(q, keep);
-          w.d[j] = ld_hint(q + slots, keep);
-          q -= 2 * slots;
+          w.d[j] = ld_hint(q + width, keep);
+          q -= 2 * width;
         }
         if (u) {
 #pragma unroll
@@ -748,8 +758,8 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
         for (int j = 0; j < U; j++)
           if (i - j >= 0) {
             w.c[j] = ld_hint(q, keep);
-            w.d[j] = ld_hint(q + slots, keep);
-            q -= 2 * slots;
+            w.d[j] = ld_hint(q + width, keep);
+            q -= 2 * width;
             if (u) w.u[j] = __ldcs(u + uo);
             uo -= ss;
           }
@@ -790,18 +800,35 @@ Buffers &buffers() {
 // The y/z sweeps (solve dimension strided, lines contiguous) by the line
 // kernel; returns false when some system does not have that shape.
 template <class T>
-bool launch_lines(const std::vector<Sys> &systems, int maxn, cudaStream_t stream, long long *kernels) {
-  long long groups = 0;
+bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long long *kernels) {
   std::vector<Sys> live;  // systems with no rows or no lines take no part
+  int maxn = 0;
   for (const Sys &s : systems) {
     if (s.ss == 1 || s.s0 != 1) return false;
     const long long nl = (long long)s.nl0 * s.nl1;
     if (s.n <= 0 || nl <= 0) continue;
-    live.push_back(s);
-    live.back().line0 = groups;
-    groups += (nl + 15) / 16;
+    maxn = std::max(maxn, s.n);
+    for (int lines : {16, (int)(nl % 16)}) {
+      if (lines == 0 || nl < lines) continue;
+      live.push_back(s);
+      live.back().glines = lines;
+      live.back().lofs = lines == 16 ? 0 : nl - nl % 16;
+    }
   }
   if (live.empty()) return true;
+  // the groups that need the most scratch first: a warp's first group then
+  // sizes its part of it, so that all of it is never more than every line's c' and d'
+  std::stable_sort(live.begin(), live.end(), [](const Sys &x, const Sys &y) {
+    return group_scratch(x.n, x.glines) > group_scratch(y.n, y.glines);
+  });
+  auto groups_of = [](const Sys &s) { return s.glines == 16 ? (long long)s.nl0 * s.nl1 / 16 : 1ll; };
+  long long groups = 0, all = 0;
+  for (Sys &s : live) {
+    s.line0 = groups;
+    s.scr0 = all;
+    groups += groups_of(s);
+    all += groups_of(s) * group_scratch(s.n, s.glines);
+  }
   static int per_sm = 0;  // resident threads, per type
   if (!per_sm) {
     int k = 0;
@@ -825,7 +852,12 @@ bool launch_lines(const std::vector<Sys> &systems, int maxn, cudaStream_t stream
     OPSB_CUDA(cudaMalloc(&B.sys, cap * sizeof(Sys)));
     B.sys_cap = cap;
   }
-  const size_t need = (size_t)slots * line;
+  long long elems = 0, left = slots / 32;  // the first group's scratch of every warp
+  for (const Sys &s : live) {
+    elems += std::min(left, groups_of(s)) * group_scratch(s.n, s.glines);
+    left -= std::min(left, groups_of(s));
+  }
+  const size_t need = (size_t)elems * sizeof(T);
   if (B.scr_bytes < need) {
     if (B.scr) cudaFree(B.scr);
     B.scr = nullptr;
@@ -835,7 +867,7 @@ bool launch_lines(const std::vector<Sys> &systems, int maxn, cudaStream_t stream
   }
   OPSB_CUDA(cudaMemcpyAsync(B.sys, live.data(), live.size() * sizeof(Sys), cudaMemcpyHostToDevice, stream));
   trid_line_kernel<T><<<(unsigned)(slots / kLineThreads), kLineThreads, kLineSmem<T>, stream>>>(
-      B.sys, (int)live.size(), groups, static_cast<T *>(B.scr), (int)slots);
+      B.sys, (int)live.size(), groups, static_cast<T *>(B.scr));
   OPSB_CUDA(cudaGetLastError());
   if (kernels) (*kernels)++;
   return true;
@@ -872,7 +904,7 @@ void launch(const std::vector<Sys> &systems, int solvedim, cudaStream_t stream, 
   int maxn = 0;
   for (const Sys &s : systems) maxn = std::max(maxn, s.n);
   if (maxn == 0) return;
-  if (launch_lines<T>(systems, maxn, stream, kernels)) return;
+  if (launch_lines<T>(systems, stream, kernels)) return;
   bool contig = true;
   for (const Sys &s : systems) contig = contig && (s.n == 0 || s.ss == 1);
   // x sweeps of lines up to 256 rows: a warp per 1, 2 or 4 lines

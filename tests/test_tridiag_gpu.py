@@ -260,3 +260,43 @@ def test_rows_of_any_scale(gpu_runtime, orc, dtype, rtol, power, sign, solvedim)
     ref = d.copy()
     oracle_solve(orc, a, b, c, ref, solvedim)
     np.testing.assert_allclose(x, ref, rtol=rtol, atol=rtol * np.abs(ref).max())
+
+
+def test_scratch_of_uneven_strided_batches(gpu_runtime, tmp_path):
+    """A few long lines beside many short ones, and systems of three lines:
+    the y sweep keeps no more scratch than every line's c' and d' (in a process
+    of its own: the scratch outlives a call), and solves them all."""
+    import subprocess
+    import sys
+    code = """
+import ctypes, sys
+import numpy as np, torch
+import oracle
+from ops_b200 import ops as O, seeded
+shapes = [(1, 256, 65536), (1, 200000, 16)] + [(1, 20001, 3)] * 40
+O.ops_init(0, 0)
+sets = []
+for i, shape in enumerate(shapes):
+    h = seeded.trid_system(shape, 1, 50 + i)
+    sets.append((h, [torch.from_numpy(v).cuda() for v in h]))
+def systems(some):
+    return [dict(a=t[0].data_ptr(), b=t[1].data_ptr(), c=t[2].data_ptr(), d=t[3].data_ptr(), u=None,
+                 dims=list(h[0].shape[::-1]), pads=list(h[0].shape[::-1])) for h, t in some]
+first = seeded.trid_system((1, 8, 16), 1, 1)
+O.trid_batch(8, 1, systems([(first, [torch.from_numpy(v).cuda() for v in first])]), None)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+O.trid_batch(8, 1, systems(sets), None)
+torch.cuda.synchronize()
+kept = free - torch.cuda.mem_get_info()[0]
+rows = sum(z * y * x for z, y, x in shapes)
+assert kept <= 16 * rows + (32 << 20), (kept, 16 * rows)
+f = oracle.lib().oracle_trid_batch_d
+for (a, b, c, d), t in sets:
+    ref = d.copy()
+    dims = (ctypes.c_int * 3)(*a.shape[::-1])
+    f(a.ctypes.data, b.ctypes.data, c.ctypes.data, ref.ctypes.data, None, 3, 1, dims, dims)
+    np.testing.assert_allclose(t[3].cpu().numpy(), ref, rtol=1e-12, atol=1e-12 * np.abs(ref).max())
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
