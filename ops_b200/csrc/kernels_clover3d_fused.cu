@@ -74,9 +74,11 @@ template <int OWN, int EDGE, int M>
 struct March {
   int X, o, m0, m1;
   bool own, live;
-  __device__ __forceinline__ March(const LoopParams &lp, int rows) {
+  __device__ __forceinline__ March(const LoopParams &lp, int rows)
+      : March(lp, rows, blockIdx.x * kWarps + (threadIdx.x >> 5)) {}
+  __device__ __forceinline__ March(const LoopParams &lp, int rows, int w) {
     constexpr int O = M == 1 ? 2 : 1;
-    const int w = blockIdx.x * kWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31;
     const int ncol = (lp.end[0] - lp.start[0] + OWN - 1) / OWN, lines = lp.end[O] - lp.start[O];
     const int rest = w / lines, c = rest % ncol;
     o = lp.start[O] + w % lines;
@@ -102,9 +104,9 @@ void launch_march(const LoopParams &lp, cudaStream_t s, F kernel) {
   const int nm = lp.end[M] - lp.start[M];
   const long long columns = (nx + OWN - 1) / OWN * no;
   const int rows = march_rows(columns, nm, HALO, 148LL * per_sm * kWarps, (long long)Runtime::kMaxRedBlocks * kWarps);
-  const long long blocks = (columns * ((nm + rows - 1) / rows) + kWarps - 1) / kWarps;
-  if (blocks > Runtime::kMaxRedBlocks && lp.nred > 0)
-    throw Error(E_UNSUPPORTED, "cloverleaf3d: mesh too large for one reduction");
+  long long blocks = (columns * ((nm + rows - 1) / rows) + kWarps - 1) / kWarps;
+  // a kernel that reduces goes over its parts with the grid's stride
+  if (lp.nred > 0) blocks = std::min<long long>(blocks, Runtime::kMaxRedBlocks);
   kernel<<<(unsigned)blocks, 32 * kWarps, 0, s>>>(lp, rows);
 }
 
@@ -145,12 +147,14 @@ struct Quad {
 // ideal_gas_kernel then field_summary_kernel. A node's kinetic term is the
 // same product at each of the eight cells around it.
 __global__ void __launch_bounds__(32 * kWarps, 5) summary_kernel(const __grid_constant__ LoopParams lp, int rows) {
-  const March<31, 0, 2> m(lp, rows);
-  const int X = min(m.X, lp.end[0]);
-  const Fld density0(lp.a[0], X), energy0(lp.a[1], X), pressure(lp.a[2], X), soundspeed(lp.a[3], X), volume(lp.a[4], X),
-      xvel0(lp.a[5], X), yvel0(lp.a[6], X), zvel0(lp.a[7], X);
   double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
-  if (m.live) {
+  // one part a warp, but more columns than kMaxRedBlocks CTAs have warps (2880 x 2880 x 8, say) take several
+  for (int w = blockIdx.x * kWarps + (threadIdx.x >> 5);; w += gridDim.x * kWarps) {
+    const March<31, 0, 2> m(lp, rows, w);
+    if (!m.live) break;
+    const int X = min(m.X, lp.end[0]);
+    const Fld density0(lp.a[0], X), energy0(lp.a[1], X), pressure(lp.a[2], X), soundspeed(lp.a[3], X),
+        volume(lp.a[4], X), xvel0(lp.a[5], X), yvel0(lp.a[6], X), zvel0(lp.a[7], X);
     const int y = m.o;
     auto kin = [](double a, double b, double c) { return 0.125 * (a * a + b * b + c * c); };
     struct Raw {  // velocities of plane z + 1 at rows y and y + 1, cell values of plane z

@@ -105,3 +105,25 @@ def test_fused_loops_leave_what_the_reference_loops_leave(gpu_runtime, tmp_path,
     assert outs[0][1].keys() == outs[1][1].keys()
     for name, data in outs[0][1].items():
         assert data == outs[1][1][name], name
+
+
+def test_mesh_of_more_columns_than_a_reduction_has_blocks(gpu_runtime):
+    """262,150 lines of 2 x 2 cells: more columns than 65,536 CTAs of four
+    warps hold. The hand-fused cycle against the reference's loops: dt exactly,
+    the sums to n * 2^-53 either way (n additions of positive terms, 2^20)."""
+    from ops_b200 import ops as O
+    ny = 262150
+    deck = apps.clover3d_deck(x_cells=2, y_cells=ny, z_cells=2, xmax=1.0, ymax=0.5 * ny, zmax=1.0,
+                              initial_timestep=0.01, timestep_rise=1.5, max_timestep=0.04, end_step=2,
+                              summary_frequency=1,
+                              states=[dict(density=0.2, energy=1.0),
+                                      dict(density=1.0, energy=2.5, geometry="cuboid", xmin=0.0, xmax=1.0,
+                                           ymin=100.0, ymax=0.4 * ny, zmin=0.0, zmax=1.0)])
+    got, _ = apps.cloverleaf3d(deck)
+    O.set_option("tiling", 0)
+    try:
+        want, _ = apps.cloverleaf3d(deck)
+    finally:
+        O.set_option("tiling", 1)
+    assert np.array_equal(got[:, 7], want[:, 7])
+    np.testing.assert_allclose(got, want, rtol=2 * 2.0 ** 20 * 2.0 ** -53, atol=0)
