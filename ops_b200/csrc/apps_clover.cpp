@@ -189,10 +189,9 @@ struct Clover {
     S2D_00_M10_STRID2D_X = strided(2, {0, 0, -1, 0}, {1, 0}, "s2D_00_M10_stride2D_x");
     S2D_00_0M1_STRID2D_Y = strided(2, {0, 0, 0, -1}, {0, 1}, "s2D_00_0M1_stride2D_y");
     if (fused) {
-      size[0] = x_cells + 5; size[1] = y_cells + 5;
-      density_n = D("fused_density"); energy_n = D("fused_energy");
-      size[0]++; size[1]++;
-      xvel_n = D("fused_xvel"); yvel_n = D("fused_yvel");
+      // the fused loops have no use for the work arrays of their own
+      density_n = work_array1; energy_n = work_array2;
+      xvel_n = work_array3; yvel_n = work_array4;
       // the reach of the fused column marches
       S2D_box = stencil(2, {-2, -2, 2, 2}, "-2,-2:2,2");
       S2D_box_X = strided(2, {-2, 0, 2, 0}, {1, 0}, "-2:2 stride2D_x");
@@ -757,6 +756,16 @@ struct Clover {
             dat(d, S2D_box, ACC_READ), dat(xv, S2D_box, ACC_READ), dat(yv, S2D_box, ACC_READ),
             dat(xout, S2D_00, ACC_WRITE), dat(yout, S2D_00, ACC_WRITE)});
   }
+  // Back to the reference's loops, with the work arrays as they start: what
+  // those loops write of them they write in each step of either direction.
+  void leave_fused() {
+    if (!fused) return;
+    fused = false;
+    for (int d : {work_array1, work_array2, work_array3, work_array4}) {
+      const std::vector<char> zeros(r.dat_data_bytes(d));
+      r.dat_set_data(d, zeros.data(), zeros.size());
+    }
+  }
   // Whether this step (its dt known) and the one after it are both followed
   // by another: the next dt is at most dt * dtrise.
   bool two_more_steps() const {
@@ -799,9 +808,9 @@ struct Clover {
   // One hydro cycle (clover_leaf.cpp:185-212). Returns true when complete.
   bool cycle() {
     step = step + 1;
-    if (keep_all && step + 1 >= end_step) fused = false;
+    if (keep_all && step + 1 >= end_step) leave_fused();
     timestep();
-    if (keep_all && !two_more_steps()) fused = false;
+    if (keep_all && !two_more_steps()) leave_fused();
     if (fused) {
       fused_step();
     } else {
@@ -872,7 +881,6 @@ extern "C" int ops_b200_app_cloverleaf(const ops_b200_clover_deck *deck, int war
     if (dump_dir) {
       for (int i = mk.dats; i < r.ndats(); i++) {
         Dat &d = r.dat(i);
-        if (d.name.compare(0, 6, "fused_") == 0) continue;  // not a dat of the reference app
         std::vector<char> buf(r.dat_data_bytes(i));  // the rank's owned part when partitioned
         r.dat_fetch_data(i, buf.data(), buf.size());
         std::string path = std::string(dump_dir) + "/" + d.name + ".bin";

@@ -237,10 +237,9 @@ struct Clover3D {
     S_00P1_00M1_00M2_STRID_Z = strided(4, {0, 0, 0, 0, 0, 1, 0, 0, 2, 0, 0, -1}, {0, 0, 1}, "z4");
 
     if (fused) {
-      size[0] = xc + 5; size[1] = yc + 5; size[2] = zc + 5;
-      density_n = D("fused_density"); energy_n = D("fused_energy");
-      size[0]++; size[1]++; size[2]++;
-      xvel_n = D("fused_xvel"); yvel_n = D("fused_yvel"); zvel_n = D("fused_zvel");
+      // the fused loops have no use for the work arrays of their own
+      density_n = work_array1; energy_n = work_array2;
+      xvel_n = work_array3; yvel_n = work_array4; zvel_n = work_array5;
       // the reach of the fused marches
       S_box = stencil(2, {-2, -2, -2, 2, 2, 2}, "-2:2");
       S_box_X = strided(2, {-2, 0, 0, 2, 0, 0}, {1, 0, 0}, "-2:2 stride x");
@@ -899,6 +898,16 @@ struct Clover3D {
          {rd(volume), rd(vol_flux_x), rd(vol_flux_y), rd(vol_flux_z), width(dir, celldx, celldy, celldz),
           rd(flux_of(dir)), rd(density1), rd(xvel1), rd(yvel1), rd(zvel1), wr(xo), wr(yo), wr(zo)});
   }
+  // Back to the reference's loops, with the work arrays as they start: what
+  // those loops write of them they write in each step of either direction.
+  void leave_fused() {
+    if (!fused) return;
+    fused = false;
+    for (int d : {work_array1, work_array2, work_array3, work_array4, work_array5}) {
+      const std::vector<char> zeros(r.dat_data_bytes(d));
+      r.dat_set_data(d, zeros.data(), zeros.size());
+    }
+  }
   // Whether this step (its dt known) and the one after it are both followed
   // by another: the next dt is at most dt * dtrise.
   bool two_more_steps() const {
@@ -946,9 +955,9 @@ struct Clover3D {
   // One hydro cycle (clover_leaf.cpp:176-210). Returns true when complete.
   bool cycle() {
     step = step + 1;
-    if (keep_all && step + 1 >= end_step) fused = false;
+    if (keep_all && step + 1 >= end_step) leave_fused();
     timestep();
-    if (keep_all && !two_more_steps()) fused = false;
+    if (keep_all && !two_more_steps()) leave_fused();
     if (fused) {
       fused_step();
     } else {
@@ -1020,7 +1029,6 @@ extern "C" int ops_b200_app_cloverleaf3d(const ops_b200_clover3d_deck *deck, int
     if (dump_dir) {
       for (int i = mk.dats; i < r.ndats(); i++) {
         Dat &d = r.dat(i);
-        if (d.name.compare(0, 6, "fused_") == 0) continue;  // not a dat of the reference app
         std::vector<char> buf(r.dat_data_bytes(i));  // the rank's owned part when partitioned
         r.dat_fetch_data(i, buf.data(), buf.size());
         std::string path = std::string(dump_dir) + "/" + d.name + ".bin";

@@ -127,3 +127,20 @@ def test_mesh_of_more_columns_than_a_reduction_has_blocks(gpu_runtime):
         O.set_option("tiling", 1)
     assert np.array_equal(got[:, 7], want[:, 7])
     np.testing.assert_allclose(got, want, rtol=2 * 2.0 ** 20 * 2.0 ** -53, atol=0)
+
+
+def test_fused_loops_take_no_storage_of_their_own(gpu_runtime):
+    """A run on the hand-fused loops after one of the same size on the
+    reference's finds all its dats among the storage that one gave back."""
+    import torch
+
+    from ops_b200 import ops as O
+    deck = deck3d(101, 103, 107, 2, 6, 0.04)
+    O.set_option("tiling", 0)
+    try:
+        apps.cloverleaf3d(deck)
+    finally:
+        O.set_option("tiling", 1)
+    free = torch.cuda.mem_get_info()[0]
+    apps.cloverleaf3d(deck)
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20  # less than one dat

@@ -102,3 +102,20 @@ def test_fused_loops_leave_what_the_reference_loops_leave(gpu_runtime, tmp_path,
     assert outs[0][1].keys() == outs[1][1].keys()
     for name, data in outs[0][1].items():
         assert data == outs[1][1][name], name
+
+
+def test_fused_loops_take_no_storage_of_their_own(gpu_runtime):
+    """A run on the hand-fused loops after one of the same size on the
+    reference's finds all its dats among the storage that one gave back."""
+    import torch
+
+    from ops_b200 import ops as O
+    deck = config2_deck(1003, 1017, 2, 3)
+    O.set_option("tiling", 0)
+    try:
+        apps.cloverleaf(deck)
+    finally:
+        O.set_option("tiling", 1)
+    free = torch.cuda.mem_get_info()[0]
+    apps.cloverleaf(deck)
+    assert free - torch.cuda.mem_get_info()[0] < 8 << 20  # less than one dat
