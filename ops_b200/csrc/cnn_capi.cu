@@ -224,6 +224,7 @@ extern "C" int ops_b200_heat_solve(const ops_b200_heat_system *sys, int method, 
     f.p = ws.p;
     f.z = ws.z;
     f.Mi = ws.Mi;
+    if (method != OPS_B200_HEAT_FCG_LEARNED_MG) f.p2 = ws.t;
     ws.solver.diag(f, sys->rx, sys->ry, s);
     heat::SolveStats st;
     cudaEvent_t e0, e1;

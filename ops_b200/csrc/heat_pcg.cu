@@ -1058,8 +1058,7 @@ struct Solver::Impl {
   long long pitch32 = 0;
   float *Kx = nullptr, *Ky = nullptr, *Mi = nullptr, *r = nullptr, *p = nullptr, *w = nullptr, *p2 = nullptr,
         *e = nullptr;
-  // the FP64 direction's second buffer, interior at p64b + its field's offset
-  double *p64b = nullptr;
+  double *p64b = nullptr;  // of `second`
   size_t p64b_n = 0;
   float *Kz = nullptr;  // 3D only
   ulonglong2 *slots = nullptr;  // k_pcg_resident's exchange, then its error word
@@ -1118,13 +1117,18 @@ struct Solver::Impl {
     return true;
   }
 
-  void ensure_p64(size_t n) {
-    if (n <= p64b_n) return;
-    cudaFree(p64b);
-    p64b = nullptr;
-    p64b_n = 0;
-    OPSB_CUDA(cudaMalloc(&p64b, n * sizeof(double)));
-    p64b_n = n;
+  // The FP64 direction's second buffer (addressed as its field's interior).
+  double *second(const Field2D &f) {
+    if (f.p2) return f.p2;
+    const size_t n = (size_t)f.pitch * f.ny;
+    if (n > p64b_n) {
+      cudaFree(p64b);
+      p64b = nullptr;
+      p64b_n = 0;
+      OPSB_CUDA(cudaMalloc(&p64b, n * sizeof(double)));
+      p64b_n = n;
+    }
+    return p64b;
   }
 
   // Partials for a grid of more than kMaxBlocks (a strip or tile is a block's
@@ -1307,8 +1311,8 @@ void Solver::pcg_fp64(const Field2D &f, double rx, double ry, bool precond, bool
   check_launch("heat solver init");
   launches_ += 2;
   if (max_iters > 0) {
-    m.ensure_p64((size_t)f.pitch * f.ny);
-    double *pb = m.p64b;
+    // z is written before the loop and after it only (k_init, k_flush)
+    double *pb = precond ? f.z : m.second(f);
     bool ran;
     if (precond && true_stop)
       ran = m.resident<double, Z_MI, STOP_TRUE>(g, f.Kx, f.Ky, f.p, f.r, f.Mi, f.u, f.z, rx, ry, m.s64, st);
@@ -1695,12 +1699,12 @@ void Solver::fcg(const Field2D &f, double rx, double ry, double eps, int max_ite
   out->initial_residual = r0;
   out->fallbacks = 0;
   bool done = h.done == 1 || r0 == 0.0;
+  double *pb = nullptr;
   if (!done) {
     // the initial residual kernel leaves done = 0 and iters = 0
-    m.ensure_p64((size_t)f.pitch * f.ny);
+    pb = m.second(f);
     precond();
   }
-  double *const pb = m.p64b;
   int rows = 1, blocks = 1;
   pw_grid(f.nx, f.ny, kPwBlocks<double>, &rows, &blocks);
   m.ensure_part(blocks);

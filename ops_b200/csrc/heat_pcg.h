@@ -35,6 +35,10 @@ struct Field2D {
   long long pitch = 0;
   const double *Kx = nullptr, *Ky = nullptr, *u0 = nullptr;
   double *u = nullptr, *r = nullptr, *w = nullptr, *p = nullptr, *z = nullptr, *Mi = nullptr;
+  // Room for a second direction (contents are lost). Without it the flexible
+  // CG and the CG without preconditioner keep a field of their own; Jacobi-PCG
+  // has `z` free between its ends.
+  double *p2 = nullptr;
 };
 
 // The 3D 7-point operator's fields: pointers address the first interior

@@ -68,3 +68,33 @@ def test_wide_cross_section_3d(gpu_runtime, method):
     st = lmg.solve3d(*k, u0, u, 5.0, 5.0, 5.0, method=getattr(lmg, method), eps=1e-8)
     # stopped on the recursive residual (PCG_TRUE) or the FP64 one; they differ by rounding, far below 1e-8 ||r0||
     assert st["converged"] and st["final_residual"] < 1.5e-8 * st["initial_residual"]
+
+
+@pytest.mark.parametrize("method", ["PCG_TRUE", "FCG_JACOBI", "FCG_MG"])
+def test_second_direction_takes_no_field_of_its_own(gpu_runtime, method):
+    """The solver's own fields are six (and the multigrid levels): the second
+    direction goes to one of them. In a process of its own, for the fields
+    outlive a solve."""
+    import subprocess
+    import sys
+    code = f"""
+import numpy as np, torch
+from ops_b200 import lmg
+def solve(n):
+    rho = np.ones((n, n))
+    en = np.random.default_rng(1).random((n, n))
+    k = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in lmg.padded_problem(rho, en)]
+    u = k[2].clone()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    lmg.solve(*k, u, 20.0, 20.0, method=lmg.{method}, eps=1e-8)
+    torch.cuda.synchronize()
+    return free - torch.cuda.mem_get_info()[0]
+solve(640)
+field = 8 * 2050 ** 2
+levels = 4 * 6 * 2080 * 2048 * 4 / 3 if {method!r} == "FCG_MG" else 0
+kept = solve(2048) + 6 * 8 * 642 ** 2
+assert kept < 6.5 * field + levels, (kept, field)
+"""
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
+    assert r.returncode == 0, r.stderr[-2000:]
