@@ -91,8 +91,8 @@ struct March {
 };
 
 // HALO: rows a march reads beyond its own.
-template <int OWN, int M, int HALO, class F>
-void launch_march(const LoopParams &lp, cudaStream_t s, F kernel) {
+template <int OWN, int M, int HALO, auto kernel>
+void launch_march(const LoopParams &lp, cudaStream_t s) {
   static int per_sm = 0;  // resident CTAs, per kernel
   if (!per_sm) {
     int n = 0;
@@ -213,7 +213,7 @@ struct ideal_gas_summary {
   __device__ void operator()(const D &density0, const D &energy0, D &pressure, D &soundspeed, const D &volume,
                              const D &xvel0, const D &yvel0, const D &zvel0, RED<double> &vol, RED<double> &mass,
                              RED<double> &ie, RED<double> &ke, RED<double> &press) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, summary_kernel); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1, summary_kernel>(lp, s); }
 };
 
 // calc_dt_kernel with calc_dt_kernel_min folded in. Point by point: the six
@@ -309,7 +309,7 @@ struct PdV_predict_pressure {
   __device__ void operator()(const D &xarea, const D &xvel0, const D &yarea, const D &yvel0, const D &zarea,
                              const D &zvel0, const D &volume, D &pressure, const D &density0, const D &viscosity,
                              const D &energy0) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, predict_march); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1, predict_march>(lp, s); }
 };
 
 // accelerate_kernel. A plane's share of a node's mass and forces is computed
@@ -388,7 +388,7 @@ struct accelerate_fused {
   __device__ void operator()(const D &density0, const D &volume, const D &pressure, const D &viscosity,
                              const D &xarea, const D &yarea, const D &zarea, const D &xvel0, const D &yvel0,
                              const D &zvel0, D &xvel1, D &yvel1, D &zvel1) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, accelerate_march); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1, accelerate_march>(lp, s); }
 };
 
 // PdV_kernel_nopredict and flux_calc_kernel{x,y,z} over the nodes; each
@@ -470,7 +470,7 @@ struct PdV_flux {
                              const D &yvel0, const D &yvel1, const D &zvel0, const D &zvel1, const D &volume,
                              const D &pressure, const D &density0, const D &viscosity, const D &energy0, D &density1,
                              D &energy1, D &vol_flux_x, D &vol_flux_y, D &vol_flux_z) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1>(lp, s, pdv_flux_march); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_march<31, 2, 1, pdv_flux_march>(lp, s); }
 };
 
 // ---- advection -------------------------------------------------------------------
@@ -640,12 +640,12 @@ __global__ void __launch_bounds__(32 * kWarps, 5) advec_cell_march(const __grid_
                                D &density0) const;                                                                  \
     static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { LAUNCH; }                                \
   };
-ADVEC_CELL(advec_cell_fused_x1, (launch_march<28, 1, 0>(lp, s, advec_cell_x_march<VOL_FIRST>)))
-ADVEC_CELL(advec_cell_fused_z1, (launch_march<32, 2, 3>(lp, s, advec_cell_march<2, VOL_FIRST>)))
-ADVEC_CELL(advec_cell_fused_y2x, (launch_march<32, 1, 3>(lp, s, advec_cell_march<1, VOL_YZ>)))
-ADVEC_CELL(advec_cell_fused_y2z, (launch_march<32, 1, 3>(lp, s, advec_cell_march<1, VOL_YX>)))
-ADVEC_CELL_LAST(advec_cell_fused_x3, (launch_march<28, 1, 0>(lp, s, advec_cell_x_march<VOL_LAST>)))
-ADVEC_CELL_LAST(advec_cell_fused_z3, (launch_march<32, 2, 3>(lp, s, advec_cell_march<2, VOL_LAST>)))
+ADVEC_CELL(advec_cell_fused_x1, (launch_march<28, 1, 0, advec_cell_x_march<VOL_FIRST>>(lp, s)))
+ADVEC_CELL(advec_cell_fused_z1, (launch_march<32, 2, 3, advec_cell_march<2, VOL_FIRST>>(lp, s)))
+ADVEC_CELL(advec_cell_fused_y2x, (launch_march<32, 1, 3, advec_cell_march<1, VOL_YZ>>(lp, s)))
+ADVEC_CELL(advec_cell_fused_y2z, (launch_march<32, 1, 3, advec_cell_march<1, VOL_YX>>(lp, s)))
+ADVEC_CELL_LAST(advec_cell_fused_x3, (launch_march<28, 1, 0, advec_cell_x_march<VOL_LAST>>(lp, s)))
+ADVEC_CELL_LAST(advec_cell_fused_z3, (launch_march<32, 2, 3, advec_cell_march<2, VOL_LAST>>(lp, s)))
 
 // One momentum sweep of the three velocities: node fluxes and masses (alike
 // for all three), momentum fluxes and updates, into other dats than the
@@ -812,12 +812,12 @@ __global__ void __launch_bounds__(32 * kWarps, 3) advec_mom_march(const __grid_c
                                const D &zvel, D &xout, D &yout, D &zout) const;                                     \
     static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { LAUNCH; }                                \
   };
-ADVEC_MOM(advec_mom_fused_x1, (launch_march<28, 1, 1>(lp, s, advec_mom_x_march<VOL_FIRST>)))
-ADVEC_MOM(advec_mom_fused_x3, (launch_march<28, 1, 1>(lp, s, advec_mom_x_march<VOL_LAST>)))
-ADVEC_MOM(advec_mom_fused_y2x, (launch_march<31, 1, 3>(lp, s, advec_mom_march<1, VOL_YZ>)))
-ADVEC_MOM(advec_mom_fused_y2z, (launch_march<31, 1, 3>(lp, s, advec_mom_march<1, VOL_YX>)))
-ADVEC_MOM(advec_mom_fused_z1, (launch_march<31, 2, 3>(lp, s, advec_mom_march<2, VOL_FIRST>)))
-ADVEC_MOM(advec_mom_fused_z3, (launch_march<31, 2, 3>(lp, s, advec_mom_march<2, VOL_LAST>)))
+ADVEC_MOM(advec_mom_fused_x1, (launch_march<28, 1, 1, advec_mom_x_march<VOL_FIRST>>(lp, s)))
+ADVEC_MOM(advec_mom_fused_x3, (launch_march<28, 1, 1, advec_mom_x_march<VOL_LAST>>(lp, s)))
+ADVEC_MOM(advec_mom_fused_y2x, (launch_march<31, 1, 3, advec_mom_march<1, VOL_YZ>>(lp, s)))
+ADVEC_MOM(advec_mom_fused_y2z, (launch_march<31, 1, 3, advec_mom_march<1, VOL_YX>>(lp, s)))
+ADVEC_MOM(advec_mom_fused_z1, (launch_march<31, 2, 3, advec_mom_march<2, VOL_FIRST>>(lp, s)))
+ADVEC_MOM(advec_mom_fused_z3, (launch_march<31, 2, 3, advec_mom_march<2, VOL_LAST>>(lp, s)))
 
 #define REG(K) OPSB_REGISTER_LOOP(K);
 REG(ideal_gas_summary) REG(calc_dt_fused) REG(PdV_predict_pressure) REG(accelerate_fused)

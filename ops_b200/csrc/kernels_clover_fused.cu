@@ -166,8 +166,8 @@ struct Strip {
 };
 
 // HALO: rows a strip reads beyond its own.
-template <int OWN, int HALO, class F>
-void launch_strips(const LoopParams &lp, cudaStream_t s, F kernel) {
+template <int OWN, int HALO, auto kernel>
+void launch_strips(const LoopParams &lp, cudaStream_t s) {
   static int per_sm = 0;  // resident CTAs, per kernel
   if (!per_sm) {
     int n = 0;
@@ -282,7 +282,7 @@ struct lagrange {
   __device__ void operator()(const D &density0, const D &volume, const D &pressure, const D &viscosity,
                              const D &xvel0, const D &yvel0, const D &xarea, const D &yarea, const D &energy0,
                              D &xvel1, D &yvel1, D &density1, D &energy1, D &vol_flux_x, D &vol_flux_y) const;
-  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<30, 2>(lp, s, lagrange_kernel); }
+  static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<30, 2, lagrange_kernel>(lp, s); }
 };
 
 // advec_cell_kernel{1,2}, 3 and 4 of an x sweep (advec_cell.cpp:38-147). The
@@ -419,13 +419,13 @@ __global__ void __launch_bounds__(32 * kWarps, 5) advec_cell_y_kernel(const __gr
     CL_LOOP(NAME##1);                                                                                          \
     __device__ void operator()(const D &vol_flux, const D &volume, const D &vertexd, const D &density,         \
                                const D &energy, const D &vol_flux_t, D &mass_flux, D &dout, D &eout) const;    \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<true>); }  \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO, KERNEL<true>>(lp, s); }  \
   };                                                                                                           \
   struct NAME##2 {                                                                                             \
     CL_LOOP(NAME##2);                                                                                          \
     __device__ void operator()(const D &vol_flux, const D &volume, const D &vertexd, const D &density,         \
                                const D &energy, D &mass_flux, D &dout, D &eout, D &d0out) const;               \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<false>); } \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO, KERNEL<false>>(lp, s); } \
   };
 ADVEC_CELL(advec_cell_fused_x, 28, 0, advec_cell_x_kernel)
 ADVEC_CELL(advec_cell_fused_y, 32, 3, advec_cell_y_kernel)
@@ -576,13 +576,13 @@ __global__ void __launch_bounds__(32 * kWarps, 4) advec_mom_y_kernel(const __gri
     CL_LOOP(NAME##1);                                                                                            \
     __device__ void operator()(const D &mass_flux, const D &volume, const D &celld, const D &density,            \
                                const D &xvel, const D &yvel, D &xout, D &yout, const D &vol_flux_t) const;       \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<true>); }    \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO, KERNEL<true>>(lp, s); }    \
   };                                                                                                             \
   struct NAME##2 {                                                                                               \
     CL_LOOP(NAME##2);                                                                                            \
     __device__ void operator()(const D &mass_flux, const D &volume, const D &celld, const D &density,            \
                                const D &xvel, const D &yvel, D &xout, D &yout) const;                            \
-    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO>(lp, s, KERNEL<false>); }   \
+    static void launch(const LoopParams &lp, dim3, dim3, cudaStream_t s) { launch_strips<OWN, HALO, KERNEL<false>>(lp, s); }   \
   };
 ADVEC_MOM(advec_mom_fused_x, 28, 1, advec_mom_x_kernel)
 ADVEC_MOM(advec_mom_fused_y, 31, 3, advec_mom_y_kernel)
