@@ -179,7 +179,10 @@ int ops_b200_dat_release_raw_data(int dat, int acc);
  * "fcg_chunks": the flexible-CG heat solves with the learned or the Jacobi
  * preconditioner replay their iterations from CUDA graphs in chunks with the
  * stopping and restart tests on the device (1, default) or run the host loop,
- * one round trip per iteration (0); both give the same iterates. */
+ * one round trip per iteration (0); both give the same iterates.
+ * "heat_wait_ms": how long, in milliseconds (default 2000), a thread block of
+ * the one-kernel PCG loop of small 2D grids waits for another before the
+ * solve ends with a timeout error; 0 lets no wait succeed. */
 int ops_b200_set_option(const char *name, int value);
 /* Counters since the last reset: kernels launched by this library, CUDA
  * graphs launched, loops queued. */

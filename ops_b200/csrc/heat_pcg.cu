@@ -18,6 +18,7 @@
 // fired every later kernel returns at entry, so a chunk of iterations that
 // runs past convergence costs only its launch latency.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -470,30 +471,33 @@ __global__ void __launch_bounds__(NT, kResident) k_to_float(Geom g, Geom g32, co
 //
 // A value travels as two 64-bit words, each with half of it and the number of
 // the exchange, so a reader knows a whole value without a fence or a counter;
-// two slots alternate, since a CTA can be one exchange ahead of another. The CTAs wait for one another, so the launch is cooperative, and
-// every wait ends after two seconds with an error.
-constexpr unsigned long long kWaitNs = 2000000000ull;
+// two slots alternate, since a CTA can be one exchange ahead of another. The
+// CTAs wait for one another, so the launch is cooperative, and a wait ends with
+// an error after the time given (option heat_wait_ms; at 0 every wait ends so):
+// the first of a CTA's that does ends the others of that CTA too, and an
+// expired CTA leaves u, r and p as they were.
 
 __device__ __forceinline__ void ll_put(ulonglong2 *slot, double v, unsigned tag) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
   asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
                : "memory");
 }
-// The value tagged `tag`; false when it did not arrive in time.
-__device__ __forceinline__ bool ll_get(const ulonglong2 *slot, unsigned tag, double *v) {
+// The value tagged `tag`, or 0 with `expired` set when it did not arrive in time
+// or another wait of the CTA had expired.
+__device__ __forceinline__ double ll_get(const ulonglong2 *slot, unsigned tag, unsigned long long wait_ns,
+                                         volatile int *expired) {
   unsigned long long t0 = 0;
   for (unsigned i = 0;; i++) {
     unsigned long long a, b;
     asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(slot) : "memory");
-    if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag) {
-      *v = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
-      return true;
-    }
+    if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag)
+      return __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
     if ((i & 255u) == 255u) {
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (!t0) t0 = now;
-      else if (now - t0 > kWaitNs) return false;
+      else if (now - t0 > wait_ns) *expired = 1;
+      if (*expired) return 0.0;
     }
   }
 }
@@ -502,7 +506,8 @@ template <class T, int Z, int STOP, int K>
 __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restrict__ Kx, const T *__restrict__ Ky,
                                                         T *__restrict__ p, T *__restrict__ r, const T *__restrict__ Mi,
                                                         T *__restrict__ u, T *__restrict__ zout, T rx, T ry, int gx,
-                                                        Scalars *s, ulonglong2 *slots, int *err) {
+                                                        Scalars *s, ulonglong2 *slots, unsigned long long wait_ns,
+                                                        int *err) {
   constexpr int NV = (STOP == STOP_TRUE && Z != Z_R) ? 2 : 1;
   __shared__ T ps[2 * K + 2][BX + 2];
   __shared__ double ws[NV * K][kWarps], sm[kWarps], tot[2];
@@ -518,6 +523,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
   const int max_iters = s->max_iters;
   const double stop = s->stop, ref = s->ref;
   if (t == 0) expired = 0;
+  // with no time to wait, the waits are for tags that nothing sets
+  const unsigned never = wait_ns ? 0u : 1u << 31;
 
   T kx0[K], kx1[K], ky0[K], ky1[K], d[K], mi[K], rv[K], uv[K], pv[K], zv[K], wv[K];
   auto row = [&](int k) { return y0 + 2 * k + ty; };
@@ -600,11 +607,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
 #pragma unroll
     for (int n = 0; n < N; n++) {
       double v = 0.0;
-      for (int b = t; b < nb; b += NT) {
-        double q = 0.0;
-        if (!ll_get(buf + (size_t)n * kTargetBlocks + b, tag, &q)) expired = 1;
-        v += q;
-      }
+      for (int b = t; b < nb; b += NT) v += ll_get(buf + (size_t)n * kTargetBlocks + b, tag ^ never, wait_ns, &expired);
       v = block_sum(v, sm);
       if (t == 0) tot[n] = v;
     }
@@ -663,15 +666,8 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
         if (tx == BX - 1) ll_put(edge(bx, by, 2 * BX + 2 * K + q, buf), zd, tag);
       }
       total(acc, std::integral_constant<int, NV>{}, tag, [&] {
-        double z = 0.0;
-        if (hv.live) {
-          if (!ll_get(hv.from + (size_t)buf * kEdge, tag, &z)) expired = 1;
-          hv.z = (T)z;
-        }
-        if (hs.live) {
-          if (!ll_get(hs.from + (size_t)buf * kEdge, tag, &z)) expired = 1;
-          hs.z = (T)z;
-        }
+        if (hv.live) hv.z = (T)ll_get(hv.from + (size_t)buf * kEdge, tag ^ never, wait_ns, &expired);
+        if (hs.live) hs.z = (T)ll_get(hs.from + (size_t)buf * kEdge, tag ^ never, wait_ns, &expired);
       });
     }
     if (expired) break;
@@ -685,6 +681,10 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
     else if (STOP == STOP_RELIABLE && e < ref) done = 3;
     else if (iters >= max_iters) done = 2;
     if (done) break;
+  }
+  if (expired) {
+    if (t == 0) *err = 1;
+    return;
   }
 #pragma unroll
   for (int k = 0; k < K; k++) {
@@ -705,7 +705,6 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
     s->iters = iters;
     s->done = done;
   }
-  if (t == 0 && expired) *err = 1;
 }
 
 // ---- flexible CG -----------------------------------------------------------
@@ -1045,6 +1044,16 @@ void check_launch(const char *what) {
 
 }  // namespace
 
+// "heat_wait_ms" option: how long a block of k_pcg_resident waits for another.
+static std::atomic<int> &wait_ms() {
+  static std::atomic<int> ms{2000};
+  return ms;
+}
+void set_wait_ms(int ms) {
+  if (ms < 0) throw Error(E_ARG, "heat_wait_ms must be >= 0");
+  wait_ms() = ms;
+}
+
 struct Solver::Impl {
   Scalars *s64 = nullptr, *s32 = nullptr;
   double *part = nullptr;
@@ -1109,7 +1118,8 @@ struct Solver::Impl {
                            : (const void *)k_pcg_resident<T, Z, STOP, 8>;
     Geom gg = g;
     int gxx = gx;
-    void *args[] = {&gg, &Kx, &Ky, &p, &r, &Mi, &u, &zout, &rx, &ry, &gxx, &s, &slots, &err};
+    unsigned long long wait_ns = (unsigned long long)wait_ms() * 1000000ull;
+    void *args[] = {&gg, &Kx, &Ky, &p, &r, &Mi, &u, &zout, &rx, &ry, &gxx, &s, &slots, &wait_ns, &err};
     OPSB_CUDA(cudaLaunchCooperativeKernel(f, dim3(gx * ((gy + K - 1) / K)), dim3(BX, BY), args, 0, st));
     OPSB_CUDA(cudaMemcpyAsync(h_flag, err, sizeof(int), cudaMemcpyDeviceToHost, st));
     OPSB_CUDA(cudaStreamSynchronize(st));

@@ -62,6 +62,11 @@ struct SolveStats {
   double true_residual = 0;    // ||u0 - A u|| at exit, FP64
 };
 
+// Limit of the waits between the blocks of a small grid's one-kernel loop, in
+// milliseconds (2000 by default); a solve whose wait expires ends with
+// E_TIMEOUT. 0 lets no wait succeed.
+void set_wait_ms(int ms);
+
 class Solver {
  public:
   Solver();

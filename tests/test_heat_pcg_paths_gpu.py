@@ -98,3 +98,29 @@ assert kept < 6.5 * field + levels, (kept, field)
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("method", ["PCG_TRUE", "MIXED"])
+def test_expired_wait_is_an_error_and_the_solver_goes_on(gpu_runtime, method):
+    """No wait of the one-kernel loop may succeed (heat_wait_ms 0): the solve
+    ends with a timeout, leaves u as it was, and the next one is as ever."""
+    import torch
+
+    from ops_b200 import _lib, lmg
+    from ops_b200 import ops as O
+    rng = np.random.default_rng(3)
+    rho = np.exp(rng.uniform(np.log(0.1), np.log(10.0), (140, 300)))
+    k = [torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in lmg.padded_problem(rho, rho)]
+    u, v = k[2].clone(), k[2].clone()
+    lmg.solve(*k, u, 20.0, 20.0, method=getattr(lmg, method), eps=1e-10)
+    O.set_option("heat_wait_ms", 0)
+    try:
+        with pytest.raises(_lib.OpsError, match="wait between thread blocks expired"):
+            lmg.solve(*k, v, 20.0, 20.0, method=getattr(lmg, method), eps=1e-10)
+    finally:
+        O.set_option("heat_wait_ms", 2000)
+    assert torch.equal(v, k[2])
+    lmg.solve(*k, v, 20.0, 20.0, method=getattr(lmg, method), eps=1e-10)
+    assert torch.equal(u, v)
+    with pytest.raises(_lib.OpsError):
+        O.set_option("heat_wait_ms", -1)
