@@ -1,6 +1,6 @@
 """The Jacobi-PCG loops of the heat solver at the edges of their kernels: the
-one-kernel loop (tiles of 128 x 2 cells, 1 to 8 of them a CTA, grids up to 1184
-tiles) and the two-kernel loop beyond it (strips of 30 columns), FP64 and
+one-kernel loop (tiles of 128 x 2 cells, 1, 2, 4 or 8 of them a CTA, one CTA an
+SM) and the two-kernel loop beyond it (strips of 30 columns), FP64 and
 mixed. Held to the FP64 residual recomputed by numpy and, as far as the two
 residuals allow them to differ, to the solution of the flexible CG with
 Jacobi (other kernels, the same solve)."""
@@ -17,12 +17,21 @@ def residual(Kx, Ky, u, u0, rx):
                     - rx * (Kx[e] * u[e] + Kx[c] * u[w]))
 
 
-# nx, ny: one cell; a tile's last column and the next CTA's first; 2, 4 and 8
-# tiles a CTA with ragged ends; the largest grid of the one-kernel loop (8 x
-# 148 tiles) and the first beyond it; strips of 30, 31 and 61 columns; more
-# strips than 4096 CTAs hold
+def one_kernel(nx, ny):
+    """Whether the grid's tiles fit one CTA an SM, 8 to a CTA at most."""
+    import torch
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    gx, gy = -(-nx // 128), -(-ny // 2)
+    return gx * gy <= 1184 and any(gx * -(-gy // k) <= sms for k in (1, 2, 4, 8))
+
+
+# nx, ny: one cell; a tile's last column and the next CTA's first; 1, 2, 4 and 8
+# tiles a CTA, with ragged ends; on 148 SMs the tallest grid of the one-kernel
+# loop 8 tiles wide (8 x 144) and the first beyond it; strips of 30, 31 and 61
+# columns; more strips than 4096 CTAs hold
 @pytest.mark.parametrize("nx,ny", [(1, 1), (128, 2), (129, 3), (127, 33), (61, 600), (257, 301), (1024, 296),
-                                   (1024, 298), (31, 2400), (150, 1190), (1230, 61), (990001, 2)])
+                                   (1024, 298), (31, 2400), (150, 1190), (1230, 61), (990001, 2), (256, 192),
+                                   (500, 511), (1024, 288), (1024, 290)])
 @pytest.mark.parametrize("method", ["PCG_TRUE", "PCG", "MIXED"])
 def test_loops_reach_the_residual(gpu_runtime, nx, ny, method):
     import torch
@@ -40,6 +49,10 @@ def test_loops_reach_the_residual(gpu_runtime, nx, ny, method):
     st = lmg.solve(*k, u, 20.0, 20.0, method=getattr(lmg, method), eps=1e-10)
     ref = lmg.solve(*k, v, 20.0, 20.0, method=lmg.FCG_JACOBI, eps=1e-12)
     assert st["converged"] and ref["converged"]
+    # the one-kernel loop is one launch, between the set-up's two and the residual (mixed: for each
+    # update the restart, the loop, the update and the residual); a chunk of the other loop is 32
+    whole = 2 + 4 * st["updates"] if method == "MIXED" else 4
+    assert st["launches"] == whole if one_kernel(nx, ny) else st["launches"] >= whole + 31
     a, b = u.cpu().numpy(), v.cpu().numpy()
     r = np.linalg.norm(residual(Kx, Ky, a, u0, 20.0))
     # PCG stops on sqrt|r.z| < eps ||r0|| (TeaLeaf's rule), so ||r|| < sqrt(max D) eps ||r0|| with

@@ -105,11 +105,25 @@ def test_python_api_path_matches_oracle(gpu_runtime, orc, graphs, fusion):
 
 
 @pytest.mark.parametrize("x0", [-1, 0, 1])
-@pytest.mark.parametrize("nx", [0, 1, 2, 59, 60, 61, 120, 121])
+@pytest.mark.parametrize("nx", [0, 1, 2, 59, 60, 61, 120, 121, 63, 64, 65, 511, 512, 513])
 @pytest.mark.parametrize("ny", [1, 2, 9, 70])
 def test_sweep_on_part_of_a_dat(gpu_runtime, x0, nx, ny):
-    """The sweep at its strips' edges (60 columns) on aligned and odd starts,
-    up to the dat's last readable points: bit-exact, nothing else written."""
+    """The sweep at the edges of its warps (64 columns) and CTAs (512) on
+    aligned and odd starts, up to the dat's last readable points: bit-exact,
+    nothing else written."""
+    sweep_part(x0, nx, ny)
+
+
+@pytest.mark.parametrize("x0", [0, 1])
+@pytest.mark.parametrize("nx,ny", [(130, 2368), (130, 2369), (130, 2375), (130, 4736), (130, 4737), (130, 4743),
+                                   (514, 1184), (514, 1185), (1500, 1500)])
+def test_sweep_rows_per_cta(gpu_runtime, x0, nx, ny):
+    """Either side of the lines between 4, 8 and 32 rows a CTA (592 CTAs), with
+    whole last CTAs and ones of a single row to one less than whole."""
+    sweep_part(x0, nx, ny)
+
+
+def sweep_part(x0, nx, ny):
     rng = np.random.default_rng(nx * 100 + ny + x0)
     f = rng.standard_normal((ny + 2, nx + x0 + 3))
     blk = O.ops_decl_block(2, "part")
