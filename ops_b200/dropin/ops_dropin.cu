@@ -341,7 +341,8 @@ ops_dat ops_decl_dat_char(ops_block block, int dim, int *size, int *base, int *d
     d->mem = host_bytes(d);
     d->data = static_cast<char *>(calloc(d->mem, 1));
     if (data) memcpy(d->data, data, d->mem);
-    d->data_d = r.data_d;
+    d->data_d = r.data_d;  // the application may write there by itself: the zeros must have landed
+    opsb::cuda_check(cudaStreamSynchronize(rt().stream()), "ops_decl_dat");
     d->name = dup(name);
     d->type = dup(type);
     d->user_managed = data != nullptr;
