@@ -180,9 +180,10 @@ int ops_b200_dat_release_raw_data(int dat, int acc);
  * preconditioner replay their iterations from CUDA graphs in chunks with the
  * stopping and restart tests on the device (1, default) or run the host loop,
  * one round trip per iteration (0); both give the same iterates.
- * "heat_wait_ms": how long, in milliseconds (default 2000), a thread block of
- * the one-kernel PCG loop of small 2D grids waits for another before the
- * solve ends with a timeout error; 0 lets no wait succeed. */
+ * "heat_wait_ms": how long, in milliseconds (default 2000), a thread of the
+ * one-kernel PCG loop of small 2D grids waits for another block's value before
+ * the solve ends with a timeout error (u, the solution, is then as it was); 0
+ * lets every wait run out. */
 int ops_b200_set_option(const char *name, int value);
 /* Counters since the last reset: kernels launched by this library, CUDA
  * graphs launched, loops queued. */

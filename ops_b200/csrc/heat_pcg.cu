@@ -473,31 +473,33 @@ __global__ void __launch_bounds__(NT, kResident) k_to_float(Geom g, Geom g32, co
 // the exchange, so a reader knows a whole value without a fence or a counter;
 // two slots alternate, since a CTA can be one exchange ahead of another. The
 // CTAs wait for one another, so the launch is cooperative, and a wait ends with
-// an error after the time given (option heat_wait_ms; at 0 every wait ends so):
-// the first of a CTA's that does ends the others of that CTA too, and an
-// expired CTA leaves u, r and p as they were.
+// an error after the limit given (option heat_wait_ms; at 0 nothing is published
+// and every wait runs out). A thread takes no further value of a sum then, so its
+// CTA stops within four limits, and leaves u, r and p as they were.
 
 __device__ __forceinline__ void ll_put(ulonglong2 *slot, double v, unsigned tag) {
   const unsigned long long b = (unsigned long long)__double_as_longlong(v), t = (unsigned long long)tag << 32;
   asm volatile("st.volatile.global.v2.u64 [%0], {%1, %2};" ::"l"(slot), "l"(t | (b & 0xffffffffull)), "l"(t | (b >> 32))
                : "memory");
 }
-// The value tagged `tag`, or 0 with `expired` set when it did not arrive in time
-// or another wait of the CTA had expired.
-__device__ __forceinline__ double ll_get(const ulonglong2 *slot, unsigned tag, unsigned long long wait_ns,
-                                         volatile int *expired) {
+// The value tagged `tag`; false when it did not arrive in time. (How often the
+// loop polls decides how soon values travel: 128^2 to 550^2 moved by up to 25 %
+// with the shape of this loop and its callers, on the same machine. This one and
+// a compile-time limit measure the same; a flag to leave early costs 5 to 10 %.)
+__device__ __forceinline__ bool ll_get(const ulonglong2 *slot, unsigned tag, double *v, unsigned long long wait_ns) {
   unsigned long long t0 = 0;
   for (unsigned i = 0;; i++) {
     unsigned long long a, b;
     asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(slot) : "memory");
-    if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag)
-      return __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+    if ((unsigned)(a >> 32) == tag && (unsigned)(b >> 32) == tag) {
+      *v = __longlong_as_double((long long)((a & 0xffffffffull) | (b << 32)));
+      return true;
+    }
     if ((i & 255u) == 255u) {
       unsigned long long now;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
       if (!t0) t0 = now;
-      else if (now - t0 > wait_ns) *expired = 1;
-      if (*expired) return 0.0;
+      else if (now - t0 > wait_ns) return false;
     }
   }
 }
@@ -516,6 +518,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
   const int tx = threadIdx.x, ty = threadIdx.y, t = tid_(), lane = t & 31, warp = t >> 5;
   const int bx = blockIdx.x % gx, by = blockIdx.x / gx, y0 = by * 2 * K, x = bx * BX + tx;
   const int gy = (g.ny + BY - 1) / BY, nb = gx * gy;  // the launched kernels' blocks
+  const int put_rows = wait_ns ? gy : 0;  // with no time to wait, nothing is published
   const long long P = g.pitch;
   const bool first = s->iters == 0;
   double rro = s->rro, rro_prev = s->rro_prev, alpha = s->alpha, beta = s->beta, pw = s->pw, e = s->err;
@@ -523,8 +526,6 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
   const int max_iters = s->max_iters;
   const double stop = s->stop, ref = s->ref;
   if (t == 0) expired = 0;
-  // with no time to wait, the waits are for tags that nothing sets
-  const unsigned never = wait_ns ? 0u : 1u << 31;
 
   T kx0[K], kx1[K], ky0[K], ky1[K], d[K], mi[K], rv[K], uv[K], pv[K], zv[K], wv[K];
   auto row = [&](int k) { return y0 + 2 * k + ty; };
@@ -601,13 +602,20 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
       const int k = q % K, vb = y0 / 2 + k;
-      if (lane == 0 && vb < gy) ll_put(buf + (size_t)(q / K) * kTargetBlocks + bx + vb * gx, v, tag);
+      if (lane == 0 && vb < put_rows) ll_put(buf + (size_t)(q / K) * kTargetBlocks + bx + vb * gx, v, tag);
     }
     meanwhile();
 #pragma unroll
     for (int n = 0; n < N; n++) {
       double v = 0.0;
-      for (int b = t; b < nb; b += NT) v += ll_get(buf + (size_t)n * kTargetBlocks + b, tag ^ never, wait_ns, &expired);
+      for (int b = t; b < nb; b += NT) {
+        double q = 0.0;
+        if (!ll_get(buf + (size_t)n * kTargetBlocks + b, tag, &q, wait_ns)) {
+          expired = 1;
+          break;
+        }
+        v += q;
+      }
       v = block_sum(v, sm);
       if (t == 0) tot[n] = v;
     }
@@ -666,8 +674,15 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
         if (tx == BX - 1) ll_put(edge(bx, by, 2 * BX + 2 * K + q, buf), zd, tag);
       }
       total(acc, std::integral_constant<int, NV>{}, tag, [&] {
-        if (hv.live) hv.z = (T)ll_get(hv.from + (size_t)buf * kEdge, tag ^ never, wait_ns, &expired);
-        if (hs.live) hs.z = (T)ll_get(hs.from + (size_t)buf * kEdge, tag ^ never, wait_ns, &expired);
+        double z = 0.0;
+        if (hv.live) {
+          if (!ll_get(hv.from + (size_t)buf * kEdge, tag, &z, wait_ns)) expired = 1;
+          hv.z = (T)z;
+        }
+        if (hs.live) {
+          if (!ll_get(hs.from + (size_t)buf * kEdge, tag, &z, wait_ns)) expired = 1;
+          hs.z = (T)z;
+        }
       });
     }
     if (expired) break;
@@ -682,20 +697,16 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
     else if (iters >= max_iters) done = 2;
     if (done) break;
   }
-  if (expired) {
-    if (t == 0) *err = 1;
-    return;
-  }
 #pragma unroll
   for (int k = 0; k < K; k++) {
-    if (!cell(x, row(k))) continue;
+    if (!cell(x, row(k)) || expired) continue;
     const long long i = (long long)row(k) * P + x;
     u[i] = uv[k];
     r[i] = rv[k];
     p[i] = pv[k];
     if (zout) zout[i] = zv[k];
   }
-  if (blockIdx.x == 0 && t == 0) {
+  if (blockIdx.x == 0 && t == 0 && !expired) {
     s->rro = rro;
     s->rro_prev = rro_prev;
     s->alpha = alpha;
@@ -705,6 +716,7 @@ __global__ void __launch_bounds__(NT, 1) k_pcg_resident(Geom g, const T *__restr
     s->iters = iters;
     s->done = done;
   }
+  if (t == 0 && expired) *err = 1;
 }
 
 // ---- flexible CG -----------------------------------------------------------
