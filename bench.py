@@ -296,12 +296,12 @@ CL_N = 3840
 #     (profiles/fused_loops_dram.md)
 #   Laplace apply_stencil at 4096^2: 227.4 MB per launch / 4096^2
 #     (profiles/laplace2d_4096_apply_stencil_dram.md)
-#   ADI 256^3 FP64 x / y / z sweeps: 649.6 / 765.5 / 909.6 MB per sweep / 256^3
+#   ADI 256^3 FP64 x / y / z sweeps: 649.8 / 733.8 / 878.2 MB per sweep / 256^3
 #     (profiles/fused_loops_dram.md)
 # Traffic grows with the cells (or unknowns) a launch processes, so a
 # launch's traffic is the figure times its cells.
 TRAFFIC_PER_CELL = {"clover": 116.0, "clover3d": 169.1, "laplace": 227.4e6 / 4096 ** 2,
-                    "adi_cube_fp64": (649.6e6 / 256 ** 3, 765.5e6 / 256 ** 3, 909.6e6 / 256 ** 3)}
+                    "adi_cube_fp64": (649.8e6 / 256 ** 3, 733.8e6 / 256 ** 3, 878.2e6 / 256 ** 3)}
 
 
 def clover_deck(steps, n=CL_N):

@@ -371,8 +371,9 @@ void Multigrid::setup(int nx, int ny, long long pitch, const double *Kx, const d
     release();
     OPSB_CUDA(cudaMalloc(&buf_, elems * sizeof(float)));
     buf_elems_ = elems;
-    // the cycle never reads the padding columns; they are zeroed once so
-    // that every word of the storage is defined
+    // the cycle loads padding columns beside a row's last cell and masks what
+    // it makes of them; they are zeroed once, since a product with a mask of 0
+    // needs a finite factor
     OPSB_CUDA(cudaMemsetAsync(buf_, 0, elems * sizeof(float), s));
   }
   float *q = buf_;

@@ -457,14 +457,16 @@ __global__ void __launch_bounds__(NT, kResident) k_to_float(Geom g, Geom g32, co
 
 
 // ---- the whole loop in one kernel, for grids that fit the registers ---------
-// Up to kTargetBlocks blocks of 128 x 2 cells (303 K cells, 550^2) an iteration
-// of the two kernels above is launch and drain latency: 14 us at 128^2, 17 us
-// at 512^2. Here a CTA keeps K such blocks, one above the other: its cells' r,
+// On small grids an iteration of the two kernels above is launch and drain
+// latency: 14 us at 128^2, 17 us at 512^2. Grids of up to kTargetBlocks blocks of
+// 128 x 2 cells that fit one CTA an SM, 8 to a CTA (on 148 SMs up to 512^2 or 1024
+// x 288), take one kernel. Here a CTA keeps K such blocks, one above the other: its cells' r,
 // u and coefficients stay in registers, the direction p in shared memory with a
 // one-cell halo, for the whole loop. CTAs exchange only z along their edges
 // and the partial sums (a neighbour's p is beta p + z, tracked in the halo):
 // 64^2 14.1 -> 3.7 us an iteration, 128^2 14.0 -> 4.5, 256^2 14.2 -> 5.4, 512^2
-// 17.3 -> 10.8 (FP64).
+// 17.3 -> 10.8 (FP64; 128^2 took 3.5 us on one B200 and 5.2 on another, 500 x 511
+// 8.0 and 11.4).
 // Each block's partial is its own, and the totals are taken, in the order that
 // the launched kernels use (publish, grid_total), so alpha, beta and every
 // iterate are the same bits as an iteration of single-cell threads gave.

@@ -1,13 +1,13 @@
 // CloverLeaf 3D: the hydro cycle's loops fused by hand, queued by the app
 // driver (apps_clover3d.cpp) in place of runs of the reference's loops, as
 // kernels_clover_fused.cu does in 2D: volumes, node masses, node fluxes,
-// energy and momentum fluxes stay in registers, and a step moves about 1000 B
-// per cell in 13 launches (plus boundary copies) instead of 2565 B in some 60.
-// Every value is computed by the reference's expressions in the reference's
+// energy and momentum fluxes stay in registers, and a step moves 1090 B per
+// cell in 12 launches (and 57 B in boundary copies) instead of 2565 B in some
+// 60. Every value is computed by the reference's expressions in the reference's
 // order, so fields and dt are the same bits; the summary's sums are taken in
-// another order. Measured at 256^3: 12.4 -> 7.7 ms of kernels a step, a
-// 4-step run with its set-up 58.5 -> 36.9 ms; with every march's loads issued
-// one row ahead of their use (Raw, Row below) 32.0 ms.
+// another order. Measured at 256^3: 12.4 -> 5.65 ms of kernels a step, copies
+// included, a 4-step run with its set-up 58.9 -> 30.5 ms (36.9 before every
+// march's loads were issued one row ahead of their use: Raw, Row below).
 //
 // Each warp marches along y or z with one column of x per lane: the marched
 // axis's neighbours are kept from row to row, x neighbours come by shuffles,
@@ -93,7 +93,7 @@ struct March {
 // HALO: rows a march reads beyond its own.
 template <int OWN, int M, int HALO, auto kernel>
 void launch_march(const LoopParams &lp, cudaStream_t s) {
-  static int per_sm = 0;  // resident CTAs, per kernel
+  static int per_sm = 0;  // resident CTAs, this kernel's
   if (!per_sm) {
     int n = 0;
     OPSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, 32 * kWarps, 0));

@@ -6,11 +6,14 @@
 // 1595 B per cell and step in 43 launches. None of those outlive the step, so
 // each kernel here computes them in registers and moves only the fields that
 // the next kernel needs: 608 B per cell and step in 9 launches plus the
-// boundary copies. Measured at 3840^2: 4.9 -> 2.37 ms of kernels a step, a
-// whole 10-step run 58.5 -> 26.1 ms (250 x 187: 14.1 -> 3.5 ms, half the
-// launches, and a queue the planner passes over). Every value is computed by the reference's expressions in
-// the reference's order (clover_flux.cuh, --fmad=false), so fields and dt are
-// the same bits.
+// boundary copies. Measured at 3840^2: 4.75 -> 2.28 ms of kernels a step, copies
+// included, a whole 10-step run with its set-up 59.0 -> 25.8 ms (250 x 187:
+// 14.2 -> 3.5 ms, half the launches, and a queue the planner passes over). Every
+// value is computed by the reference's expressions in the reference's order
+// (clover_flux.cuh, --fmad=false), so fields and dt are the same bits.
+// The sweeps wait for their loads: 70 to 102 registers a thread leave 24 to 39 %
+// of an SM's warps, which issue in 32 to 52 % of the cycles, the FP64 pipe 14 to
+// 28 % busy.
 //
 // The stencil loops march up columns. A warp owns a strip of columns, one per
 // lane, and keeps the rows it needs in registers: values of other rows come

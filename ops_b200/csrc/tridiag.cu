@@ -345,7 +345,9 @@ __global__ void __launch_bounds__(kTileThreads, kCtasPerSm) trid_tile_kernel(con
 // lines' 4 n loads in flight at once. Its time is its instructions (FP64 chains
 // and reduction steps): with the short reciprocal and one of them a reduced row
 // and step instead of two, 256^3 FP64 0.248 -> 0.168 ms, FP32 0.135 -> 0.120, the
-// 64-block batch 0.837 -> 0.587 and 0.480 -> 0.402.
+// 64-block batch 0.837 -> 0.587 and 0.480 -> 0.402, each sweep repeated by itself.
+// Right after a z sweep, as in an ADI step, 256^3 FP64 takes 0.205 ms and the FP64
+// batch 0.748.
 constexpr int kWarpLines = 8;  // warps per CTA
 
 template <int R>
@@ -542,10 +544,10 @@ __global__ void __launch_bounds__(32 * kWarpLines, sizeof(T) == 4 ? 3 : 2)
 // (kScratchBytes; a CTA an SM at least), each warp reuses its own part group after
 // group, the scratch is marked evict-last and everything else evict-first. HBM then sees the
 // compulsory 40 B per FP64 unknown (48 with _Inc). With every line in flight
-// the scratch went through HBM too (68 to 77 B). 256^3 FP64: y sweep 0.213 ->
-// 0.167 ms, z sweep (_Inc) 0.289 -> 0.209 ms; the 64-block batch's 0.548 -> 0.478
-// and 0.655 -> 0.544 ms, in FP32 0.297 -> 0.273 and 0.432 -> 0.307 ms. Scratches of
-// 60 to 400 MB measured within 7 % of one another, 40 MB 1.3x slower.
+// the scratch went through HBM too (68 to 77 B; now 43.7 and 52.3). In an ADI step
+// at 256^3 FP64: y sweep 0.213 -> 0.162 ms, z sweep (_Inc) 0.289 -> 0.209 ms; the
+// 64-block FP64 batch's 0.548 -> 0.443 and 0.655 -> 0.497 ms. Limits of 60 to 400 MB
+// measured within 7 % of one another, 40 MB 1.3x slower.
 constexpr size_t kScratchBytes = 64ull << 20;
 
 __device__ __forceinline__ uint64_t policy_last() {
@@ -601,7 +603,7 @@ __device__ __forceinline__ int magnitude(float x) { return __float_as_int(x) & 0
 // elimination from the bottom is as sound as the rows are; a line whose c' pass
 // it (a vanished pivot leaves infinity or NaN) is solved again from the top
 // alone, a lane a line, in the two lanes' scratch. Diagonally dominant rows
-// have |c'| <= 1.
+// have |c'| <= 1. (The maximum costs 0.1 to 0.2 % of an ADI step.)
 constexpr float kGrowth = 16.0f;
 constexpr int kLineThreads = 128, kLineRows = 8, kLineStages = 3;
 
