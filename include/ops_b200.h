@@ -452,7 +452,8 @@ typedef struct ops_b200_trid_system {
 } ops_b200_trid_system;
 
 /* Solves all lines along `solvedim` of `nsys` system sets, of any shapes, in
- * one launch (elem_size 8 = double, 4 = float) on `stream` (cudaStream_t,
+ * one launch, or two where y/z lines of up to 16 rows (32 in FP32) come in
+ * great number beside longer ones (elem_size 8 = double, 4 = float) on `stream` (cudaStream_t,
  * NULL = default stream). Lines along x (contiguous) run the partition
  * method in shared memory, up to 512 points; lines along y/z (strided,
  * neighbouring lines contiguous) are eliminated from both ends at once, any

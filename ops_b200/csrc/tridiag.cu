@@ -786,6 +786,78 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
   }
 }
 
+// Short lines in great number. A group of the line kernel costs the latency of
+// its stages and exchanges however few its rows are, and an SM has few groups
+// in flight. Here a thread solves a line, from the top: its 4 N coefficients are
+// all loaded at once, c' and d' take their place in registers, and nothing else
+// moves. 1,000,000 lines, FP64: of 3 rows 24 us against 135 in the line kernel, of
+// 7 rows 61 against 163, of 16 rows 118 against 182; FP32 of 7 rows 28 against 114,
+// of 32 rows 159 against 193. In FP64 20 rows no longer fit the registers (_Inc 295
+// us against 257).
+template <class T>
+constexpr int kShortRows = sizeof(T) == 4 ? 32 : 16;
+// From a line for every thread of a CTA an SM on; below that the two are alike up
+// to 8 rows, and the line kernel's two lanes a line are faster beyond.
+constexpr long long kShortLines = 148LL * kLineThreads;
+
+template <class T, int N>
+__global__ void __launch_bounds__(kLineThreads) trid_short_kernel(const Sys *__restrict__ sys, int nsys,
+                                                                  long long lines) {
+  for (long long g = (long long)blockIdx.x * kLineThreads + threadIdx.x; g < lines;
+       g += (long long)gridDim.x * kLineThreads) {
+    int lo = 0, hi = nsys - 1;  // last system whose first line is <= g
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (sys[mid].line0 <= g) lo = mid;
+      else hi = mid - 1;
+    }
+    const Sys &s = sys[lo];
+    const long long l = g - s.line0, base = (l % s.nl0) * s.s0 + (l / s.nl0) * s.s1, ss = s.ss;
+    const int n = s.n;
+    const T *a = reinterpret_cast<const T *>(s.a) + base, *b = reinterpret_cast<const T *>(s.b) + base;
+    const T *c = reinterpret_cast<const T *>(s.c) + base;
+    T *d = reinterpret_cast<T *>(s.d) + base;
+    T *u = s.u ? reinterpret_cast<T *>(s.u) + base : nullptr;
+    T v[N][4];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if (i < n) {
+        v[i][0] = i ? __ldcs(a + i * ss) : T(0);
+        v[i][1] = __ldcs(b + i * ss);
+        v[i][2] = __ldcs(c + i * ss);
+        v[i][3] = __ldcs((const T *)d + i * ss);
+      }
+    T cp[N], dp[N], x = T(0), pc = T(0);
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if (i < n) {
+        T r;
+        recip_times(v[i][1] - v[i][0] * pc, v[i][2], r, pc);
+        x = (v[i][3] - v[i][0] * x) * r;
+        cp[i] = pc;
+        dp[i] = x;
+      }
+    // x is the last row's
+    if (!u) {
+#pragma unroll
+      for (int i = N - 1; i >= 0; i--) {
+        if (i < n - 1) x = dp[i] - cp[i] * x;
+        if (i < n) __stcs(d + i * ss, x);
+      }
+      continue;
+    }
+    T w[N];
+#pragma unroll
+    for (int i = 0; i < N; i++)
+      if (i < n) w[i] = __ldcs(u + i * ss);
+#pragma unroll
+    for (int i = N - 1; i >= 0; i--) {
+      if (i < n - 1) x = dp[i] - cp[i] * x;
+      if (i < n) __stcs(u + i * ss, w[i] + x);
+    }
+  }
+}
+
 // Device copies of the work description, grown as needed.
 struct Buffers {
   Sys *sys = nullptr;
@@ -799,16 +871,27 @@ Buffers &buffers() {
   return b;
 }
 
-// The y/z sweeps (solve dimension strided, lines contiguous) by the line
-// kernel; returns false when some system does not have that shape.
+// The y/z sweeps (solve dimension strided, lines contiguous) by the line kernel,
+// and in great number the short ones by a launch of their own; returns false
+// when some system does not have that shape.
 template <class T>
 bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long long *kernels) {
-  std::vector<Sys> live;  // systems with no rows or no lines take no part
-  int maxn = 0;
+  std::vector<Sys> live, shorts;  // systems with no rows or no lines take no part
+  long long short_lines = 0;
+  int maxn = 0, short_n = 0;
   for (const Sys &s : systems) {
     if (s.ss == 1 || s.s0 != 1) return false;
     const long long nl = (long long)s.nl0 * s.nl1;
-    if (s.n <= 0 || nl <= 0) continue;
+    if (s.n <= 0 || s.n > kShortRows<T> || nl <= 0) continue;
+    shorts.push_back(s);
+    shorts.back().line0 = short_lines;
+    short_lines += nl;
+    short_n = std::max(short_n, s.n);
+  }
+  if (short_lines < kShortLines) shorts.clear();
+  for (const Sys &s : systems) {
+    const long long nl = (long long)s.nl0 * s.nl1;
+    if (s.n <= 0 || nl <= 0 || (s.n <= kShortRows<T> && !shorts.empty())) continue;
     maxn = std::max(maxn, s.n);
     for (int lines : {16, (int)(nl % 16)}) {
       if (lines == 0 || nl < lines) continue;
@@ -817,7 +900,7 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
       live.back().lofs = lines == 16 ? 0 : nl - nl % 16;
     }
   }
-  if (live.empty()) return true;
+  if (live.empty() && shorts.empty()) return true;
   // the groups that need the most scratch first: a warp's first group then
   // sizes its part of it, so that all of it is never more than every line's c' and d'
   std::stable_sort(live.begin(), live.end(), [](const Sys &x, const Sys &y) {
@@ -830,6 +913,31 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
     s.scr0 = all;
     groups += groups_of(s);
     all += groups_of(s) * group_scratch(s.n, s.glines);
+  }
+  const int nlive = (int)live.size(), nshort = (int)shorts.size();
+  live.insert(live.end(), shorts.begin(), shorts.end());
+  Buffers &B = buffers();
+  if (B.sys_cap < live.size()) {
+    if (B.sys) cudaFree(B.sys);
+    B.sys = nullptr;
+    B.sys_cap = 0;
+    const size_t cap = std::max<size_t>(live.size(), 64);
+    OPSB_CUDA(cudaMalloc(&B.sys, cap * sizeof(Sys)));
+    B.sys_cap = cap;
+  }
+  OPSB_CUDA(cudaMemcpyAsync(B.sys, live.data(), live.size() * sizeof(Sys), cudaMemcpyHostToDevice, stream));
+  live.resize(nlive);
+  if (nshort) {
+    const Sys *at = B.sys + nlive;
+    const unsigned grid = (unsigned)std::min<long long>((short_lines + kLineThreads - 1) / kLineThreads, 1 << 20);
+    if (short_n <= 4) trid_short_kernel<T, 4><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    else if (short_n <= 8) trid_short_kernel<T, 8><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    else if (short_n <= 12) trid_short_kernel<T, 12><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    else if (short_n <= 16) trid_short_kernel<T, 16><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    else trid_short_kernel<T, kShortRows<T>><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    OPSB_CUDA(cudaGetLastError());
+    if (kernels) (*kernels)++;
+    if (!nlive) return true;
   }
   static int per_sm = 0;  // resident threads, per type
   if (!per_sm) {
@@ -845,15 +953,6 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
   const long long fit = (long long)(kScratchBytes / line) / 148 / kLineThreads * kLineThreads;
   long long slots = 148 * std::max<long long>(kLineThreads, std::min<long long>(per_sm, fit));
   slots = std::min(slots, (32 * groups + kLineThreads - 1) / kLineThreads * kLineThreads);
-  Buffers &B = buffers();
-  if (B.sys_cap < live.size()) {
-    if (B.sys) cudaFree(B.sys);
-    B.sys = nullptr;
-    B.sys_cap = 0;
-    const size_t cap = std::max<size_t>(live.size(), 64);
-    OPSB_CUDA(cudaMalloc(&B.sys, cap * sizeof(Sys)));
-    B.sys_cap = cap;
-  }
   long long elems = 0, left = slots / 32;  // the first group's scratch of every warp
   for (const Sys &s : live) {
     elems += std::min(left, groups_of(s)) * group_scratch(s.n, s.glines);
@@ -867,9 +966,8 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
     OPSB_CUDA(cudaMalloc(&B.scr, need));
     B.scr_bytes = need;
   }
-  OPSB_CUDA(cudaMemcpyAsync(B.sys, live.data(), live.size() * sizeof(Sys), cudaMemcpyHostToDevice, stream));
   trid_line_kernel<T><<<(unsigned)(slots / kLineThreads), kLineThreads, kLineSmem<T>, stream>>>(
-      B.sys, (int)live.size(), groups, static_cast<T *>(B.scr));
+      B.sys, nlive, groups, static_cast<T *>(B.scr));
   OPSB_CUDA(cudaGetLastError());
   if (kernels) (*kernels)++;
   return true;

@@ -300,3 +300,35 @@ for (a, b, c, d), t in sets:
 """
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.parametrize("dtype,rtol", [(np.float64, 1e-12), (np.float32, 2e-4)])
+@pytest.mark.parametrize("inc", [False, True])
+@pytest.mark.parametrize("n", [1, 2, 4, 5, 8, 9, 15, 16, 17, 31, 32, 33])
+def test_short_lines_in_great_number(gpu_runtime, orc, dtype, rtol, inc, n):
+    """Short strided lines, more than one for every thread of a CTA an SM, at
+    the edges of their kernel's sizes, along y and along z, alone and beside
+    shorter and longer systems. a_0 and c_{n-1} are not read."""
+    import torch
+    for solvedim, shapes in ((1, [(3, n, 6500)]), (2, [(n, 200, 100)]),
+                             (1, [(1, n, 19000), (2, 70, 33), (1, 1, 5), (1, 3, 700), (1, n, 17)])):
+        sets, systems = [], []
+        for i, shape in enumerate(shapes):
+            a, b, c, d = seeded.trid_system(shape, solvedim, 90 + n + i, dtype)
+            u = seeded.uniform(7 + i, np.arange(d.size, dtype=np.uint64), -1, 1).reshape(shape).astype(dtype)
+            an, cn, ax = a.copy(), c.copy(), 2 - solvedim
+            an[(slice(None),) * ax + (0,)] = np.nan
+            cn[(slice(None),) * ax + (-1,)] = np.nan
+            t = [torch.from_numpy(v).cuda() for v in (an, b, cn, d, u)]
+            sets.append(((a, b, c, d, u), t))
+            systems.append(dict(a=t[0].data_ptr(), b=t[1].data_ptr(), c=t[2].data_ptr(), d=t[3].data_ptr(),
+                                u=t[4].data_ptr() if inc else None, dims=list(shape[::-1]), pads=list(shape[::-1])))
+        O.trid_batch(np.dtype(dtype).itemsize, solvedim, systems, None)
+        torch.cuda.synchronize()
+        for (a, b, c, d, u), t in sets:
+            ref = d.copy()
+            oracle_solve(orc, a, b, c, ref, solvedim)
+            if inc:
+                assert np.array_equal(t[3].cpu().numpy(), d)
+                ref = u + ref
+            np.testing.assert_allclose(t[4 if inc else 3].cpu().numpy(), ref, rtol=rtol, atol=rtol * np.abs(ref).max())
