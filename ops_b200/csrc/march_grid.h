@@ -10,11 +10,12 @@ namespace opsb {
 // strips that fill whole waves win, and of those the long ones. (CloverLeaf 2D
 // at 3840^2 with strips of 64 rows ran 3.3 waves in the time of 4, the heat
 // solver's 2048^2 direction kernel 1.4 waves in the time of 2.) At most
-// `most` strips.
+// `most` strips. The loop goes over the strip lengths, about 2 sqrt(n) of them:
+// over every number of strips it took 0.2 ms of a solve on 5 x 40,000 cells.
 inline int march_rows(long long columns, int n, int halo, long long resident, long long most = 1LL << 40) {
   int best = n;
   double cost = 1e300;
-  for (int c = 1; c <= n; c++) {
+  for (int c = 1; c <= n;) {
     const int rows = (n + c - 1) / c;
     if (rows < 2 && n > 1) break;
     const long long strips = columns * ((n + rows - 1) / rows);
@@ -26,6 +27,8 @@ inline int march_rows(long long columns, int n, int halo, long long resident, lo
       cost = t;
       best = rows;
     }
+    if (rows < 2) break;
+    c = (n + rows - 2) / (rows - 1);  // the next number of strips that have fewer rows
   }
   return best;
 }
