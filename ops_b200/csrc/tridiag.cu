@@ -796,8 +796,9 @@ __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__re
 // us against 257).
 template <class T>
 constexpr int kShortRows = sizeof(T) == 4 ? 32 : 16;
-// From a line for every thread of a CTA an SM on; below that the two are alike up
-// to 8 rows, and the line kernel's two lanes a line are faster beyond.
+// From a line for every thread of a CTA an SM on, and any number where no line of
+// the batch is longer than 8 rows; fewer lines of more rows are faster with the
+// line kernel's two lanes each, and a second launch for them would cost more.
 constexpr long long kShortLines = 148LL * kLineThreads;
 
 template <class T, int N>
@@ -888,7 +889,9 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
     short_lines += nl;
     short_n = std::max(short_n, s.n);
   }
-  if (short_lines < kShortLines) shorts.clear();
+  bool longer = false;
+  for (const Sys &s : systems) longer |= s.n > 8;
+  if (short_lines < kShortLines && longer) shorts.clear();
   for (const Sys &s : systems) {
     const long long nl = (long long)s.nl0 * s.nl1;
     if (s.n <= 0 || nl <= 0 || (s.n <= kShortRows<T> && !shorts.empty())) continue;
@@ -930,7 +933,8 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
   if (nshort) {
     const Sys *at = B.sys + nlive;
     const unsigned grid = (unsigned)std::min<long long>((short_lines + kLineThreads - 1) / kLineThreads, 1 << 20);
-    if (short_n <= 4) trid_short_kernel<T, 4><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    if (short_n <= 2) trid_short_kernel<T, 2><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
+    else if (short_n <= 4) trid_short_kernel<T, 4><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
     else if (short_n <= 8) trid_short_kernel<T, 8><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
     else if (short_n <= 12) trid_short_kernel<T, 12><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
     else if (short_n <= 16) trid_short_kernel<T, 16><<<grid, kLineThreads, 0, stream>>>(at, nshort, short_lines);
