@@ -595,8 +595,8 @@ __device__ __forceinline__ int magnitude(float x) { return __float_as_int(x) & 0
 // and substitute outwards. So a line's chain is half as long and the lines
 // whose c' and d' fit L2 keep twice the threads busy. The rows ahead come by
 // cp.async into the thread's own column of a ring of kLineStages stages of
-// kLineRows rows (no barrier: nobody else reads it); the backward pass reads
-// c' and d' kLineRows rows ahead into registers.
+// U rows (no barrier: nobody else reads it); the backward pass reads c' and d' U
+// rows ahead into registers.
 //
 // A line may have pivots from the top only (b_{n-1} = 0, say). While |c'| stays
 // within kGrowth a pivot's rounding error is that of its row's entries, so the
@@ -605,18 +605,23 @@ __device__ __forceinline__ int magnitude(float x) { return __float_as_int(x) & 0
 // alone, a lane a line, in the two lanes' scratch. Diagonally dominant rows
 // have |c'| <= 1. (The maximum costs 0.1 to 0.2 % of an ADI step.)
 constexpr float kGrowth = 16.0f;
-constexpr int kLineThreads = 128, kLineRows = 8, kLineStages = 3;
+constexpr int kLineThreads = 128, kLineStages = 3;
+// U is 8, which leaves an SM 2 CTAs (FP64) or 3, and 4, with 4 to 6 of them, where
+// lines of up to 64 rows fill more than a wave of the former: a wave more or less
+// counts for more there than the loads ahead. 300,000 lines FP64 of 24 rows 75 ->
+// 62 us, of 64 rows 167 -> 159, of 128 rows 335 -> 347; 65,536 lines FP32 of 48 rows
+// 26 -> 23.5.
+constexpr int kFewRows = 64;
 
 // Scratch of a group: c' and d' of its lines' halves.
 __host__ __device__ inline long long group_scratch(int n, int glines) { return (n + 1) / 2 * 4ll * glines; }
 
-template <class T>
-constexpr int kLineSmem = kLineStages * kLineRows * 4 * kLineThreads * (int)sizeof(T);
+template <class T, int U>
+constexpr int kLineSmem = kLineStages * U * 4 * kLineThreads * (int)sizeof(T);
 
-template <class T>
+template <class T, int U>
 __global__ void __launch_bounds__(kLineThreads) trid_line_kernel(const Sys *__restrict__ sys, int nsys,
                                                                  long long groups, T *scr) {
-  constexpr int U = kLineRows;
   extern __shared__ __align__(16) unsigned char smraw[];
   T *ring = reinterpret_cast<T *>(smraw) + threadIdx.x;  // element (stage, row, array) every kLineThreads
   const uint64_t keep = policy_last(), pass = policy_first();
@@ -872,6 +877,53 @@ Buffers &buffers() {
   return b;
 }
 
+// Threads of trid_line_kernel<T, U> that an SM holds.
+template <class T, int U>
+int line_threads() {
+  static int per_sm = 0;
+  if (!per_sm) {
+    int k = 0;
+    OPSB_CUDA(cudaFuncSetAttribute(trid_line_kernel<T, U>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   kLineSmem<T, U>));
+    OPSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, trid_line_kernel<T, U>, kLineThreads,
+                                                            kLineSmem<T, U>));
+    per_sm = std::max(k, 1) * kLineThreads;
+  }
+  return per_sm;
+}
+
+// Groups of a system's entry of the line kernel.
+long long groups_of(const Sys &s) { return s.glines == 16 ? (long long)s.nl0 * s.nl1 / 16 : 1ll; }
+
+// The line kernel over `live`, whose entries are on the device.
+template <class T, int U>
+void launch_groups(const std::vector<Sys> &live, long long groups, int maxn, cudaStream_t stream) {
+  // threads: what is resident, no more than kScratchBytes hold half lines for
+  // (but a CTA an SM at least), nor than there are groups
+  const int rows = (maxn + 1) / 2;
+  const size_t line = 2 * sizeof(T) * (size_t)rows;
+  const long long fit = (long long)(kScratchBytes / line) / 148 / kLineThreads * kLineThreads;
+  long long slots = 148 * std::max<long long>(kLineThreads, std::min<long long>(line_threads<T, U>(), fit));
+  slots = std::min(slots, (32 * groups + kLineThreads - 1) / kLineThreads * kLineThreads);
+  long long elems = 0, left = slots / 32;  // the first group's scratch of every warp
+  for (const Sys &s : live) {
+    elems += std::min(left, groups_of(s)) * group_scratch(s.n, s.glines);
+    left -= std::min(left, groups_of(s));
+  }
+  const size_t need = (size_t)elems * sizeof(T);
+  Buffers &B = buffers();
+  if (B.scr_bytes < need) {
+    if (B.scr) cudaFree(B.scr);
+    B.scr = nullptr;
+    B.scr_bytes = 0;
+    OPSB_CUDA(cudaMalloc(&B.scr, need));
+    B.scr_bytes = need;
+  }
+  trid_line_kernel<T, U><<<(unsigned)(slots / kLineThreads), kLineThreads, kLineSmem<T, U>, stream>>>(
+      B.sys, (int)live.size(), groups, static_cast<T *>(B.scr));
+  OPSB_CUDA(cudaGetLastError());
+}
+
 // The y/z sweeps (solve dimension strided, lines contiguous) by the line kernel,
 // and in great number the short ones by a launch of their own; returns false
 // when some system does not have that shape.
@@ -909,7 +961,6 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
   std::stable_sort(live.begin(), live.end(), [](const Sys &x, const Sys &y) {
     return group_scratch(x.n, x.glines) > group_scratch(y.n, y.glines);
   });
-  auto groups_of = [](const Sys &s) { return s.glines == 16 ? (long long)s.nl0 * s.nl1 / 16 : 1ll; };
   long long groups = 0, all = 0;
   for (Sys &s : live) {
     s.line0 = groups;
@@ -943,36 +994,11 @@ bool launch_lines(const std::vector<Sys> &systems, cudaStream_t stream, long lon
     if (kernels) (*kernels)++;
     if (!nlive) return true;
   }
-  static int per_sm = 0;  // resident threads, per type
-  if (!per_sm) {
-    int k = 0;
-    OPSB_CUDA(cudaFuncSetAttribute(trid_line_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLineSmem<T>));
-    OPSB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, trid_line_kernel<T>, kLineThreads, kLineSmem<T>));
-    per_sm = std::max(k, 1) * kLineThreads;
-  }
-  // threads: what is resident, no more than kScratchBytes hold half lines for
-  // (but a CTA an SM at least), nor than there are groups
-  const int rows = (maxn + 1) / 2;
-  const size_t line = 2 * sizeof(T) * (size_t)rows;
-  const long long fit = (long long)(kScratchBytes / line) / 148 / kLineThreads * kLineThreads;
-  long long slots = 148 * std::max<long long>(kLineThreads, std::min<long long>(per_sm, fit));
-  slots = std::min(slots, (32 * groups + kLineThreads - 1) / kLineThreads * kLineThreads);
-  long long elems = 0, left = slots / 32;  // the first group's scratch of every warp
-  for (const Sys &s : live) {
-    elems += std::min(left, groups_of(s)) * group_scratch(s.n, s.glines);
-    left -= std::min(left, groups_of(s));
-  }
-  const size_t need = (size_t)elems * sizeof(T);
-  if (B.scr_bytes < need) {
-    if (B.scr) cudaFree(B.scr);
-    B.scr = nullptr;
-    B.scr_bytes = 0;
-    OPSB_CUDA(cudaMalloc(&B.scr, need));
-    B.scr_bytes = need;
-  }
-  trid_line_kernel<T><<<(unsigned)(slots / kLineThreads), kLineThreads, kLineSmem<T>, stream>>>(
-      B.sys, nlive, groups, static_cast<T *>(B.scr));
-  OPSB_CUDA(cudaGetLastError());
+  // a wave of the kernel with U = 8: line_threads<T, 8>() / 32 groups an SM
+  if (maxn <= kFewRows && groups > 148LL * (line_threads<T, 8>() / 32))
+    launch_groups<T, 4>(live, groups, maxn, stream);
+  else
+    launch_groups<T, 8>(live, groups, maxn, stream);
   if (kernels) (*kernels)++;
   return true;
 }

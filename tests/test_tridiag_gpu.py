@@ -332,3 +332,21 @@ def test_short_lines_in_great_number(gpu_runtime, orc, dtype, rtol, inc, n):
                 assert np.array_equal(t[3].cpu().numpy(), d)
                 ref = u + ref
             np.testing.assert_allclose(t[4 if inc else 3].cpu().numpy(), ref, rtol=rtol, atol=rtol * np.abs(ref).max())
+
+
+@pytest.mark.parametrize("dtype,rtol", [(np.float64, 1e-12), (np.float32, 2e-4)])
+@pytest.mark.parametrize("inc", [False, True])
+@pytest.mark.parametrize("n", [17, 33, 39, 40, 41, 63, 64, 65])
+def test_more_than_a_wave_of_lines_of_few_rows(gpu_runtime, orc, dtype, rtol, inc, n):
+    """Lines of up to 64 rows, more than a wave of the line kernel's usual
+    stages: stages of four rows, at the edges of a half line's."""
+    shape = (3, n, 10001)
+    a, b, c, d = seeded.trid_system(shape, 1, 60 + n, dtype)
+    u = seeded.uniform(5, np.arange(d.size, dtype=np.uint64), -1, 1).reshape(shape).astype(dtype) if inc else None
+    x, ug = run_gpu(a, b, c, d, 1, u=u, pad=(0, 0, 3))
+    ref = d.copy()
+    oracle_solve(orc, a, b, c, ref, 1)
+    if inc:
+        assert np.array_equal(x, d)
+        x, ref = ug, u + ref
+    np.testing.assert_allclose(x, ref, rtol=rtol, atol=rtol * np.abs(ref).max())
