@@ -603,7 +603,9 @@ __device__ __forceinline__ int magnitude(float x) { return __float_as_int(x) & 0
 // elimination from the bottom is as sound as the rows are; a line whose c' pass
 // it (a vanished pivot leaves infinity or NaN) is solved again from the top
 // alone, a lane a line, in the two lanes' scratch. Diagonally dominant rows
-// have |c'| <= 1. (The maximum costs 0.1 to 0.2 % of an ADI step.)
+// have |c'| <= 1. (The maximum costs 0.1 to 0.2 % of an ADI step. Where every line
+// is solved again, 256^3 FP64 takes 1.75 ms instead of 0.17; the loops' loads in
+// batches of eight rows, in or out of line, cost ordinary lines 20 %.)
 constexpr float kGrowth = 16.0f;
 constexpr int kLineThreads = 128, kLineStages = 3;
 // U is 8, which leaves an SM 2 CTAs (FP64) or 3, and 4, with 4 to 6 of them, where
